@@ -143,12 +143,15 @@ def _mixed(case):
 
 
 def _design(seed, w, precision):
-    """A handle that has run: the design before last and its displacements, the design in hand in pinned memory."""
+    """A handle, the design in hand in pinned memory and its volume, which is the volume to keep; the handle holds the design before it."""
     p = _problem(w, precision)
     before, c = _coefficients(seed, [n + w.order for n in w.partition])
+    p.put("coeff", c)
+    p.coeff_to_density()
+    volume = p.volume()
     p.put("coeff", before)
     p.coeff_to_density()
-    return p, _pinned(c)
+    return p, _pinned(c), volume
 
 
 def _warm(state, solve, oc):
@@ -172,15 +175,15 @@ def prepare(case, seed):
     if kind == "batch":
         solve, parts = _mixed(case), []
         for k, w in enumerate(workloads.batch_cantilevers(case["n"], seed0=case["seed0"])):
-            p, c = _design(seed + 100 * k, w, 2)
-            part = dict(p=p, c=c, oc=dict(vgoal=w.vgoal))
+            p, c, volume = _design(seed + 100 * k, w, 2)
+            part = dict(p=p, c=c, oc=dict(vgoal=volume))
             _warm(part, solve, part["oc"])
             part["out"] = {n: _view(p, n) for n in ("u", "coeff", "csens")}
             parts.append(part)
         return dict(kind=kind, parts=parts, solve=solve)
     if kind == "loads":
         w = _workload("cantilever", case["nx"], case["ny"], case["nz"], 3)
-        p, c = _design(seed, w, 2)
+        p, _, _ = _design(seed, w, 2)
         p.multi_reserve(case["nrhs"])
         p.update_operators()
         p.put("multi_f", workloads.patch_loads(w.nx, w.ny, w.nz, case["nrhs"], seed0=seed, patch=8 if min(w.ny, w.nz) > 16 else 2))
@@ -189,23 +192,21 @@ def prepare(case, seed):
         return dict(kind=kind, p=p, nrhs=case["nrhs"], opts=o, u0=_pinned(np.zeros(p.size("multi_u"))), rel=np.zeros(case["nrhs"]),
                     out=_view(p, "multi_u"))
     w = _workload(case["wl"], case["nx"], case["ny"], case["nz"], case["order"])
-    oc = dict(vgoal=w.vgoal)
+    p, c, volume = _design(seed, w, 2 if kind in ("iter", "chain") else 1)
+    oc = dict(vgoal=volume)
     if kind == "iter":
-        p, c = _design(seed, w, 2)
         state = dict(kind=kind, p=p, c=c, solve=_mixed(case), oc=oc)
         _warm(state, state["solve"], oc)
         state["out"] = {n: _view(p, n) for n in ("u", "sens", "csens", "coeff", "rho")}
         return state
     if kind == "chain":
-        p, c = _design(seed, w, 2)
         p.put("u", _field(seed, w))
         return dict(kind=kind, p=p, c=c, oc=oc, out={n: _view(p, n) for n in ("sens", "csens", "volcsens", "coeff", "rho")})
-    p, c = _design(seed, w, 1)
     state = dict(kind=kind, p=p, c=c, u0=_pinned(np.zeros(3 * p.nv)))
     if kind == "mma":
         state["mma"] = capi.MMA.for_problem(p, m=1, lb=0.0, ub=1.0)
         p.volume_csens(scale=1e3)
-        state["vgoal"] = w.vgoal
+        state["vgoal"] = volume
         state["out"] = {n: _view(p, n) for n in ("u", "sens", "csens", "coeff")}
         state["x"] = torch.empty(state["mma"].n, dtype=torch.float64, device="cuda")
     elif kind == "pcg":

@@ -242,16 +242,15 @@ void level_residual(topo_handle* h, int l) {
 template <typename T>
 void gs_level(topo_handle* h, int l, int sweeps, bool reverse) {
   DevLevel& L = h->lv[l];
+  if (l > 0) {
+    count_launch(launch_stencil_gs<T>(h->stream, L.d, P<T>::st(L), L.vmask, P<T>::U(L), P<T>::F(L), sweeps, reverse));
+    return;
+  }
   for (int s = 0; s < sweeps; ++s)
     for (int cc = 0; cc < 8; ++cc) {
-      const int col = reverse ? 7 - cc : cc;
-      if (l == 0) {
-        EventPair* ev = prof_begin(h, P<T>::fam_smooth);
-        launch_fine_gs<T>(h->stream, L.d, P<T>::rhop(h), L.vmask, P<T>::U(L), P<T>::F(L), col, reverse);
-        prof_end(h, ev);
-      } else {
-        launch_stencil_gs<T>(h->stream, L.d, P<T>::st(L), L.vmask, P<T>::U(L), P<T>::F(L), col, reverse);
-      }
+      EventPair* ev = prof_begin(h, P<T>::fam_smooth);
+      launch_fine_gs<T>(h->stream, L.d, P<T>::rhop(h), L.vmask, P<T>::U(L), P<T>::F(L), reverse ? 7 - cc : cc, reverse);
+      prof_end(h, ev);
       count_launch();
     }
 }

@@ -59,6 +59,173 @@ __device__ __forceinline__ void stencil_row(const LevelDims& d, const T* __restr
 }
 
 
+// ---------------------------------------------------------------------------
+// Point-block Gauss-Seidel on a stencil level.  A vertex is nine lanes of a
+// warp, (row, neighbour z plane): each forms the products of nine neighbours
+// side by side, and the row's sum then passes through its three lanes in
+// neighbour order, so every sum and quotient is bit for bit the one a thread
+// walking the 27 neighbours forms.  A warp takes three vertices.  The thread-per-vertex form
+// (k_stencil_gs) waits for 243 products on the FP64 pipe with a colour's 80 to
+// 1500 vertices in a handful of CTAs: 51 us a colour on a level of 637 vertices,
+// here 5.5 us in the cluster form.
+// ---------------------------------------------------------------------------
+constexpr int GS_PER_WARP = 3;                        // vertices of a warp (27 of its lanes)
+constexpr int GS_WARPS = 8;                           // warps of a CTA
+constexpr int GS_PER_CTA = GS_PER_WARP * GS_WARPS;    // vertices of a CTA
+
+struct GsColour {  // vertices x = cx + 2i, y = cy + 2j, z = cz + 2k of a level
+  int cx, cy, cz, hx, hy, cnt;
+};
+__host__ __device__ inline GsColour gs_colour(const LevelDims& d, int colour) {
+  GsColour c;
+  c.cx = colour & 1;
+  c.cy = (colour >> 1) & 1;
+  c.cz = colour >> 2;
+  c.hx = (d.vx - c.cx + 1) / 2;
+  c.hy = (d.vy - c.cy + 1) / 2;
+  c.cnt = c.hx * c.hy * ((d.vz - c.cz + 1) / 2);
+  return c;
+}
+
+// s / d with rc = 1 / d computed ahead of time: the product with the correctly
+// rounded reciprocal, corrected by its exact remainder, which gives the
+// correctly rounded quotient (Markstein 1990) without a division's latency on
+// the critical path.
+template <typename T>
+__device__ __forceinline__ T div_by(T s, T d, T rc) {
+  const T q = s * rc;
+  const T e = fma(fma(-q, d, s), rc, q);
+  return isfinite(e) ? e : q;
+}
+
+// What a lane's share of a vertex update needs besides u.
+template <typename T>
+struct GsLane {
+  T c[27];       // stencil coefficients of (row, z plane): neighbour (y, x) major, component minor
+  T S[3], rc, f; // block entries (row, .), 1 / S(row, row), right-hand side of the row
+  int v, at;     // the vertex (-1: none) and its neighbour (-1, -1, plane) in the level
+  unsigned ok;   // in-plane neighbours inside the level
+};
+
+template <typename T>
+__device__ __forceinline__ void gs_load(const LevelDims& d, const T* __restrict__ st, StIdx si,
+                                        const uint8_t* __restrict__ vmask, const T* __restrict__ f, GsColour g, int t,
+                                        int row, int part, GsLane<T>& L) {
+  L.v = -1;
+  L.ok = 0;
+  L.f = L.S[0] = L.S[1] = L.S[2] = T(0);
+  L.rc = T(1);
+  if (t < 0 || t >= g.cnt) return;
+  const int q = t / g.hx, x = g.cx + 2 * (t - q * g.hx), qz = q / g.hy, y = g.cy + 2 * (q - qz * g.hy), z = g.cz + 2 * qz;
+  const int v = x + d.vx * (y + d.vy * z);
+  if (!(vmask[v] & 8)) return;
+  L.v = v;
+  const int64_t ss = si.stride(), nv = d.nv;
+  const T* sb = st + si.base(v);
+  const int nz = z + part - 1;
+  L.at = (x - 1) + d.vx * ((y - 1) + d.vy * nz);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int nx = x + k % 3 - 1, ny = y + k / 3 - 1;
+    const bool ok = nz >= 0 && nz < d.vz && nx >= 0 && ny >= 0 && nx < d.vx && ny < d.vy;
+    L.ok |= ok ? 1u << k : 0u;
+    const T* s = sb + (int64_t)((9 * part + k) * 9 + 3 * row) * ss;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) L.c[3 * k + j] = ok ? s[j * ss] : T(0);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) L.S[j] = sb[(int64_t)(13 * 9 + 3 * row + j) * ss];
+  L.rc = T(1) / (row == 0 ? L.S[0] : row == 1 ? L.S[1] : L.S[2]);
+  L.f = f[row * nv + v];
+}
+
+// Updates the warp's vertices; every lane of the warp must call it.
+template <typename T>
+__device__ __forceinline__ void gs_update(const LevelDims& d, T* u, const GsLane<T>& L, int lane, int row, int part,
+                                          bool reverse) {
+  const int64_t nv = d.nv;
+  T t[9], own = T(0);
+  if (L.v >= 0) {
+    T w[27];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int n = L.at + k % 3 + d.vx * (k / 3);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) w[3 * k + j] = (L.ok >> k) & 1u ? __ldcg(u + j * nv + n) : T(0);
+    }
+    own = __ldcg(u + row * nv + L.v);
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+      t[k] = fma(L.c[3 * k + 2], w[3 * k + 2], fma(L.c[3 * k], w[3 * k], L.c[3 * k + 1] * w[3 * k + 1]));
+  }
+  const int b9 = lane - 3 * row - part, b3 = lane - part;  // first lane of the vertex, of its row
+  T o = T(0);
+#pragma unroll
+  for (int ph = 0; ph < 3; ++ph) {
+    if (ph > 0) {
+      const T in = __shfl_sync(0xffffffffu, o, (b3 + ph - 1) & 31);
+      if (part == ph) o = in;
+    }
+    if (part == ph && L.v >= 0) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k)
+        if ((L.ok >> k) & 1u) o += t[k];
+    }
+  }
+  const T r = L.f - __shfl_sync(0xffffffffu, o, (b3 + 2) & 31);
+  // du of the rows in turn (0, 1, 2; reverse: 2, 1, 0); a lane's du is its row's
+  const T Sd = row == 0 ? L.S[0] : row == 1 ? L.S[1] : L.S[2];
+  const int first = reverse ? 2 : 0, last = 2 - first;
+  const T df_ = div_by(r, Sd, L.rc);  // right for row `first`
+  const T d1 = __shfl_sync(0xffffffffu, df_, (b9 + 3 * first) & 31);
+  const T Sf = reverse ? L.S[2] : L.S[0];
+  const T dm = div_by(fma(-Sf, d1, r), Sd, L.rc);  // right for row 1
+  const T d2 = __shfl_sync(0xffffffffu, dm, (b9 + 3) & 31);
+  // the last row subtracts by column: 0, 1 forward, 1, 2 in reverse
+  const T rl = reverse ? fma(-Sf, d1, fma(-L.S[1], d2, r)) : fma(-L.S[1], d2, fma(-Sf, d1, r));
+  const T dl = div_by(rl, Sd, L.rc);
+  const T du = row == first ? df_ : row == last ? dl : dm;
+  if (L.v >= 0 && part == 0) __stcg(u + row * nv + L.v, own + du);
+}
+
+// One colour, one launch.
+template <typename T>
+__global__ void __launch_bounds__(32 * GS_WARPS) k_stencil_gs9(LevelDims d, const T* __restrict__ st, StIdx si,
+                                                               const uint8_t* __restrict__ vmask, T* u,
+                                                               const T* __restrict__ f, int colour, bool reverse) {
+  const int lane = threadIdx.x & 31, g = lane / 9, j = lane - 9 * g, row = j / 3, part = j - 3 * row;
+  const int t = (blockIdx.x * GS_WARPS + (threadIdx.x >> 5)) * GS_PER_WARP + g;
+  GsLane<T> L;
+  gs_load<T>(d, st, si, vmask, f, gs_colour(d, colour), g < GS_PER_WARP ? t : -1, row, part, L);
+  gs_update<T>(d, u, L, lane, row, part, reverse);
+}
+
+// All colours of all sweeps in one launch of one thread-block cluster, a
+// cluster barrier between colours: for levels whose colours hold no more
+// vertices than the cluster updates at once.  The stencil part of the next
+// colour is loaded before the wait, so a colour costs the barrier, the
+// L2 latency of u and the FP64 products of its few vertices.
+template <typename T>
+__global__ void __launch_bounds__(32 * GS_WARPS) k_stencil_gs_cluster(LevelDims d, const T* __restrict__ st, StIdx si,
+                                                                      const uint8_t* __restrict__ vmask, T* u,
+                                                                      const T* __restrict__ f, int sweeps,
+                                                                      bool reverse) {
+  const int lane = threadIdx.x & 31, g = lane / 9, j = lane - 9 * g, row = j / 3, part = j - 3 * row;
+  // consecutive groups of three vertices go to different CTAs (SMs)
+  const int t = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * GS_PER_WARP + g;
+  for (int k = 0; k < 8 * sweeps; ++k) {
+    GsLane<T> L;
+    gs_load<T>(d, st, si, vmask, f, gs_colour(d, reverse ? 7 - (k & 7) : (k & 7)), g < GS_PER_WARP ? t : -1, row, part,
+               L);
+    if (k > 0) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    gs_update<T>(d, u, L, lane, row, part, reverse);
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  }
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// Thread per vertex: every lane of a warp carries products, which pays where a
+// colour has enough vertices to fill the chip by itself (GS_THREAD_MIN).
 template <typename T>
 __global__ void k_stencil_gs(LevelDims d, const T* __restrict__ st, StIdx si, const uint8_t* __restrict__ vmask,
                              T* u, const T* __restrict__ f, int cx, int cy, int cz, int hx, int hy,
@@ -337,14 +504,76 @@ template void launch_cheb_zero_stored<double>(cudaStream_t, int64_t, const uint8
 template void launch_cheb_zero_stored<float>(cudaStream_t, int64_t, const uint8_t*, const float*, const float*,
                                              float*, float*, const double*, int);
 
+// CTAs of the cluster k_stencil_gs_cluster runs in: 16 where the device can
+// place such a cluster (more SMs share the FP64 work of a colour), else 8.
 template <typename T>
-void launch_stencil_gs(cudaStream_t s, const LevelDims& d, const T* st, const uint8_t* vmask, T* u,
-                       const T* f, int colour, bool reverse) {
-  const int cx = colour & 1, cy = (colour >> 1) & 1, cz = colour >> 2;
-  const int hx = (d.vx - cx + 1) / 2, hy = (d.vy - cy + 1) / 2, hz = (d.vz - cz + 1) / 2;
-  const int64_t cnt = (int64_t)hx * hy * hz;
-  if (cnt <= 0) return;
-  k_stencil_gs<T><<<nblk(cnt, 128), 128, 0, s>>>(d, st, st_idx<T>(d), vmask, u, f, cx, cy, cz, hx, hy, cnt, reverse);
+static int gs_cluster_size() {
+  static PerDeviceOnce once;
+  static std::atomic<int> size[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 8;
+  const cudaError_t e = once_per_device(once, [&]() -> cudaError_t {
+    int n = 0;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(16);
+    c.blockDim = dim3(32 * GS_WARPS);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 16;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    const bool big = cudaFuncSetAttribute(k_stencil_gs_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                         cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&n, k_stencil_gs_cluster<T>, &c) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    size[dev] = big ? 16 : 8;
+    return cudaSuccess;
+  });
+  return e == cudaSuccess ? size[dev].load() : 8;
+}
+
+// A colour of at least this many vertices runs thread per vertex.  FP64, us a
+// colour, nine lanes against one thread a vertex: 400 vertices 10.4 / 24.7,
+// 1,200 12.2 / 24.7, 8,800 29.5 / 45.8, 20,000 58.4 / 53.6, 29,000 83 / 57.
+constexpr int GS_THREAD_MIN = 16384;
+
+// `sweeps` Gauss-Seidel sweeps, colours 0..7 or 7..0.  Returns the launches made.
+template <typename T>
+int launch_stencil_gs(cudaStream_t s, const LevelDims& d, const T* st, const uint8_t* vmask, T* u,
+                      const T* f, int sweeps, bool reverse) {
+  if (sweeps <= 0 || d.nv <= 0) return 0;
+  const GsColour big = gs_colour(d, 0);  // the largest colour
+  const int cl = gs_cluster_size<T>();
+  if (big.cnt <= cl * GS_PER_CTA) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(cl);
+    c.blockDim = dim3(32 * GS_WARPS);
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k_stencil_gs_cluster<T>, d, st, st_idx<T>(d), vmask, u, f, sweeps, reverse);
+    return 1;
+  }
+  int n = 0;
+  for (int sw = 0; sw < sweeps; ++sw)
+    for (int cc = 0; cc < 8; ++cc) {
+      const int col = reverse ? 7 - cc : cc;
+      const GsColour g = gs_colour(d, col);
+      if (g.cnt <= 0) continue;
+      if (big.cnt >= GS_THREAD_MIN)
+        k_stencil_gs<T><<<nblk(g.cnt, 128), 128, 0, s>>>(d, st, st_idx<T>(d), vmask, u, f, g.cx, g.cy, g.cz, g.hx, g.hy,
+                                                       g.cnt, reverse);
+      else
+        k_stencil_gs9<T><<<nblk(g.cnt, GS_PER_CTA), 32 * GS_WARPS, 0, s>>>(d, st, st_idx<T>(d), vmask, u, f, col,
+                                                                          reverse);
+      ++n;
+    }
+  return n;
 }
 
 template <typename T>
@@ -1218,10 +1447,10 @@ template void launch_stencil_apply<double>(cudaStream_t, const LevelDims&, const
                                            const double*, double*, bool, int);
 template void launch_stencil_apply<float>(cudaStream_t, const LevelDims&, const float*, const float*,
                                           const float*, float*, bool, int);
-template void launch_stencil_gs<double>(cudaStream_t, const LevelDims&, const double*, const uint8_t*,
-                                        double*, const double*, int, bool);
-template void launch_stencil_gs<float>(cudaStream_t, const LevelDims&, const float*, const uint8_t*,
-                                       float*, const float*, int, bool);
+template int launch_stencil_gs<double>(cudaStream_t, const LevelDims&, const double*, const uint8_t*,
+                                       double*, const double*, int, bool);
+template int launch_stencil_gs<float>(cudaStream_t, const LevelDims&, const float*, const uint8_t*,
+                                      float*, const float*, int, bool);
 template void launch_stencil_diag_inv<double>(cudaStream_t, const LevelDims&, const double*,
                                               const uint8_t*, double*);
 template void launch_stencil_diag_inv<float>(cudaStream_t, const LevelDims&, const float*,

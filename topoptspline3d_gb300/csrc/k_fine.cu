@@ -1433,16 +1433,11 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// Row block of vertex (x,y,z): out = sum over incident elements of rho^p Ke[a,:] u_e,
-// S = diagonal 3x3 block.  Template arguments fix whether S is needed.
-template <typename T, bool NEED_S>
+// Row block of vertex (x,y,z): out = sum over incident elements of rho^p Ke[a,:] u_e.
+template <typename T>
 __device__ __forceinline__ void fine_row(const LevelDims& d, const T* __restrict__ rhop,
-                                         const T* __restrict__ u, int x, int y, int z, T out[3],
-                                         T S[9]) {
+                                         const T* __restrict__ u, int x, int y, int z, T out[3]) {
   out[0] = out[1] = out[2] = T(0);
-  if (NEED_S)
-#pragma unroll
-    for (int i = 0; i < 9; ++i) S[i] = T(0);
   const int64_t nv = d.nv;
 #pragma unroll
   for (int w = 0; w < 8; ++w) {
@@ -1462,12 +1457,6 @@ __device__ __forceinline__ void fine_row(const LevelDims& d, const T* __restrict
       s2 += ke<T>(r0 + 48) * u0 + ke<T>(r0 + 49) * u1 + ke<T>(r0 + 50) * u2;
     }
     out[0] += pe * s0; out[1] += pe * s1; out[2] += pe * s2;
-    if (NEED_S) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) S[3 * i + j] += pe * ke<T>((3 * a + i) * 24 + 3 * a + j);
-    }
   }
 }
 
@@ -1483,7 +1472,7 @@ __global__ void __launch_bounds__(256) k_fine_apply(LevelDims d, const T* __rest
   const int y = (int)(t % d.vy), z = (int)(t / d.vy);
   const uint8_t m = vmask[v];
   T o[3] = {T(0), T(0), T(0)};
-  if (m & 7) fine_row<T, false>(d, rhop, u, x, y, z, o, nullptr);
+  if (m & 7) fine_row<T>(d, rhop, u, x, y, z, o);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const bool fr = (m >> c) & 1;
@@ -1494,32 +1483,34 @@ __global__ void __launch_bounds__(256) k_fine_apply(LevelDims d, const T* __rest
 
 // One colour of the 8-colour point-block Gauss-Seidel sweep.  Forward: DOFs
 // 0,1,2 (grid/Grid.cu:1830-1838); reverse: DOFs 2,1,0 (adjoint sweep).
-template <typename T>
-__device__ __forceinline__ void block_update(T* u, int64_t nv, int64_t v, const T r[3], const T S[9],
-                                             uint8_t fb, bool reverse) {
-  T du[3] = {T(0), T(0), T(0)};
-  if (!reverse) {
+// A CTA takes 32 vertices.  Warp w forms the row products of the vertices'
+// incident element w (its constants are the instructions' own operands), the
+// sums over the elements and the diagonal block are then formed in element
+// order by one warp a sum, and warp 0 substitutes.  The arithmetic is that of a
+// thread that walks the eight elements, which had 31 CTAs for a colour of a
+// 48x24x24 grid: 71 us there, 14.1 us here (the FP64 pipe alone needs 4 us).
+template <typename T, int W>
+__device__ __forceinline__ void gs_element_rows(const T* __restrict__ u, int64_t nv, int64_t v0, int vx, int64_t vxy,
+                                                T s[3]) {
+  constexpr int a = 7 - W;
+  s[0] = s[1] = s[2] = T(0);
+  T ue[24];  // all loads in flight at once
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      if (!((fb >> i) & 1)) continue;
-      T s = r[i];
-#pragma unroll
-      for (int j = 0; j < i; ++j) s -= S[3 * i + j] * du[j];
-      du[i] = s / S[4 * i];
-    }
-  } else {
-#pragma unroll
-    for (int i = 2; i >= 0; --i) {
-      if (!((fb >> i) & 1)) continue;
-      T s = r[i];
-#pragma unroll
-      for (int j = i + 1; j < 3; ++j) s -= S[3 * i + j] * du[j];
-      du[i] = s / S[4 * i];
-    }
+  for (int b = 0; b < 8; ++b) {
+    const T* ub = u + v0 + (b & 1) + (int64_t)vx * ((b >> 1) & 1) + vxy * (b >> 2);
+    ue[3 * b] = ub[0];
+    ue[3 * b + 1] = ub[nv];
+    ue[3 * b + 2] = ub[2 * nv];
   }
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-    if ((fb >> i) & 1) u[i * nv + v] += du[i];
+  for (int b = 0; b < 8; ++b) {
+    const T u0 = ue[3 * b], u1 = ue[3 * b + 1], u2 = ue[3 * b + 2];
+    constexpr int r0 = (3 * a) * 24;
+    const int q = r0 + 3 * b;
+    s[0] += ke<T>(q) * u0 + ke<T>(q + 1) * u1 + ke<T>(q + 2) * u2;
+    s[1] += ke<T>(q + 24) * u0 + ke<T>(q + 25) * u1 + ke<T>(q + 26) * u2;
+    s[2] += ke<T>(q + 48) * u0 + ke<T>(q + 49) * u1 + ke<T>(q + 50) * u2;
+  }
 }
 
 template <typename T>
@@ -1527,20 +1518,101 @@ __global__ void __launch_bounds__(256) k_fine_gs(LevelDims d, const T* __restric
                                                  const uint8_t* __restrict__ vmask, T* u,
                                                  const T* __restrict__ f, int cx, int cy, int cz,
                                                  int hx, int hy, int64_t cnt, bool reverse) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cnt) return;
-  const int x = cx + 2 * (int)(t % hx);
-  const int64_t t2 = t / hx;
+  __shared__ T ss[8][3][32];  // element w's row sums
+  __shared__ T sp[8][32];     // its rho^p (0: none)
+  __shared__ T sr[3][32];     // residual
+  __shared__ T sS[6][32];     // diagonal block: S00 S11 S22, then the off-diagonal entries the sweep reads
+  __shared__ T sc[3][32];     // 1 / S00, S11, S22
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t t = (int64_t)blockIdx.x * 32 + lane;
+  const bool in = t < cnt;
+  const int64_t tc = in ? t : 0;
+  const int x = cx + 2 * (int)(tc % hx);
+  const int64_t t2 = tc / hx;
   const int y = cy + 2 * (int)(t2 % hy), z = cz + 2 * (int)(t2 / hy);
   const int64_t v = x + (int64_t)d.vx * (y + (int64_t)d.vy * z);
-  const uint8_t m = vmask[v];
+  const uint8_t m = in ? vmask[v] : 0;
   const uint8_t fb = (m & 8) ? (m & 7) : 0;
-  if (!fb) return;
-  T o[3], S[9], r[3];
-  fine_row<T, true>(d, rhop, u, x, y, z, o, S);
+  const int ex = x - 1 + (w & 1), ey = y - 1 + ((w >> 1) & 1), ez = z - 1 + (w >> 2);
+  T pe = T(0), s[3] = {T(0), T(0), T(0)};
+  if (fb && ex >= 0 && ey >= 0 && ez >= 0 && ex < d.ex && ey < d.ey && ez < d.ez)
+    pe = rhop[ex + (int64_t)d.ex * (ey + (int64_t)d.ey * ez)];
+  if (pe != T(0)) {
+    const int64_t v0 = ex + (int64_t)d.vx * (ey + (int64_t)d.vy * ez), vxy = (int64_t)d.vx * d.vy;
+    switch (w) {
+      case 0: gs_element_rows<T, 0>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 1: gs_element_rows<T, 1>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 2: gs_element_rows<T, 2>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 3: gs_element_rows<T, 3>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 4: gs_element_rows<T, 4>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 5: gs_element_rows<T, 5>(u, d.nv, v0, d.vx, vxy, s); break;
+      case 6: gs_element_rows<T, 6>(u, d.nv, v0, d.vx, vxy, s); break;
+      default: gs_element_rows<T, 7>(u, d.nv, v0, d.vx, vxy, s); break;
+    }
+  }
+  sp[w][lane] = pe;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) r[c] = f[c * d.nv + v] - o[c];
-  block_update<T>(u, d.nv, v, r, S, fb, reverse);
+  for (int c = 0; c < 3; ++c) ss[w][c][lane] = s[c];
+  __syncthreads();
+  // sums in element order: warps 0-2 the rows, warps 3-5 the diagonal entries
+  // and their reciprocals, warps 6 and 7 the others
+  if (w < 3) {
+    T o = T(0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const T p = sp[e][lane];
+      if (p != T(0)) o += p * ss[e][w][lane];
+    }
+    sr[w][lane] = fb ? f[w * d.nv + v] - o : T(0);
+  } else if (w < 6) {
+    T S = T(0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int a = 7 - e;
+      const T k = w == 3 ? ke<T>(3 * a * 25) : w == 4 ? ke<T>((3 * a + 1) * 25) : ke<T>((3 * a + 2) * 25);
+      S += sp[e][lane] * k;
+    }
+    sS[w - 3][lane] = S;
+    sc[w - 3][lane] = T(1) / S;
+  } else {
+    // forward: S10, S20, S21; reverse: S01, S02, S12 (warp 6: two of them)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (w == 7 && q) break;
+      T S = T(0);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int a = 7 - e, r = 3 * a * 25;  // entry (3a, 3a)
+        const T kf = w == 7 ? ke<T>(r + 49) : q ? ke<T>(r + 48) : ke<T>(r + 24);
+        const T kr = w == 7 ? ke<T>(r + 26) : q ? ke<T>(r + 2) : ke<T>(r + 1);
+        S += sp[e][lane] * (reverse ? kr : kf);
+      }
+      sS[w == 7 ? 5 : 3 + q][lane] = S;
+    }
+  }
+  __syncthreads();
+  if (w > 0 || !fb) return;
+  // s / d by the reciprocal and its exact remainder: the correctly rounded
+  // quotient (Markstein 1990)
+  auto quot = [](T n, T den, T rc) {
+    const T q = n * rc;
+    const T e = fma(fma(-q, den, n), rc, q);
+    return isfinite(e) ? e : q;
+  };
+  const T S01 = sS[3][lane], S02 = sS[4][lane], S12 = sS[5][lane];  // (transposed forward)
+  T du[3] = {T(0), T(0), T(0)};
+  if (!reverse) {
+    if (fb & 1) du[0] = quot(sr[0][lane], sS[0][lane], sc[0][lane]);
+    if (fb & 2) du[1] = quot(sr[1][lane] - S01 * du[0], sS[1][lane], sc[1][lane]);
+    if (fb & 4) du[2] = quot((sr[2][lane] - S02 * du[0]) - S12 * du[1], sS[2][lane], sc[2][lane]);
+  } else {
+    if (fb & 4) du[2] = quot(sr[2][lane], sS[2][lane], sc[2][lane]);
+    if (fb & 2) du[1] = quot(sr[1][lane] - S12 * du[2], sS[1][lane], sc[1][lane]);
+    if (fb & 1) du[0] = quot((sr[0][lane] - S01 * du[1]) - S02 * du[2], sS[0][lane], sc[0][lane]);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if ((fb >> i) & 1) u[i * d.nv + v] += du[i];
 }
 
 // Inverse of the free-DOF part of each diagonal 3x3 block (Chebyshev): [9][nv]
@@ -1884,8 +1956,7 @@ void launch_fine_gs(cudaStream_t s, const LevelDims& d, const T* rhop, const uin
   const int hx = (d.vx - cx + 1) / 2, hy = (d.vy - cy + 1) / 2, hz = (d.vz - cz + 1) / 2;
   const int64_t cnt = (int64_t)hx * hy * hz;
   if (cnt <= 0) return;
-  k_fine_gs<T><<<blocks_for(cnt, 256), 256, 0, s>>>(d, rhop, vmask, u, f, cx, cy, cz, hx, hy, cnt,
-                                                    reverse);
+  k_fine_gs<T><<<blocks_for(cnt, 32), 256, 0, s>>>(d, rhop, vmask, u, f, cx, cy, cz, hx, hy, cnt, reverse);
 }
 
 template <typename T>

@@ -205,8 +205,8 @@ template <typename T>
 void launch_stencil_apply(cudaStream_t s, const LevelDims& d, const T* st, const T* u, const T* f,
                           T* out, bool residual, int nb = 1);
 template <typename T>
-void launch_stencil_gs(cudaStream_t s, const LevelDims& d, const T* st, const uint8_t* vmask, T* u,
-                       const T* f, int colour, bool reverse);
+int launch_stencil_gs(cudaStream_t s, const LevelDims& d, const T* st, const uint8_t* vmask, T* u,
+                      const T* f, int sweeps, bool reverse);
 template <typename T>
 void launch_stencil_diag_inv(cudaStream_t s, const LevelDims& d, const T* st, const uint8_t* vmask,
                              T* dinv);

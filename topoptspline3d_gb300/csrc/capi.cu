@@ -37,19 +37,6 @@ using namespace topo;
 #define TOPO_FUSED_DOT_TICKET 1
 #endif
 
-// CTAs per SM of the coarsest inversion when it runs on the side stream next
-// to the solve's set-up kernels: one up to TOPO_GJ_SIDE_LARGE_N unknowns
-// (256x128x128: n = 675, where the set-up kernels need the SMs as much as the
-// inversion: two CTAs per SM there ran the design iteration at 26.0-26.3
-// against 25.7 ms), two above, where the inversion outlasts the set-up by far
-// (n = 1617: about 6 against 1 ms)
-#ifndef TOPO_GJ_SIDE_PER_SM
-#define TOPO_GJ_SIDE_PER_SM 1
-#endif
-#ifndef TOPO_GJ_SIDE_LARGE_N
-#define TOPO_GJ_SIDE_LARGE_N 1000
-#endif
-
 #include "handle.h"
 
 // z-march depth argument of the handle's FP32 fine-kernel launches
@@ -1278,7 +1265,7 @@ int topo_create(const topo_config* cfg, const uint8_t* eactive, topo_handle** ou
     else {
       A(dalloc(hp, &h->A, (int64_t)h->ndense * h->ndense));
       A(dalloc(hp, &h->A32, (int64_t)h->ndense * h->ndense));
-      A(dalloc(hp, &h->gjwork, 128 * (int64_t)h->ndense + 32 * 32));  // block, panels in FP64 and split
+      A(dalloc(hp, &h->gjwork, 128 * (int64_t)h->ndense + 8 * 32 * 32));  // panels and diagonal blocks of the inversion
       A(dalloc(hp, &h->coarse64tmp, 243 * dl.nv));
     }
     std::vector<double> T;
@@ -1695,11 +1682,11 @@ int topo_update_operators(topo_handle* h) {
       st = h->coarse64tmp;
     }
     launch_dense_from_stencil(h->stream, Lc.d, st, h->A);
-    count_launch(2);
+    count_launch();
     CKL();
     // FP32-only operators: the matrix comes from FP32 stencils; the updates
     // in double-float keep twice their precision on the FP32 pipe
-    if (h->defer_coarse) {  // on the side stream, one CTA per SM, joined later
+    if (h->defer_coarse) {  // on the side stream, joined later
       if (!h->side) {
         CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&h->ev_ops, cudaEventDisableTiming));
@@ -1708,14 +1695,11 @@ int topo_update_operators(topo_handle* h) {
       }
       CK(cudaEventRecord(h->ev_ops, h->stream));
       CK(cudaStreamWaitEvent(h->side, h->ev_ops, 0));
-      const int e = coarsest_invert(h->side, h->ndense, h->A, h->gjwork, h->status, !b64,
-                                    h->ndense > TOPO_GJ_SIDE_LARGE_N ? 2 : TOPO_GJ_SIDE_PER_SM);
+      const int e = coarsest_invert(h->side, h->ndense, h->A, h->A32, h->gjwork, h->status, !b64);
       count_launch();
       if (e != (int)cudaSuccess)
         return fail(h, TOPO_E_CUDA, "coarsest inversion launch failed: %s", cudaGetErrorString((cudaError_t)e));
       CK(cudaMemcpyAsync(h->hstat, h->status, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->side));
-      launch_to_float(h->side, h->A, h->A32, (int64_t)h->ndense * h->ndense);
-      count_launch();
       CK(cudaEventRecord(h->ev_coarse, h->side));
       h->coarse_pending = h->coarse_unchecked = true;
       for (auto& l : h->lv) { l.lmax = 0; l.lmax32 = 0; }
@@ -1724,7 +1708,7 @@ int topo_update_operators(topo_handle* h) {
       h->ops_ready = true;
       return TOPO_OK;
     }
-    int e = coarsest_invert(h->stream, h->ndense, h->A, h->gjwork, h->status, !b64);
+    int e = coarsest_invert(h->stream, h->ndense, h->A, h->A32, h->gjwork, h->status, !b64);
     count_launch();
     if (e != (int)cudaSuccess)
       return fail(h, TOPO_E_CUDA, "coarsest inversion launch failed: %s", cudaGetErrorString((cudaError_t)e));
@@ -1736,8 +1720,6 @@ int topo_update_operators(topo_handle* h) {
       return fail(h, TOPO_E_SINGULAR, "coarsest matrix indefinite at pivot %d", hstat[1] - 1);
     }
     h->coarse_dropped = hstat[0];
-    launch_to_float(h->stream, h->A, h->A32, (int64_t)h->ndense * h->ndense);
-    count_launch();
     CKL();
   }
   for (auto& l : h->lv) { l.lmax = 0; l.lmax32 = 0; }

@@ -1070,60 +1070,13 @@ __global__ void k_symmetrize(int n, double* A) {
   A[(int64_t)j * n + i] = s;
 }
 
-// In-place Gauss-Jordan inverse of a symmetric positive (semi-)definite matrix
-// (no pivoting needed), one cooperative launch; two grid barriers per pivot.
-// A pivot below 1e-10 of the largest diagonal entry belongs to a null
-// direction (a floating part of the domain): its row and column are dropped,
-// which gives the inverse of the remaining DOFs, as the reference's
+// Blocked Gauss-Jordan inversion (in place, SPD matrix), for matrices too large
+// for k_gj_sweep.  A pivot below 1e-10 of the largest diagonal entry belongs to
+// a null direction (a floating part of the domain): its row and column are
+// dropped, which gives the inverse of the remaining DOFs, as the reference's
 // pseudo-inverse does for its coarsest system (grid/Grid.cpp:3657, 4072).
 // status[0] counts dropped pivots; a clearly negative pivot sets status[1] = k+1
-// and every block stops at the same step (all threads read the same pivot).
-__global__ void k_gauss_jordan(int n, double* A, int* status) {
-  cg::grid_group grid = cg::this_grid();
-  const int64_t nn = (int64_t)n * n;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t tid0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double dmax = 0.0;
-  for (int k = 0; k < n; ++k) dmax = fmax(dmax, fabs(A[(int64_t)k * n + k]));
-  const double tol = 1e-10 * dmax;
-  for (int k = 0; k < n; ++k) {
-    const double p = A[(int64_t)k * n + k];
-    if (p < -tol) {
-      if (tid0 == 0) status[1] = k + 1;
-      return;
-    }
-    if (p <= tol) {  // drop DOF k
-      for (int64_t g = tid0; g < 2 * (int64_t)n; g += stride) {
-        if (g < n) A[(int64_t)k * n + g] = 0.0;
-        else A[(g - n) * n + k] = 0.0;
-      }
-      if (tid0 == 0) status[0] += 1;
-      grid.sync();
-      continue;
-    }
-    const double rp = 1.0 / p;
-    for (int64_t g = tid0; g < nn; g += stride) {
-      const int i = (int)(g / n), j = (int)(g % n);
-      if (i == k || j == k) continue;
-      A[g] -= A[(int64_t)i * n + k] * A[(int64_t)k * n + j] * rp;
-    }
-    grid.sync();
-    for (int64_t g = tid0; g < 2 * (int64_t)n; g += stride) {
-      if (g < n) {
-        const int j = (int)g;
-        if (j != k) A[(int64_t)k * n + j] *= rp;
-        else A[(int64_t)k * n + k] = rp;
-      } else {
-        const int i = (int)(g - n);
-        if (i != k) A[(int64_t)i * n + k] *= -rp;
-      }
-    }
-    grid.sync();
-  }
-}
-
-// Blocked Gauss-Jordan inversion (in place, SPD matrix, same pivot-drop rule as
-// k_gauss_jordan).  For each panel K of GJB pivots: one CTA inverts the
+// and every block stops at the same step.  For each panel K of GJB pivots: one CTA inverts the
 // diagonal block D = A[K,K] pivot by pivot in shared memory (dropping pivots
 // <= tol); all CTAs form the row panel P = D^-1 A[K,:] and copy the column panel
 // C = A[:,K]; then every element gets its rank-GJB update
@@ -1341,6 +1294,317 @@ __global__ void __launch_bounds__(256) k_gj_blocked(int n, double* __restrict__ 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Inversion of the coarsest matrix by symmetric sweeps, the lower triangle held
+// on chip.  Sweeping a panel K of 32 pivots maps a symmetric A to
+//   A_KK <- -A_KK^-1,  A_iK <- W_i = A_iK A_KK^-1,  A_ij <- A_ij - W_i A_Kj,
+// which is symmetric again, and sweeping every panel leaves -A^-1, so only the
+// 32 x 32 tiles (i, j), i >= j, are kept: half the rank-32 updates of
+// Gauss-Jordan on the full matrix.  Each CTA owns consecutive tiles of that
+// triangle in shared memory for the whole inversion (n = 1617: nine tiles a
+// SM, n = 675: two), so a panel moves only the panel itself through L2:
+//   B: W_j = C_j D, eight rows of a tile at a time spread over all CTAs, with
+//      C_j = A_jK and D = A_KK^-1 published by the phase before;
+//   C: every tile's update; the owners of the next panel's tiles publish them.
+// CTA 0 owns no tile: during C it forms the next diagonal tile from the
+// published parts and inverts it.  Two grid barriers a panel.
+// Everything is double-float arithmetic on the FP32 pipe, for matrices that come
+// from FP32 stencils: even the conversions of a form with FP64 panels cost more
+// than the panels (n = 675: 0.65 against 0.36 ms).  Its bounds: at n = 675 the
+// chain of a panel (C for the diagonal tile 3 us, its inversion 7 us, B 2 us,
+// barriers 2.5 us), at n = 1617 the updates (480 FP32 instructions an element
+// and panel).  Against k_gj_blocked<true>: n = 336 0.64 -> 0.18 ms, 675
+// 1.31 -> 0.36 ms, 1617 5.17 -> 1.6 ms; ||A X - 1|| no larger on coarsest matrices
+// of designs (n = 675: 6.6e-13 against 8.0e-13).
+// The pivot-drop rule and status are k_gj_blocked's.
+// ---------------------------------------------------------------------------
+constexpr int GJT = GJB * GJB;         // elements of a tile
+constexpr int GJP = GJB + 1;           // pitch of a tile row in shared memory
+constexpr int GJ_TILE = GJB * GJP;     // shared elements of an owned tile
+constexpr int GJ_THREADS = 512;
+constexpr int SB = 4;                  // pivots a step of the diagonal block's inversion
+constexpr int GJ_SWEEP_SMEM = 212 * 1024;  // dynamic shared memory a CTA may take (227 KB less the static arrays)
+
+__device__ __forceinline__ df df_ldcg(const df* p) {
+  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return df(v.x, v.y);
+}
+__device__ __forceinline__ df df_shfl(df v, int l) {
+  return df(__shfl_sync(0xffffffffu, v.hi, l), __shfl_sync(0xffffffffu, v.lo, l));
+}
+__device__ __forceinline__ df df_neg(df v) { return df(-v.hi, -v.lo); }
+// acc - a b: TwoProd, TwoSum and one renormalisation
+__device__ __forceinline__ df df_nfma(df acc, df a, df b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  e = __fmaf_rn(a.lo, b.hi, e);
+  const float t = __fsub_rn(acc.hi, p), z = __fsub_rn(t, acc.hi);
+  const float r = __fsub_rn(__fsub_rn(acc.hi, __fsub_rn(t, z)), __fadd_rn(p, z));
+  return df_fast2sum(t, __fadd_rn(r, __fsub_rn(acc.lo, e)));
+}
+// 1/p: FP32 estimate, one Newton step with its second-order term
+__device__ __forceinline__ df df_rcp(df p) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(p.hi));
+  const float e = __fmaf_rn(-p.lo, r, __fmaf_rn(-p.hi, r, 1.f));
+  return df_fast2sum(r, __fmul_rn(r, __fmaf_rn(e, e, e)));
+}
+
+// Inverts the kb x kb symmetric block in the lower triangle of sd (rows and
+// columns from kb on are zero) and writes the full inverse to out[GJT].
+// Called by all threads of a CTA.  k0: index of the first pivot (status).
+// Four pivots at a time: warp 0 sweeps them on their own four columns, held in
+// registers (lane r: row r), so a pivot costs shuffles and arithmetic but no
+// barrier, and the other elements then get their rank-4 update from all warps.
+// (One barrier a pivot took twice as long.)
+__device__ __forceinline__ void sweep_block(df (*sd)[GJP], df (*sv)[SB][GJB], int kb, int k0, float tol, int* status,
+                                            df* out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const df zero(0.f, 0.f);
+  // this thread's element of the lower triangle with the four panel rows taken
+  // out: rows r and 27 - r of that 28-row triangle together hold 29
+  constexpr int R = GJB - SB;
+  static_assert((R / 2) * (R + 1) <= GJ_THREADS, "one element a thread");
+  const int pr = tid / (R + 1), pk = tid - pr * (R + 1);
+  const bool mine = tid < (R / 2) * (R + 1);
+  const int r28 = pk <= pr ? pr : R - 1 - pr, c28 = pk <= pr ? pk : pk - pr - 1;
+  for (int j = 0; j < kb; j += SB) {
+    __syncthreads();
+    if (warp == 0) {
+      df v[SB];
+#pragma unroll
+      for (int q = 0; q < SB; ++q) v[q] = lane >= j + q ? sd[lane][j + q] : sd[j + q][lane];
+#pragma unroll
+      for (int q = 0; q < SB; ++q) {
+        if (j + q >= kb) {
+          sv[0][q][lane] = sv[1][q][lane] = zero;
+          continue;
+        }
+        const df p = df_shfl(v[q], j + q);
+        const bool drop = p.hi <= tol;
+        df rp = df_rcp(p);
+        if (drop) rp = zero;
+        const df w = drop ? zero : v[q] * rp;
+        const df m = lane == j + q ? df_neg(rp) : w;  // the swept column; the pivot row gets 0 - (-rp) a
+        sv[0][q][lane] = v[q];
+        sv[1][q][lane] = m;
+#pragma unroll
+        for (int i = 0; i < SB; ++i) {
+          if (i == q) continue;
+          const df s = df_shfl(v[q], j + i);
+          v[i] = df_nfma(lane == j + q ? zero : v[i], m, s);
+        }
+        v[q] = m;
+        if (drop && lane == 0) {
+          if (p.hi < -tol) status[1] = k0 + j + q + 1;
+          else status[0] += 1;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < SB; ++q)
+        if (lane >= j + q) sd[lane][j + q] = v[q];
+        else if (lane < j) sd[j + q][lane] = v[q];
+    }
+    __syncthreads();
+    if (mine) {
+      const int r = r28 < j ? r28 : r28 + SB, c = c28 < j ? c28 : c28 + SB;
+      df x = sd[r][c];
+#pragma unroll
+      for (int q = 0; q < SB; ++q) x = df_nfma(x, sv[1][q][r], sv[0][q][c]);
+      sd[r][c] = x;
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < GJT; e += GJ_THREADS) {
+    const int r = e / GJB, c = e % GJB;
+    out[e] = df_neg(r >= c ? sd[r][c] : sd[c][r]);
+  }
+}
+
+__global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __restrict__ A, float* __restrict__ A32,
+                                                         double* __restrict__ work, int* __restrict__ status) {
+  cg::grid_group grid = cg::this_grid();
+  extern __shared__ __align__(16) unsigned char gj_smem[];
+  df* sW = reinterpret_cast<df*>(gj_smem);  // [2][GJT] staged W_i, [r][m]
+  df* sC = sW + 2 * GJT;                   // [2][GJT] staged C_j transposed, [m][c]
+  df* sT = sC + 2 * GJT;                   // owned tiles [r][c], pitch GJP
+  __shared__ df sd[GJB][GJP];
+  __shared__ df sv[2][SB][GJB];
+  __shared__ double smax[GJ_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = (n + GJB - 1) / GJB;
+  // published panels: C_j transposed ([2][nt][m][r]), W_j ([nt][r][m]), the
+  // inverse block ([2]) and the next but one diagonal tile ([2])
+  df* Cg = reinterpret_cast<df*>(work);
+  df* Wg = Cg + (int64_t)2 * nt * GJT;
+  df* Dg = Wg + (int64_t)nt * GJT;
+  df* Qg = Dg + 2 * GJT;
+  double dmax = 0.0;
+  for (int k = tid; k < n; k += GJ_THREADS) dmax = fmax(dmax, fabs(A[(int64_t)k * n + k]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  if (lane == 0) smax[warp] = dmax;
+  __syncthreads();
+  for (int k = 0; k < GJ_THREADS / 32; ++k) dmax = fmax(dmax, smax[k]);
+  const float tol = (float)(1e-10 * dmax);
+  // tiles t0 .. t1 of the triangle in row order; CTA 0 has none unless alone
+  const int nb = (int)gridDim.x, own = nb > 1 ? nb - 1 : 1, me = nb > 1 ? (int)blockIdx.x - 1 : 0;
+  const int64_t ntri = (int64_t)nt * (nt + 1) / 2;
+  const int t0 = me < 0 ? 0 : (int)(ntri * me / own), t1 = me < 0 ? 0 : (int)(ntri * (me + 1) / own);
+  int i0 = (int)((sqrtf(8.f * (float)t0 + 1.f) - 1.f) * 0.5f);
+  while ((i0 + 1) * (i0 + 2) / 2 <= t0) ++i0;
+  while (i0 * (i0 + 1) / 2 > t0) --i0;
+  const int j0 = t0 - i0 * (i0 + 1) / 2;
+  // publishes tile (i, j) where panel q or the diagonal after it needs it
+  auto publish = [&](const df* T, int i, int j, int q) {
+    if (q < nt && (i == q) != (j == q)) {  // C_m transposed, m the other index
+      df* dst = Cg + ((int64_t)(q & 1) * nt + (i == q ? j : i)) * GJT;
+      for (int e = tid; e < GJT; e += GJ_THREADS) {
+        const int m = e / GJB, r = e % GJB;
+        dst[e] = T[i == q ? m * GJP + r : r * GJP + m];
+      }
+    }
+    if (i == j && i == q + 1)
+      for (int e = tid; e < GJT; e += GJ_THREADS) Qg[(i & 1) * GJT + e] = T[(e / GJB) * GJP + e % GJB];
+  };
+  // the symmetric part of A, as k_symmetrize forms it
+  auto entry = [&](int r, int c) { return r < n && c < n ? 0.5 * (A[(int64_t)r * n + c] + A[(int64_t)c * n + r]) : 0.0; };
+  {
+    int i = i0, j = j0;
+    for (int t = t0; t < t1; ++t) {
+      df* T = sT + (int64_t)(t - t0) * GJ_TILE;
+      for (int e = tid; e < GJT; e += GJ_THREADS)
+        T[(e / GJB) * GJP + e % GJB] = df_from(entry(i * GJB + e / GJB, j * GJB + e % GJB));
+      __syncthreads();
+      publish(T, i, j, 0);
+      if (++j > i) { ++i; j = 0; }
+    }
+  }
+  if (blockIdx.x == 0) {
+    for (int e = tid; e < GJT; e += GJ_THREADS) sd[e / GJB][e % GJB] = df_from(entry(e / GJB, e % GJB));
+    sweep_block(sd, sv, min(GJB, n), 0, tol, status, Dg);
+  }
+  grid.sync();
+  for (int k = 0; k < nt; ++k) {
+    if (__ldcg(status + 1)) return;  // indefinite pivot: every CTA sees it after the barrier
+    const df* Ck = Cg + (int64_t)(k & 1) * nt * GJT;
+    const df* Dk = Dg + (k & 1) * GJT;
+    // ---- B: W_j = C_j D, eight rows of one tile a unit: half the products of
+    // an element a thread, the halves added through shared memory
+    if ((int)blockIdx.x < 4 * nt) {
+      df* D = sW;
+      df* H = sC;
+#pragma unroll
+      for (int q = 0; q < GJT / GJ_THREADS; ++q) D[tid + q * GJ_THREADS] = df_ldcg(Dk + tid + q * GJ_THREADS);
+      const int rr = warp & 7, half = warp >> 3;
+      for (int u = blockIdx.x; u < 4 * nt; u += nb) {
+        const int j = u >> 2, r = (u & 3) * 8 + rr;
+        df c[GJB / 2];
+#pragma unroll
+        for (int m = 0; m < GJB / 2; ++m) c[m] = df_ldcg(Ck + (int64_t)j * GJT + (half * (GJB / 2) + m) * GJB + r);
+        __syncthreads();
+        df a(0), b(0);  // two chains
+#pragma unroll
+        for (int m = 0; m < GJB / 2; m += 2) {
+          a = df_nfma(a, c[m], D[(half * (GJB / 2) + m) * GJB + lane]);
+          b = df_nfma(b, c[m + 1], D[(half * (GJB / 2) + m + 1) * GJB + lane]);
+        }
+        a = a + b;
+        if (half) H[rr * GJB + lane] = a;
+        __syncthreads();
+        if (!half && j != k) Wg[(int64_t)j * GJT + r * GJB + lane] = df_neg(a + H[rr * GJB + lane]);
+      }
+    }
+    grid.sync();
+    // ---- C: the tiles' updates; CTA 0 inverts the next diagonal block
+    const int k1 = k + 1;
+    auto stage = [&](int buf, int i, int j) {
+      const char* w = reinterpret_cast<const char*>(Wg + (int64_t)i * GJT);
+      const char* c = reinterpret_cast<const char*>(Ck + (int64_t)j * GJT);
+      const unsigned dw = (unsigned)__cvta_generic_to_shared(sW + buf * GJT), dc = (unsigned)__cvta_generic_to_shared(sC + buf * GJT);
+      static_assert(GJT * 8 == GJ_THREADS * 16, "one 16-byte copy a thread and operand");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dw + tid * 16), "l"(w + tid * 16));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dc + tid * 16), "l"(c + tid * 16));
+    };
+    // T -= W C^T for the staged pair; two rows of one column a thread
+    auto update = [&](df* T, int buf) {
+      const df* W = sW + buf * GJT + warp * GJB;
+      const df* C = sC + buf * GJT + lane;
+      df* t = T + warp * GJP + lane;
+      df v0 = t[0], v1 = t[16 * GJP], w0(0), w1(0);  // even and odd m apart: shorter sums, smaller error
+#pragma unroll 4
+      for (int m = 0; m < GJB; m += 2) {
+        const df c = C[m * GJB], e = C[(m + 1) * GJB];
+        v0 = df_nfma(v0, W[m], c);
+        v1 = df_nfma(v1, W[16 * GJB + m], c);
+        w0 = df_nfma(w0, W[m + 1], e);
+        w1 = df_nfma(w1, W[16 * GJB + m + 1], e);
+      }
+      t[0] = v0 + w0;
+      t[16 * GJP] = v1 + w1;
+    };
+    if (blockIdx.x == 0 && k1 < nt) {
+      stage(0, k1, k1);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      df* T = &sd[0][0];
+      for (int e = tid; e < GJT; e += GJ_THREADS) T[(e / GJB) * GJP + e % GJB] = df_ldcg(Qg + (k1 & 1) * GJT + e);
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
+      update(T, 0);
+      sweep_block(sd, sv, min(GJB, n - k1 * GJB), k1 * GJB, tol, status, Dg + (k1 & 1) * GJT);
+    }
+    int i = i0, j = j0;
+    if (t0 < t1 && i != k && j != k) stage(0, i, j);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int t = t0; t < t1; ++t) {
+      const int buf = (t - t0) & 1, in = j + 1 > i ? i + 1 : i, jn = j + 1 > i ? 0 : j + 1;
+      if (t + 1 < t1 && in != k && jn != k) stage(buf ^ 1, in, jn);
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
+      __syncthreads();
+      df* T = sT + (int64_t)(t - t0) * GJ_TILE;
+      if (i != k && j != k) {
+        update(T, buf);
+      } else if (i == j) {  // -D
+        for (int e = tid; e < GJT; e += GJ_THREADS) T[(e / GJB) * GJP + e % GJB] = df_neg(df_ldcg(Dk + e));
+      } else {  // W_i, or W_j transposed
+        const df* W = Wg + (int64_t)(j == k ? i : j) * GJT;
+        for (int e = tid; e < GJT; e += GJ_THREADS) {
+          const int a = e / GJB, b = e % GJB;
+          T[j == k ? a * GJP + b : b * GJP + a] = df_ldcg(W + e);
+        }
+      }
+      __syncthreads();
+      publish(T, i, j, k1);
+      i = in;
+      j = jn;
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    grid.sync();
+  }
+  // ---- A <- the inverse, both triangles, and its FP32 copy
+  int i = i0, j = j0;
+  for (int t = t0; t < t1; ++t) {
+    const df* T = sT + (int64_t)(t - t0) * GJ_TILE;
+    for (int e = tid; e < GJT; e += GJ_THREADS) {
+      const int a = e / GJB, b = e % GJB;
+      int r = i * GJB + a, c = j * GJB + b;
+      if (r < n && c < n && (i != j || r >= c)) {
+        const double v = -df_to(T[a * GJP + b]);
+        A[(int64_t)r * n + c] = v;
+        A32[(int64_t)r * n + c] = (float)v;
+      }
+      r = i * GJB + b;
+      c = j * GJB + a;
+      if (r < n && c < n && (i != j || r > c)) {
+        const double v = -df_to(T[b * GJP + a]);
+        A[(int64_t)c * n + r] = v;
+        A32[(int64_t)c * n + r] = (float)v;
+      }
+    }
+    if (++j > i) { ++i; j = 0; }
+  }
+}
+
 __global__ void k_to_float(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)a[i];
@@ -1404,34 +1668,45 @@ void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const double*
   const int64_t n = 3 * d.nv;
   cudaMemsetAsync(A, 0, sizeof(double) * n * n, s);
   k_dense_from_stencil<<<nblk(243 * d.nv, 256), 256, 0, s>>>(d, st, A);
-  k_symmetrize<<<nblk(n * n, 256), 256, 0, s>>>((int)n, A);
 }
 
-int coarsest_invert(cudaStream_t s, int n, double* A, double* work, int* status_dev, bool df_update,
-                    int max_per_sm) {
+// A: the coarsest matrix (its symmetric part is inverted in place), A32: the
+// inverse in FP32.  df_update: the sweeps where the triangle fits into the SMs'
+// shared memory (n up to about 2,500).  Else, and for FP64 operators, the
+// blocked Gauss-Jordan on A in place.
+int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update) {
   int dev = 0, nsm = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int threads = 256;
-  if (work) {  // blocked form: GJB-pivot panels, rank-GJB updates
-    void* fn = df_update ? (void*)k_gj_blocked<true> : (void*)k_gj_blocked<false>;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
-    if (per_sm < 1) return (int)cudaErrorCooperativeLaunchTooLarge;
-    const int tiles = ((n + GJB - 1) / GJB) * ((n + GJB - 1) / GJB);
-    const int blocks = std::max(1, std::min(tiles, nsm * std::min(per_sm, std::max(1, max_per_sm))));
-    cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
-    void* args[] = {&n, &A, &work, &status_dev};
-    return (int)cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, 0, s);
+  if (df_update) {
+    const int64_t nt = (n + GJB - 1) / GJB, ntri = nt * (nt + 1) / 2;
+    const int blocks = nt == 1 ? 1 : (int)std::min<int64_t>(nsm, ntri + 1);
+    const int64_t own = nt == 1 ? 1 : (ntri + blocks - 2) / (blocks - 1);
+    const int64_t smem = 8 * (4 * GJT + own * GJ_TILE);
+    if (smem <= GJ_SWEEP_SMEM) {
+      static PerDeviceOnce once;
+      const cudaError_t e = once_per_device(once, []() -> cudaError_t {
+        return cudaFuncSetAttribute(k_gj_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SWEEP_SMEM);
+      });
+      if (e != cudaSuccess) return (int)e;
+      cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
+      void* args[] = {&n, &A, &A32, &work, &status_dev};
+      return (int)cudaLaunchCooperativeKernel((void*)k_gj_sweep, dim3(blocks), dim3(GJ_THREADS), args, (size_t)smem, s);
+    }
   }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gauss_jordan, threads, 0);
+  k_symmetrize<<<nblk((int64_t)n * n, 256), 256, 0, s>>>(n, A);
+  void* fn = df_update ? (void*)k_gj_blocked<true> : (void*)k_gj_blocked<false>;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
   if (per_sm < 1) return (int)cudaErrorCooperativeLaunchTooLarge;
-  int64_t want = ((int64_t)n * n + threads - 1) / threads;
-  int blocks = (int)std::min<int64_t>(want, (int64_t)nsm * std::min(per_sm, 2));
-  if (blocks < 1) blocks = 1;
+  const int tiles = ((n + GJB - 1) / GJB) * ((n + GJB - 1) / GJB);
+  const int blocks = std::max(1, std::min(tiles, nsm * std::min(per_sm, 2)));
   cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
-  void* args[] = {&n, &A, &status_dev};
-  return (int)cudaLaunchCooperativeKernel((void*)k_gauss_jordan, dim3(blocks), dim3(threads), args,
-                                          0, s);
+  void* args[] = {&n, &A, &work, &status_dev};
+  const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, 0, s);
+  if (e != cudaSuccess) return (int)e;
+  launch_to_float(s, A, A32, (int64_t)n * n);
+  return (int)cudaGetLastError();
 }
 
 void launch_to_float(cudaStream_t s, const double* a, float* b, int64_t n) {

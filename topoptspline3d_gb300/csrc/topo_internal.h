@@ -227,12 +227,10 @@ template <typename T>
 void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                                const uint8_t* vmask, const T* kel, T* st);
 void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const double* st, double* A);
-// work: the blocked kernel's panels (GJB*GJB + 4*GJB*n doubles; null selects
-// the unblocked kernel); df_update: rank-GJB updates in double-float arithmetic.
-// max_per_sm caps the blocked form's CTAs per SM (it runs beside other work
-// on a second stream with 1).
-int coarsest_invert(cudaStream_t s, int n, double* A, double* work, int* status_dev, bool df_update = false,
-                    int max_per_sm = 2);
+// Inverts the symmetric part of A in place and writes its FP32 copy to A32.
+// work: published panels (128 n + 8192 doubles); df_update: in double-float
+// arithmetic (matrices from FP32 stencils).
+int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update);
 void launch_to_float(cudaStream_t s, const double* a, float* b, int64_t n);
 template <typename T>
 void launch_dense_gemv(cudaStream_t s, int n, const T* Ainv, const T* f_soa, T* u_soa, int64_t nv, int nb = 1);

@@ -2647,7 +2647,8 @@ int topo_multi_reserve(topo_handle* h, int capacity) {
     if (rc == TOPO_OK) rc = alloc((void**)v, n64);
   for (float** v : {&m->x32, &m->d32, &m->q32})
     if (rc == TOPO_OK) rc = alloc((void**)v, n64 / 2);
-  if (rc == TOPO_OK) rc = alloc((void**)&m->part, (size_t)capacity * 256 * sizeof(double));
+  if (rc == TOPO_OK) rc = alloc((void**)&m->part, (size_t)capacity * 512 * sizeof(double));
+  if (rc == TOPO_OK) rc = alloc((void**)&m->ctr, (size_t)capacity * sizeof(unsigned));
   if (rc == TOPO_OK) rc = alloc((void**)&m->sc, (size_t)capacity * 16 * sizeof(double));
   if (rc != TOPO_OK) {
     for (void* p : m->allocs) cudaFree(p);
@@ -2708,9 +2709,9 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
   CK(cudaEventRecord(e0, h->stream));
   // r = f - A x, ||r||^2, ||f||^2 per right-hand side
   fine64(h, L0.d, m.x, m.f, m.r, true, nb);
-  launch_bdot<double>(h->stream, m.r, m.r, n3, nb, m.part, slot(B_RR));
-  launch_bdot<double>(h->stream, m.f, m.f, n3, nb, m.part, slot(B_FF));
-  count_launch(5);
+  launch_bdot<double>(h->stream, m.r, m.r, n3, nb, m.part, m.ctr, slot(B_RR));
+  launch_bdot<double>(h->stream, m.f, m.f, n3, nb, m.part, m.ctr, slot(B_FF));
+  count_launch(3);
   std::vector<double> rr(nb), ff(nb);
   CK(cudaMemcpyAsync(rr.data(), slot(B_RR), sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaMemcpyAsync(ff.data(), slot(B_FF), sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
@@ -2742,39 +2743,37 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
       float* r32 = L0.F32;
       float* z32 = L0.U32;
       CK(cudaMemsetAsync(m.x32, 0, sizeof(float) * n3 * nb, h->stream));
-      launch_bdot<float>(h->stream, r32, r32, n3, nb, m.part, slot(I_FF));
+      launch_bdot<float>(h->stream, r32, r32, n3, nb, m.part, m.ctr, slot(I_FF));
       CK(cudaMemcpyAsync(slot(I_RR), slot(I_FF), sizeof(double) * nb, cudaMemcpyDeviceToDevice, h->stream));
-      count_launch(2);
+      count_launch();
       for (int j = 0; j < inner_max; ++j) {
         if (!cheb_zero_start(TOPO_SMOOTH_CHEBYSHEV, o->pre, cp))
           CK(cudaMemsetAsync(z32, 0, sizeof(float) * n3 * nb, h->stream));
         vcycle32(h, o->pre, o->post, TOPO_SMOOTH_CHEBYSHEV, cp, true);
         ++nvc;
-        launch_bdot<float>(h->stream, r32, z32, n3, nb, m.part, slot(I_RZ));
+        launch_bdot<float>(h->stream, r32, z32, n3, nb, m.part, m.ctr, slot(I_RZ));
         launch_bbeta(h->stream, nb, slot(I_RZ), slot(I_ZERO), slot(I_RZOLD), j == 0, slot(I_BETA));
         launch_bdir<float>(h->stream, n3, nb, z32, m.d32, slot(I_BETA));
         launch_fine_apply<float>(h->stream, L0.d, h->rhop32, L0.vmask, m.d32, nullptr, m.q32, false, nb,
                                  tz32_arg(h));
-        launch_bdot<float>(h->stream, m.d32, m.q32, n3, nb, m.part, slot(I_DQ));
+        launch_bdot<float>(h->stream, m.d32, m.q32, n3, nb, m.part, m.ctr, slot(I_DQ));
         launch_balpha(h->stream, nb, slot(I_RZ), slot(I_DQ), slot(I_RR), slot(I_FF), inner_rtol * inner_rtol,
                       slot(I_ALPHA), slot(I_RZOLD));
-        launch_bupdate<float>(h->stream, n3, nb, m.x32, r32, nullptr, m.d32, m.q32, slot(I_ALPHA));
-        launch_bdot<float>(h->stream, r32, r32, n3, nb, m.part, slot(I_RR));
-        count_launch(14);
+        launch_bupdate<float>(h->stream, n3, nb, m.x32, r32, nullptr, m.d32, m.q32, slot(I_ALPHA), m.part, m.ctr,
+                              slot(I_RR));
+        count_launch(7);
       }
       k_to_double<float><<<nb256(n3 * nb), 256, 0, h->stream>>>(n3 * nb, m.x32, m.z);
     }
-    launch_bdot<double>(h->stream, m.r, m.z, n3, nb, m.part, slot(B_RZ));
-    if (it > 0) launch_bdot<double>(h->stream, m.z, m.rold, n3, nb, m.part, slot(B_ZROLD));
+    launch_bdot<double>(h->stream, m.r, m.z, n3, nb, m.part, m.ctr, slot(B_RZ), it > 0 ? m.rold : nullptr, slot(B_ZROLD));
     launch_bbeta(h->stream, nb, slot(B_RZ), slot(B_ZROLD), slot(B_RZOLD), it == 0, slot(B_BETA));
     launch_bdir<double>(h->stream, n3, nb, m.z, m.d, slot(B_BETA));
     fine64(h, L0.d, m.d, nullptr, m.q, false, nb);
-    launch_bdot<double>(h->stream, m.d, m.q, n3, nb, m.part, slot(B_DQ));
+    launch_bdot<double>(h->stream, m.d, m.q, n3, nb, m.part, m.ctr, slot(B_DQ));
     launch_balpha(h->stream, nb, slot(B_RZ), slot(B_DQ), slot(B_RR), slot(B_FF), rtol2, slot(B_ALPHA),
                   slot(B_RZOLD));
-    launch_bupdate<double>(h->stream, n3, nb, m.x, m.r, m.rold, m.d, m.q, slot(B_ALPHA));
-    launch_bdot<double>(h->stream, m.r, m.r, n3, nb, m.part, slot(B_RR));
-    count_launch(it > 0 ? 16 : 14);
+    launch_bupdate<double>(h->stream, n3, nb, m.x, m.r, m.rold, m.d, m.q, slot(B_ALPHA), m.part, m.ctr, slot(B_RR));
+    count_launch(9);
     CKL();
     CK(cudaMemcpyAsync(rr.data(), slot(B_RR), sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
@@ -2784,8 +2783,8 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
   }
   // true FP64 residuals of the final iterates
   fine64(h, L0.d, m.x, m.f, m.r, true, nb);
-  launch_bdot<double>(h->stream, m.r, m.r, n3, nb, m.part, slot(B_RR));
-  count_launch(3);
+  launch_bdot<double>(h->stream, m.r, m.r, n3, nb, m.part, m.ctr, slot(B_RR));
+  count_launch(2);
   CK(cudaMemcpyAsync(rr.data(), slot(B_RR), sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaEventRecord(e1, h->stream));
   CK(cudaEventSynchronize(e1));

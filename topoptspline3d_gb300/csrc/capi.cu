@@ -206,7 +206,11 @@ void level_apply(topo_handle* h, int l, const T* u, const T* f, T* out, bool res
   DevLevel& L = h->lv[l];
   if (l == 0) {
     EventPair* ev = prof_begin(h, P<T>::fam_apply);
-    if (sizeof(T) == 8 && h->fine_df)
+    if (sizeof(T) == 8 && h->fine_fx())
+      launch_fine_apply_fx(h->stream, L.d, reinterpret_cast<const double*>(P<T>::rhop(h)), L.vmask,
+                           reinterpret_cast<const double*>(u), reinterpret_cast<const double*>(f),
+                           reinterpret_cast<double*>(out), residual, h->nb, h->tz64);
+    else if (sizeof(T) == 8 && h->fine_df)
       launch_fine_apply_df(h->stream, L.d, reinterpret_cast<const double*>(P<T>::rhop(h)), L.vmask,
                            reinterpret_cast<const double*>(u), reinterpret_cast<const double*>(f),
                            reinterpret_cast<double*>(out), residual, h->nb, h->tz64);
@@ -284,7 +288,13 @@ void cheb_level(topo_handle* h, int l, const ChebParams& cp, bool zero_start, bo
     } else if (l == 0) {
       const bool dots = last_dots && k == cp.degree - 1;
       EventPair* ev = prof_begin(h, P<T>::fam_smooth);
-      const int np = launch_fine_cheb<T>(
+      int np = 0;
+      if constexpr (sizeof(T) == 8) {
+        if (h->fine_fx())
+          launch_fine_cheb_fx(h->stream, L.d, P<T>::rhop(h), L.vmask, ua, P<T>::F(L), ub, P<T>::dinv(L), P<T>::cd(L),
+                              coef, k == 0, h->nb, h->tz64);
+      }
+      if (sizeof(T) == 4 || !h->fine_fx()) np = launch_fine_cheb<T>(
           h->stream, L.d, P<T>::rhop(h), L.vmask, ua, P<T>::F(L), ub, P<T>::dinv(L), P<T>::cd(L), coef, k == 0,
           h->nb, sizeof(T) == 4 ? tz32_arg(h) : h->tz64, d_in_u && k == 1, dots ? h->vdot : nullptr, h->fdot_cap,
           h->vdot_out, TOPO_FUSED_DOT_TICKET ? h->ctr : nullptr);
@@ -670,6 +680,20 @@ __global__ void k_cheb_table(const double* lam, int nl, double lo, double hi, in
   }
 }
 
+// A power step's product on level 0.
+template <typename T>
+void fine_product(topo_handle* h, const T* x, T* y) {
+  DevLevel& L = h->lv[0];
+  if constexpr (sizeof(T) == 8) {
+    if (h->fine_fx()) {
+      launch_fine_apply_fx(h->stream, L.d, P<T>::rhop(h), L.vmask, x, nullptr, y, false, 1, h->tz64);
+      return;
+    }
+  }
+  launch_fine_apply<T>(h->stream, L.d, P<T>::rhop(h), L.vmask, x, nullptr, y, false, 1,
+                       sizeof(T) == 4 ? tz32_arg(h) : h->tz64);
+}
+
 // Largest eigenvalue of D^-1 A of every level whose bound is stale, by power
 // iteration.  First estimate of a level: 12 steps from the deterministic start
 // (as the oracle).  After an operator update: 4 steps from the previous
@@ -714,8 +738,7 @@ int estimate_bounds(topo_handle* h) {
     double* sl = h->sc + S_PW + 2 * r.l;
     for (int it = 0; it < k; ++it) {
       launch_dot<T>(h->stream, r.x, r.x, n3, h->partial, sl, h->ctr);
-      if (r.l == 0) launch_fine_apply<T>(h->stream, L.d, P<T>::rhop(h), L.vmask, r.x, nullptr, r.y, false, 1,
-                                         sizeof(T) == 4 ? tz32_arg(h) : h->tz64);
+      if (r.l == 0) fine_product<T>(h, r.x, r.y);
       else launch_stencil_apply<T>(h->stream, L.d, P<T>::st(L), r.x, nullptr, r.y, false);
       k_dinv_apply<T><<<nb256(L.d.nv), 256, 0, h->stream>>>(L.d.nv, P<T>::dinv(L), r.y, r.z, sl,
                                                            sizeof(T) == 4 && r.l == 0);
@@ -1757,6 +1780,7 @@ int topo_apply_fine(topo_handle* h, int precision) {
 
 int topo_residual(topo_handle* h, int level) {
   DEVICE_SCOPE(h);
+  RefOps ref_ops(h);
   RET(check_ready(h, level > 0));
   if (level < 0 || level >= (int)h->lv.size()) return TOPO_E_BAD_INPUT;
   RET(update_penalised_if_stale(h));
@@ -1826,6 +1850,7 @@ int topo_coarsest_solve(topo_handle* h) {
 
 int topo_vcycle(topo_handle* h, int pre, int post, double* relres) {
   DEVICE_SCOPE(h);
+  RefOps ref_ops(h);
   RET(check_ready(h, true));
   if (!h->ops64) return fail(h, TOPO_E_STATE, "FP64 operators not built");
   ChebParams cp;
@@ -1898,6 +1923,7 @@ static int solve_impl(topo_handle* h, const topo_solve_opts* o, topo_solve_stats
   RET(check_ready(h, true));
   h->energy_ready = false;
   if (!o || o->rtol <= 0 || o->max_iter < 0 || o->pre < 0 || o->post < 0) return TOPO_E_BAD_INPUT;
+  RefOps ref_ops(h, o->mode == TOPO_SOLVE_VCYCLE);
   DevLevel& L0 = h->lv[0];
   const int64_t n3 = 3 * L0.d.nv;
   ChebParams cp;
@@ -2303,7 +2329,7 @@ int topo_spline_adjoint(topo_handle* h) {
 // FP64 fine operator on a batch of vectors, in the handle's fine arithmetic.
 static void fine64(topo_handle* h, const LevelDims& d, const double* u, const double* f, double* out, bool residual,
                    int nb) {
-  if (h->fine_df) launch_fine_apply_df(h->stream, d, h->rhop, h->lv[0].vmask, u, f, out, residual, nb, h->tz64);
+  if (h->fine_fx()) launch_fine_apply_fx(h->stream, d, h->rhop, h->lv[0].vmask, u, f, out, residual, nb, h->tz64);
   else launch_fine_apply<double>(h->stream, d, h->rhop, h->lv[0].vmask, u, f, out, residual, nb, h->tz64);
 }
 
@@ -2458,7 +2484,7 @@ int topo_autotune(topo_handle* h, const topo_solve_opts* base, topo_solve_opts* 
     for (int rep = 0; rep < 2; ++rep) {
       CK(cudaEventRecord(a, h->stream));
       for (int i = 0; i < 5; ++i) {
-        if (h->fine_df) launch_fine_apply_df(h->stream, L0.d, h->rhop, L0.vmask, h->work, nullptr, L0.R, false, 1, tzs[k]);
+        if (h->fine_fx()) launch_fine_apply_fx(h->stream, L0.d, h->rhop, L0.vmask, h->work, nullptr, L0.R, false, 1, tzs[k]);
         else launch_fine_apply<double>(h->stream, L0.d, h->rhop, L0.vmask, h->work, nullptr, L0.R, false, 1, tzs[k]);
       }
       CK(cudaEventRecord(b, h->stream));

@@ -54,7 +54,8 @@ struct topo_handle {
   topo::UNetState* unet = nullptr;  // learned preconditioner (topo_unet_enable)
   bool mat_registered = false;      // holds a reference on the device's element constants
   int nb = 1;                       // right-hand sides the level vectors hold (multi-RHS solve)
-  int fine_df = 1;                  // FP64 fine operator in double-float arithmetic (topo_set_fine_arithmetic)
+  int fine_df = 1;                  // FP64 fine operator emulated (fixed point or double-float), topo_set_fine_arithmetic
+  bool ref_ops = false;             // inside the reference-mode entry points (RefOps)
   int tz32 = 16, tz64 = 16;         // z-march depth of the fine kernels, FP32 / FP64 (topo_autotune)
   bool fine_tc = false;             // FP32 fine element products on the tensor cores (topo_set_fine_tensor_cores)
   // the coarsest inverse is recomputed at every coarse_every-th operator
@@ -204,4 +205,22 @@ struct topo_handle {
   bool prof = false;
   std::vector<topo::EventPair> evs[TOPO_K_COUNT];
   std::vector<topo::EventPair> evpool;
+  // The FP64 fine operator of the CG solvers runs in fixed point (k_fine_fx).
+  bool fine_fx() const { return fine_df && !ref_ops; }
 };
+
+namespace topo {
+// Scope of the reference-mode entry points (topo_vcycle, topo_residual, repeated
+// V-cycles as a solve): double-float residuals and FP64 smoothing.  Their
+// callers compare residuals of nearly converged fields between runs; a residual
+// is a difference of nearly equal numbers there, so any other rounding of K u
+// shows in its last digits.
+struct RefOps {
+  topo_handle* h;
+  bool prev;
+  RefOps(topo_handle* hh, bool on = true) : h(hh), prev(hh ? hh->ref_ops : false) { if (h && on) h->ref_ops = true; }
+  ~RefOps() { if (h) h->ref_ops = prev; }
+  RefOps(const RefOps&) = delete;
+  RefOps& operator=(const RefOps&) = delete;
+};
+}  // namespace topo

@@ -56,6 +56,7 @@ void upload_template(const double* Ke576, double lam, double mu, double h) {
     mdf[i].y = (float)(m64[i] - (double)mdf[i].x);
   }
   cudaMemcpyToSymbol(cModalDF, mdf, sizeof(mdf));
+  upload_fx(lam, mu, h);
 }
 
 // ---------------------------------------------------------------------------

@@ -168,6 +168,14 @@ int launch_fine_apply_dot(cudaStream_t s, const LevelDims& d, const T* rhop, con
 void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
                           const double* u, const double* f, double* out, bool residual, int nb = 1, int tz = 0,
                           double* energy = nullptr);
+// FP64 vectors, 64-bit fixed-point arithmetic (k_fine_fx): K u or f - K u, and
+// the Chebyshev step of launch_fine_cheb<double>
+void launch_fine_apply_fx(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
+                          const double* u, const double* f, double* out, bool residual, int nb = 1, int tz = 0);
+void launch_fine_cheb_fx(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
+                         const double* u, const double* f, double* uout, const double* dinv, double* dvec,
+                         const double* coef, bool first, int nb, int tz);
+void upload_fx(double lam, double mu, double h);
 template <typename T>
 void launch_fine_gs(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, T* u,
                     const T* f, int colour, bool reverse);

@@ -1274,8 +1274,9 @@ int topo_create(const topo_config* cfg, const uint8_t* eactive, topo_handle** ou
     A(dalloc(hp, &h->dKe, 576));
     A(dalloc(hp, &h->partial, 2048)); A(dalloc(hp, &h->sc, S_COUNT)); A(dalloc(hp, &h->status, 4));
     // partials of the fused fine-operator dot: one per CTA of 32 x 8 element
-    // tiles (31 x 7 owned vertices) at z-march depths of 4 and more
-    h->fdot_cap = (int)std::min<int64_t>(1 << 24, (int64_t)((d0.vx + 30) / 31) * ((d0.vy + 6) / 7) * ((d0.vz + 3) / 4));
+    // tiles (31 x 7 owned vertices) at z-march depths of 4 and more, or where
+    // the z blocks fill the chip
+    h->fdot_cap = (int)std::min<int64_t>(1 << 24, FINE_FILL_CTAS + (int64_t)((d0.vx + 30) / 31) * ((d0.vy + 6) / 7) * ((d0.vz + 3) / 4));
     A(dalloc(hp, &h->fdot, h->fdot_cap));
     A(dalloc(hp, &h->vdot, h->fdot_cap));
     A(dalloc(hp, &h->ctr, 1));

@@ -63,14 +63,13 @@ struct FxCheb {
 template <int MODE, bool VOID>
 __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __restrict__ rhop,
                                                    const uint8_t* __restrict__ vmask, const double* __restrict__ u,
-                                                   const double* __restrict__ f, double* __restrict__ out, int TZ,
+                                                   const double* __restrict__ f, double* __restrict__ out, int zblk,
                                                    FxCheb ch) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxSmem& sm = *reinterpret_cast<FxSmem*>(fx_smem);
   const int t = threadIdx.x, i = t % TX, j = t / TX;
-  const int zblk = fine_zblocks(d.vz, TZ);
   const int rhs = blockIdx.z / zblk, kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TX - 1), y0 = blockIdx.y * (TY - 1), zb0 = kz * TZ;
+  const int x0 = blockIdx.x * (TX - 1), y0 = blockIdx.y * (TY - 1), zb0 = fine_zblock(d.vz, zblk, kz);
   const int64_t nv = d.nv, plane_n = (int64_t)d.vx * d.vy;
   u += (int64_t)rhs * 3 * nv;
   if (MODE >= 1) f += (int64_t)rhs * 3 * nv;
@@ -78,42 +77,64 @@ __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __
   double* __restrict__ dv = MODE == 2 ? ch.dvec + (int64_t)rhs * 3 * nv : nullptr;
   const int gx = x0 + i, gy = y0 + j;  // owned vertex (x, y) and element (x - 1, y - 1)
   const bool own = i < TX - 1 && j < TY - 1 && gx < d.vx && gy < d.vy;
-  const int zb1 = fine_zblock_end(d.vz, TZ, kz);
+  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
   int z0 = zb0, zend = zb1;  // the planes marched: [zb0, zb1) less the void (LevelDims::colz)
   if (VOID) {
     const int2 cz = d.colz[blockIdx.x + gridDim.x * blockIdx.y];
     z0 = min(max(zb0, cz.x), zb1);
     zend = max(z0, min(zb1, cz.y + 2));
   }
-  // the owned vertex of plane p with its element forces y (fixed DOFs: none)
-  auto finish = [&](int p, const double y[3]) {
-    const int64_t v = gx + (int64_t)d.vx * gy + plane_n * p;
-    const uint8_t m = vmask[v];
+  // What the owned vertex of plane p needs besides its element forces.  Loaded
+  // before the step's first barrier, so that the loads' latency passes there.
+  struct Vertex {
+    int64_t v;
+    uint8_t m;
+    double f[3], di[MODE == 2 ? 9 : 1], d[3], u[3];
+  };
+  auto load_vertex = [&](int p, Vertex& V) {
+    V.v = gx + (int64_t)d.vx * gy + plane_n * p;
+    V.m = vmask[V.v];
+    if (MODE >= 1) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) V.f[c] = f[c * nv + V.v];
+    }
+    if (MODE == 2) {
+#pragma unroll
+      for (int c = 0; c < 9; ++c) V.di[c] = ch.dinv[c * nv + V.v];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        V.d[c] = ch.first ? 0.0 : dv[c * nv + V.v];
+        V.u[c] = u[c * nv + V.v];
+      }
+    }
+  };
+  // the vertex with its element forces y (fixed DOFs: none)
+  auto finish = [&](const Vertex& V, const double y[3]) {
     if (MODE < 2) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const bool fr = (m >> c) & 1;
-        out[c * nv + v] = MODE == 1 ? (fr ? f[c * nv + v] - y[c] : 0.0) : (fr ? y[c] : 0.0);
+        const bool fr = (V.m >> c) & 1;
+        out[c * nv + V.v] = MODE == 1 ? (fr ? V.f[c] - y[c] : 0.0) : (fr ? y[c] : 0.0);
       }
     } else {
       double r[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) r[c] = ((m >> c) & 1) ? f[c * nv + v] - y[c] : 0.0;
+      for (int c = 0; c < 3; ++c) r[c] = ((V.m >> c) & 1) ? V.f[c] - y[c] : 0.0;
       const double c_old = __ldg(ch.coef), c_new = __ldg(ch.coef + 1);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double z = ch.dinv[(3 * c) * nv + v] * r[0] + ch.dinv[(3 * c + 1) * nv + v] * r[1] +
-                         ch.dinv[(3 * c + 2) * nv + v] * r[2];
-        const double dn = ch.first ? c_new * z : c_old * dv[c * nv + v] + c_new * z;
-        dv[c * nv + v] = dn;
-        out[c * nv + v] = u[c * nv + v] + dn;
+        const double z = V.di[3 * c] * r[0] + V.di[3 * c + 1] * r[1] + V.di[3 * c + 2] * r[2];
+        const double dn = ch.first ? c_new * z : c_old * V.d[c] + c_new * z;
+        dv[c * nv + V.v] = dn;
+        out[c * nv + V.v] = V.u[c] + dn;
       }
     }
   };
   if (VOID && own) {  // void planes see no forces
     const double none[3] = {0.0, 0.0, 0.0};
-    for (int p = zb0; p < z0; ++p) finish(p, none);
-    for (int p = zend; p < zb1; ++p) finish(p, none);
+    Vertex V;
+    for (int p = zb0; p < z0; ++p) { load_vertex(p, V); finish(V, none); }
+    for (int p = zend; p < zb1; ++p) { load_vertex(p, V); finish(V, none); }
   }
   if (z0 >= zend) return;  // the whole CTA
   int pxy[KS];  // this thread's staged vertices, in-plane (-1: outside the domain)
@@ -168,6 +189,8 @@ __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __
   // step st: finish vertex plane st - 1 (layers st - 2 and st - 1), compute element layer st
   for (int st = z0 - 1; st <= zend; ++st) {
     const double pe = pe_n;
+    Vertex V;
+    if (st - 1 >= z0 && own) load_vertex(st - 1, V);
     if (st < zend) {
       prefetch(st + 2);
       if (st + 1 < zend) pe_n = load_pe(st + 1);
@@ -189,7 +212,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __
         top[c] = fx_down(own1[1][c], ye - oe + 1) + fx_down(r1[c], ye - re + 1);
       }
       te = ye + 1;
-      if (st - 1 >= z0) finish(st - 1, y);
+      if (st - 1 >= z0) finish(V, y);
     }
     if (st == zend) break;
     __syncthreads();  // C
@@ -264,9 +287,9 @@ void launch(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_
   once_per_device(once[vd ? 1 : 0], [&]() -> cudaError_t {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSmem));
   });
-  const int TZ = tz > 0 ? tz : 16;
-  const dim3 g((d.vx + TX - 2) / (TX - 1), (d.vy + TY - 2) / (TY - 1), (unsigned)(fine_zblocks(d.vz, TZ) * nb));
-  fn<<<g, NT, sizeof(FxSmem), s>>>(d, rhop, vmask, u, f, out, TZ, ch);
+  const int gx = (d.vx + TX - 2) / (TX - 1), gy = (d.vy + TY - 2) / (TY - 1);
+  const int zblk = fine_zblocks(d.vz, tz > 0 ? tz : 16, (int64_t)gx * gy * nb);
+  fn<<<dim3(gx, gy, zblk * nb), NT, sizeof(FxSmem), s>>>(d, rhop, vmask, u, f, out, zblk, ch);
 }
 
 }  // namespace

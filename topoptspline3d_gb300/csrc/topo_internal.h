@@ -75,14 +75,22 @@ inline int fine_rows_flag(int rows) {
   return rows == 4 ? TOPO_FINE_ROWS4_FLAG : rows == 16 ? TOPO_FINE_ROWS16_FLAG : 0;
 }
 
-// z blocks of the fine z-marching kernels: blocks of tz vertex planes, the
-// last one also taking the remainder (up to 2 tz - 1 planes) rather than a
-// short block of its own, which would recompute a whole element layer below
-// it for a few planes.  Block k covers planes [k tz, fine_zblock_end(k)).
-__host__ __device__ inline int fine_zblocks(int vz, int tz) { return vz / tz > 1 ? vz / tz : 1; }
-__host__ __device__ inline int fine_zblock_end(int vz, int tz, int k) {
-  return k + 1 >= fine_zblocks(vz, tz) ? vz : (k + 1) * tz;
+// z blocks of the fine z-marching kernels over `tiles` columns of CTAs (all
+// right-hand sides): vz / tz of them, more where that leaves the chip idle, up
+// to two CTAs on each of the 152 SMs or one plane a block.  A block of few
+// planes recomputes the element layer below it, but a march costs 2 to 5 us a
+// plane whatever the grid (16x8x8: FP32 step 11.9 us with 4 planes a block,
+// 8.1 with 1; fixed-point step 30.5 / 14.1; 77x44x42 with 304 CTAs 38 us, with
+// 441 43 us).  The planes are dealt evenly: block k covers [fine_zblock(k),
+// fine_zblock(k + 1)); a last block that takes the remainder of vz / tz marches
+// up to twice as long as the others (77x44x42, 4 planes: 57 us).
+constexpr int FINE_FILL_CTAS = 304;
+inline int fine_zblocks(int vz, int tz, int64_t tiles) {
+  const int64_t by_depth = vz / tz > 1 ? vz / tz : 1, fill = FINE_FILL_CTAS / (tiles > 0 ? tiles : 1);
+  const int64_t most = fill < vz ? fill : vz;
+  return (int)(by_depth > most ? by_depth : most);
 }
+__host__ __device__ inline int fine_zblock(int vz, int zblk, int k) { return k * vz / zblk; }
 
 // Vertex tile of the fine z-marching kernels: a CTA owns FINE_TILE_X - 1 by
 // FINE_TILE_Y - 1 vertex columns and computes the FINE_TILE_X x FINE_TILE_Y

@@ -41,7 +41,7 @@ namespace cg = cooperative_groups;
 namespace topo {
 
 constexpr int kMmaMaxM = 4;        // constraints handled by the GPU kernel
-constexpr int kMmaBlock = 256;
+constexpr int kMmaBlock = 256;     // threads of a CTA, at most (mma_alloc)
 constexpr int kMmaWarps = kMmaBlock / 32;
 constexpr int kMmaSlots = 32;      // reduction slots per grid-wide reduction
 constexpr double kStepFrac = 0.99; // asym_clamp_factor, optimization/mma_t.h:20
@@ -85,7 +85,7 @@ __device__ __forceinline__ void grid_reduce(cg::grid_group& grid, double* v, int
   double* slot = part + (size_t)(rs & 1) * kMmaSlots * gridDim.x;
   for (int k = threadIdx.x; k < nk; k += blockDim.x) {
     double t = wsum[0][k];
-    for (int w = 1; w < kMmaWarps; ++w) t = k < ns ? t + wsum[w][k] : fmax(t, wsum[w][k]);
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) t = k < ns ? t + wsum[w][k] : fmax(t, wsum[w][k]);
     slot[(size_t)k * gridDim.x + blockIdx.x] = t;
   }
   grid.sync();
@@ -126,16 +126,18 @@ __device__ void small_solve(double (&A)[K][K], double (&r)[K]) {
 }
 
 // Scalar rows of the KKT error at step t (optimization/mma_t.cu:597-660); vsum,
-// vmax are the reduced per-variable terms and gsum the proxy constraints.
-template <int M>
-__device__ void kkt_scalars(const MmaArgs& A, MmaScalars<M>& S, double t, double damp, double vsum,
+// vmax are the reduced per-variable terms and gsum the proxy constraints.  HERE:
+// at the current point (t = 0), without reading the direction.
+template <int M, bool HERE>
+__device__ void kkt_scalars(const MmaArgs& A, const MmaScalars<M>& S, double t, double damp, double vsum,
                             double vmax, const double* gsum, double* err2, double* errinf) {
   double e2 = vsum, ei = fmax(-10.0, vmax);
   double lt[M], la = 0.0;
-  for (int i = 0; i < M; ++i) { lt[i] = S.lam[i] + t * S.dl[i]; la += lt[i] * A.a[i]; }
-  const double zt = S.z + t * S.dz, zetat = S.zeta + t * S.dzeta;
+  auto at = [t](double v, const double& d) { return HERE ? v : v + t * d; };
+  for (int i = 0; i < M; ++i) { lt[i] = at(S.lam[i], S.dl[i]); la += lt[i] * A.a[i]; }
+  const double zt = at(S.z, S.dz), zetat = at(S.zeta, S.dzeta);
   for (int i = 0; i < M; ++i) {
-    const double yt = S.y[i] + t * S.dy[i], mt = S.mu[i] + t * S.dmu[i], st = S.s[i] + t * S.ds[i];
+    const double yt = at(S.y[i], S.dy[i]), mt = at(S.mu[i], S.dmu[i]), st = at(S.s[i], S.ds[i]);
     const double rey = A.c[i] + A.d[i] * yt - lt[i] - mt;
     const double relam = (gsum[i] - A.a[i] * zt - yt + st - S.b[i]) / damp;
     const double remu = mt * yt - S.eps;
@@ -272,9 +274,11 @@ __global__ void __launch_bounds__(kMmaBlock) k_mma_update(MmaArgs A) {
           S.ds[i] = eps / S.lam[i] - S.s[i] / S.lam[i] * S.dl[i] - S.s[i];
         }
         S.dzeta = eps / S.z - S.zeta - (S.zeta / S.z) * S.dz;
-        // the error at the current point (damping 1) records lambda for p/q lambda
+      } else if (threadIdx.x == 32) {
+        // beside it, the error at the current point (damping 1), which records
+        // lambda for p/q lambda
         double e2, ei;
-        kkt_scalars<M>(A, S, 0.0, 1.0, red[kV], red[kX], red + kG, &e2, &ei);
+        kkt_scalars<M, true>(A, S, 0.0, 1.0, red[kV], red[kX], red + kG, &e2, &ei);
         S.old_err = e2;
         for (int i = 0; i < M; ++i) S.lampq[i] = S.lam[i];
       }
@@ -304,16 +308,22 @@ __global__ void __launch_bounds__(kMmaBlock) k_mma_update(MmaArgs A) {
         v[2] = fmax(v[2], fmax((-1.0 / kStepFrac) * dxij / xij, (-1.0 / kStepFrac) * detaj / etaj));
       }
       grid_reduce(grid, v, 0, 3, A.part, rs, wsum, red);
-      if (threadIdx.x == 0) {
-        double t3 = red[2];
-        for (int i = 0; i < M; ++i) {
-          t3 = fmax(t3, (-1.0 / kStepFrac) * S.dy[i] / S.y[i]);
-          t3 = fmax(t3, (-1.0 / kStepFrac) * S.dl[i] / S.lam[i]);
-          t3 = fmax(t3, (-1.0 / kStepFrac) * S.dmu[i] / S.mu[i]);
-          t3 = fmax(t3, (-1.0 / kStepFrac) * S.ds[i] / S.s[i]);
+      double t3 = red[2];
+      if (threadIdx.x < 32) {  // one quotient a lane
+        const int i = threadIdx.x >> 2, w = threadIdx.x & 3;
+        double num = 0.0, den = 1.0;
+        if (i < M) {
+          num = w == 0 ? S.dy[i] : w == 1 ? S.dl[i] : w == 2 ? S.dmu[i] : S.ds[i];
+          den = w == 0 ? S.y[i] : w == 1 ? S.lam[i] : w == 2 ? S.mu[i] : S.s[i];
+        } else if (i == M && w < 2) {
+          num = w ? S.dzeta : S.dz;
+          den = w ? S.zeta : S.z;
         }
-        t3 = fmax(t3, (-1.0 / kStepFrac) * S.dz / S.z);
-        t3 = fmax(t3, (-1.0 / kStepFrac) * S.dzeta / S.zeta);
+        // (the idle lanes' 0 is below red[2]'s floor in the step: max(.., 1))
+        t3 = fmax(t3, (-1.0 / kStepFrac) * num / den);
+        for (int o = 16; o > 0; o >>= 1) t3 = fmax(t3, __shfl_xor_sync(0xffffffffu, t3, o));
+      }
+      if (threadIdx.x == 0) {
         S.step = 1.0 / fmax(fmax(red[0], red[1]), fmax(t3, 1.0));
         S.new_err = 1e30;
         S.new_inf = 1e30;
@@ -348,7 +358,7 @@ __global__ void __launch_bounds__(kMmaBlock) k_mma_update(MmaArgs A) {
         grid_reduce(grid, v, M + 1, 1, A.part, rs, wsum, red);
         if (threadIdx.x == 0) {
           double e2, ei;
-          kkt_scalars<M>(A, S, t, S.damp, red[M], red[M + 1], red, &e2, &ei);
+          kkt_scalars<M, false>(A, S, t, S.damp, red[M], red[M + 1], red, &e2, &ei);
           S.new_err = e2;
           S.new_inf = ei;
           for (int i = 0; i < M; ++i) S.lampq[i] = lt[i];
@@ -458,7 +468,7 @@ struct topo_mma {
   double *x, *xold, *xmin, *xmax, *L, *U, *alpha, *beta, *lastdx, *xi, *eta, *p, *q, *Dx, *dlx, *dx, *dxi,
       *deta, *part, *stats, *lbub;
   double c[kMmaMaxM], d[kMmaMaxM];
-  int nblocks = 1;
+  int nblocks = 1, threads = kMmaBlock;
   int stop_counter = 0;
   bool initialised = false;
   std::string err;
@@ -497,8 +507,13 @@ static int mma_alloc(topo_mma* o) {
   }
   if (rc != TOPO_OK || per_sm < 1) return mma_fail(o, TOPO_E_CUDA, "cooperative occupancy query failed");
   // One CTA per SM at most: enough threads for the design sizes the spline
-  // lattices give, and a cheaper grid barrier than a fully populated grid.
-  const long long want = ((long long)o->n + kMmaBlock - 1) / kMmaBlock;
+  // lattices give, and a cheaper grid barrier than a fully populated grid.  A
+  // variable's Newton step has some 30 FP64 divisions, which the warps of an SM
+  // take one after another, so few variables are spread over small CTAs (n =
+  // 637: 4.0 ms an update on 3 CTAs of 256 threads, 2.7 on 10 of 64).
+  o->threads = 64;
+  while (o->threads < kMmaBlock && (long long)o->n > (long long)o->threads * sms) o->threads *= 2;
+  const long long want = ((long long)o->n + o->threads - 1) / o->threads;
   o->nblocks = (int)std::max(1LL, std::min<long long>(want, (long long)sms * std::min(per_sm, 1)));
   const size_t n = o->n, m1 = o->m + 1;
   const size_t total = 16 * n + 2 * m1 * n + 2 * (size_t)kMmaSlots * o->nblocks + 8 + 2 * n;
@@ -659,7 +674,7 @@ int topo_mma_update(topo_mma* o, const double* df_dev, const double* const* dg_d
     case 3: fn = (const void*)k_mma_update<3>; break;
     default: fn = (const void*)k_mma_update<4>; break;
   }
-  MCK(cudaLaunchCooperativeKernel(fn, dim3(o->nblocks), dim3(kMmaBlock), args, 0, o->stream));
+  MCK(cudaLaunchCooperativeKernel(fn, dim3(o->nblocks), dim3(o->threads), args, 0, o->stream));
   count_launch();
   double hs[5];
   MCK(cudaMemcpyAsync(hs, o->stats, sizeof(hs), cudaMemcpyDeviceToHost, o->stream));

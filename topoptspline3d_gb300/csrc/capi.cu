@@ -166,7 +166,7 @@ template <> struct P<double> {
   static double* U2(DevLevel& L) { return L.U2; }
   static double* F(DevLevel& L) { return L.F; }
   static double* R(DevLevel& L) { return L.R; }
-  static double* st(DevLevel& L) { return L.stencil; }
+  static double* st(DevLevel& L) { return L.stencilv ? L.stencilv : L.stencil; }
   static double* dinv(DevLevel& L) { return L.dinv; }
   static double* cd(DevLevel& L) { return L.cd; }
   static double* rhop(topo_handle* h) { return h->rhop; }
@@ -1241,6 +1241,7 @@ int topo_create(const topo_config* cfg, const uint8_t* eactive, topo_handle** ou
     if (l > 0) {
       A(dalloc(hp, &L.kel, 576 * ne)); A(dalloc(hp, &L.kel32, 576 * ne));
       A(dalloc(hp, &L.stencil, 243 * nv));
+      if (stencil_by_vertex(L.d)) A(dalloc(hp, &L.stencilv, 243 * nv));
       // FP32: room for the tiled layout (243 x 32 values per started group of 32 vertices)
       A(dalloc(hp, &L.stencil32, 243 * ((nv + 31) / 32 * 32)));
     }
@@ -1290,7 +1291,6 @@ int topo_create(const topo_config* cfg, const uint8_t* eactive, topo_handle** ou
       A(dalloc(hp, &h->A, (int64_t)h->ndense * h->ndense));
       A(dalloc(hp, &h->A32, (int64_t)h->ndense * h->ndense));
       A(dalloc(hp, &h->gjwork, 128 * (int64_t)h->ndense + 8 * 32 * 32));  // panels and diagonal blocks of the inversion
-      A(dalloc(hp, &h->coarse64tmp, 243 * dl.nv));
     }
     std::vector<double> T;
     galerkin_tables(h->Ke, h->lv[1].d.factor, T);
@@ -1686,7 +1686,8 @@ int topo_update_operators(topo_handle* h) {
       if (b32) launch_galerkin_dyadic_t<float>(h->stream, Fl.d, C.d, Fl.eactive, Fl.kel32, C.kel32);
       count_launch((b64 ? 1 : 0) + (b32 ? 1 : 0));
     }
-    if (b64) launch_assemble_stencil_t<double>(h->stream, C.d, C.eactive, C.vmask, C.kel, C.stencil);
+    if (b64) launch_assemble_stencil_t<double>(h->stream, C.d, C.eactive, C.vmask, C.kel, P<double>::st(C),
+                                                       C.stencilv ? C.stencil : nullptr);
     if (b32) launch_assemble_stencil_t<float>(h->stream, C.d, C.eactive, C.vmask, C.kel32, C.stencil32);
     count_launch((b64 ? 1 : 0) + (b32 ? 1 : 0));
     CKL();
@@ -1698,14 +1699,8 @@ int topo_update_operators(topo_handle* h) {
     h->coarse_age = 0;
     h->coarse_valid = true;
     DevLevel& Lc = h->lv.back();
-    const double* st = Lc.stencil;
-    if (!b64) {  // FP64 copy of the FP32 coarsest stencil
-      CK(cudaMemsetAsync(h->coarse64tmp, 0, sizeof(double) * 243 * Lc.d.nv, h->stream));
-      launch_f2d_add(h->stream, Lc.stencil32, h->coarse64tmp, 243 * Lc.d.nv);
-      count_launch();
-      st = h->coarse64tmp;
-    }
-    launch_dense_from_stencil(h->stream, Lc.d, st, h->A);
+    if (b64) launch_dense_from_stencil<double>(h->stream, Lc.d, P<double>::st(Lc), h->A);
+    else launch_dense_from_stencil<float>(h->stream, Lc.d, Lc.stencil32, h->A);
     count_launch();
     CKL();
     // FP32-only operators: the matrix comes from FP32 stencils; the updates
@@ -1800,7 +1795,7 @@ int topo_apply_level(topo_handle* h, int level, int precision) {
   const int64_t n3 = 3 * L.d.nv;
   if (precision == 0) {
     if (!h->ops64) return fail(h, TOPO_E_STATE, "FP64 operators not built (topo_set_operator_precision)");
-    launch_stencil_apply<double>(h->stream, L.d, L.stencil, L.U, nullptr, L.R, false, 1);
+    launch_stencil_apply<double>(h->stream, L.d, P<double>::st(L), L.U, nullptr, L.R, false, 1);
     count_launch();
   } else {
     if (!h->ops32) return fail(h, TOPO_E_STATE, "FP32 operators not built (topo_set_operator_precision)");

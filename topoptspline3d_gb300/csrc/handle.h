@@ -164,7 +164,6 @@ struct topo_handle {
   double* A = nullptr;
   float* A32 = nullptr;
   double* gjwork = nullptr;  // panels of the blocked Gauss-Jordan inversion
-  double* coarse64tmp = nullptr;  // FP64 copy of an FP32 coarsest stencil
   int* status = nullptr;
   // first coarse level: elements whose fine elements touch fixed DOFs
   int* gal_fixed = nullptr;

@@ -16,23 +16,31 @@ static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) 
 // Coarse levels below this vertex count run the warp-per-vertex stencil kernels.
 constexpr int64_t STENCIL_WARP_MAX_NV = 32768;
 
-// Where stencil coefficient q (neighbour k times 9 plus block entry, 0..242) of
-// vertex v lives: base(v) + q * stride().  [243][nv] for FP64 and for the small
-// levels; tiled for the FP32 levels the row kernels serve (vertex count at
-// least STENCIL_WARP_MAX_NV): the 243 x 32 coefficients of each group of 32
-// vertices lie together, so a warp of consecutive vertices reads one
-// contiguous block instead of 243 arrays.  A tiled array holds 243 x 32
-// values per started group of 32 vertices.
+// Where entry e (0..8) of vertex v's block for neighbour k (0..26) lives:
+// base(v) + k ks() + e es().
+//  form 0: [27][9][nv], FP64 levels of STENCIL_WARP_MAX_NV vertices and more
+//  form 1: the same in tiles, FP32 levels of that size, which the row kernels
+//    serve: the 243 x 32 coefficients of each group of 32 vertices lie together,
+//    so a warp of consecutive vertices reads one contiguous block instead of 243
+//    arrays (243 x 32 values per started group)
+//  form 2: [nv][9][27], the smaller levels, where a warp takes one vertex and
+//    lane k its neighbour k: nine reads of 27 consecutive values.  In form 0
+//    each of the 243 values was a sector of its own, eight times the bytes
+//    through L2 (FP32 Chebyshev step on 18,500 vertices 8.5 -> 6.7 us, eight
+//    right-hand sides on 4,200 12.2 -> 8.4 us).
 struct StIdx {
   int64_t nv;
-  bool tiled;
-  __device__ __forceinline__ int64_t base(int64_t v) const { return tiled ? (v >> 5) * (243 * 32) + (v & 31) : v; }
-  __device__ __forceinline__ int64_t stride() const { return tiled ? 32 : nv; }
+  int form;
+  __device__ __forceinline__ int64_t base(int64_t v) const {
+    return form == 1 ? (v >> 5) * (243 * 32) + (v & 31) : form == 2 ? v * 243 : v;
+  }
+  __device__ __forceinline__ int64_t ks() const { return form == 1 ? 9 * 32 : form == 2 ? 1 : 9 * nv; }
+  __device__ __forceinline__ int64_t es() const { return form == 1 ? 32 : form == 2 ? 27 : nv; }
 };
 
 template <typename T>
 StIdx st_idx(const LevelDims& d) {
-  return StIdx{d.nv, sizeof(T) == 4 && d.nv >= STENCIL_WARP_MAX_NV};
+  return StIdx{d.nv, d.nv < STENCIL_WARP_MAX_NV ? 2 : sizeof(T) == 4 ? 1 : 0};
 }
 
 // ---------------------------------------------------------------------------
@@ -43,7 +51,7 @@ __device__ __forceinline__ void stencil_row(const LevelDims& d, const T* __restr
                                             const T* __restrict__ u, int x, int y, int z, int64_t v,
                                             T o[3]) {
   o[0] = o[1] = o[2] = T(0);
-  const int64_t nv = d.nv, ss = si.stride();
+  const int64_t nv = d.nv, ss = si.es(), sk = si.ks();
   const T* sb = st + si.base(v);
 #pragma unroll
   for (int k = 0; k < 27; ++k) {
@@ -51,7 +59,7 @@ __device__ __forceinline__ void stencil_row(const LevelDims& d, const T* __restr
     if (nx < 0 || ny < 0 || nz < 0 || nx >= d.vx || ny >= d.vy || nz >= d.vz) continue;
     const int64_t n = nx + (int64_t)d.vx * (ny + (int64_t)d.vy * nz);
     const T u0 = u[n], u1 = u[nv + n], u2 = u[2 * nv + n];
-    const T* s = sb + (int64_t)(k * 9) * ss;
+    const T* s = sb + k * sk;
     o[0] += s[0] * u0 + s[ss] * u1 + s[2 * ss] * u2;
     o[1] += s[3 * ss] * u0 + s[4 * ss] * u1 + s[5 * ss] * u2;
     o[2] += s[6 * ss] * u0 + s[7 * ss] * u1 + s[8 * ss] * u2;
@@ -120,7 +128,7 @@ __device__ __forceinline__ void gs_load(const LevelDims& d, const T* __restrict_
   const int v = x + d.vx * (y + d.vy * z);
   if (!(vmask[v] & 8)) return;
   L.v = v;
-  const int64_t ss = si.stride(), nv = d.nv;
+  const int64_t ss = si.es(), sk = si.ks(), nv = d.nv;
   const T* sb = st + si.base(v);
   const int nz = z + part - 1;
   L.at = (x - 1) + d.vx * ((y - 1) + d.vy * nz);
@@ -129,12 +137,12 @@ __device__ __forceinline__ void gs_load(const LevelDims& d, const T* __restrict_
     const int nx = x + k % 3 - 1, ny = y + k / 3 - 1;
     const bool ok = nz >= 0 && nz < d.vz && nx >= 0 && ny >= 0 && nx < d.vx && ny < d.vy;
     L.ok |= ok ? 1u << k : 0u;
-    const T* s = sb + (int64_t)((9 * part + k) * 9 + 3 * row) * ss;
+    const T* s = sb + (9 * part + k) * sk + 3 * row * ss;
 #pragma unroll
     for (int j = 0; j < 3; ++j) L.c[3 * k + j] = ok ? s[j * ss] : T(0);
   }
 #pragma unroll
-  for (int j = 0; j < 3; ++j) L.S[j] = sb[(int64_t)(13 * 9 + 3 * row + j) * ss];
+  for (int j = 0; j < 3; ++j) L.S[j] = sb[13 * sk + (3 * row + j) * ss];
   L.rc = T(1) / (row == 0 ? L.S[0] : row == 1 ? L.S[1] : L.S[2]);
   L.f = f[row * nv + v];
 }
@@ -240,7 +248,7 @@ __global__ void k_stencil_gs(LevelDims d, const T* __restrict__ st, StIdx si, co
   T o[3], S[9], r[3];
   stencil_row<T>(d, st, si, u, x, y, z, v, o);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) S[k] = st[si.base(v) + (int64_t)(13 * 9 + k) * si.stride()];
+  for (int k = 0; k < 9; ++k) S[k] = st[si.base(v) + 13 * si.ks() + k * si.es()];
 #pragma unroll
   for (int c = 0; c < 3; ++c) r[c] = f[c * d.nv + v] - o[c];
   T du[3] = {T(0), T(0), T(0)};
@@ -272,7 +280,7 @@ __global__ void k_stencil_diag_inv(LevelDims d, const T* __restrict__ st, StIdx 
   if (v >= d.nv) return;
   T S[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) S[k] = st[si.base(v) + (int64_t)(13 * 9 + k) * si.stride()];
+  for (int k = 0; k < 9; ++k) S[k] = st[si.base(v) + 13 * si.ks() + k * si.es()];
   const T a = S[0], b = S[1], c = S[2], dd = S[4], e = S[5], f = S[8];
   const T A0 = dd * f - e * e, A1 = c * e - b * f, A2 = b * e - c * dd;
   const T det = a * A0 + b * A1 + c * A2;
@@ -293,14 +301,14 @@ template <typename T>
 __device__ __forceinline__ T stencil_row_i(const LevelDims& d, const T* __restrict__ st, StIdx si,
                                            const T* __restrict__ u, int x, int y, int z, int64_t v, int row) {
   T o = T(0);
-  const int64_t nv = d.nv, ss = si.stride();
-  const T* sb = st + si.base(v);
+  const int64_t nv = d.nv, ss = si.es(), sk = si.ks();
+  const T* sb = st + si.base(v) + 3 * row * ss;
 #pragma unroll
   for (int k = 0; k < 27; ++k) {
     const int nx = x + k % 3 - 1, ny = y + k / 3 % 3 - 1, nz = z + k / 9 - 1;
     if (nx < 0 || ny < 0 || nz < 0 || nx >= d.vx || ny >= d.vy || nz >= d.vz) continue;
     const int64_t n = nx + (int64_t)d.vx * (ny + (int64_t)d.vy * nz);
-    const T* s = sb + (int64_t)(k * 9 + 3 * row) * ss;
+    const T* s = sb + k * sk;
     o += s[0] * u[n] + s[ss] * u[nv + n] + s[2 * ss] * u[2 * nv + n];
   }
   return o;
@@ -370,19 +378,18 @@ constexpr int WV = 8;  // vertices (warps) per 256-thread CTA
 template <typename T>
 __device__ __forceinline__ void stencil_warp_rows(const LevelDims& d, const T* __restrict__ st,
                                                   const T* __restrict__ u, int64_t v, int lane, T o[3]) {
-  const int x = (int)(v % d.vx);
-  const int64_t t = v / d.vx;
-  const int y = (int)(t % d.vy), z = (int)(t / d.vy);
+  const int iv = (int)v, t = iv / d.vx, x = iv - t * d.vx, z = t / d.vy, y = t - z * d.vy;
   o[0] = o[1] = o[2] = T(0);
   if (lane < 27) {
-    const int nx = x + lane % 3 - 1, ny = y + lane / 3 % 3 - 1, nz = z + lane / 9 - 1;
+    const int kz = lane / 9, ky = (lane - 9 * kz) / 3, kx = lane - 9 * kz - 3 * ky;
+    const int nx = x + kx - 1, ny = y + ky - 1, nz = z + kz - 1;
     if (nx >= 0 && ny >= 0 && nz >= 0 && nx < d.vx && ny < d.vy && nz < d.vz) {
-      const int64_t n = nx + (int64_t)d.vx * (ny + (int64_t)d.vy * nz), nv = d.nv;
+      const int n = nx + d.vx * (ny + d.vy * nz), nv = (int)d.nv;
       const T u0 = u[n], u1 = u[nv + n], u2 = u[2 * nv + n];
-      const T* sk = st + (int64_t)(lane * 9) * nv + v;
+      const T* sk = st + (int64_t)iv * 243 + lane;  // form 2 (StIdx)
 #pragma unroll
       for (int row = 0; row < 3; ++row)
-        o[row] = sk[(3 * row) * nv] * u0 + sk[(3 * row + 1) * nv] * u1 + sk[(3 * row + 2) * nv] * u2;
+        o[row] = sk[27 * (3 * row)] * u0 + sk[27 * (3 * row + 1)] * u1 + sk[27 * (3 * row + 2)] * u2;
     }
   }
 #pragma unroll
@@ -996,15 +1003,17 @@ __global__ void __launch_bounds__(576) k_galerkin_dyadic(LevelDims fd, LevelDims
   kel_c[ce * 576 + ent] = acc;
 }
 
-// Stencil assembly from element matrices: thread per (neighbour d, vertex v).
+// Stencil assembly from element matrices: thread per (neighbour d, vertex v),
+// consecutive threads along what the layout stores together.  planes: also the
+// [243][nv] form that callers read (FP64, null: none).
 template <typename T>
 __global__ void k_assemble_stencil(LevelDims d, const uint8_t* __restrict__ eactive,
                                    const uint8_t* __restrict__ vmask, const T* __restrict__ kel,
-                                   T* __restrict__ st, StIdx si) {
+                                   T* __restrict__ st, StIdx si, T* __restrict__ planes) {
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= 27 * d.nv) return;
-  const int k = (int)(gid / d.nv);
-  const int64_t v = gid % d.nv;
+  const int k = (int)(si.form == 2 ? gid % 27 : gid / d.nv);
+  const int64_t v = si.form == 2 ? gid / 27 : gid % d.nv;
   const int x = (int)(v % d.vx);
   const int64_t t = v / d.vx;
   const int y = (int)(t % d.vy), z = (int)(t / d.vy);
@@ -1040,24 +1049,26 @@ __global__ void k_assemble_stencil(LevelDims d, const uint8_t* __restrict__ eact
     blk[0] = T(1); blk[4] = T(1); blk[8] = T(1);
   }
 #pragma unroll
-  for (int q = 0; q < 9; ++q) st[si.base(v) + (int64_t)(k * 9 + q) * si.stride()] = blk[q];
+  for (int q = 0; q < 9; ++q) {
+    st[si.base(v) + k * si.ks() + q * si.es()] = blk[q];
+    if (planes) planes[(int64_t)(k * 9 + q) * d.nv + v] = blk[q];
+  }
 }
 
-__global__ void k_dense_from_stencil(LevelDims d, const double* __restrict__ st,
-                                     double* __restrict__ A) {
+template <typename T>
+__global__ void k_dense_from_stencil(LevelDims d, const T* __restrict__ st, StIdx si, double* __restrict__ A) {
   const int64_t n = 3 * d.nv;
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= 243 * d.nv) return;
-  const int q = (int)(gid / d.nv);  // k*9 + 3i + j
-  const int64_t v = gid % d.nv;
-  const int k = q / 9, i = (q % 9) / 3, j = q % 3;
+  const int64_t v = gid / 243;
+  const int q = (int)(gid - v * 243), e = q / 27, k = q - 27 * e, i = e / 3, j = e - 3 * i;
   const int x = (int)(v % d.vx);
   const int64_t t = v / d.vx;
   const int y = (int)(t % d.vy), z = (int)(t / d.vy);
   const int nx = x + k % 3 - 1, ny = y + k / 3 % 3 - 1, nz = z + k / 9 - 1;
   if (nx < 0 || ny < 0 || nz < 0 || nx >= d.vx || ny >= d.vy || nz >= d.vz) return;
   const int64_t nb = nx + (int64_t)d.vx * (ny + (int64_t)d.vy * nz);
-  A[(3 * v + i) * n + 3 * nb + j] = st[(int64_t)q * d.nv + v];
+  A[(3 * v + i) * n + 3 * nb + j] = (double)st[si.base(v) + k * si.ks() + e * si.es()];
 }
 
 __global__ void k_symmetrize(int n, double* A) {
@@ -1660,14 +1671,17 @@ void launch_galerkin_dyadic_t(cudaStream_t s, const LevelDims& fd, const LevelDi
 
 template <typename T>
 void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                               const uint8_t* vmask, const T* kel, T* st) {
-  k_assemble_stencil<T><<<nblk(27 * d.nv, 256), 256, 0, s>>>(d, eactive, vmask, kel, st, st_idx<T>(d));
+                               const uint8_t* vmask, const T* kel, T* st, T* planes) {
+  k_assemble_stencil<T><<<nblk(27 * d.nv, 256), 256, 0, s>>>(d, eactive, vmask, kel, st, st_idx<T>(d), planes);
 }
 
-void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const double* st, double* A) {
+bool stencil_by_vertex(const LevelDims& d) { return d.nv < STENCIL_WARP_MAX_NV; }
+
+template <typename T>
+void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const T* st, double* A) {
   const int64_t n = 3 * d.nv;
   cudaMemsetAsync(A, 0, sizeof(double) * n * n, s);
-  k_dense_from_stencil<<<nblk(243 * d.nv, 256), 256, 0, s>>>(d, st, A);
+  k_dense_from_stencil<T><<<nblk(243 * d.nv, 256), 256, 0, s>>>(d, st, st_idx<T>(d), A);
 }
 
 // A: the coarsest matrix (its symmetric part is inverted in place), A32: the
@@ -1743,9 +1757,11 @@ template void launch_galerkin_dyadic_t<double>(cudaStream_t, const LevelDims&, c
 template void launch_galerkin_dyadic_t<float>(cudaStream_t, const LevelDims&, const LevelDims&,
                                               const uint8_t*, const float*, float*);
 template void launch_assemble_stencil_t<double>(cudaStream_t, const LevelDims&, const uint8_t*,
-                                                const uint8_t*, const double*, double*);
+                                                const uint8_t*, const double*, double*, double*);
 template void launch_assemble_stencil_t<float>(cudaStream_t, const LevelDims&, const uint8_t*,
-                                               const uint8_t*, const float*, float*);
+                                               const uint8_t*, const float*, float*, float*);
+template void launch_dense_from_stencil<double>(cudaStream_t, const LevelDims&, const double*, double*);
+template void launch_dense_from_stencil<float>(cudaStream_t, const LevelDims&, const float*, double*);
 template void launch_dense_gemv<double>(cudaStream_t, int, const double*, const double*, double*,
                                         int64_t, int);
 template void launch_dense_gemv<float>(cudaStream_t, int, const float*, const float*, float*, int64_t, int);

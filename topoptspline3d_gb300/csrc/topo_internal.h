@@ -123,8 +123,9 @@ struct DevLevel {
   float *U32 = nullptr, *F32 = nullptr, *R32 = nullptr;  // FP32 [3nv]
   double* kel = nullptr;        // coarse: FP64 element matrices [ne][576]
   float* kel32 = nullptr;       // coarse: FP32 element matrices [ne][576]
-  double* stencil = nullptr;    // coarse: FP64 [243][nv]
-  float* stencil32 = nullptr;   // coarse: FP32 [243][nv], tiled on levels of 32,768 vertices or more (StIdx)
+  double* stencil = nullptr;    // coarse: FP64 [243][nv], as callers read it
+  double* stencilv = nullptr;   // coarse: the kernels' copy on small levels, by vertex (StIdx form 2; else null)
+  float* stencil32 = nullptr;   // coarse: FP32, by vertex on small levels, tiled on the others (StIdx)
   double* dinv = nullptr;       // FP64 inverse diagonal blocks [9][nv] (Chebyshev)
   float* dinv32 = nullptr;      // FP32 inverse diagonal blocks [9][nv]; level 0: packed symmetric (float4 d00 d01 d02 d11 [nv], float2 d12 d22 [nv])
   double* cd = nullptr;         // FP64 Chebyshev direction [3nv]
@@ -241,8 +242,11 @@ void launch_galerkin_dyadic_t(cudaStream_t s, const LevelDims& fd, const LevelDi
                               const uint8_t* eactive_f, const T* kel_f, T* kel_c);
 template <typename T>
 void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                               const uint8_t* vmask, const T* kel, T* st);
-void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const double* st, double* A);
+                               const uint8_t* vmask, const T* kel, T* st, T* planes = nullptr);
+// whether a level's stencils are stored by vertex
+bool stencil_by_vertex(const LevelDims& d);
+template <typename T>
+void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const T* st, double* A);
 // Inverts the symmetric part of A in place and writes its FP32 copy to A32.
 // work: published panels (128 n + 8192 doubles); df_update: in double-float
 // arithmetic (matrices from FP32 stencils).

@@ -1917,7 +1917,6 @@ static int tc_wait_status(topo_handle* h) {
 
 static int solve_impl(topo_handle* h, const topo_solve_opts* o, topo_solve_stats* stats) {
   RET(check_ready(h, true));
-  h->energy_ready = false;
   if (!o || o->rtol <= 0 || o->max_iter < 0 || o->pre < 0 || o->post < 0) return TOPO_E_BAD_INPUT;
   RefOps ref_ops(h, o->mode == TOPO_SOLVE_VCYCLE);
   DevLevel& L0 = h->lv[0];
@@ -2183,17 +2182,7 @@ static int solve_impl(topo_handle* h, const topo_solve_opts* o, topo_solve_stats
     return fail(h, TOPO_E_BAD_INPUT, "unknown solve mode %d", o->mode);
   }
   if (o->mode != TOPO_SOLVE_VCYCLE && fn != 0.0) {
-    // true FP64 residual of the final iterate (with the element energies of
-    // the sensitivity when a design iteration asks for them)
-    if (h->want_energy && h->fine_df && h->nb == 1) {
-      EventPair* ev = prof_begin(h, P<double>::fam_apply);
-      launch_fine_apply_df(h->stream, L0.d, h->rhop, L0.vmask, L0.U, L0.F, L0.R, true, 1, h->tz64, h->sens);
-      prof_end(h, ev);
-      count_launch();
-      h->energy_ready = true;
-    } else {
-      level_residual<double>(h, 0);
-    }
+    level_residual<double>(h, 0);  // true FP64 residual of the final iterate
     launch_dot<double>(h->stream, L0.R, L0.R, n3, h->partial, h->sc + S_RR, h->ctr);
     count_launch();
     if (cap) {
@@ -2245,16 +2234,22 @@ int topo_volume(topo_handle* h, int refden, double* v) {
   return TOPO_OK;
 }
 
-int topo_sensitivity(topo_handle* h) {
-  DEVICE_SCOPE(h);
-  if (!h) return TOPO_E_BAD_INPUT;
+// Element sensitivities; from_rhop: with rho^(p-1) as rhop / rho (a design
+// iteration, where rhop is the operator's)
+static int sensitivity(topo_handle* h, bool from_rhop) {
   const DevLevel& L = h->lv[0];
-  launch_sensitivity(h->stream, L.d, L.eactive, h->rho, L.U, h->cfg.power_penalty, h->lam, h->mu,
-                     h->cfg.h, h->sens);
+  launch_sensitivity(h->stream, L.d, L.eactive, h->rho, from_rhop ? h->rhop : nullptr, L.U, h->cfg.power_penalty,
+                     h->lam, h->mu, h->cfg.h, h->sens);
   count_launch();
   if (h->ref_fp32) { launch_round_f32(h->stream, L.d.ne, h->sens); count_launch(); }
   CKL();
   return TOPO_OK;
+}
+
+int topo_sensitivity(topo_handle* h) {
+  DEVICE_SCOPE(h);
+  if (!h) return TOPO_E_BAD_INPUT;
+  return sensitivity(h, false);
 }
 
 }  // extern "C"
@@ -3379,19 +3374,10 @@ int iteration_graph_launch(topo_handle* h, const topo_iter_opts* o) {
       h->iter_waited = false;
       h->d_outer_body = h->d_inner_body = h->d_oc_body = h->d_if_body = 0;
       topo_solve_stats ss{};
-      h->want_energy = true;
-      rc = topo_solve(h, &so, &ss);
-      h->want_energy = false;
+      rc = h->fine_df ? topo_solve(h, &so, &ss) : TOPO_E_STATE;  // (native FP64: the host sequence)
       double c = 0;
       if (rc == TOPO_OK) rc = topo_compliance(h, &c);
-      if (rc == TOPO_OK && h->energy_ready) {
-        launch_sensitivity_from_energy(h->stream, L0.d.ne, L0.eactive, h->rho, h->cfg.power_penalty, h->sens);
-        count_launch();
-        if (h->ref_fp32) { launch_round_f32(h->stream, L0.d.ne, h->sens); count_launch(); }
-        h->energy_ready = false;
-      } else if (rc == TOPO_OK) {
-        rc = TOPO_E_STATE;
-      }
+      if (rc == TOPO_OK) rc = sensitivity(h, true);
       if (rc == TOPO_OK) rc = topo_filter(h, o->filter_radius > 0 ? o->filter_radius : 2.0);
       if (rc == TOPO_OK) rc = topo_spline_adjoint(h);
       topo_oc_stats ocs{};
@@ -3476,21 +3462,11 @@ int topo_design_iteration(topo_handle* h, const topo_iter_opts* o, topo_iter_sta
   const int urc = topo_update_operators(h);
   h->defer_coarse = false;
   RET(urc);
-  h->want_energy = true;
   int rc = topo_solve(h, &o->solve, &st.solve);
-  h->want_energy = false;
   if (rc != TOPO_OK && rc != TOPO_E_NOT_CONVERGED) return rc;
   RET(topo_compliance(h, &st.compliance));
   if (!std::isfinite(st.compliance)) return fail(h, TOPO_E_NONFINITE, "compliance is not finite");
-  if (h->energy_ready) {  // u is the solve's final iterate, rho unchanged since
-    const DevLevel& L = h->lv[0];
-    launch_sensitivity_from_energy(h->stream, L.d.ne, L.eactive, h->rho, h->cfg.power_penalty, h->sens);
-    count_launch();
-    if (h->ref_fp32) { launch_round_f32(h->stream, L.d.ne, h->sens); count_launch(); }
-    h->energy_ready = false;
-  } else {
-    RET(topo_sensitivity(h));
-  }
+  RET(sensitivity(h, o->solve.mode != TOPO_SOLVE_VCYCLE && h->fine_df));
   RET(topo_filter(h, o->filter_radius > 0 ? o->filter_radius : 2.0));
   RET(topo_spline_adjoint(h));
   topo_oc_stats oc{};

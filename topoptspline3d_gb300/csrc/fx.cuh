@@ -77,6 +77,16 @@ __host__ __device__ __forceinline__ double fx_to(int64_t y, int F) {
   return fx_double((b & 0x800fffffffffffffull) | ((uint64_t)e << 52));
 }
 
+// v 2^k (below the normal range: 0)
+__host__ __device__ __forceinline__ double fx_scale(double v, int k) {
+  const uint64_t b = fx_bits(v);
+  const int e0 = (int)(b >> 52) & 0x7ff, e = e0 + k;
+  if (e0 == 0x7ff) return v;
+  if (e0 == 0 || e <= 0) return 0.0;
+  if (e >= 0x7ff) return fx_double((b & 0x8000000000000000ull) | 0x7ff0000000000000ull);
+  return fx_double((b & 0x800fffffffffffffull) | ((uint64_t)e << 52));
+}
+
 // p in units of 2^(x - 1081): below 2^59 for exponents up to x
 __host__ __device__ __forceinline__ int64_t fx_factor(double p, int x) {
   const uint64_t b = fx_bits(p);
@@ -103,15 +113,9 @@ __host__ __device__ __forceinline__ int fx_clz(unsigned v) {
 }
 
 // In: v[3][8] nodal displacements, component i in units of 2^(ei - 1079),
-// |v| <= 2^57.  Out: nodal forces, and their exponent is returned.  The modes
-// and their coefficients are modal_element's (k_fine.cu).
-__host__ __device__ __forceinline__ int fx_element(int64_t v[3][8], int e0, int e1, int e2, double pe,
-                                                   const FxConst& k) {
-  const double pE = pe * k.e, pF = pe * k.f, pG = pe * k.g;
-  const int xe = (int)(fx_bits(pE) >> 52) & 0x7ff, xf = (int)(fx_bits(pF) >> 52) & 0x7ff,
-            xg = (int)(fx_bits(pG) >> 52) & 0x7ff;
-  const int x = xe > xf ? (xe > xg ? xe : xg) : (xf > xg ? xf : xg);
-  const int64_t E = fx_factor(pE, x), F = fx_factor(pF, x), G = fx_factor(pG, x);
+// |v| <= 2^57.  Out: modes 1 to 7 of each component, in units of 2^(X - 1079)
+// with the largest just below 2^60; X is returned (FX_ZERO: all zero).
+__host__ __device__ __forceinline__ int fx_modes(int64_t v[3][8], int e0, int e1, int e2) {
   int sh[3], X[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -138,13 +142,26 @@ __host__ __device__ __forceinline__ int fx_element(int64_t v[3][8], int e0, int 
     X[i] = lz < 64 ? (i == 0 ? e0 : i == 1 ? e1 : e2) - sh[i] : FX_ZERO;
   }
   const int XX = X[0] > X[1] ? (X[0] > X[2] ? X[0] : X[2]) : (X[1] > X[2] ? X[1] : X[2]);
-  int64_t(*c)[8] = v;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const int r = XX - X[i] < 63 ? XX - X[i] : 63;
 #pragma unroll
-    for (int m = 1; m < 8; ++m) c[i][m] = (int64_t)((uint64_t)c[i][m] << sh[i]) >> r;
+    for (int m = 1; m < 8; ++m) v[i][m] = (int64_t)((uint64_t)v[i][m] << sh[i]) >> r;
   }
+  return XX;
+}
+
+// In: v as for fx_modes.  Out: nodal forces, and their exponent is returned.
+// The modes and their coefficients are modal_element's (k_fine.cu).
+__host__ __device__ __forceinline__ int fx_element(int64_t v[3][8], int e0, int e1, int e2, double pe,
+                                                   const FxConst& k) {
+  const double pE = pe * k.e, pF = pe * k.f, pG = pe * k.g;
+  const int xe = (int)(fx_bits(pE) >> 52) & 0x7ff, xf = (int)(fx_bits(pF) >> 52) & 0x7ff,
+            xg = (int)(fx_bits(pG) >> 52) & 0x7ff;
+  const int x = xe > xf ? (xe > xg ? xe : xg) : (xf > xg ? xf : xg);
+  const int64_t E = fx_factor(pE, x), F = fx_factor(pF, x), G = fx_factor(pG, x);
+  const int XX = fx_modes(v, e0, e1, e2);
+  int64_t(*c)[8] = v;
   // constant part of the gradient (three times the coefficients of the others)
   const int64_t t = fx_mul(c[0][1] + c[1][2] + c[2][4], E);
   const int64_t sxy = 3 * fx_mul(c[0][2] + c[1][1], F), sxz = 3 * fx_mul(c[0][4] + c[2][1], F),

@@ -194,9 +194,6 @@ struct topo_handle {
   double* hsc = nullptr;   // pinned host mirror
   int64_t active_elements = 0, gs_padded_elements = 0;
   bool bc_set = false, ops_ready = false;
-  // design iteration: the solve's final residual also writes element energies
-  // into sens (want_energy), and says so (energy_ready)
-  bool want_energy = false, energy_ready = false;
   int op_precision = 3;    // bit0 FP64 operators, bit1 FP32 operators
   bool ref_fp32 = false;   // reference precision: rho, coefficients, sensitivities kept in FP32, rho^p by powf
   bool ops64 = false, ops32 = false;

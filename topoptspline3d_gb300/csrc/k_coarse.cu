@@ -447,6 +447,61 @@ __global__ void __launch_bounds__(32 * WV) k_stencil_cheb_warp(LevelDims d, cons
   }
 }
 
+// The FP64 step on the small levels, nine lanes a vertex as in gs_load: the warp
+// form above spends a warp's FP64 issue (16 clocks) on every one of its 15
+// shuffle additions and leaves a sixth of its lanes idle; here three vertices
+// share a warp and a row is finished by two additions (9,537 and 1,377
+// vertices, mean: 16.0 -> 11.2 us).
+__global__ void __launch_bounds__(32 * GS_WARPS) k_stencil_cheb9(LevelDims d, const double* __restrict__ st, StIdx si,
+                                                                 const double* __restrict__ u,
+                                                                 const double* __restrict__ f,
+                                                                 double* __restrict__ uout,
+                                                                 const double* __restrict__ dinv,
+                                                                 double* __restrict__ dv,
+                                                                 const double* __restrict__ coef, bool first) {
+  const int64_t bo = (int64_t)blockIdx.y * 3 * d.nv;  // right-hand side of the batch
+  u += bo;
+  f += bo;
+  uout += bo;
+  dv += bo;
+  const int lane = threadIdx.x & 31, g = lane / 9, j9 = lane - 9 * g, row = j9 / 3, part = j9 - 3 * row;
+  const int nv = (int)d.nv, v = (blockIdx.x * GS_WARPS + (threadIdx.x >> 5)) * GS_PER_WARP + g;
+  const bool ok = g < GS_PER_WARP && v < nv;
+  double a[3] = {0.0, 0.0, 0.0}, fr = 0.0, un = 0.0, dn = 0.0, di[3] = {0.0, 0.0, 0.0};
+  const int i = row * nv + v;
+  if (ok) {
+    fr = f[i];
+    un = u[i];
+    dn = first ? 0.0 : dv[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) di[c] = dinv[(3 * row + c) * (int64_t)nv + v];
+    const int t = v / d.vx, x = v - t * d.vx, z = t / d.vy, y = t - z * d.vy, nz = z + part - 1;
+    const int64_t es = si.es(), ks = si.ks();
+    const double* sb = st + si.base(v) + 3 * row * es + 9 * part * ks;
+    if (nz >= 0 && nz < d.vz) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const int nx = x + k % 3 - 1, ny = y + k / 3 - 1;
+        if (nx < 0 || ny < 0 || nx >= d.vx || ny >= d.vy) continue;
+        const int n = nx + d.vx * (ny + d.vy * nz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] += sb[k * ks + c * es] * u[c * nv + n];
+      }
+    }
+  }
+  const double s = (a[0] + a[1]) + a[2];
+  const int b9 = lane - j9, b3 = lane - part;
+  const double r = fr - ((__shfl_sync(0xffffffffu, s, b3 & 31) + __shfl_sync(0xffffffffu, s, (b3 + 1) & 31)) +
+                         __shfl_sync(0xffffffffu, s, (b3 + 2) & 31));
+  const double r0 = __shfl_sync(0xffffffffu, r, b9 & 31), r1 = __shfl_sync(0xffffffffu, r, (b9 + 3) & 31),
+               r2 = __shfl_sync(0xffffffffu, r, (b9 + 6) & 31);
+  if (!ok || part) return;
+  const double z = di[0] * r0 + di[1] * r1 + di[2] * r2, c_old = __ldg(coef), c_new = __ldg(coef + 1);
+  dn = first ? c_new * z : c_old * dn + c_new * z;
+  dv[i] = dn;
+  uout[i] = un + dn;
+}
+
 // Levels with fewer vertices than this use the warp-per-vertex kernels.
 
 template <typename T>
@@ -461,6 +516,13 @@ void launch_stencil_apply(cudaStream_t s, const LevelDims& d, const T* st, const
 template <typename T>
 void launch_stencil_cheb(cudaStream_t s, const LevelDims& d, const T* st, const T* u, const T* f, T* uout,
                          const T* dinv, T* dvec, const double* coef, bool first, int nb) {
+  if constexpr (sizeof(T) == 8) {
+    if (d.nv < STENCIL_WARP_MAX_NV) {
+      k_stencil_cheb9<<<dim3(nblk(d.nv, GS_PER_CTA), nb), 32 * GS_WARPS, 0, s>>>(d, st, st_idx<T>(d), u, f, uout, dinv,
+                                                                                dvec, coef, first);
+      return;
+    }
+  }
   if (d.nv < STENCIL_WARP_MAX_NV)
     k_stencil_cheb_warp<T><<<dim3(nblk(d.nv, WV), nb), 32 * WV, 0, s>>>(d, st, u, f, uout, dinv, dvec, coef, first);
   else

@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "df.cuh"
+#include "fx.cuh"
 #include "topo_internal.h"
 
 namespace topo {
@@ -438,105 +439,84 @@ void launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eact
 }
 
 // Element sensitivity g_e = -p rho^(p-1) u_e^T Ke u_e (optimization/optimization.cu:96-159),
-// with u_e^T Ke u_e evaluated in the sum-factorised modal form: Walsh-Hadamard
-// coefficients of the nodal values, the displacement gradient split over the
-// orthogonal functions {1, X, Y, Z, YZ, XZ, XY} of the reference cube, and the
-// isotropic energy of each part weighted by the function's L2 norm.  The
-// energy is formed in double-float arithmetic (about 1e-14 relative, on the
-// FP32 pipe); only the final scaling by -p rho^(p-1) (h/2)^3 runs in FP64.
-template <typename T>
-__device__ __forceinline__ T cst(double v);
-template <>
-__device__ __forceinline__ double cst<double>(double v) { return v; }
-template <>
-__device__ __forceinline__ df cst<df>(double v) { return df_from(v); }
-__device__ __forceinline__ double to_double(double v) { return v; }
-__device__ __forceinline__ double to_double(df v) { return df_to(v); }
+// with u_e^T Ke u_e in the modal form of the fine operator: the transforms of
+// the nodal values are exact, on 64-bit integers (fx.cuh), and the modes enter
+// the isotropic energy as double-float numbers on the FP32 pipe (48 bits of the
+// element's largest mode).  rhop: take rho^(p-1) as rhop / rho (a design
+// iteration, whose operator was built from rhop), else from rho.
+// Bound by instructions, about 1,700 an element.  The double-float form spent
+// them on its transforms and on FP64 conversions, three FP64 operations a nodal
+// value (191x95x93: 413 us, here 99).
+struct SensConst {
+  float2 e, f, g;  // FxConst as (hi, lo) floats
+};
 
-template <typename T>
-__device__ __forceinline__ void hadamard8(T v[8]) {
-#pragma unroll
-  for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (!(i & h)) {
-        const T a = v[i], b = v[i | h];
-        v[i] = a + b;
-        v[i | h] = b - a;
-      }
+// a mode in units of 2^-60
+__device__ __forceinline__ df mode_df(int64_t c) {
+  c += 1 << 13;
+  const float hi = __int2float_rn((int)(c >> 38)), lo = __int2float_rn((int)((c >> 14) & 0xffffff));
+  return df_fast2sum(hi * 0x1p-22f, lo * 0x1p-46f);
 }
+__device__ __forceinline__ void add_sq(df& s, df v) { s += v * v; }
 
-// 0.5 lam tr(G)^2 + mu |sym G|^2 with lam2 = lam / 2
-template <typename T>
-__device__ __forceinline__ T energy_part(const T G[3][3], T lam2, T mu) {
-  const T half = cst<T>(0.5), two = cst<T>(2.0);
-  const T tr = G[0][0] + G[1][1] + G[2][2];
-  T ee = G[0][0] * G[0][0] + G[1][1] * G[1][1] + G[2][2] * G[2][2];
-  const T e01 = half * (G[0][1] + G[1][0]), e02 = half * (G[0][2] + G[2][0]), e12 = half * (G[1][2] + G[2][1]);
-  ee += two * (e01 * e01 + e02 * e02 + e12 * e12);
-  return lam2 * tr * tr + mu * ee;
-}
-
-template <typename T>
-__global__ void k_sensitivity(LevelDims d, const uint8_t* __restrict__ eactive,
-                              const double* __restrict__ rho, const double* __restrict__ u,
-                              double penal, double lam, double mu, double h, double* __restrict__ sens) {
+__global__ void __launch_bounds__(128) k_sensitivity(LevelDims d, const uint8_t* __restrict__ eactive,
+                                                     const double* __restrict__ rho, const double* __restrict__ rhop,
+                                                     const double* __restrict__ u, double penal, SensConst k,
+                                                     double* __restrict__ sens) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= d.ne) return;
   if (!eactive[e]) { sens[e] = 0.0; return; }
   const int x = (int)(e % d.ex);
   const int64_t t = e / d.ex;
   const int y = (int)(t % d.ey), z = (int)(t / d.ey);
-  // c[i][S]: modal coefficient of component i for mode S (bit0 x, bit1 y, bit2 z),
-  // with sign convention H[a][S] = prod_{k in S} (2 a_k - 1); scaled by 2/h * 1/8.
-  T c[3][8];
+  int64_t c[3][8];
+  int E[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
+    int ei[8];
+    E[i] = 0;
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
       const int64_t v = (x + (a & 1)) + (int64_t)d.vx * ((y + ((a >> 1) & 1)) + (int64_t)d.vy * (z + (a >> 2)));
-      c[i][a] = cst<T>(u[i * d.nv + v]);
+      c[i][a] = fx_split(u[i * d.nv + v], ei[a]);
+      E[i] = max(E[i], ei[a]);
     }
-    hadamard8<T>(c[i]);
+#pragma unroll
+    for (int a = 0; a < 8; ++a) c[i][a] = fx_down(c[i][a], E[i] - ei[a]);
   }
-  const T sc = cst<T>(2.0 / h / 8.0), lam2 = cst<T>(0.5 * lam), muT = cst<T>(mu), zero = cst<T>(0.0);
-  T tot = zero;
-#pragma unroll
-  for (int f = 0; f < 7; ++f) {
-    T G[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        G[i][j] = ((f >> j) & 1) ? zero : sc * c[i][f | (1 << j)];
-    const int nbits = (f & 1) + ((f >> 1) & 1) + ((f >> 2) & 1);
-    const T nf = cst<T>(nbits == 0 ? 8.0 : (nbits == 1 ? 8.0 / 3.0 : 8.0 / 9.0));
-    tot += nf * energy_part<T>(G, lam2, muT);
-  }
-  const double hh = 0.5 * h;
-  const double q = 2.0 * hh * hh * hh * to_double(tot);  // u_e^T Ke u_e
-  sens[e] = -penal * simp_pow(rho[e], penal - 1.0) * q;
+  const bool bad = max(max(E[0], E[1]), E[2]) >= 0x7ff;
+  const int X = fx_modes(c, E[0], E[1], E[2]);
+  df se(0), sf(0), sg(0), s(0);
+  // constant part of the gradient (weight 3)
+  add_sq(se, mode_df(c[0][1] + c[1][2] + c[2][4]));
+  add_sq(s, mode_df(c[0][1])); add_sq(s, mode_df(c[1][2])); add_sq(s, mode_df(c[2][4]));
+  sf += s + s;
+  add_sq(sf, mode_df(c[0][2] + c[1][1])); add_sq(sf, mode_df(c[0][4] + c[2][1])); add_sq(sf, mode_df(c[1][4] + c[2][2]));
+  se = se + se + se;
+  // X, Y and Z parts
+  add_sq(se, mode_df(c[1][3] + c[2][5])); add_sq(se, mode_df(c[0][3] + c[2][6])); add_sq(se, mode_df(c[0][5] + c[1][6]));
+  add_sq(sf, mode_df(c[0][3])); add_sq(sf, mode_df(c[1][3])); add_sq(sf, mode_df(c[0][5]));
+  add_sq(sf, mode_df(c[2][5])); add_sq(sf, mode_df(c[1][6])); add_sq(sf, mode_df(c[2][6]));
+  sf = sf + sf + sf;
+  add_sq(sf, mode_df(c[1][5] + c[2][3])); add_sq(sf, mode_df(c[0][6] + c[2][3])); add_sq(sf, mode_df(c[0][6] + c[1][5]));
+  add_sq(sg, mode_df(c[0][7])); add_sq(sg, mode_df(c[1][7])); add_sq(sg, mode_df(c[2][7]));
+  const df w = se * df(k.e.x, k.e.y) + sf * df(k.f.x, k.f.y) + sg * df(k.g.x, k.g.y);
+  double q = fx_scale(df_to(w), 2 * (X - 1019));  // u_e^T Ke u_e
+  if (bad) q = __longlong_as_double(0x7ff8000000000000ll);
+  const double r = rho[e];
+  if (rhop) sens[e] = r > 0.0 ? -penal * (rhop[e] * q) / r : 0.0;
+  else sens[e] = -penal * simp_pow(r, penal - 1.0) * q;
 }
 
 void launch_sensitivity(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                        const double* rho, const double* u, double penal, double lam, double mu,
+                        const double* rho, const double* rhop, const double* u, double penal, double lam, double mu,
                         double h, double* sens) {
-  k_sensitivity<df><<<nblk(d.ne, 128), 128, 0, s>>>(d, eactive, rho, u, penal, lam, mu, h, sens);
-}
-
-// The same sensitivity from element energies E = u_e . (rho^p Ke u_e) that the
-// solve's final residual kernel wrote: -p rho^(p-1) u_e^T Ke u_e = -p E / rho.
-__global__ void k_sensitivity_from_energy(int64_t ne, const uint8_t* __restrict__ eactive,
-                                          const double* __restrict__ rho, double penal, double* __restrict__ sens) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const double r = rho[e];
-  sens[e] = (eactive[e] && r > 0.0) ? -penal * sens[e] / r : 0.0;
-}
-
-void launch_sensitivity_from_energy(cudaStream_t s, int64_t ne, const uint8_t* eactive, const double* rho,
-                                    double penal, double* sens) {
-  k_sensitivity_from_energy<<<nblk(ne, 256), 256, 0, s>>>(ne, eactive, rho, penal, sens);
+  auto split = [](double v) {
+    const float hi = (float)v;
+    return make_float2(hi, (float)(v - (double)hi));
+  };
+  const SensConst k{split(lam * h / 48.0), split(mu * h / 48.0), split((lam + 4.0 * mu) * h / 144.0)};
+  k_sensitivity<<<nblk(d.ne, 128), 128, 0, s>>>(d, eactive, rho, rhop, u, penal, k, sens);
 }
 
 // Sensitivity filter (grid/Grid.cu:4130-4229): normalised average over the ball

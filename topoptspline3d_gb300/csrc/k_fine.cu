@@ -195,10 +195,8 @@ __device__ __forceinline__ void wht3_bwd<df>(df g[3][8]) {
 }
 
 // In: c[3][8] nodal values per component.  Out: c[3][8] nodal forces of pe*Ke*u.
-// EN: also *energy = u . (pe Ke u) = sum over modes of (transformed u) . (modal
-// force), since the backward transform is the forward one's transpose.
-template <typename T, bool EN = false>
-__device__ __forceinline__ void modal_element(T c[3][8], T pe, T* energy = nullptr) {
+template <typename T>
+__device__ __forceinline__ void modal_element(T c[3][8], T pe) {
   wht3_fwd<T>(c);
   const T L = modal_c<T>(0) * pe, M = modal_c<T>(1) * pe;
   const T k0 = modal_c<T>(2), k1 = modal_c<T>(3), k2 = modal_c<T>(4);
@@ -248,14 +246,6 @@ __device__ __forceinline__ void modal_element(T c[3][8], T pe, T* energy = nullp
   {  // YZ, XZ, XY parts all act on the XYZ mode
     const T kk = k2 * (L + T(4) * M);
     g[0][7] = kk * c[0][7]; g[1][7] = kk * c[1][7]; g[2][7] = kk * c[2][7];
-  }
-  if constexpr (EN) {
-    T e = T(0);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int a = 1; a < 8; ++a) e += c[i][a] * g[i][a];  // g[i][0] = 0: rigid translation
-    *energy = e;
   }
   wht3_bwd<T>(g);
 #pragma unroll
@@ -1288,7 +1278,7 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
                                                             const uint8_t* __restrict__ vmask,
                                                             const double* __restrict__ u,
                                                             const double* __restrict__ f, double* __restrict__ out,
-                                                            int zblk, double* __restrict__ energy) {
+                                                            int zblk) {
   using S = DfSmem<TXE, TYE>;
   constexpr int NT = S::NT, PX = S::PX, NP = S::NP;
   extern __shared__ __align__(32) unsigned char modal_smem[];
@@ -1306,8 +1296,7 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
   const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
   int z0, zend;  // the planes marched: [zb0, zb1) less the void
   fine_active_planes<VOID>(d, zb0, zb1, z0, zend);
-  // Void planes [pa, pb): the owned vertices get the output for zero forces;
-  // MODE 3 writes zero energy for this thread's owned elements of those layers.
+  // Void planes [pa, pb): the owned vertices get the output for zero forces.
   auto void_planes = [&](int pa, int pb) {
     for (int p = pa; p < pb; ++p) {
       if (own) {
@@ -1316,9 +1305,6 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
 #pragma unroll
         for (int c = 0; c < 3; ++c) out[c * nv + v] = (MODE >= 1 && ((m >> c) & 1)) ? f[c * nv + v] : 0.0;
       }
-      const int ex = gx - 1, ey = gy - 1;
-      if (MODE == 3 && i > 0 && j > 0 && ex < d.ex && ey < d.ey && p < d.ez)
-        energy[ex + (int64_t)d.ex * (ey + (int64_t)d.ey * p)] = 0.0;
     }
   };
   if (VOID) {
@@ -1367,9 +1353,6 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
         df pe(0);
         if (ex >= 0 && ey >= 0 && ez >= 0 && ex < d.ex && ey < d.ey && ez < d.ez)
           pe = df_from(rhop[ex + (int64_t)d.ex * (ey + (int64_t)d.ey * ez)]);
-        // MODE 3 writes u_e . (rho^p Ke u_e) of the elements this CTA owns (its
-        // first element row / column and layer belong to the neighbouring tiles)
-        const bool own_e = MODE == 3 && i > 0 && j > 0 && ez >= z0 && ex < d.ex && ey < d.ey && ez < d.ez;
         if (pe != df(0)) {
           df c[3][8];
 #pragma unroll
@@ -1379,13 +1362,7 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
             const float4 h = sm.phi[cs][k], l = sm.plo[cs][k];
             c[0][a] = df(h.x, l.x); c[1][a] = df(h.y, l.y); c[2][a] = df(h.z, l.z);
           }
-          if (MODE == 3) {
-            df en;
-            modal_element<df, true>(c, pe, &en);
-            if (own_e) energy[ex + (int64_t)d.ex * (ey + (int64_t)d.ey * ez)] = df_to(en);
-          } else {
-            modal_element<df>(c, pe);
-          }
+          modal_element<df>(c, pe);
 #pragma unroll
           for (int a = 0; a < 8; ++a) {
             sm.fhi[a][t] = make_float4(c[0][a].hi, c[1][a].hi, c[2][a].hi, 0.f);
@@ -1397,7 +1374,6 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
             sm.fhi[a][t] = make_float4(0.f, 0.f, 0.f, 0.f);
             sm.flo[a][t] = make_float4(0.f, 0.f, 0.f, 0.f);
           }
-          if (own_e) energy[ex + (int64_t)d.ex * (ey + (int64_t)d.ey * ez)] = 0.0;
         }
       }
       __syncthreads();
@@ -1820,8 +1796,7 @@ template int launch_fine_apply_dot<double>(cudaStream_t, const LevelDims&, const
 
 template <bool VOID>
 static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
-                                   const double* u, const double* f, double* out, bool residual, int nb, int tz,
-                                   double* energy) {
+                                   const double* u, const double* f, double* out, bool residual, int nb, int tz) {
   if (tz <= 0) tz = MODAL_TZ;
   const int gx = (d.vx + MODAL_TXE - 2) / (MODAL_TXE - 1), gy = (d.vy + MODAL_TYE - 2) / (MODAL_TYE - 1);
   const int zblk = fine_zblocks(d.vz, tz, (int64_t)gx * gy * nb);
@@ -1835,24 +1810,18 @@ static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const dou
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_fine_modal_df<MODAL_TXE, MODAL_TYE, 1, VOID>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_fine_modal_df<MODAL_TXE, MODAL_TYE, 3, VOID>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return e;
   });
-  if (residual && energy)
-    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 3, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk, energy);
-  else if (residual)
-    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 1, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk, nullptr);
+  if (residual)
+    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 1, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk);
   else
-    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 0, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk, nullptr);
+    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 0, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk);
 }
 
 void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
-                          const double* u, const double* f, double* out, bool residual, int nb, int tz,
-                          double* energy) {
-  if (d.colz && d.colz_void) launch_fine_apply_df_v<true>(s, d, rhop, vmask, u, f, out, residual, nb, tz, energy);
-  else launch_fine_apply_df_v<false>(s, d, rhop, vmask, u, f, out, residual, nb, tz, energy);
+                          const double* u, const double* f, double* out, bool residual, int nb, int tz) {
+  if (d.colz && d.colz_void) launch_fine_apply_df_v<true>(s, d, rhop, vmask, u, f, out, residual, nb, tz);
+  else launch_fine_apply_df_v<false>(s, d, rhop, vmask, u, f, out, residual, nb, tz);
 }
 
 // One fused Chebyshev step on level 0: uout = u + d with d = c_old d + c_new Dinv (f - K u)

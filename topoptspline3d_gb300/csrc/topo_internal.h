@@ -173,10 +173,8 @@ template <typename T>
 int launch_fine_apply_dot(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, const T* u,
                           T* out, int tz, double* partial, int cap, double* dot = nullptr, unsigned* ctr = nullptr);
 // FP64 vectors, double-float arithmetic (k_fine_modal_df)
-// energy (residual only, one right-hand side): per-element u_e . (rho^p Ke u_e)
 void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
-                          const double* u, const double* f, double* out, bool residual, int nb = 1, int tz = 0,
-                          double* energy = nullptr);
+                          const double* u, const double* f, double* out, bool residual, int nb = 1, int tz = 0);
 // FP64 vectors, 64-bit fixed-point arithmetic (k_fine_fx): K u or f - K u, and
 // the Chebyshev step of launch_fine_cheb<double>
 void launch_fine_apply_fx(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
@@ -317,12 +315,10 @@ void launch_coeff_to_density(cudaStream_t s, const LevelDims& d, const uint8_t* 
 void launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                          const SplineDev& sp, const float2* coeff_df, double rho_min, double* partial,
                          double* out, double* Btmp);
+// sens = -p rho^(p-1) u_e^T Ke u_e; rhop (may be null): rho^(p-1) as rhop / rho
 void launch_sensitivity(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                        const double* rho, const double* u, double penal, double lam, double mu,
+                        const double* rho, const double* rhop, const double* u, double penal, double lam, double mu,
                         double h, double* sens);
-// sens = -p E / rho in place, from element energies E = u_e . (rho^p Ke u_e)
-void launch_sensitivity_from_energy(cudaStream_t s, int64_t ne, const uint8_t* eactive, const double* rho,
-                                    double penal, double* sens);
 // The same filter in double-float, in place on sens (sens_df: ne float2 scratch;
 // wts: the weights split into (hi, lo) floats)
 void launch_filter_df(cudaStream_t s, const LevelDims& d, const uint8_t* eactive, double* sens,

@@ -274,7 +274,7 @@ __device__ __forceinline__ void fine_active_planes(const LevelDims& d, int zb0, 
 }
 
 // y = K(rho) u (or f - K u) on level 0.  A CTA owns a (TXE-1) x (TYE-1) column of
-// vertices over one of zblk blocks of vertex planes and marches in z.  Vertex planes are staged in
+// vertices over one block of vertex planes (ZSplit) and marches in z.  Vertex planes are staged in
 // shared memory by asynchronous copies (cp.async, zero-filled outside the
 // domain) two planes ahead of use in a 3-slot ring; per element layer the CTA
 // computes its TXE x TYE elements (one per thread) into shared memory, and each
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE 
     k_fine_modal(LevelDims d, const T* __restrict__ rhop,
                                                          const uint8_t* __restrict__ vmask,
                                                          const T* __restrict__ u, const T* __restrict__ f,
-                                                         T* __restrict__ out, int zblk, ChebArgs ch) {
+                                                         T* __restrict__ out, ZSplit zs, ChebArgs ch) {
   using S = ModalSmem<T, TXE, TYE>;
   constexpr int NT = S::NT, PX = S::PX, NP = S::NP;
   extern __shared__ __align__(32) unsigned char modal_smem[];
@@ -417,16 +417,16 @@ __global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE 
   const int t = threadIdx.x, i = t % TXE, j = t / TXE;
   // blockIdx.z enumerates (right-hand side, z block): vectors of a batch of
   // right-hand sides are stored one after another, the operator is shared
-  const int rhs = blockIdx.z / zblk;
-  const int kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = fine_zblock(d.vz, zblk, kz);
+  const int rhs = blockIdx.z / zs.n;
+  const int kz = blockIdx.z - rhs * zs.n;
+  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = zs.begin(kz);
   const int64_t nv = d.nv;
   u += (int64_t)rhs * 3 * nv;
   if (f) f += (int64_t)rhs * 3 * nv;
   out += (int64_t)rhs * 3 * nv;
   const int gx = x0 + i, gy = y0 + j;  // owned vertex (x, y) and element (x-1, y-1)
   const bool own = (i < TXE - 1) && (j < TYE - 1) && gx < d.vx && gy < d.vy;
-  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
+  const int zb1 = zs.end(kz, zb0);
   int z0, zend;  // the planes marched: [zb0, zb1) less the void
   fine_active_planes<VOID>(d, zb0, zb1, z0, zend);
   T acc0 = T(0), acc1 = T(0), acc2 = T(0);
@@ -683,7 +683,7 @@ template <int TYE, int MODE, bool I32, bool VOID>
 __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ? TOPO_FINE32_CHEB_THREADS_PER_SM
                                                                                : TOPO_FINE32_THREADS_PER_SM))
     k_fine_modal32(LevelDims d, const float* __restrict__ rhop, const uint8_t* __restrict__ vmask,
-                   const float* __restrict__ u, const float* __restrict__ f, float* __restrict__ out, int zblk,
+                   const float* __restrict__ u, const float* __restrict__ f, float* __restrict__ out, ZSplit zs,
                    ChebArgs ch) {
   // MODE 3: the Chebyshev step of MODE 2 that also sums f.out.  I32: vertex and
   // element offsets within one right-hand side in 32-bit arithmetic (3 nv and
@@ -699,10 +699,10 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
     sm.coef[0] = float(ch.coef[0]);
     sm.coef[1] = float(ch.coef[1]);
   }
-  const int rhs = blockIdx.z / zblk;
-  const int kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = fine_zblock(d.vz, zblk, kz);
-  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
+  const int rhs = blockIdx.z / zs.n;
+  const int kz = blockIdx.z - rhs * zs.n;
+  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = zs.begin(kz);
+  const int zb1 = zs.end(kz, zb0);
   const I nv = (I)d.nv;
   u += (int64_t)rhs * 3 * d.nv;
   if (f) f += (int64_t)rhs * 3 * d.nv;
@@ -967,7 +967,7 @@ cudaError_t fine_tc_error(int* flag) {
 template <int TYE, int MODE, bool I32>
 __global__ void __launch_bounds__(32 * TYE, 3)
     k_fine_tc32(LevelDims d, const float* __restrict__ rhop, const uint8_t* __restrict__ vmask,
-                const float* __restrict__ u, const float* __restrict__ f, float* __restrict__ out, int zblk,
+                const float* __restrict__ u, const float* __restrict__ f, float* __restrict__ out, ZSplit zs,
                 ChebArgs ch) {
   static_assert(TYE == 8, "two M = 128 tiles of 32 x 4 elements per layer");
   constexpr bool CHEB = MODE >= 2, DOTS = MODE == 3;
@@ -1015,10 +1015,10 @@ __global__ void __launch_bounds__(32 * TYE, 3)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = sm.tmem;
 
-  const int rhs = blockIdx.z / zblk;
-  const int kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TXE - 2), y0 = blockIdx.y * (TYE - 1), zb0 = fine_zblock(d.vz, zblk, kz);
-  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
+  const int rhs = blockIdx.z / zs.n;
+  const int kz = blockIdx.z - rhs * zs.n;
+  const int x0 = blockIdx.x * (TXE - 2), y0 = blockIdx.y * (TYE - 1), zb0 = zs.begin(kz);
+  const int zb1 = zs.end(kz, zb0);
   const I nv = (I)d.nv;
   u += (int64_t)rhs * 3 * d.nv;
   if (f) f += (int64_t)rhs * 3 * d.nv;
@@ -1278,22 +1278,22 @@ __global__ void __launch_bounds__(TXE* TYE) k_fine_modal_df(LevelDims d, const d
                                                             const uint8_t* __restrict__ vmask,
                                                             const double* __restrict__ u,
                                                             const double* __restrict__ f, double* __restrict__ out,
-                                                            int zblk) {
+                                                            ZSplit zs) {
   using S = DfSmem<TXE, TYE>;
   constexpr int NT = S::NT, PX = S::PX, NP = S::NP;
   extern __shared__ __align__(32) unsigned char modal_smem[];
   S& sm = *reinterpret_cast<S*>(modal_smem);
   const int t = threadIdx.x, i = t % TXE, j = t / TXE;
-  const int rhs = blockIdx.z / zblk;
-  const int kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = fine_zblock(d.vz, zblk, kz);
+  const int rhs = blockIdx.z / zs.n;
+  const int kz = blockIdx.z - rhs * zs.n;
+  const int x0 = blockIdx.x * (TXE - 1), y0 = blockIdx.y * (TYE - 1), zb0 = zs.begin(kz);
   const int64_t nv = d.nv;
   u += (int64_t)rhs * 3 * nv;
   if (f) f += (int64_t)rhs * 3 * nv;
   out += (int64_t)rhs * 3 * nv;
   const int gx = x0 + i, gy = y0 + j;
   const bool own = (i < TXE - 1) && (j < TYE - 1) && gx < d.vx && gy < d.vy;
-  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
+  const int zb1 = zs.end(kz, zb0);
   int z0, zend;  // the planes marched: [zb0, zb1) less the void
   fine_active_planes<VOID>(d, zb0, zb1, z0, zend);
   // Void planes [pa, pb): the owned vertices get the output for zero forces.
@@ -1687,7 +1687,7 @@ dim3 modal_grid(const LevelDims& d, int tz, int nb) {
 // One launch of the FP32 modal kernel with a CTA tile of ROWS element rows.
 template <int ROWS, int MODE, bool VOID>
 void launch_modal32_rows(cudaStream_t s, const LevelDims& d, const float* rhop, const uint8_t* vmask, const float* u,
-                         const float* f, float* out, int zblk, const dim3& grid, const ChebArgs& ch) {
+                         const float* f, float* out, const ZSplit& zs, const dim3& grid, const ChebArgs& ch) {
   const size_t smem = sizeof(Modal32Smem<ROWS>);
   static PerDeviceOnce once;
   once_per_device(once, [smem] {
@@ -1698,12 +1698,10 @@ void launch_modal32_rows(cudaStream_t s, const LevelDims& d, const float* rhop, 
                                (int)smem);
     return e;
   });
-  // (MODE 3 keeps 64-bit offsets: with 32-bit ones it spilled 32 bytes and
-  // ran 122 against 118 us at 256x128x128, where modes 0-2 gained 4-9 us)
-  if (MODE != 3 && 3 * d.nv < ((int64_t)1 << 31) && d.ne < ((int64_t)1 << 31))
-    k_fine_modal32<ROWS, MODE, true, VOID><<<grid, 32 * ROWS, smem, s>>>(d, rhop, vmask, u, f, out, zblk, ch);
+  if (3 * d.nv < ((int64_t)1 << 31) && d.ne < ((int64_t)1 << 31))
+    k_fine_modal32<ROWS, MODE, true, VOID><<<grid, 32 * ROWS, smem, s>>>(d, rhop, vmask, u, f, out, zs, ch);
   else
-    k_fine_modal32<ROWS, MODE, false, VOID><<<grid, 32 * ROWS, smem, s>>>(d, rhop, vmask, u, f, out, zblk, ch);
+    k_fine_modal32<ROWS, MODE, false, VOID><<<grid, 32 * ROWS, smem, s>>>(d, rhop, vmask, u, f, out, zs, ch);
 }
 
 // One launch of the modal operator in mode MODE: the single-barrier kernel for
@@ -1715,15 +1713,16 @@ void launch_modal_v(cudaStream_t s, const LevelDims& d, const T* rhop, const uin
                     T* out, int tz, int nb, const ChebArgs& ch) {
   const dim3 grid = modal_grid<T>(d, tz, nb);
   const bool tc = modal_tc<T>(d, tz) && !VOID;
-  const int rows = modal_rows<T>(d, tz), zblk = (int)grid.z / nb;
+  const int rows = modal_rows<T>(d, tz), nzb = (int)grid.z / nb;
+  const ZSplit zs(d.vz, nzb);
   constexpr int TYE = modal_tye<T>();
   if constexpr (sizeof(T) == 4 && !VOID) {
     if (!tc && rows == 4) {
-      launch_modal32_rows<4, MODE, false>(s, d, rhop, vmask, u, f, out, zblk, grid, ch);
+      launch_modal32_rows<4, MODE, false>(s, d, rhop, vmask, u, f, out, zs, grid, ch);
       return;
     }
     if (!tc && rows == 16) {
-      launch_modal32_rows<16, MODE, false>(s, d, rhop, vmask, u, f, out, zblk, grid, ch);
+      launch_modal32_rows<16, MODE, false>(s, d, rhop, vmask, u, f, out, zs, grid, ch);
       return;
     }
   }
@@ -1740,14 +1739,14 @@ void launch_modal_v(cudaStream_t s, const LevelDims& d, const T* rhop, const uin
         return e;
       });
       if (MODE != 3 && 3 * d.nv < ((int64_t)1 << 31) && d.ne < ((int64_t)1 << 31))
-        k_fine_tc32<TYE, MODE, true><<<grid, 32 * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zblk, ch);
+        k_fine_tc32<TYE, MODE, true><<<grid, 32 * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zs, ch);
       else
-        k_fine_tc32<TYE, MODE, false><<<grid, 32 * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zblk, ch);
+        k_fine_tc32<TYE, MODE, false><<<grid, 32 * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zs, ch);
       return;
     }
   }
   if constexpr (sizeof(T) == 4) {
-    launch_modal32_rows<TYE, MODE, VOID>(s, d, rhop, vmask, u, f, out, zblk, grid, ch);
+    launch_modal32_rows<TYE, MODE, VOID>(s, d, rhop, vmask, u, f, out, zs, grid, ch);
   } else {
     const size_t smem = sizeof(ModalSmem<T, MODAL_TXE, TYE>);
     static PerDeviceOnce once;
@@ -1755,7 +1754,7 @@ void launch_modal_v(cudaStream_t s, const LevelDims& d, const T* rhop, const uin
       return cudaFuncSetAttribute(k_fine_modal<T, MODAL_TXE, TYE, MODE, VOID>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
-    k_fine_modal<T, MODAL_TXE, TYE, MODE, VOID><<<grid, MODAL_TXE * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zblk,
+    k_fine_modal<T, MODAL_TXE, TYE, MODE, VOID><<<grid, MODAL_TXE * TYE, smem, s>>>(d, rhop, vmask, u, f, out, zs,
                                                                                      ch);
   }
 }
@@ -1799,8 +1798,8 @@ static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const dou
                                    const double* u, const double* f, double* out, bool residual, int nb, int tz) {
   if (tz <= 0) tz = MODAL_TZ;
   const int gx = (d.vx + MODAL_TXE - 2) / (MODAL_TXE - 1), gy = (d.vy + MODAL_TYE - 2) / (MODAL_TYE - 1);
-  const int zblk = fine_zblocks(d.vz, tz, (int64_t)gx * gy * nb);
-  const dim3 grid(gx, gy, zblk * nb);
+  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz, (int64_t)gx * gy * nb));
+  const dim3 grid(gx, gy, zs.n * nb);
   constexpr int NT = MODAL_TXE * MODAL_TYE;
   const size_t smem = sizeof(DfSmem<MODAL_TXE, MODAL_TYE>);
   static PerDeviceOnce once;
@@ -1813,9 +1812,9 @@ static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const dou
     return e;
   });
   if (residual)
-    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 1, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk);
+    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 1, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zs);
   else
-    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 0, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zblk);
+    k_fine_modal_df<MODAL_TXE, MODAL_TYE, 0, VOID><<<grid, NT, smem, s>>>(d, rhop, vmask, u, f, out, zs);
 }
 
 void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,

@@ -63,13 +63,13 @@ struct FxCheb {
 template <int MODE, bool VOID>
 __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __restrict__ rhop,
                                                    const uint8_t* __restrict__ vmask, const double* __restrict__ u,
-                                                   const double* __restrict__ f, double* __restrict__ out, int zblk,
+                                                   const double* __restrict__ f, double* __restrict__ out, ZSplit zs,
                                                    FxCheb ch) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxSmem& sm = *reinterpret_cast<FxSmem*>(fx_smem);
   const int t = threadIdx.x, i = t % TX, j = t / TX;
-  const int rhs = blockIdx.z / zblk, kz = blockIdx.z - rhs * zblk;
-  const int x0 = blockIdx.x * (TX - 1), y0 = blockIdx.y * (TY - 1), zb0 = fine_zblock(d.vz, zblk, kz);
+  const int rhs = blockIdx.z / zs.n, kz = blockIdx.z - rhs * zs.n;
+  const int x0 = blockIdx.x * (TX - 1), y0 = blockIdx.y * (TY - 1), zb0 = zs.begin(kz);
   const int64_t nv = d.nv, plane_n = (int64_t)d.vx * d.vy;
   u += (int64_t)rhs * 3 * nv;
   if (MODE >= 1) f += (int64_t)rhs * 3 * nv;
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __
   double* __restrict__ dv = MODE == 2 ? ch.dvec + (int64_t)rhs * 3 * nv : nullptr;
   const int gx = x0 + i, gy = y0 + j;  // owned vertex (x, y) and element (x - 1, y - 1)
   const bool own = i < TX - 1 && j < TY - 1 && gx < d.vx && gy < d.vy;
-  const int zb1 = fine_zblock(d.vz, zblk, kz + 1);
+  const int zb1 = zs.end(kz, zb0);
   int z0 = zb0, zend = zb1;  // the planes marched: [zb0, zb1) less the void (LevelDims::colz)
   if (VOID) {
     const int2 cz = d.colz[blockIdx.x + gridDim.x * blockIdx.y];
@@ -288,8 +288,8 @@ void launch(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSmem));
   });
   const int gx = (d.vx + TX - 2) / (TX - 1), gy = (d.vy + TY - 2) / (TY - 1);
-  const int zblk = fine_zblocks(d.vz, tz > 0 ? tz : 16, (int64_t)gx * gy * nb);
-  fn<<<dim3(gx, gy, zblk * nb), NT, sizeof(FxSmem), s>>>(d, rhop, vmask, u, f, out, zblk, ch);
+  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz > 0 ? tz : 16, (int64_t)gx * gy * nb));
+  fn<<<dim3(gx, gy, zs.n * nb), NT, sizeof(FxSmem), s>>>(d, rhop, vmask, u, f, out, zs, ch);
 }
 
 }  // namespace

@@ -81,16 +81,24 @@ inline int fine_rows_flag(int rows) {
 // planes recomputes the element layer below it, but a march costs 2 to 5 us a
 // plane whatever the grid (16x8x8: FP32 step 11.9 us with 4 planes a block,
 // 8.1 with 1; fixed-point step 30.5 / 14.1; 77x44x42 with 304 CTAs 38 us, with
-// 441 43 us).  The planes are dealt evenly: block k covers [fine_zblock(k),
-// fine_zblock(k + 1)); a last block that takes the remainder of vz / tz marches
-// up to twice as long as the others (77x44x42, 4 planes: 57 us).
+// 441 43 us).  The planes are dealt evenly (ZSplit); a last block that takes
+// the remainder of vz / tz marches up to twice as long as the others (77x44x42,
+// 4 planes: 57 us).
 constexpr int FINE_FILL_CTAS = 304;
 inline int fine_zblocks(int vz, int tz, int64_t tiles) {
   const int64_t by_depth = vz / tz > 1 ? vz / tz : 1, fill = FINE_FILL_CTAS / (tiles > 0 ? tiles : 1);
   const int64_t most = fill < vz ? fill : vz;
   return (int)(by_depth > most ? by_depth : most);
 }
-__host__ __device__ inline int fine_zblock(int vz, int zblk, int k) { return k * vz / zblk; }
+// n blocks of vz planes: the first r of them have q + 1, the others q (worked
+// out on the host: a division in the FP32 kernel costs it a register, and the
+// Chebyshev step of 256x128x128 then spills, 107 against 104 us)
+struct ZSplit {
+  int n, q, r;
+  ZSplit(int vz, int blocks) : n(blocks), q(vz / blocks), r(vz % blocks) {}
+  __host__ __device__ int begin(int k) const { return k * q + (k < r ? k : r); }
+  __host__ __device__ int end(int k, int begin_k) const { return begin_k + q + (k < r ? 1 : 0); }
+};
 
 // Vertex tile of the fine z-marching kernels: a CTA owns FINE_TILE_X - 1 by
 // FINE_TILE_Y - 1 vertex columns and computes the FINE_TILE_X x FINE_TILE_Y

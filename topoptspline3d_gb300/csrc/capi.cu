@@ -297,14 +297,15 @@ void cheb_level(topo_handle* h, int l, const ChebParams& cp, bool zero_start, bo
       if (sizeof(T) == 4 || !h->fine_fx()) np = launch_fine_cheb<T>(
           h->stream, L.d, P<T>::rhop(h), L.vmask, ua, P<T>::F(L), ub, P<T>::dinv(L), P<T>::cd(L), coef, k == 0,
           h->nb, sizeof(T) == 4 ? tz32_arg(h) : h->tz64, d_in_u && k == 1, dots ? h->vdot : nullptr, h->fdot_cap,
-          h->vdot_out, TOPO_FUSED_DOT_TICKET ? h->ctr : nullptr);
+          h->vdot_out, TOPO_FUSED_DOT_TICKET ? h->ctr : nullptr, h->vdot_ratio);
       if (np > 0 && !TOPO_FUSED_DOT_TICKET) {
-        launch_sum_partials(h->stream, h->vdot, np, h->vdot_out);
+        launch_sum_partials(h->stream, h->vdot, np, h->vdot_out, h->vdot_ratio);
         count_launch();
       }
       prof_end(h, ev);
       if (dots && np == 0) {  // r.z of the cycle's result (F is r, the output is z), unfused
-        launch_dot<T>(h->stream, P<T>::F(L), ub, 3 * L.d.nv, h->partial, h->vdot_out, h->ctr);
+        launch_dot<T>(h->stream, P<T>::F(L), ub, 3 * L.d.nv, h->partial, h->vdot_out, h->ctr,
+                      h->vdot_ratio);
         count_launch();
       }
     } else {
@@ -462,30 +463,6 @@ __global__ void k_power_start(int64_t nv, const uint8_t* vmask, T* x) {
   x[i] = (T)v;
 }
 
-// z = s D^-1 r with s = 1/sqrt(*nrm2) (the power iteration's normalisation of
-// its vector, applied after the operator, which is linear).  D^-1 is [9][nv],
-// or with sym the packed symmetric layout of level 0's FP32 inverse (float4
-// d00 d01 d02 d11 per vertex, then float2 d12 d22).
-template <typename T>
-__global__ void k_dinv_apply(int64_t nv, const T* dinv, const T* r, T* z, const double* nrm2, bool sym) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  const T sc = (T)rsqrt(*nrm2);
-  const T r0 = r[v] * sc, r1 = r[nv + v] * sc, r2 = r[2 * nv + v] * sc;
-  if constexpr (sizeof(T) == 4) {
-    if (sym) {
-      const float4 a = reinterpret_cast<const float4*>(dinv)[v];
-      const float2 b = reinterpret_cast<const float2*>(dinv + 4 * nv)[v];
-      z[v] = a.x * r0 + a.y * r1 + a.z * r2;
-      z[nv + v] = a.y * r0 + a.w * r1 + b.x * r2;
-      z[2 * nv + v] = a.z * r0 + b.x * r1 + b.y * r2;
-      return;
-    }
-  }
-  for (int i = 0; i < 3; ++i)
-    z[i * nv + v] = dinv[(3 * i) * nv + v] * r0 + dinv[(3 * i + 1) * nv + v] * r1 + dinv[(3 * i + 2) * nv + v] * r2;
-}
-
 template <typename T>
 __global__ void k_to_double(int64_t n, const T* a, double* b) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -494,35 +471,9 @@ __global__ void k_to_double(int64_t n, const T* a, double* b) {
 
 inline unsigned nb256(int64_t n) { return (unsigned)((n + 255) / 256); }
 
-// Loop control of the device-side inner CG (slots loop[0..3]: iterations of
-// this solve, ||b|| reference, first non-finite iteration (1-based, 0 none),
-// iterations summed over the solve).  Start: zero the count, take ||b|| from
-// the outer residual (1 if that is 0) and test ||r|| / ||b|| > rtol.
-__global__ void k_loop_start(double* loop, const double* rr_outer, const double* rr, double rtol, int maxit,
-                             cudaGraphConditionalHandle hc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double bo = sqrt(*rr_outer);
-  const double bn = bo > 0 ? bo : 1.0;
-  loop[0] = 0.0;
-  loop[1] = bn;
-  cudaGraphSetConditional(hc, (sqrt(*rr) / bn > rtol && 0 < maxit) ? 1u : 0u);
-}
-
-// End of one iteration: count it and test again; a non-finite ||r|| stops the
-// loop and is recorded.
-__global__ void k_loop_step(double* loop, const double* rr, double rtol, int maxit, cudaGraphConditionalHandle hc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double it = loop[0] + 1.0;
-  loop[0] = it;
-  loop[3] += 1.0;
-  const double rn = sqrt(*rr);
-  unsigned go = 0;
-  if (!isfinite(rn)) {
-    if (loop[2] == 0.0) loop[2] = it;
-  } else {
-    go = (rn / loop[1] > rtol && it < (double)maxit) ? 1u : 0u;
-  }
-  cudaGraphSetConditional(hc, go);
+// Start of a device-side CG loop whose set-up is outside its graph.
+__global__ void k_loop_start(const double* bb, const double* rr, LoopCtl lc) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) loop_start(lc, *bb, *rr);
 }
 
 // OC bisection on the device (slots oc[0..5]: lo, hi, threshold of the
@@ -559,13 +510,6 @@ __global__ void k_ocl_step(double* oc, const double* vol, double den, double vgo
   }
   if (go) oc[2] = 0.5 * (lo + hi);
   cudaGraphSetConditional(hc, go ? 1u : 0u);
-}
-
-// beta = (r.z - z.rold) / rold.z after the first iteration (the host loop's
-// scalar ratio, taken when the iteration counter is past 0).
-__global__ void k_loop_beta(const double* loop, double* sc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (loop[0] > 0.0) sc[S_BETA] = (sc[S_RZ] - sc[S_ZROLD]) / sc[S_RZOLD];
 }
 
 int read_scalars(topo_handle* h, int first, int count);
@@ -703,7 +647,7 @@ void fine_product(topo_handle* h, const T* x, T* y) {
 // back to back with their own scalar slots, so all levels cost one host read
 // (two when a warm estimate dropped).
 // One step: with s = 1/|x|, z = D^-1 A (s x) = s D^-1 (A x) and the Rayleigh
-// estimate (s x).z = s (x.z); x <- z.  Work vectors: the level's R, U2 and
+// estimate (s x).z = s (x.z); x <- z.  The operator, then one kernel for the rest.  Work vectors: the level's R, U2 and
 // Chebyshev direction buffers (all free outside a V-cycle).
 template <typename T>
 int estimate_bounds(topo_handle* h) {
@@ -732,19 +676,22 @@ int estimate_bounds(topo_handle* h) {
     runs.push_back(r);
   }
   if (runs.empty()) return TOPO_OK;
-  auto power_steps = [&](Run& r, int k) {
+  auto power_steps = [&](Run& r, int k, bool first) {
     DevLevel& L = h->lv[r.l];
     const int64_t n3 = 3 * L.d.nv;
     double* sl = h->sc + S_PW + 2 * r.l;
+    double* nrm = h->sc + S_PZ + r.l;
+    if (first) {
+      launch_dot<T>(h->stream, r.x, r.x, n3, h->partial, nrm, h->ctr);
+      count_launch();
+    }
     for (int it = 0; it < k; ++it) {
-      launch_dot<T>(h->stream, r.x, r.x, n3, h->partial, sl, h->ctr);
       if (r.l == 0) fine_product<T>(h, r.x, r.y);
       else launch_stencil_apply<T>(h->stream, L.d, P<T>::st(L), r.x, nullptr, r.y, false);
-      k_dinv_apply<T><<<nb256(L.d.nv), 256, 0, h->stream>>>(L.d.nv, P<T>::dinv(L), r.y, r.z, sl,
-                                                           sizeof(T) == 4 && r.l == 0);
-      launch_dot<T>(h->stream, r.x, r.z, n3, h->partial, sl + 1, h->ctr);
+      launch_power_step<T>(h->stream, L.d.nv, P<T>::dinv(L), sizeof(T) == 4 && r.l == 0, r.x, r.y, r.z, h->partial,
+                           nrm, sl, sl + 1, h->ctr);
       std::swap(r.x, r.z);
-      count_launch(4);
+      count_launch(2);
     }
   };
   auto read_all = [&]() -> int {
@@ -760,7 +707,7 @@ int estimate_bounds(topo_handle* h) {
     mask |= 1u << r.l;
     warm |= r.warm ? 1u << r.l : 0u;
   }
-  for (Run& r : runs) power_steps(r, r.warm ? 4 : 12);
+  for (Run& r : runs) power_steps(r, r.warm ? 4 : 12, true);
   if (h->iter_capture) {
     // inside a captured design iteration: the restart test on the device and
     // one conditional node per level for its 8 more steps (an even count, so
@@ -778,7 +725,7 @@ int estimate_bounds(topo_handle* h) {
     for (Run& r : runs) {
       long long per = 0;
       RET(capture_cond_node(h, conds.c[r.l], cudaGraphCondTypeIf, [&]() -> int {
-        power_steps(r, 8);
+        power_steps(r, 8, false);
         return TOPO_OK;
       }, &per));
       h->d_if_body = per;
@@ -788,7 +735,7 @@ int estimate_bounds(topo_handle* h) {
     bool more = false;
     for (Run& r : runs)
       if (r.warm && r.lam < 0.95 * P<T>::lprev(h->lv[r.l])) {
-        power_steps(r, 8);
+        power_steps(r, 8, false);
         more = true;
       }
     if (more) RET(read_all());
@@ -843,37 +790,34 @@ int read_scalars(topo_handle* h, int first, int count) {
 // `it` is the iteration number when the host runs the loop; it is -1 when the
 // loop runs on the device (a graphed solve), where the iteration counter in
 // the loop slots `loop` (the inner loop's by default) tells the first
-// iteration from the others.
+// iteration from the others and hc is the loop's condition.  alpha and beta are
+// written by the blocks that finish d.q and r.z (beta of a first iteration is
+// written from stale slots and not read).
 template <typename T, typename Prec>
 int fcg_body(topo_handle* h, T* x, T* r, T* d, T* q, T* rold, T* z, double* sc, Prec&& prec, bool prec_dots,
-             int it, double* loop = nullptr) {
-  if (!loop) loop = h->sc + S_LOOP;
+             int it, LoopCtl lc = LoopCtl{}) {
+  double* loop = lc.loop;
   DevLevel& L0 = h->lv[0];
   const int64_t n3 = 3 * L0.d.nv;
   RET(prec(r, z));
-  if (!prec_dots) {  // else the preconditioner left r.z and z.rold in the scalar slots
-    launch_dot<T>(h->stream, r, z, n3, h->partial, sc + S_RZ, h->ctr);
+  if (!prec_dots) {  // else the preconditioner left r.z and beta in the scalar slots
+    if (it == 0)
+      launch_dot<T>(h->stream, r, z, n3, h->partial, sc + S_RZ, h->ctr);
+    else  // (rold is not read on the device loop's first iteration)
+      launch_dot2<T>(h->stream, r, z, rold, n3, h->partial, sc + S_RZ, sc + S_ZROLD, h->ctr,
+                     it < 0 ? loop : nullptr, SumRatio{sc + S_RZ, sc + S_ZROLD, sc + S_RZOLD, sc + S_BETA});
     count_launch();
-    if (it != 0) {  // (on the device loop's first iteration the kernel returns at once)
-      launch_dot<T>(h->stream, z, rold, n3, h->partial, sc + S_ZROLD, h->ctr, it < 0 ? loop : nullptr);
-      count_launch();
-    }
-  }
-  if (it < 0) {
-    k_loop_beta<<<1, 32, 0, h->stream>>>(loop, sc);
-    count_launch();
-  } else if (it > 0) {
-    launch_scalar_ratio(h->stream, sc, S_RZ, S_ZROLD, S_RZOLD, S_BETA);
   }
   launch_pcg_dir<T>(h->stream, z, d, sc, S_BETA, it == 0, n3, it < 0 ? loop : nullptr);
   // q = A d with d.q: fused into the FP32 operator's epilogue
   int nparts = 0;
+  const SumRatio alpha{sc + S_RZ, nullptr, sc + S_DQ, sc + S_ALPHA};
   if (sizeof(T) == 4 && h->fdot && h->nb == 1) {
     EventPair* ev = prof_begin(h, P<T>::fam_apply);
     nparts = launch_fine_apply_dot<T>(h->stream, L0.d, P<T>::rhop(h), L0.vmask, d, q, tz32_arg(h), h->fdot,
-                                      h->fdot_cap, sc + S_DQ, TOPO_FUSED_DOT_TICKET ? h->ctr : nullptr);
+                                      h->fdot_cap, sc + S_DQ, TOPO_FUSED_DOT_TICKET ? h->ctr : nullptr, alpha);
     if (nparts > 0 && !TOPO_FUSED_DOT_TICKET) {
-      launch_sum_partials(h->stream, h->fdot, nparts, sc + S_DQ);
+      launch_sum_partials(h->stream, h->fdot, nparts, sc + S_DQ, alpha);
       count_launch();
     }
     prof_end(h, ev);
@@ -882,16 +826,14 @@ int fcg_body(topo_handle* h, T* x, T* r, T* d, T* q, T* rold, T* z, double* sc, 
     count_launch();
   } else {
     level_apply<T>(h, 0, d, nullptr, q, false);
-    launch_dot<T>(h->stream, d, q, n3, h->partial, sc + S_DQ, h->ctr);
+    launch_dot<T>(h->stream, d, q, n3, h->partial, sc + S_DQ, h->ctr, alpha);
     count_launch();
   }
-  launch_scalar_ratio(h->stream, sc, S_RZ, -1, S_DQ, S_ALPHA);
   // x += alpha d, rold = r, r -= alpha q with r.r of the new residual; rold
   // is not kept when the preconditioner runs the plain (Fletcher-Reeves) form
-  launch_pcg_update_rr<T>(h->stream, x, r, (prec_dots && h->inner_fr) ? nullptr : rold, d, q, sc, S_ALPHA, n3,
-                          h->partial, sc + S_RR, h->ctr);
-  CK(cudaMemcpyAsync(sc + S_RZOLD, sc + S_RZ, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  count_launch(it > 0 ? 4 : 3);
+  launch_pcg_update_rr<T>(h->stream, x, r, (prec_dots && h->inner_fr) ? nullptr : rold, d, q, sc, S_ALPHA, S_RZ, S_RZOLD,
+                          n3, h->partial, sc + S_RR, h->ctr, lc);
+  count_launch(2);
   CKL();
   return TOPO_OK;
 }
@@ -1022,8 +964,8 @@ int capture_nested_loop(topo_handle* h, Setup&& setup, Body&& body, long long* p
 
 // The FP32 inner CG of the mixed solve, z = CG(r) from x = 0, as one CUDA
 // graph: set-up (r in FP32, x = 0, r.r and the stopping test), a WHILE node
-// whose body is one CG iteration (fcg_body) closed by a kernel that counts the
-// iteration and sets the loop condition, and the copy of x to FP64 in z.  The
+// whose body is one CG iteration (fcg_body, whose last kernel counts the
+// iteration and sets the loop condition), and the copy of x to FP64 in z.  The
 // iterations are the host loop's, kernel for kernel, with the same stopping
 // rule (||r|| / ||b|| > rtol and fewer than maxit iterations; ||b|| is the
 // outer residual's norm, 1 if that is 0) decided on the device, so the host
@@ -1040,17 +982,14 @@ int inner_cg_graphed(topo_handle* h, const double* rin, double* zout, double rto
                          (double)(uintptr_t)h->x32, (double)(uintptr_t)h->d32, (double)(uintptr_t)h->q32,
                          (double)tz32_arg(h), (double)(uintptr_t)h->fdot, (double)h->fdot_cap});
   auto setup = [&](cudaGraphConditionalHandle hc) -> int {
-    launch_d2f(h->stream, rin, L0.F32, n3);
-    CK(cudaMemsetAsync(h->x32, 0, sizeof(float) * n3, h->stream));
-    launch_dot<float>(h->stream, L0.F32, L0.F32, n3, h->partial, sc + S_RR, h->ctr);
-    k_loop_start<<<1, 32, 0, h->stream>>>(h->sc + S_LOOP, h->sc + S_RR, sc + S_RR, rtol, maxit, hc);
-    count_launch(3);
+    launch_inner_start(h->stream, rin, L0.F32, h->x32, n3, h->partial, sc + S_RR, h->sc + S_RR, h->ctr,
+                       LoopCtl{h->sc + S_LOOP, rtol, maxit, hc});
+    count_launch();
     return TOPO_OK;
   };
   auto body = [&](cudaGraphConditionalHandle hc) -> int {
-    RET(fcg_body<float>(h, h->x32, L0.F32, h->d32, h->q32, h->rold32, L0.U32, sc, prec, true, -1));
-    k_loop_step<<<1, 32, 0, h->stream>>>(h->sc + S_LOOP, sc + S_RR, rtol, maxit, hc);
-    count_launch();
+    RET(fcg_body<float>(h, h->x32, L0.F32, h->d32, h->q32, h->rold32, L0.U32, sc, prec, true, -1,
+                        LoopCtl{h->sc + S_LOOP, rtol, maxit, hc}));
     return TOPO_OK;
   };
   auto tail = [&]() -> int {  // z = x in FP64 after the loop
@@ -1079,8 +1018,8 @@ int inner_cg_graphed(topo_handle* h, const double* rin, double* zout, double rto
 // The outer FP64 flexible CG of the mixed solve as one CUDA graph: a WHILE
 // node whose body is one outer iteration (fcg_body: the FP32 preconditioner,
 // one V-cycle or the inner CG as a nested WHILE node, then the FP64 matvec,
-// step and update) closed by a kernel that counts the iteration and sets the
-// loop condition on the outer loop slots.  The stopping rule is the host
+// step and update, whose last block counts the iteration and sets the loop
+// condition on the outer loop slots).  The stopping rule is the host
 // loop's (||r|| / ||F|| > rtol and fewer than maxit iterations) decided on
 // the device, so the host waits for the GPU once per solve instead of once
 // per outer iteration.  The set-up (r = f - A x and r.r in sc[S_RR], F.F in
@@ -1097,14 +1036,13 @@ int outer_cg_graphed(topo_handle* h, double rtol, int maxit, Prec&& prec, std::v
                          (double)tz32_arg(h), (double)(uintptr_t)h->fdot, (double)h->fdot_cap});
   auto setup = [&](cudaGraphConditionalHandle hc) -> int {
     CK(cudaMemsetAsync(loop + 2, 0, 2 * sizeof(double), h->stream));
-    k_loop_start<<<1, 32, 0, h->stream>>>(loop, h->sc + S_FF, h->sc + S_RR, rtol, maxit, hc);
+    k_loop_start<<<1, 32, 0, h->stream>>>(h->sc + S_FF, h->sc + S_RR, LoopCtl{loop, rtol, maxit, hc});
     count_launch();
     return TOPO_OK;
   };
   auto body = [&](cudaGraphConditionalHandle hc) -> int {
-    RET(fcg_body<double>(h, h->x, h->r, h->d, h->q, h->rold, L0.U, h->sc, prec, false, -1, loop));
-    k_loop_step<<<1, 32, 0, h->stream>>>(loop, h->sc + S_RR, rtol, maxit, hc);
-    count_launch();
+    RET(fcg_body<double>(h, h->x, h->r, h->d, h->q, h->rold, L0.U, h->sc, prec, false, -1,
+                         LoopCtl{loop, rtol, maxit, hc}));
     return TOPO_OK;
   };
   if (h->iter_capture) {  // inside a captured design iteration: a nested WHILE node
@@ -2040,16 +1978,16 @@ static int solve_impl(topo_handle* h, const topo_solve_opts* o, topo_solve_stats
       h->vdot_on = vdots && !net_on;
       h->inner_fr = h->vdot_on;
       h->vdot_out = s_rz;
-      if (h->inner_fr) CK(cudaMemsetAsync(s_zr, 0, sizeof(double), h->stream));
+      h->vdot_ratio = SumRatio{s_rz, nullptr, h->sc + 8 + S_RZOLD, h->sc + 8 + S_BETA};  // z.rold = 0
       const int rc = vcycle_prec<float>(h, r, o->pre, o->post, o->smoother, cp);
       const bool fused = h->vdot_on;
       h->vdot_on = false;
       RET(rc);
       RET(net(r, L0.U32));
       if (!fused) {
-        launch_dot<float>(h->stream, r, L0.U32, n3, h->partial, s_rz, h->ctr);
-        launch_dot<float>(h->stream, L0.U32, h->rold32, n3, h->partial, s_zr, h->ctr);
-        count_launch(2);
+        launch_dot2<float>(h->stream, r, L0.U32, h->rold32, n3, h->partial, s_rz, s_zr, h->ctr, nullptr,
+                           SumRatio{s_rz, s_zr, h->sc + 8 + S_RZOLD, h->sc + 8 + S_BETA});
+        count_launch();
       }
       return TOPO_OK;
     };

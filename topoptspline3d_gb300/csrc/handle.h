@@ -35,7 +35,9 @@ enum Slot {
   S_LAM = S_OLOOP + 4, S_LPREV = S_LAM + 2 * S_MAXLEV,
   // results of a graphed design iteration: compliance F.U, the density sum
   // after the OC update, levels whose power iteration restarted
-  S_DI = S_LPREV + 2 * S_MAXLEV, S_COUNT = S_DI + 3
+  S_DI = S_LPREV + 2 * S_MAXLEV,
+  // |x|^2 of each level's power-iteration vector, for the next step
+  S_PZ = S_DI + 3, S_COUNT = S_PZ + S_MAXLEV
 };
 
 // Chebyshev step coefficients (c_old, c_new) in device memory: per precision
@@ -188,6 +190,7 @@ struct topo_handle {
   double* vdot = nullptr;
   bool vdot_on = false;
   double* vdot_out = nullptr;
+  topo::SumRatio vdot_ratio{};  // written after it (the inner CG's beta)
   bool inner_fr = false;  // inner CG in Fletcher-Reeves form (z.rold taken as 0)
   double* chebc = nullptr;          // Chebyshev coefficient table (device)
   double* sc = nullptr;    // device scalar slots

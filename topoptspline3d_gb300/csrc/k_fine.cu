@@ -292,6 +292,7 @@ struct ChebArgs {
   int d_is_u;        // MODE 2, FP32: d equals u on entry (the step after a zero start); dvec is not read
   double* dot;       // with ctr: the last CTA sums the partials into *dot
   unsigned* ctr;     // zeroed ticket counter (reset by the last CTA)
+  SumRatio rt;       // written after *dot
 };
 
 // Sum of v over the CTA (valid in thread 0); every thread must call it.
@@ -300,7 +301,8 @@ __device__ __forceinline__ double modal_block_sum(double v);
 // After thread 0 of every CTA published its partial: the CTA that takes the last
 // ticket sums the n partials in index order (independent of which CTA is last)
 // into *out and resets the counter.  Every thread must call it.
-__device__ __forceinline__ void modal_finish_sum(const double* partial, int64_t n, double* out, unsigned* ctr) {
+__device__ __forceinline__ void modal_finish_sum(const double* partial, int64_t n, double* out, unsigned* ctr,
+                                                 const SumRatio& rt) {
   __shared__ bool last;
   if (threadIdx.x == 0) {  // thread 0 wrote the block's partial: fence, then take a ticket
     __threadfence();
@@ -314,6 +316,7 @@ __device__ __forceinline__ void modal_finish_sum(const double* partial, int64_t 
   s = modal_block_sum(s);
   if (threadIdx.x == 0) {
     *out = s;
+    write_ratio(rt);
     *ctr = 0u;
   }
 }
@@ -878,7 +881,7 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   if ((MODE == 0 || DOTS) && ch.dotp) {
     const double bs = modal_block_sum((double)dsum);
     if (t == 0) ch.dotp[cta] = bs;
-    if (ch.ctr) modal_finish_sum(ch.dotp, (int64_t)gridDim.x * gridDim.y * gridDim.z, ch.dot, ch.ctr);
+    if (ch.ctr) modal_finish_sum(ch.dotp, (int64_t)gridDim.x * gridDim.y * gridDim.z, ch.dot, ch.ctr, ch.rt);
   }
 }
 
@@ -1250,7 +1253,7 @@ __global__ void __launch_bounds__(32 * TYE, 3)
   if ((MODE == 0 || DOTS) && ch.dotp) {
     const double bs = modal_block_sum((double)dsum);
     if (t == 0) ch.dotp[cta] = bs;
-    if (ch.ctr) modal_finish_sum(ch.dotp, (int64_t)gridDim.x * gridDim.y * gridDim.z, ch.dot, ch.ctr);
+    if (ch.ctr) modal_finish_sum(ch.dotp, (int64_t)gridDim.x * gridDim.y * gridDim.z, ch.dot, ch.ctr, ch.rt);
   }
 }
 
@@ -1779,19 +1782,19 @@ void launch_fine_apply(cudaStream_t s, const LevelDims& d, const T* rhop, const 
 // CTAs than the cap partial slots.
 template <typename T>
 int launch_fine_apply_dot(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, const T* u,
-                          T* out, int tz, double* partial, int cap, double* dot, unsigned* ctr) {
+                          T* out, int tz, double* partial, int cap, double* dot, unsigned* ctr, SumRatio rt) {
   const dim3 grid = modal_grid<T>(d, tz, 1);
   const int64_t nparts = (int64_t)grid.x * grid.y * grid.z;
   if (nparts > cap) return 0;
-  const ChebArgs ch{nullptr, nullptr, nullptr, 0, partial, 0, dot, dot ? ctr : nullptr};
+  const ChebArgs ch{nullptr, nullptr, nullptr, 0, partial, 0, dot, dot ? ctr : nullptr, rt};
   launch_modal<T, 0>(s, d, rhop, vmask, u, nullptr, out, tz, 1, ch);
   return (int)nparts;
 }
 
 template int launch_fine_apply_dot<float>(cudaStream_t, const LevelDims&, const float*, const uint8_t*,
-                                          const float*, float*, int, double*, int, double*, unsigned*);
+                                          const float*, float*, int, double*, int, double*, unsigned*, SumRatio);
 template int launch_fine_apply_dot<double>(cudaStream_t, const LevelDims&, const double*, const uint8_t*,
-                                           const double*, double*, int, double*, int, double*, unsigned*);
+                                           const double*, double*, int, double*, int, double*, unsigned*, SumRatio);
 
 template <bool VOID>
 static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
@@ -1828,7 +1831,7 @@ void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop
 template <typename T>
 int launch_fine_cheb(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, const T* u,
                      const T* f, T* uout, const T* dinv, T* dvec, const double* coef, bool first, int nb,
-                     int tz, bool d_is_u, double* dot_fo, int cap, double* dot, unsigned* ctr) {
+                     int tz, bool d_is_u, double* dot_fo, int cap, double* dot, unsigned* ctr, SumRatio rt) {
   // the FP64 kernel always reads d and has no fused dots
   int nparts = 0;
   if (sizeof(T) == 4 && dot_fo && nb == 1) {
@@ -1836,7 +1839,7 @@ int launch_fine_cheb(cudaStream_t s, const LevelDims& d, const T* rhop, const ui
     nparts = (int64_t)grid.x * grid.y * grid.z <= cap ? (int)(grid.x * grid.y * grid.z) : 0;
   }
   const ChebArgs ch{dinv, dvec, coef, first ? 1 : 0, nparts ? dot_fo : nullptr,
-                    (d_is_u && sizeof(T) == 4) ? 1 : 0, dot, (nparts && dot) ? ctr : nullptr};
+                    (d_is_u && sizeof(T) == 4) ? 1 : 0, dot, (nparts && dot) ? ctr : nullptr, rt};
   if constexpr (sizeof(T) == 4) {
     if (nparts) {  // the step with the fused sums is its own instantiation
       launch_modal<T, 3>(s, d, rhop, vmask, u, f, uout, tz, nb, ch);
@@ -1849,10 +1852,11 @@ int launch_fine_cheb(cudaStream_t s, const LevelDims& d, const T* rhop, const ui
 
 template int launch_fine_cheb<double>(cudaStream_t, const LevelDims&, const double*, const uint8_t*,
                                       const double*, const double*, double*, const double*, double*,
-                                      const double*, bool, int, int, bool, double*, int, double*, unsigned*);
+                                      const double*, bool, int, int, bool, double*, int, double*, unsigned*,
+                                      SumRatio);
 template int launch_fine_cheb<float>(cudaStream_t, const LevelDims&, const float*, const uint8_t*,
                                      const float*, const float*, float*, const float*, float*, const double*,
-                                     bool, int, int, bool, double*, int, double*, unsigned*);
+                                     bool, int, int, bool, double*, int, double*, unsigned*, SumRatio);
 
 // First Chebyshev step from a zero iterate (every pre-smoothing sweep of a
 // preconditioning V-cycle starts from u = 0): K u vanishes, so r = f on the

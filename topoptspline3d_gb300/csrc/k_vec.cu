@@ -44,50 +44,88 @@ __device__ __forceinline__ double block_sum(double v) {
 // partials in index order (the order of k_finalize_sum, so the result does not
 // depend on which block finishes last) and resets the counter for the next use.
 // Saves the separate finalising launch.  ctr: one counter per stream in order.
-__device__ __forceinline__ void finish_sum(const double* partial, int nb, double* out, unsigned* ctr) {
+// One call sums K sets of partials, set k at partial + k nb, into *out[k] (null:
+// not wanted); true in thread 0 of the last block, which goes on from there.
+template <int K>
+__device__ __forceinline__ bool finish_sums(const double* partial, int nb, double* const (&out)[K], unsigned* ctr) {
   __shared__ bool last;
-  if (threadIdx.x == 0) {  // thread 0 wrote the block's partial: fence, then take a ticket
+  if (threadIdx.x == 0) {  // thread 0 wrote the block's partials: fence, then take a ticket
     __threadfence();
     last = atomicAdd(ctr, 1u) == (unsigned)(nb - 1);
     if (last) __threadfence();
   }
   __syncthreads();
-  if (!last) return;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s += __ldcg(partial + i);
-  s = block_sum(s);
-  if (threadIdx.x == 0) {
-    *out = s;
-    *ctr = 0u;
+  if (!last) return false;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (!out[k]) continue;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += __ldcg(partial + (int64_t)k * nb + i);
+    s = block_sum(s);
+    __syncthreads();  // block_sum's shared words are free again
+    if (threadIdx.x == 0) *out[k] = s;
   }
+  if (threadIdx.x == 0) *ctr = 0u;
+  return threadIdx.x == 0;
 }
 
 // Per-thread partial sums are accumulated in the vector's precision (FP32
 // vectors: a few dozen terms per thread, inside the FP32 inner solver only) and
 // combined in FP64 across threads and blocks.  With ctr the last block also
-// writes the total to out.  With skip_if_zero the whole grid does nothing while
-// *skip_if_zero is 0 (a device-side loop's first iteration).
+// writes the total to out, and the ratio after it.
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) k_dot_partial(const T* __restrict__ a, const T* __restrict__ b,
                                                              int64_t n, double* __restrict__ partial,
                                                              double* __restrict__ out = nullptr,
                                                              unsigned* __restrict__ ctr = nullptr,
-                                                             const double* __restrict__ skip_if_zero = nullptr) {
-  if (skip_if_zero && *skip_if_zero == 0.0) return;
+                                                             SumRatio rt = SumRatio{}) {
   T s = T(0);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     s += a[i] * (b ? b[i] : T(1));
   const double bs = block_sum((double)s);
   if (threadIdx.x == 0) partial[blockIdx.x] = bs;
-  if (ctr) finish_sum(partial, gridDim.x, out, ctr);
+  if (ctr) {
+    double* const outs[1] = {out};
+    if (finish_sums(partial, gridDim.x, outs, ctr)) write_ratio(rt);
+  }
 }
 
-__global__ void __launch_bounds__(RED_THREADS) k_finalize_sum(const double* __restrict__ partial, int nb,
-                                                              double* __restrict__ out) {
+// The flexible CG's r.z and z.rold (a.b and b.c) with one read of z and one
+// launch: k_dot_partial's sums in the same order.  The FP64 vectors of an outer
+// step are read once less (n = 92 k: 2 x 7.9 us -> one launch).
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) k_dot2(const T* __restrict__ a, const T* __restrict__ b,
+                                                      const T* __restrict__ c, int64_t n,
+                                                      double* __restrict__ partial, double* out_ab, double* out_bc,
+                                                      unsigned* __restrict__ ctr,
+                                                      const double* __restrict__ skip_if_zero, SumRatio rt) {
+  const bool two = !(skip_if_zero && *skip_if_zero == 0.0);  // the same in every thread of the grid
+  T s = T(0), t = T(0);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T bi = b[i];
+    s += a[i] * bi;
+    if (two) t += bi * c[i];
+  }
+  const double bs = block_sum((double)s);
+  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
+  if (two) {
+    __syncthreads();  // block_sum's shared words are free again
+    const double bt = block_sum((double)t);
+    if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = bt;
+  }
+  double* const outs[2] = {out_ab, two ? out_bc : nullptr};
+  if (finish_sums(partial, gridDim.x, outs, ctr) && two) write_ratio(rt);
+}
+
+__global__ void __launch_bounds__(RED_THREADS) k_finalize_sum(const double* __restrict__ partial, int nb, double* out,
+                                                              SumRatio rt) {
   double s = 0.0;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) s += partial[i];
   s = block_sum(s);
-  if (threadIdx.x == 0) *out = s;
+  if (threadIdx.x == 0) {
+    *out = s;
+    write_ratio(rt);
+  }
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_maxabs_partial(const double* __restrict__ a, int64_t n,
@@ -117,24 +155,30 @@ __global__ void k_finalize_max(const double* __restrict__ partial, int nb, doubl
 
 template <typename T>
 void launch_dot(cudaStream_t s, const T* a, const T* b, int64_t n, double* partial, double* out, unsigned* ctr,
-                const double* skip_if_zero) {
+                SumRatio rt) {
   const int nb = reduce_blocks(n);
   if (ctr) {
-    k_dot_partial<T><<<nb, RED_THREADS, 0, s>>>(a, b, n, partial, out, ctr, skip_if_zero);
+    k_dot_partial<T><<<nb, RED_THREADS, 0, s>>>(a, b, n, partial, out, ctr, rt);
   } else {
     k_dot_partial<T><<<nb, RED_THREADS, 0, s>>>(a, b, n, partial);
-    k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out);
+    k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out, rt);
   }
 }
 
-void launch_sum_partials(cudaStream_t s, const double* partial, int nb, double* out) {
-  k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out);
+template <typename T>
+void launch_dot2(cudaStream_t s, const T* a, const T* b, const T* c, int64_t n, double* partial, double* out_ab,
+                 double* out_bc, unsigned* ctr, const double* skip_if_zero, SumRatio rt) {
+  k_dot2<T><<<reduce_blocks(n), RED_THREADS, 0, s>>>(a, b, c, n, partial, out_ab, out_bc, ctr, skip_if_zero, rt);
+}
+
+void launch_sum_partials(cudaStream_t s, const double* partial, int nb, double* out, SumRatio rt) {
+  k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out, rt);
 }
 
 void launch_sum(cudaStream_t s, const double* a, int64_t n, double* partial, double* out) {
   const int nb = reduce_blocks(n);
   k_dot_partial<double><<<nb, RED_THREADS, 0, s>>>(a, nullptr, n, partial);
-  k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out);
+  k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, out, SumRatio{});
 }
 
 void launch_maxabs(cudaStream_t s, const double* a, int64_t n, double* partial, double* out) {
@@ -183,17 +227,6 @@ void launch_f2d_add(cudaStream_t s, const float* a, double* b, int64_t n) {
   k_f2d_add<<<nblk(n, 256), 256, 0, s>>>(a, b, n);
 }
 
-// The CG step scalars are formed once by a one-thread kernel (an FP64 division
-// per vector element is expensive on this part) and read by the vector kernels.
-// sc[out] = (sc[num] - (sub >= 0 ? sc[sub] : 0)) / sc[den]
-__global__ void k_scalar_ratio(double* sc, int num, int sub, int den, int out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) sc[out] = (sc[num] - (sub >= 0 ? sc[sub] : 0.0)) / sc[den];
-}
-
-void launch_scalar_ratio(cudaStream_t s, double* sc, int num, int sub, int den, int out) {
-  k_scalar_ratio<<<1, 32, 0, s>>>(sc, num, sub, den, out);
-}
-
 // d = z + beta d (beta = sc[beta_slot]), or d = z.  With first_if_zero the
 // choice is made on the device: d = z when *first_if_zero is 0 (an iteration
 // counter).
@@ -236,13 +269,16 @@ void launch_pcg_dir(cudaStream_t s, const T* z, T* d, const double* sc, int beta
 // in the vectors' precision, combined in FP64 in a fixed order (deterministic).
 // Each thread moves 16-byte packs (4 floats / 2 doubles) so enough bytes are in
 // flight to stream at HBM bandwidth; the tail past the last whole pack is scalar.
-
+// The last block also closes the iteration (the r.z kept for the next beta, the
+// device loop's count and test): every block has read alpha by then, and a
+// copy node and a one-thread kernel are saved per iteration.
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) k_pcg_update_rr(T* __restrict__ x, T* __restrict__ r,
                                                                T* __restrict__ rold, const T* __restrict__ d,
-                                                               const T* __restrict__ q, const double* __restrict__ sc,
-                                                               int alpha_slot, int64_t n, double* __restrict__ partial,
-                                                               int packed, double* __restrict__ rr, unsigned* __restrict__ ctr) {
+                                                               const T* __restrict__ q, double* sc, int alpha_slot,
+                                                               int rz_slot, int rzold_slot, int64_t n,
+                                                               double* __restrict__ partial, int packed, double* rr,
+                                                               unsigned* __restrict__ ctr, LoopCtl lc) {
   constexpr int W = 16 / sizeof(T);
   using P = Pack16<T, W>;
   const T alpha = (T)sc[alpha_slot];
@@ -273,31 +309,127 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update_rr(T* __restrict__ x
   }
   const double bs = block_sum((double)acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = bs;
-  if (ctr) finish_sum(partial, gridDim.x, rr, ctr);
+  double* const outs[1] = {rr};
+  if (finish_sums(partial, gridDim.x, outs, ctr)) {
+    sc[rzold_slot] = sc[rz_slot];
+    if (lc.loop) loop_step(lc, *rr);
+  }
 }
 
 template <typename T>
-void launch_pcg_update_rr(cudaStream_t s, T* x, T* r, T* rold, const T* d, const T* q, const double* sc,
-                          int alpha_slot, int64_t n, double* partial, double* rr, unsigned* ctr) {
+void launch_pcg_update_rr(cudaStream_t s, T* x, T* r, T* rold, const T* d, const T* q, double* sc,
+                          int alpha_slot, int rz_slot, int rzold_slot, int64_t n, double* partial, double* rr,
+                          unsigned* ctr, LoopCtl lc) {
   // 16-byte packs when all five vectors start on 16-byte boundaries
   const uintptr_t al = (uintptr_t)x | (uintptr_t)r | (uintptr_t)rold | (uintptr_t)d | (uintptr_t)q;
   const int nb = reduce_blocks(n);
-  k_pcg_update_rr<T><<<nb, RED_THREADS, 0, s>>>(x, r, rold, d, q, sc, alpha_slot, n, partial, (al & 15) == 0,
-                                                 rr, ctr);
-  if (!ctr) k_finalize_sum<<<1, RED_THREADS, 0, s>>>(partial, nb, rr);
+  k_pcg_update_rr<T><<<nb, RED_THREADS, 0, s>>>(x, r, rold, d, q, sc, alpha_slot, rz_slot, rzold_slot, n, partial,
+                                                 (al & 15) == 0, rr, ctr, lc);
+}
+
+// Start of an inner CG: the FP64 residual rounded to FP32, x = 0, the rounded
+// residual's squared norm (k_dot_partial's sum, term by term) and the loop's
+// start in one pass instead of a conversion, a fill, a dot and a one-thread
+// kernel that each wait for the one before (4 launches of 1.4 us and more per
+// outer step; the vector is read once instead of twice).
+__global__ void __launch_bounds__(RED_THREADS) k_inner_start(const double* __restrict__ r, float* __restrict__ r32,
+                                                             float* __restrict__ x32, int64_t n,
+                                                             double* __restrict__ partial, double* rr,
+                                                             const double* bb, unsigned* __restrict__ ctr,
+                                                             LoopCtl lc) {
+  float s = 0.f;
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float v = (float)r[i];
+    r32[i] = v;
+    x32[i] = 0.f;
+    s += v * v;
+  }
+  const double bs = block_sum((double)s);
+  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
+  double* const outs[1] = {rr};
+  if (finish_sums(partial, gridDim.x, outs, ctr)) loop_start(lc, *bb, *rr);
+}
+
+void launch_inner_start(cudaStream_t s, const double* r, float* r32, float* x32, int64_t n, double* partial,
+                        double* rr, const double* bb, unsigned* ctr, LoopCtl lc) {
+  k_inner_start<<<reduce_blocks(n), RED_THREADS, 0, s>>>(r, r32, x32, n, partial, rr, bb, ctr, lc);
+}
+
+// A power step after the operator: the block inverse, the normalisation of x
+// (applied here, the operator being linear) and both sums the step needs, x.z
+// for the Rayleigh estimate and z.z for the next normalisation.  The blocks
+// take the old norm before their ticket, so the last one may replace it.  Two
+// launches a step (with the operator) instead of four: at small levels each
+// one is a launch and a wait of 3 to 8 us for a few KB of vectors.  As many
+// blocks as vertices fill, up to the reduction's bound (a block's FP64 sums
+// cost more than the loop's own work beyond that).
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) k_power_step(int64_t nv, const T* __restrict__ dinv, bool sym,
+                                                            const T* __restrict__ x, const T* __restrict__ y,
+                                                            T* __restrict__ z, double* __restrict__ partial,
+                                                            double* nrm, double* xx, double* xz,
+                                                            unsigned* __restrict__ ctr) {
+  const double n2 = *nrm;
+  const T sc = (T)rsqrt(n2);
+  T sxz = T(0), szz = T(0);
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
+    const T r0 = y[v] * sc, r1 = y[nv + v] * sc, r2 = y[2 * nv + v] * sc;
+    T z0, z1, z2;
+    bool done = false;
+    if constexpr (sizeof(T) == 4) {
+      if (sym) {
+        const float4 a = reinterpret_cast<const float4*>(dinv)[v];
+        const float2 b = reinterpret_cast<const float2*>(dinv + 4 * nv)[v];
+        z0 = a.x * r0 + a.y * r1 + a.z * r2;
+        z1 = a.y * r0 + a.w * r1 + b.x * r2;
+        z2 = a.z * r0 + b.x * r1 + b.y * r2;
+        done = true;
+      }
+    }
+    if (!done) {
+      z0 = dinv[v] * r0 + dinv[nv + v] * r1 + dinv[2 * nv + v] * r2;
+      z1 = dinv[3 * nv + v] * r0 + dinv[4 * nv + v] * r1 + dinv[5 * nv + v] * r2;
+      z2 = dinv[6 * nv + v] * r0 + dinv[7 * nv + v] * r1 + dinv[8 * nv + v] * r2;
+    }
+    sxz += x[v] * z0 + x[nv + v] * z1 + x[2 * nv + v] * z2;
+    szz += z0 * z0 + z1 * z1 + z2 * z2;
+    z[v] = z0;
+    z[nv + v] = z1;
+    z[2 * nv + v] = z2;
+  }
+  const double b0 = block_sum((double)sxz);
+  if (threadIdx.x == 0) partial[blockIdx.x] = b0;
+  __syncthreads();  // block_sum's shared words are free again
+  const double b1 = block_sum((double)szz);
+  if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = b1;
+  double* const outs[2] = {xz, nrm};
+  if (finish_sums(partial, gridDim.x, outs, ctr)) *xx = n2;
+}
+
+template <typename T>
+void launch_power_step(cudaStream_t s, int64_t nv, const T* dinv, bool sym, const T* x, const T* y, T* z,
+                       double* partial, double* nrm, double* xx, double* xz, unsigned* ctr) {
+  const int nb = (int)std::min<int64_t>(nblk(nv, RED_THREADS), RED_MAX_BLOCKS);
+  k_power_step<T><<<nb, RED_THREADS, 0, s>>>(nv, dinv, sym, x, y, z, partial, nrm, xx, xz, ctr);
 }
 
 template void launch_pcg_update_rr<double>(cudaStream_t, double*, double*, double*, const double*, const double*,
-                                           const double*, int, int64_t, double*, double*, unsigned*);
+                                           double*, int, int, int, int64_t, double*, double*, unsigned*, LoopCtl);
 template void launch_pcg_update_rr<float>(cudaStream_t, float*, float*, float*, const float*, const float*,
-                                          const double*, int, int64_t, double*, double*, unsigned*);
-
-
-
+                                          double*, int, int, int, int64_t, double*, double*, unsigned*, LoopCtl);
+template void launch_power_step<double>(cudaStream_t, int64_t, const double*, bool, const double*, const double*,
+                                        double*, double*, double*, double*, double*, unsigned*);
+template void launch_power_step<float>(cudaStream_t, int64_t, const float*, bool, const float*, const float*, float*,
+                                       double*, double*, double*, double*, unsigned*);
 template void launch_dot<double>(cudaStream_t, const double*, const double*, int64_t, double*, double*, unsigned*,
-                                  const double*);
+                                  SumRatio);
 template void launch_dot<float>(cudaStream_t, const float*, const float*, int64_t, double*, double*, unsigned*,
-                                 const double*);
+                                 SumRatio);
+template void launch_dot2<double>(cudaStream_t, const double*, const double*, const double*, int64_t, double*, double*,
+                                  double*, unsigned*, const double*, SumRatio);
+template void launch_dot2<float>(cudaStream_t, const float*, const float*, const float*, int64_t, double*, double*,
+                                 double*, unsigned*, const double*, SumRatio);
 template void launch_fill<double>(cudaStream_t, double*, double, int64_t);
 template void launch_fill<float>(cudaStream_t, float*, float, int64_t);
 template void launch_copy<double>(cudaStream_t, const double*, double*, int64_t);

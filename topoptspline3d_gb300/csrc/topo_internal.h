@@ -173,13 +173,66 @@ struct Stream {
 template <typename T>
 void launch_fine_apply(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask,
                        const T* u, const T* f, T* out, bool residual, int nb = 1, int tz = 0);
+// A CG scalar that the block finishing a sum writes after the sum itself:
+// *out = (*num - *sub) / *den (sub may be null, and num, sub or den the sum just
+// written).  Taken there, the step's alpha and beta need no launch of their own
+// (1.4 us each inside a graph) and are divided once, not per vector element.
+struct SumRatio {
+  const double* num = nullptr;
+  const double* sub = nullptr;
+  const double* den = nullptr;
+  double* out = nullptr;  // null: no ratio
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void write_ratio(const SumRatio& q) {
+  if (q.out) *q.out = (*q.num - (q.sub ? *q.sub : 0.0)) / *q.den;
+}
+#endif
+
+// Control of a CG loop on the device through a conditional graph node (slots
+// loop[0..3]: iterations of this solve, ||b|| reference, first non-finite
+// iteration (1-based, 0 none), iterations summed over the solve).
+struct LoopCtl {
+  double* loop = nullptr;  // null: the host runs the loop
+  double rtol = 0;
+  int maxit = 0;
+  cudaGraphConditionalHandle hc = 0;
+};
+#ifdef __CUDACC__
+// Start, one thread: zero the count, take ||b|| from the squared norm bb (1 if
+// that is 0) and test ||r|| / ||b|| > rtol.
+__device__ __forceinline__ void loop_start(const LoopCtl& c, double bb, double rr) {
+  const double bo = sqrt(bb);
+  const double bn = bo > 0 ? bo : 1.0;
+  c.loop[0] = 0.0;
+  c.loop[1] = bn;
+  cudaGraphSetConditional(c.hc, (sqrt(rr) / bn > c.rtol && 0 < c.maxit) ? 1u : 0u);
+}
+// End of an iteration, one thread: count it and test again; a non-finite ||r||
+// stops the loop and is recorded.
+__device__ __forceinline__ void loop_step(const LoopCtl& c, double rr) {
+  const double it = c.loop[0] + 1.0;
+  c.loop[0] = it;
+  c.loop[3] += 1.0;
+  const double rn = sqrt(rr);
+  unsigned go = 0;
+  if (!isfinite(rn)) {
+    if (c.loop[2] == 0.0) c.loop[2] = it;
+  } else {
+    go = (rn / c.loop[1] > c.rtol && it < (double)c.maxit) ? 1u : 0u;
+  }
+  cudaGraphSetConditional(c.hc, go);
+}
+#endif
+
 // out = K u (level 0, one right-hand side) with per-CTA partial sums of u.out
 // in partial; with dot and ctr (a zeroed counter) the last CTA also writes
-// their total to *dot.  Returns the number of partials, or 0, launching
+// their total to *dot, and the ratio after it.  Returns the number of partials, or 0, launching
 // nothing, when the kernel would need more than cap partial slots.
 template <typename T>
 int launch_fine_apply_dot(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, const T* u,
-                          T* out, int tz, double* partial, int cap, double* dot = nullptr, unsigned* ctr = nullptr);
+                          T* out, int tz, double* partial, int cap, double* dot = nullptr, unsigned* ctr = nullptr,
+                          SumRatio rt = SumRatio{});
 // FP64 vectors, double-float arithmetic (k_fine_modal_df)
 void launch_fine_apply_df(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_t* vmask,
                           const double* u, const double* f, double* out, bool residual, int nb = 1, int tz = 0);
@@ -199,13 +252,13 @@ void launch_fine_diag_inv(cudaStream_t s, const LevelDims& d, const T* rhop, con
                           T* dinv);
 // FP32, one right-hand side: with dot_fo the kernel also leaves per-CTA partial
 // sums of f.uout in dot_fo, and with dot and ctr (a zeroed counter) the last
-// CTA writes their total to *dot.  Returns the number of partials, or 0 when
+// CTA writes their total to *dot, and the ratio after it.  Returns the number of partials, or 0 when
 // none were formed (FP64, a batch, or more CTAs than cap).
 template <typename T>
 int launch_fine_cheb(cudaStream_t s, const LevelDims& d, const T* rhop, const uint8_t* vmask, const T* u,
                      const T* f, T* uout, const T* dinv, T* dvec, const double* coef, bool first,
                      int nb = 1, int tz = 0, bool d_is_u = false, double* dot_fo = nullptr, int cap = 0,
-                     double* dot = nullptr, unsigned* ctr = nullptr);
+                     double* dot = nullptr, unsigned* ctr = nullptr, SumRatio rt = SumRatio{});
 template <typename T>
 void launch_stencil_cheb(cudaStream_t s, const LevelDims& d, const T* st, const T* u, const T* f, T* uout,
                          const T* dinv, T* dvec, const double* coef, bool first, int nb = 1);
@@ -263,13 +316,20 @@ void launch_dense_gemv(cudaStream_t s, int n, const T* Ainv, const T* f_soa, T* 
 
 // vectors and reductions (k_vec.cu)
 int reduce_blocks(int64_t n);
-// *out = sum of partial[0 .. nb) in index order (one CTA)
-void launch_sum_partials(cudaStream_t s, const double* partial, int nb, double* out);
+// *out = sum of partial[0 .. nb) in index order (one CTA), then the ratio
+void launch_sum_partials(cudaStream_t s, const double* partial, int nb, double* out, SumRatio rt = SumRatio{});
 // ctr (optional): a zeroed counter; the last block then writes out itself (one
-// launch).  skip_if_zero (with ctr): no work while *skip_if_zero is 0.
+// launch).  The ratio is written after the sum.
 template <typename T>
 void launch_dot(cudaStream_t s, const T* a, const T* b, int64_t n, double* partial, double* out,
-                unsigned* ctr = nullptr, const double* skip_if_zero = nullptr);
+                unsigned* ctr = nullptr, SumRatio rt = SumRatio{});
+// Both dots of a flexible CG step in one pass over b: *out_ab = a.b and
+// *out_bc = b.c, then the ratio.  While *skip_if_zero is 0 (a device loop's
+// first iteration; null: never) c is not read and *out_bc not written.
+// partial holds 2 x reduce_blocks(n).
+template <typename T>
+void launch_dot2(cudaStream_t s, const T* a, const T* b, const T* c, int64_t n, double* partial, double* out_ab,
+                 double* out_bc, unsigned* ctr, const double* skip_if_zero, SumRatio rt);
 // b == nullptr sums a.
 void launch_sum(cudaStream_t s, const double* a, int64_t n, double* partial, double* out);
 void launch_axpby(cudaStream_t s, double a, const double* x, double b, double* y, int64_t n);
@@ -280,15 +340,27 @@ void launch_copy(cudaStream_t s, const T* a, T* b, int64_t n);
 void launch_d2f(cudaStream_t s, const double* a, float* b, int64_t n);
 void launch_f2d_add(cudaStream_t s, const float* a, double* b, int64_t n);
 // PCG helpers with device-resident scalars (sc: double scalar slots)
-void launch_scalar_ratio(cudaStream_t s, double* sc, int num, int sub, int den, int out);
 template <typename T>
 void launch_pcg_dir(cudaStream_t s, const T* z, T* d, const double* sc, int beta_slot, bool first, int64_t n,
                     const double* first_if_zero = nullptr);
-// launch_pcg_update fused with rr = r.r of the updated residual (2 launches);
-// rold may be null (not kept)
+// x += alpha d, r -= alpha q and rr = r.r of the updated residual in one launch
+// (ctr: a zeroed counter); rold may be null (not kept).  Its last block closes
+// the CG iteration: sc[rzold_slot] = sc[rz_slot] and, with lc.loop, loop_step.
 template <typename T>
-void launch_pcg_update_rr(cudaStream_t s, T* x, T* r, T* rold, const T* d, const T* q, const double* sc,
-                          int alpha_slot, int64_t n, double* partial, double* rr, unsigned* ctr = nullptr);
+void launch_pcg_update_rr(cudaStream_t s, T* x, T* r, T* rold, const T* d, const T* q, double* sc,
+                          int alpha_slot, int rz_slot, int rzold_slot, int64_t n, double* partial, double* rr,
+                          unsigned* ctr, LoopCtl lc = LoopCtl{});
+// Start of an inner CG in one launch: r32 = r in FP32, x32 = 0, rr = r32.r32
+// (the FP32 launch_dot's sum) and, from its last block, loop_start with *bb.
+void launch_inner_start(cudaStream_t s, const double* r, float* r32, float* x32, int64_t n, double* partial,
+                        double* rr, const double* bb, unsigned* ctr, LoopCtl lc);
+// A power step after y = A x (n = 3 nv): z = s D^-1 y with s = 1/|x|, *xx = x.x,
+// *xz = x.z and, for the next step, *nrm = z.z; *nrm holds x.x on entry.  dinv:
+// [9][nv], or with sym the packed symmetric FP32 layout (float4 d00 d01 d02 d11
+// per vertex, then float2 d12 d22).  partial holds 2 x reduce_blocks(n).
+template <typename T>
+void launch_power_step(cudaStream_t s, int64_t nv, const T* dinv, bool sym, const T* x, const T* y, T* z,
+                       double* partial, double* nrm, double* xx, double* xz, unsigned* ctr);
 // out = sum of nb partials in a fixed order
 
 // design chain (k_design.cu)

@@ -489,29 +489,6 @@ __global__ void k_ocl_start(double* oc, const double* gmax, cudaGraphConditional
   cudaGraphSetConditional(hc, 1u);
 }
 
-// After a trial of volume *vol: the volume fraction, the new bracket and the
-// loop test of the reference (repeat while |V - vgoal| > 1e-4 and itn++ < 30,
-// at most 32 trials); the next threshold when it repeats.
-__global__ void k_ocl_step(double* oc, const double* vol, double den, double vgoal, cudaGraphConditionalHandle hc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double thres = oc[2];
-  const double V = *vol / den;
-  oc[3] = V;
-  oc[4] += 1.0;
-  double lo = oc[0], hi = oc[1];
-  if (V > vgoal) lo = thres;
-  else if (V < vgoal) hi = thres;
-  oc[0] = lo;
-  oc[1] = hi;
-  bool go = fabs(V - vgoal) > 1e-4;
-  if (go) {
-    go = oc[5] < 30.0;
-    oc[5] += 1.0;
-  }
-  if (go) oc[2] = 0.5 * (lo + hi);
-  cudaGraphSetConditional(hc, go ? 1u : 0u);
-}
-
 int read_scalars(topo_handle* h, int first, int count);
 
 // Inside a capture on h->stream: a conditional node of `type` (IF or WHILE)
@@ -2919,8 +2896,8 @@ WorstState*& handle_worst_slot(topo_handle* h) { return h->worst; }
 
 // The OC bisection of topo_oc_update as one CUDA graph: start (bracket [0,
 // max |dc|] from the device slot S_TMP), a WHILE node whose body is one trial
-// (coefficients at the threshold, their volume) closed by the bracket update
-// and loop test, and the second application when asked.  The trials, their
+// (coefficients at the threshold, their volume, whose last block takes the
+// bracket's step and sets the loop test), and the second application when asked.  The trials, their
 // thresholds and the stopping rule are the host loop's, decided on the
 // device; the trial count and final threshold are left in the OC slots.
 static int oc_bisection_graphed(topo_handle* h, const topo_oc_opts* o, int64_t nc, double den) {
@@ -2943,10 +2920,9 @@ static int oc_bisection_graphed(topo_handle* h, const topo_oc_opts* o, int64_t n
   auto body = [&](cudaGraphConditionalHandle hc) -> int {
     launch_oc_trial(h->stream, nc, h->coeff_old, h->csens, 0.0, o->damp, o->step, o->cmin, o->cmax, h->coeff,
                     h->coeff_df, oc + 2);
-    launch_trial_volume(h->stream, L.d, L.eactive, h->sd, h->coeff_df, h->cfg.min_density, h->partial,
-                        h->sc + S_TMP, h->adj1);
-    k_ocl_step<<<1, 32, 0, h->stream>>>(oc, h->sc + S_TMP, den, o->vgoal, hc);
-    count_launch(5);
+    count_launch(1 + launch_trial_volume(h->stream, L.d, L.eactive, h->sd, h->coeff_df, h->cfg.min_density,
+                                         h->partial, h->sc + S_TMP, h->adj1, h->ctr,
+                                         OcStep{oc, den, o->vgoal, hc}));
     return TOPO_OK;
   };
   auto tail = [&]() -> int {
@@ -3021,9 +2997,8 @@ int topo_oc_update(topo_handle* h, const topo_oc_opts* o, topo_oc_stats* stats) 
     thres = 0.5 * (lo + hi);
     launch_oc_trial(h->stream, nc, h->coeff_old, h->csens, thres, o->damp, o->step, o->cmin, o->cmax, h->coeff,
                     h->coeff_df);
-    launch_trial_volume(h->stream, L.d, L.eactive, h->sd, h->coeff_df, h->cfg.min_density, h->partial,
-                        h->sc + S_TMP, h->adj1);
-    count_launch(4);
+    count_launch(1 + launch_trial_volume(h->stream, L.d, L.eactive, h->sd, h->coeff_df, h->cfg.min_density,
+                                         h->partial, h->sc + S_TMP, h->adj1, h->ctr));
     CKL();
     RET(read_scalars(h, S_TMP, 1));
     V = h->hsc[S_TMP] / den;

@@ -27,18 +27,44 @@ __device__ __forceinline__ double simp_pow(double v, double p) {
 }
 
 constexpr int VOL_THREADS = 256;
+constexpr int VOL_BLOCKS = 2048;  // partial sums of a trial volume
 
-__global__ void k_sum_partials(const double* __restrict__ partial, int nb, double* __restrict__ out) {
-  __shared__ double sh[256];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s += partial[i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+// End of a trial volume: the CTA's FP64 sum r of its threads' values becomes a
+// partial, and the CTA with the last ticket adds the nb partials (in an order
+// that does not depend on which CTA is last) into *out and, in a device-side
+// bisection, takes the bracket's step.  Done here it costs the trial neither a
+// one-CTA kernel nor a one-thread one.  Every thread calls it.
+__device__ __forceinline__ void finish_volume(double s, double* partial, double* out, unsigned* ctr, const OcStep& st) {
+  __shared__ double ws[32];
+  __shared__ bool last;
+  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto cta_sum = [&](double v) {  // valid in thread 0
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) ws[w] = v;
     __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x == 0)
+      for (int q = 0; q < nw; ++q) r += ws[q];
+    return r;
+  };
+  const double r = cta_sum(s);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = r;
+    __threadfence();
+    last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    if (last) __threadfence();
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  __syncthreads();
+  if (!last) return;
+  double t = 0.0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) t += __ldcg(partial + q);
+  t = cta_sum(t);
+  if (threadIdx.x == 0) {
+    *out = t;
+    *ctr = 0u;
+    if (st.oc) oc_step(st, t);
+  }
 }
 
 // Separable evaluation, pass 1: B[z][y][i] = sum_{s,t} c[i, iy+s, iz+t] Ny[y][s] Nz[z][t]
@@ -149,7 +175,8 @@ __global__ void k_density_from_B(LevelDims d, const uint8_t* __restrict__ eactiv
 
 __global__ void __launch_bounds__(VOL_THREADS) k_volume_from_B(LevelDims d, const uint8_t* __restrict__ eactive,
                                                                SplineDev sp, const float2* __restrict__ B,
-                                                               double rho_min, double* __restrict__ partial) {
+                                                               double rho_min, double* partial, double* out,
+                                                               unsigned* ctr, OcStep st) {
   const df lo = df_from(rho_min), one(1.f, 0.f);
   df sd(0);
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < d.ne; e += (int64_t)gridDim.x * blockDim.x) {
@@ -161,17 +188,7 @@ __global__ void __launch_bounds__(VOL_THREADS) k_volume_from_B(LevelDims d, cons
     if (df_lt(one, v)) v = one;
     sd += v;
   }
-  double s = df_to(sd);
-  __shared__ double ws[VOL_THREADS / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int w = 0; w < VOL_THREADS / 32; ++w) r += ws[w];
-    partial[blockIdx.x] = r;
-  }
+  finish_volume(df_to(sd), partial, out, ctr, st);
 }
 
 // (hi, lo) float split of n doubles
@@ -182,16 +199,23 @@ __global__ void k_to_df(int64_t n, const double* __restrict__ a, float2* __restr
   b[i] = make_float2(v.hi, v.lo);
 }
 
-// Pass 1 in double-float, separable, one CTA per (element layer z, chunk of
-// SEP_Y element rows y): first C[j][i] = sum_t c[i, j, iz+t] Nz[z][t] for the
-// y-basis indices j the chunk's rows use, into shared memory, then
-// B[z][y][i] = sum_s Ny[y][s] C[iy+s][i] (0 where y or z is outside the spline
-// range).  The products and their order are those of k_spline_yz_df (inner
-// sum over t, outer over s); each coefficient is read once per CTA instead of
-// once per output.  The shared table holds cap_j y-basis rows; a chunk whose
-// rows use more (a spline partition finer than the elements) forms its
-// outputs straight from the coefficients.
-constexpr int SEP_Y = 16;
+// Both passes for a chunk of element rows in one CTA, in double-float.  A chunk
+// is up to ych rows y of an element layer z.  C[j][i] = sum_t c[i, j, iz+t]
+// Nz[z][t] for the y-basis indices j the rows use and then B[y][i] = sum_s
+// Ny[y][s] C[iy+s][i] go to shared memory (the products and their order are
+// those of k_spline_yz_df: inner sum over t, outer over s), and each thread
+// evaluates its element column x on the chunk's rows with the column's basis
+// index and weights in registers (values as spline_from_B).  The table C holds
+// cap_j y-basis rows; a chunk whose rows use more (a spline partition finer
+// than the elements) forms B straight from the coefficients.
+// B never goes to global memory and the two passes are one launch.  A trial
+// volume is bound by latency at small grids and by the double-float chains of
+// a few rows per thread at large ones: the rows of a chunk are independent, so
+// four of them are in flight per thread, with no barrier between rows.
+constexpr int ROW_MAX = 1024;  // elements of a row, one thread each
+constexpr int CHUNK_Y = 16;    // most rows of a chunk (a warp holds their y-basis indices)
+// CTAs aimed at by shortening the chunks of small grids: four on each SM
+constexpr int CHUNK_CTAS = 608;
 
 __device__ __forceinline__ df spline_yz_at(const LevelDims& d, const SplineDev& sp, const float2* __restrict__ coeff,
                                            int i, int y, int iz, const df* nz) {
@@ -210,232 +234,186 @@ __device__ __forceinline__ df spline_yz_at(const LevelDims& d, const SplineDev& 
   return v;
 }
 
-__global__ void __launch_bounds__(256) k_spline_yz_sep(LevelDims d, SplineDev sp, const float2* __restrict__ coeff,
-                                                       float2* __restrict__ B, int cap_j) {
-  extern __shared__ float2 sC[];  // [j - jlo][nb0]
-  __shared__ int sj[2];
-  const int z = blockIdx.x, y0 = blockIdx.y * SEP_Y, y1 = min(y0 + SEP_Y, d.ey);
-  const int nbx = sp.nb[0], nby = sp.nb[1], k = sp.order;
-  const int iz = sp.i0[2][z];
-  float2* Bz = B + (int64_t)nbx * d.ey * z;
-  if (iz < 0) {
-    for (int q = threadIdx.x; q < nbx * (y1 - y0); q += blockDim.x) Bz[nbx * y0 + q] = make_float2(0.f, 0.f);
-    return;
-  }
-  if (threadIdx.x == 0) {  // y-basis indices of the chunk's rows
-    int lo = nby, hi = -1;
-    for (int y = y0; y < y1; ++y) {
-      const int iy = sp.i0[1][y];
-      if (iy >= 0) { lo = min(lo, iy); hi = max(hi, iy + k - 1); }
-    }
-    sj[0] = lo;
-    sj[1] = hi;
-  }
-  __syncthreads();
-  const int jlo = sj[0], nj = sj[1] - sj[0] + 1;
-  df nz[MAX_ORDER];
-#pragma unroll
-  for (int t = 0; t < MAX_ORDER; ++t) {
-    const float2 n = t < k ? sp.Ndf[2][z * k + t] : make_float2(0.f, 0.f);
-    nz[t] = df(n.x, n.y);
-  }
-  if (nj > cap_j) {  // (uniform over the CTA)
-    for (int q = threadIdx.x; q < nbx * (y1 - y0); q += blockDim.x) {
-      const df v = spline_yz_at(d, sp, coeff, q % nbx, y0 + q / nbx, iz, nz);
-      Bz[nbx * y0 + q] = make_float2(v.hi, v.lo);
-    }
-    return;
-  }
-  for (int q = threadIdx.x; q < nbx * nj; q += blockDim.x) {
-    const int i = q % nbx, j = jlo + q / nbx;
-    df a(0);
-    for (int t = 0; t < k; ++t) {
-      const float2 c = coeff[i + (int64_t)nbx * (j + (int64_t)nby * (iz + t))];
-      a += df(c.x, c.y) * nz[t];
-    }
-    sC[q] = make_float2(a.hi, a.lo);
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < nbx * (y1 - y0); q += blockDim.x) {
-    const int i = q % nbx, y = y0 + q / nbx;
-    const int iy = sp.i0[1][y];
-    df v(0);
-    if (iy >= 0) {
-      for (int s2 = 0; s2 < k; ++s2) {
-        const float2 ns = sp.Ndf[1][y * k + s2];
-        const float2 a = sC[i + nbx * (iy - jlo + s2)];
-        v += df(ns.x, ns.y) * df(a.x, a.y);
-      }
-    }
-    Bz[nbx * y0 + q] = make_float2(v.hi, v.lo);
-  }
-}
-
-// Pass 2 one element row (y, z) at a time, one thread per element column x
-// (the CTA is the row's width rounded up to whole warps): the row's pass-1
-// values B[z][y][:] are staged in shared memory, the next row's values and
-// activity flags are loaded while this row's elements are evaluated, and each
-// thread keeps its column's basis index and weights in registers for all rows
-// (values as spline_from_B).  Rows of at most ROW_MAX elements.
-constexpr int ROW_MAX = 1024;
-
-__device__ __forceinline__ df row_value(const float2* sB, int ix, const df* nx, int k, bool in) {
-  if (!in) return df_from(-0.2);
-  df v(0);
-  for (int r = 0; r < k; ++r) {
-    const float2 bb = sB[ix + r];
-    v += nx[r] * df(bb.x, bb.y);
-  }
-  return v;
-}
-
-// MODE 0: volume partial sums (clamped values of active elements, per CTA);
+// MODE 0: volume of the clamped values of active elements (partial, *out, st);
 // MODE 1: densities rho, rho^p (FP64 and FP32) of every element.
 template <int MODE>
-__global__ void __launch_bounds__(ROW_MAX) k_spline_rows(LevelDims d, const uint8_t* __restrict__ eactive,
-                                                         SplineDev sp, const float2* __restrict__ B,
-                                                         double rho_min, double penal,
-                                                         double* __restrict__ partial, double* __restrict__ rho,
-                                                         double* __restrict__ rhop, float* __restrict__ rhop32) {
-  extern __shared__ float2 sB[];  // nb0
-  const int nbx = sp.nb[0], ex = d.ex, nrows = d.ey * d.ez, k = sp.order;
-  const int x = threadIdx.x;
+__global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const uint8_t* __restrict__ eactive,
+                                                           SplineDev sp, const float2* __restrict__ coeff, int ych,
+                                                           int cap_j, double rho_min, double penal,
+                                                           double* __restrict__ rho, double* __restrict__ rhop,
+                                                           float* __restrict__ rhop32, double* partial, double* out,
+                                                           unsigned* ctr, OcStep st) {
+  extern __shared__ float2 sC[];  // [cap_j][nb0], then B: [ych][nb0]
+  const int nbx = sp.nb[0], nby = sp.nb[1], ex = d.ex, k = sp.order;
+  float2* sB = sC + (size_t)nbx * cap_j;
+  const int x = threadIdx.x, lane = threadIdx.x & 31;
   const bool col = x < ex;
-  // the column's basis index and weights, for every row
   int ix = -1;
   df nx[MAX_ORDER];
 #pragma unroll
   for (int r = 0; r < MAX_ORDER; ++r) nx[r] = df(0);
   if (col) {
     ix = sp.i0[0][x];
-    for (int r = 0; r < k; ++r) {
-      const float2 n = sp.Ndf[0][x * k + r];
-      nx[r] = df(n.x, n.y);
-    }
-  }
-  const df lo = df_from(rho_min), one(1.f, 0.f);
-  df sd(0);
-  float2 pb[4];
-  uint8_t pa = 0;
-  auto fetch = [&](int row) {
-    const float2* b = B + (int64_t)nbx * row;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = x + q * (int)blockDim.x;
-      pb[q] = i < nbx ? b[i] : make_float2(0.f, 0.f);
-    }
-    pa = col ? eactive[x + (int64_t)ex * row] : 0;
-  };
-  int row = blockIdx.x;
-  if (row < nrows) fetch(row);
-  for (; row < nrows; row += gridDim.x) {
-    __syncthreads();  // the previous row's readers are done with sB
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = x + q * (int)blockDim.x;
-      if (i < nbx) sB[i] = pb[q];
-    }
-    const uint8_t act = pa;
-    __syncthreads();
-    if (row + (int)gridDim.x < nrows) fetch(row + gridDim.x);
-    if (!col) continue;
-    const int y = row % d.ey, z = row / d.ey;
-    const bool in = ix >= 0 && sp.i0[1][y] >= 0 && sp.i0[2][z] >= 0;
-    if (MODE == 0) {
-      if (!act) continue;
-      df v = row_value(sB, ix, nx, k, in);
-      if (df_lt(v, lo)) v = lo;
-      if (df_lt(one, v)) v = one;
-      sd += v;
-    } else {
-      const int64_t e = x + (int64_t)ex * row;
-      if (!act) {
-        rho[e] = 0.0; rhop[e] = 0.0; rhop32[e] = 0.0f;
-        continue;
+    for (int r = 0; r < MAX_ORDER; ++r)
+      if (r < k) {
+        const float2 n = sp.Ndf[0][x * k + r];
+        nx[r] = df(n.x, n.y);
       }
-      const double v = fmin(fmax(df_to(row_value(sB, ix, nx, k, in)), rho_min), 1.0);
-      const double vp = simp_pow(v, penal);
-      rho[e] = v; rhop[e] = vp; rhop32[e] = (float)vp;
+  }
+  const df lo = df_from(rho_min), one(1.f, 0.f), outside = df_from(-0.2);
+  df sd(0);
+  const int ncy = (d.ey + ych - 1) / ych, nchunk = ncy * d.ez;
+  for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
+    const int z = c / ncy, y0 = (c - z * ncy) * ych, ny = min(ych, d.ey - y0);
+    const int64_t e0 = x + (int64_t)ex * (y0 + (int64_t)d.ey * z);
+    unsigned act = 0;  // the column's activity flags, a bit per row
+    if (col) {
+#pragma unroll 4
+      for (int r = 0; r < ny; ++r) act |= (eactive[e0 + (int64_t)ex * r] ? 1u : 0u) << r;
+    }
+    const int iz = sp.i0[2][z];
+    // lane r holds row r's first y-basis index (every warp the same)
+    const int iy = lane < ny ? sp.i0[1][y0 + lane] : -1;
+    const int jlo = __reduce_min_sync(0xffffffffu, iy >= 0 ? iy : nby);
+    const int nj = __reduce_max_sync(0xffffffffu, iy >= 0 ? iy + k : jlo) - jlo;
+    df nz[MAX_ORDER];
+#pragma unroll
+    for (int t = 0; t < MAX_ORDER; ++t) {
+      const float2 n = t < k ? sp.Ndf[2][z * k + t] : make_float2(0.f, 0.f);
+      nz[t] = df(n.x, n.y);
+    }
+    __syncthreads();  // the previous chunk's readers are done
+    if (iz >= 0 && nj > cap_j) {  // (uniform over the CTA)
+      for (int q = threadIdx.x; q < nbx * ny; q += blockDim.x) {
+        const df v = spline_yz_at(d, sp, coeff, q % nbx, y0 + q / nbx, iz, nz);
+        sB[q] = make_float2(v.hi, v.lo);
+      }
+    } else if (iz >= 0) {
+      for (int q = threadIdx.x; q < nbx * nj; q += blockDim.x) {
+        const int j = q / nbx, i = q - j * nbx;
+        const float2* cq = coeff + i + (int64_t)nbx * (jlo + j + (int64_t)nby * iz);
+        df a(0);
+#pragma unroll
+        for (int t = 0; t < MAX_ORDER; ++t)
+          if (t < k) {
+            const float2 cf = cq[(int64_t)nbx * nby * t];
+            a += df(cf.x, cf.y) * nz[t];
+          }
+        sC[q] = make_float2(a.hi, a.lo);
+      }
+      __syncthreads();
+      for (int q = threadIdx.x; q < nbx * ny; q += blockDim.x) {
+        const int r = q / nbx, i = q - r * nbx, y = y0 + r;
+        const int iyr = sp.i0[1][y];
+        df v(0);
+        if (iyr >= 0) {
+          for (int s2 = 0; s2 < k; ++s2) {
+            const float2 ns = sp.Ndf[1][y * k + s2];
+            const float2 a = sC[i + nbx * (iyr - jlo + s2)];
+            v += df(ns.x, ns.y) * df(a.x, a.y);
+          }
+        }
+        sB[q] = make_float2(v.hi, v.lo);
+      }
+    }
+    __syncthreads();
+    for (int r0 = 0; r0 < ny; r0 += 4) {  // uniform: every lane takes part in the shuffles
+      df v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + q;
+        const int iyr = __shfl_sync(0xffffffffu, iy, r);  // (r < CHUNK_Y; -1 past the chunk)
+        const bool in = ix >= 0 && iz >= 0 && iyr >= 0;
+        v[q] = in ? df(0) : outside;
+        if (in) {
+          const float2* b = sB + nbx * r + ix;
+#pragma unroll
+          for (int t = 0; t < MAX_ORDER; ++t)
+            if (t < k) {
+              const float2 bb = b[t];
+              v[q] += nx[t] * df(bb.x, bb.y);
+            }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + q;
+        if (MODE == 0) {
+          if (!((act >> r) & 1u)) continue;
+          if (df_lt(v[q], lo)) v[q] = lo;
+          if (df_lt(one, v[q])) v[q] = one;
+          sd += v[q];
+        } else {
+          if (!col || r >= ny) continue;
+          const int64_t e = e0 + (int64_t)ex * r;
+          const bool on = (act >> r) & 1u;
+          const double vr = on ? fmin(fmax(df_to(v[q]), rho_min), 1.0) : 0.0;
+          const double vp = on ? simp_pow(vr, penal) : 0.0;
+          rho[e] = vr; rhop[e] = vp; rhop32[e] = (float)vp;
+        }
+      }
     }
   }
-  if (MODE != 0) return;
-  double s = df_to(sd);
-  __shared__ double ws[ROW_MAX / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += ws[w];
-    partial[blockIdx.x] = r;
-  }
+  if (MODE == 0) finish_volume(df_to(sd), partial, out, ctr, st);
 }
 
-// Pass 1 through the separable kernel when its layer table fits in shared
-// memory (returns false otherwise).
-static bool spline_yz_sep(cudaStream_t s, const LevelDims& d, const SplineDev& sp, const float2* coeff_df,
-                          float2* B) {
-  // rows of SEP_Y elements span SEP_Y + order - 1 y-basis indices when the
-  // partition is no finer than the elements (the kernel checks each chunk)
-  const int cap_j = std::min(sp.nb[1], SEP_Y + sp.order - 1);
-  const size_t smem = sizeof(float2) * (size_t)sp.nb[0] * cap_j;
-  if (sp.order > MAX_ORDER || smem > 200 * 1024) return false;
+// Rows of at most ROW_MAX elements and orders up to MAX_ORDER whose tables fit
+// in shared memory go to k_spline_chunks (returns false otherwise).  Chunks of
+// CHUNK_Y rows share the z contraction best; a grid with fewer than CHUNK_CTAS
+// of them takes shorter ones down to one row, and tables of more than 96 KB
+// (two CTAs on an SM) shorten them too.
+template <int MODE>
+static bool spline_chunks(cudaStream_t s, const LevelDims& d, const uint8_t* eactive, const SplineDev& sp,
+                          const float2* coeff_df, double rho_min, double penal, double* rho, double* rhop,
+                          float* rhop32, double* partial, double* out, unsigned* ctr, const OcStep& st) {
+  if (d.ex > ROW_MAX || sp.order > MAX_ORDER) return false;
+  int ych = (int)std::min<int64_t>(CHUNK_Y, std::max<int64_t>(1, (int64_t)d.ey * d.ez / CHUNK_CTAS));
+  auto cap = [&](int r) { return std::min(sp.nb[1], r + sp.order - 1); };
+  auto bytes = [&](int r) { return sizeof(float2) * (size_t)sp.nb[0] * (cap(r) + r); };
+  while (ych > 1 && bytes(ych) > 96 * 1024) --ych;
+  const size_t smem = bytes(ych);
+  if (smem > 200 * 1024) return false;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_spline_yz_sep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+      cudaFuncSetAttribute(k_spline_chunks<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  k_spline_yz_sep<<<dim3(d.ez, (d.ey + SEP_Y - 1) / SEP_Y), 256, smem, s>>>(d, sp, coeff_df, B, cap_j);
+  const int nb = (int)std::min<int64_t>(VOL_BLOCKS, (int64_t)((d.ey + ych - 1) / ych) * d.ez);
+  k_spline_chunks<MODE><<<nb, (d.ex + 31) / 32 * 32, smem, s>>>(d, eactive, sp, coeff_df, ych, cap(ych), rho_min,
+                                                                penal, rho, rhop, rhop32, partial, out, ctr, st);
   return true;
 }
-
-static int rows_threads(const LevelDims& d) { return std::min(ROW_MAX, (d.ex + 31) / 32 * 32); }
-
-// Rows fit the row kernel: at most ROW_MAX elements, a staged row of basis
-// values within 4 per thread, spline order at most MAX_ORDER.
-static bool rows_fit(const LevelDims& d, const SplineDev& sp) {
-  return d.ex <= ROW_MAX && sp.nb[0] <= 4 * rows_threads(d) && sp.order <= MAX_ORDER;
-}
-
-static int rows_blocks(const LevelDims& d) { return (int)std::min<int64_t>(1024, (int64_t)d.ey * d.ez); }
 
 void launch_coeff_to_density(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                              const SplineDev& sp, const double* coeff, double rho_min, double penal,
                              double* rho, double* rhop, float* rhop32, double* Btmp, float2* coeff_df) {
   const int64_t nB = (int64_t)sp.nb[0] * d.ey * d.ez;
   const int64_t nc = (int64_t)sp.nb[0] * sp.nb[1] * sp.nb[2];
-  float2* B = reinterpret_cast<float2*>(Btmp);  // nB (hi, lo) pairs in the nB-double scratch
-  bool sep = false;
   if (coeff_df) {
     k_to_df<<<nblk(nc, 256), 256, 0, s>>>(nc, coeff, coeff_df);
-    sep = spline_yz_sep(s, d, sp, coeff_df, B);
+    if (spline_chunks<1>(s, d, eactive, sp, coeff_df, rho_min, penal, rho, rhop, rhop32, nullptr, nullptr, nullptr,
+                         OcStep{}))
+      return;
   }
-  if (!sep) k_spline_yz<<<nblk(nB, 256), 256, 0, s>>>(d, sp, coeff, B);
-  if (rows_fit(d, sp))
-    k_spline_rows<1><<<rows_blocks(d), rows_threads(d), sizeof(float2) * sp.nb[0], s>>>(
-        d, eactive, sp, B, rho_min, penal, nullptr, rho, rhop, rhop32);
-  else
-    k_density_from_B<<<nblk(d.ne, 256), 256, 0, s>>>(d, eactive, sp, B, rho_min, penal, rho, rhop, rhop32);
+  float2* B = reinterpret_cast<float2*>(Btmp);  // nB (hi, lo) pairs in the nB-double scratch
+  k_spline_yz<<<nblk(nB, 256), 256, 0, s>>>(d, sp, coeff, B);
+  k_density_from_B<<<nblk(d.ne, 256), 256, 0, s>>>(d, eactive, sp, B, rho_min, penal, rho, rhop, rhop32);
 }
 
-void launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                         const SplineDev& sp, const float2* coeff_df, double rho_min, double* partial,
-                         double* out, double* Btmp) {
+int launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
+                        const SplineDev& sp, const float2* coeff_df, double rho_min, double* partial,
+                        double* out, double* Btmp, unsigned* ctr, OcStep st) {
+  if (spline_chunks<0>(s, d, eactive, sp, coeff_df, rho_min, 0.0, nullptr, nullptr, nullptr, partial, out, ctr, st))
+    return 1;
   const int64_t nB = (int64_t)sp.nb[0] * d.ey * d.ez;
   float2* B = reinterpret_cast<float2*>(Btmp);  // nB (hi, lo) pairs in the nB-double scratch
-  if (!spline_yz_sep(s, d, sp, coeff_df, B)) k_spline_yz_df<<<nblk(nB, 256), 256, 0, s>>>(d, sp, coeff_df, B);
-  int nb;
-  if (rows_fit(d, sp)) {
-    nb = rows_blocks(d);
-    k_spline_rows<0><<<nb, rows_threads(d), sizeof(float2) * sp.nb[0], s>>>(d, eactive, sp, B, rho_min, 0.0, partial,
-                                                                           nullptr, nullptr, nullptr);
-  } else {  // two elements per thread at most (up to 2048 partials)
-    nb = (int)std::min<int64_t>(2048, (d.ne + VOL_THREADS * 2 - 1) / (VOL_THREADS * 2));
-    if (nb < 1) nb = 1;
-    k_volume_from_B<<<nb, VOL_THREADS, 0, s>>>(d, eactive, sp, B, rho_min, partial);
-  }
-  k_sum_partials<<<1, 256, 0, s>>>(partial, nb, out);
+  k_spline_yz_df<<<nblk(nB, 256), 256, 0, s>>>(d, sp, coeff_df, B);
+  // two elements per thread at most
+  const int nb = (int)std::min<int64_t>(VOL_BLOCKS, (d.ne + VOL_THREADS * 2 - 1) / (VOL_THREADS * 2));
+  k_volume_from_B<<<nb < 1 ? 1 : nb, VOL_THREADS, 0, s>>>(d, eactive, sp, B, rho_min, partial, out, ctr, st);
+  return 2;
 }
 
 // Element sensitivity g_e = -p rho^(p-1) u_e^T Ke u_e (optimization/optimization.cu:96-159),

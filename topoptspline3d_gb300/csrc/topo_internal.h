@@ -391,10 +391,43 @@ void spline_tables(int order, const int* partition, const double* bmin, const do
 void launch_coeff_to_density(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                              const SplineDev& sp, const double* coeff, double rho_min, double penal,
                              double* rho, double* rhop, float* rhop32, double* Btmp, float2* coeff_df = nullptr);
+// The step of a device-side OC bisection after a trial (slots oc[0..5]: lo, hi,
+// threshold of the current trial, its volume fraction, trials, repeats), one
+// thread: the volume fraction, the new bracket and the loop test of the
+// reference (repeat while |V - vgoal| > 1e-4 and itn++ < 30, at most 32
+// trials); the next threshold when it repeats.
+struct OcStep {
+  double* oc = nullptr;  // null: the host runs the bisection
+  double den = 1, vgoal = 0;
+  cudaGraphConditionalHandle hc = 0;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void oc_step(const OcStep& s, double vol) {
+  double* oc = s.oc;
+  const double thres = oc[2];
+  const double V = vol / s.den;
+  oc[3] = V;
+  oc[4] += 1.0;
+  double lo = oc[0], hi = oc[1];
+  if (V > s.vgoal) lo = thres;
+  else if (V < s.vgoal) hi = thres;
+  oc[0] = lo;
+  oc[1] = hi;
+  bool go = fabs(V - s.vgoal) > 1e-4;
+  if (go) {
+    go = oc[5] < 30.0;
+    oc[5] += 1.0;
+  }
+  if (go) oc[2] = 0.5 * (lo + hi);
+  cudaGraphSetConditional(s.hc, go ? 1u : 0u);
+}
+#endif
 // coeff_df: the trial coefficients split into (hi, lo) floats (from launch_oc_trial)
-void launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
-                         const SplineDev& sp, const float2* coeff_df, double rho_min, double* partial,
-                         double* out, double* Btmp);
+// *out: its volume, with ctr a zeroed counter and partial 2048 doubles; st: see
+// OcStep.  Returns the kernels launched.
+int launch_trial_volume(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
+                        const SplineDev& sp, const float2* coeff_df, double rho_min, double* partial,
+                        double* out, double* Btmp, unsigned* ctr, OcStep st = OcStep{});
 // sens = -p rho^(p-1) u_e^T Ke u_e; rhop (may be null): rho^(p-1) as rhop / rho
 void launch_sensitivity(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                         const double* rho, const double* rhop, const double* u, double penal, double lam, double mu,

@@ -217,15 +217,17 @@ constexpr int CHUNK_Y = 16;    // most rows of a chunk (a warp holds their y-bas
 // CTAs aimed at by shortening the chunks of small grids: four on each SM
 constexpr int CHUNK_CTAS = 608;
 
+template <int K>
 __device__ __forceinline__ df spline_yz_at(const LevelDims& d, const SplineDev& sp, const float2* __restrict__ coeff,
                                            int i, int y, int iz, const df* nz) {
-  const int iy = sp.i0[1][y], k = sp.order, nbx = sp.nb[0];
+  const int iy = sp.i0[1][y], nbx = sp.nb[0];
   df v(0);
   if (iy < 0) return v;
-  for (int s2 = 0; s2 < k; ++s2) {
-    const float2 ns = sp.Ndf[1][y * k + s2];
+  for (int s2 = 0; s2 < K; ++s2) {
+    const float2 ns = sp.Ndf[1][y * K + s2];
     df a(0);
-    for (int t = 0; t < k; ++t) {
+#pragma unroll
+    for (int t = 0; t < K; ++t) {
       const float2 c = coeff[i + (int64_t)nbx * ((iy + s2) + (int64_t)sp.nb[1] * (iz + t))];
       a += df(c.x, c.y) * nz[t];
     }
@@ -236,30 +238,30 @@ __device__ __forceinline__ df spline_yz_at(const LevelDims& d, const SplineDev& 
 
 // MODE 0: volume of the clamped values of active elements (partial, *out, st);
 // MODE 1: densities rho, rho^p (FP64 and FP32) of every element.
-template <int MODE>
+// K: the spline order.  ip: penal as a whole number from 0 to 8, or -1.
+template <int MODE, int K>
 __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const uint8_t* __restrict__ eactive,
                                                            SplineDev sp, const float2* __restrict__ coeff, int ych,
                                                            int cap_j, double rho_min, double penal,
-                                                           double* __restrict__ rho, double* __restrict__ rhop,
+                                                           int ip, double* __restrict__ rho, double* __restrict__ rhop,
                                                            float* __restrict__ rhop32, double* partial, double* out,
                                                            unsigned* ctr, OcStep st) {
   extern __shared__ float2 sC[];  // [cap_j][nb0], then B: [ych][nb0]
-  const int nbx = sp.nb[0], nby = sp.nb[1], ex = d.ex, k = sp.order;
+  const int nbx = sp.nb[0], nby = sp.nb[1], ex = d.ex;
   float2* sB = sC + (size_t)nbx * cap_j;
   const int x = threadIdx.x, lane = threadIdx.x & 31;
   const bool col = x < ex;
   int ix = -1;
-  df nx[MAX_ORDER];
+  df nx[K];
 #pragma unroll
-  for (int r = 0; r < MAX_ORDER; ++r) nx[r] = df(0);
+  for (int r = 0; r < K; ++r) nx[r] = df(0);
   if (col) {
     ix = sp.i0[0][x];
 #pragma unroll
-    for (int r = 0; r < MAX_ORDER; ++r)
-      if (r < k) {
-        const float2 n = sp.Ndf[0][x * k + r];
-        nx[r] = df(n.x, n.y);
-      }
+    for (int r = 0; r < K; ++r) {
+      const float2 n = sp.Ndf[0][x * K + r];
+      nx[r] = df(n.x, n.y);
+    }
   }
   const df lo = df_from(rho_min), one(1.f, 0.f), outside = df_from(-0.2);
   df sd(0);
@@ -269,24 +271,25 @@ __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const ui
     const int64_t e0 = x + (int64_t)ex * (y0 + (int64_t)d.ey * z);
     unsigned act = 0;  // the column's activity flags, a bit per row
     if (col) {
-#pragma unroll 4
-      for (int r = 0; r < ny; ++r) act |= (eactive[e0 + (int64_t)ex * r] ? 1u : 0u) << r;
+#pragma unroll
+      for (int r = 0; r < CHUNK_Y; ++r)  // all in flight together
+        if (r < ny) act |= (eactive[e0 + (int64_t)ex * r] ? 1u : 0u) << r;
     }
     const int iz = sp.i0[2][z];
     // lane r holds row r's first y-basis index (every warp the same)
     const int iy = lane < ny ? sp.i0[1][y0 + lane] : -1;
     const int jlo = __reduce_min_sync(0xffffffffu, iy >= 0 ? iy : nby);
-    const int nj = __reduce_max_sync(0xffffffffu, iy >= 0 ? iy + k : jlo) - jlo;
-    df nz[MAX_ORDER];
+    const int nj = __reduce_max_sync(0xffffffffu, iy >= 0 ? iy + K : jlo) - jlo;
+    df nz[K];
 #pragma unroll
-    for (int t = 0; t < MAX_ORDER; ++t) {
-      const float2 n = t < k ? sp.Ndf[2][z * k + t] : make_float2(0.f, 0.f);
+    for (int t = 0; t < K; ++t) {
+      const float2 n = sp.Ndf[2][z * K + t];
       nz[t] = df(n.x, n.y);
     }
     __syncthreads();  // the previous chunk's readers are done
     if (iz >= 0 && nj > cap_j) {  // (uniform over the CTA)
       for (int q = threadIdx.x; q < nbx * ny; q += blockDim.x) {
-        const df v = spline_yz_at(d, sp, coeff, q % nbx, y0 + q / nbx, iz, nz);
+        const df v = spline_yz_at<K>(d, sp, coeff, q % nbx, y0 + q / nbx, iz, nz);
         sB[q] = make_float2(v.hi, v.lo);
       }
     } else if (iz >= 0) {
@@ -295,11 +298,10 @@ __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const ui
         const float2* cq = coeff + i + (int64_t)nbx * (jlo + j + (int64_t)nby * iz);
         df a(0);
 #pragma unroll
-        for (int t = 0; t < MAX_ORDER; ++t)
-          if (t < k) {
-            const float2 cf = cq[(int64_t)nbx * nby * t];
-            a += df(cf.x, cf.y) * nz[t];
-          }
+        for (int t = 0; t < K; ++t) {
+          const float2 cf = cq[(int64_t)nbx * nby * t];
+          a += df(cf.x, cf.y) * nz[t];
+        }
         sC[q] = make_float2(a.hi, a.lo);
       }
       __syncthreads();
@@ -308,8 +310,9 @@ __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const ui
         const int iyr = sp.i0[1][y];
         df v(0);
         if (iyr >= 0) {
-          for (int s2 = 0; s2 < k; ++s2) {
-            const float2 ns = sp.Ndf[1][y * k + s2];
+#pragma unroll
+          for (int s2 = 0; s2 < K; ++s2) {
+            const float2 ns = sp.Ndf[1][y * K + s2];
             const float2 a = sC[i + nbx * (iyr - jlo + s2)];
             v += df(ns.x, ns.y) * df(a.x, a.y);
           }
@@ -329,11 +332,10 @@ __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const ui
         if (in) {
           const float2* b = sB + nbx * r + ix;
 #pragma unroll
-          for (int t = 0; t < MAX_ORDER; ++t)
-            if (t < k) {
-              const float2 bb = b[t];
-              v[q] += nx[t] * df(bb.x, bb.y);
-            }
+          for (int t = 0; t < K; ++t) {
+            const float2 bb = b[t];
+            v[q] += nx[t] * df(bb.x, bb.y);
+          }
         }
       }
 #pragma unroll
@@ -348,8 +350,18 @@ __global__ void __launch_bounds__(ROW_MAX) k_spline_chunks(LevelDims d, const ui
           if (!col || r >= ny) continue;
           const int64_t e = e0 + (int64_t)ex * r;
           const bool on = (act >> r) & 1u;
-          const double vr = on ? fmin(fmax(df_to(v[q]), rho_min), 1.0) : 0.0;
-          const double vp = on ? simp_pow(vr, penal) : 0.0;
+          // clamped before the conversion: FP64 compares run on the same pipe as
+          // the conversion and the power, which bound this mode (a NaN is rho_min)
+          const double vr = !on ? 0.0 : !df_lt(lo, v[q]) ? rho_min : df_lt(v[q], one) ? df_to(v[q]) : 1.0;
+          double vp = 0.0;
+          if (on) {
+            if (ip >= 0) {
+              vp = ip > 0 ? vr : 1.0;
+              for (int p = 1; p < ip; ++p) vp *= vr;
+            } else {
+              vp = pow(vr, penal);
+            }
+          }
           rho[e] = vr; rhop[e] = vp; rhop32[e] = (float)vp;
         }
       }
@@ -367,22 +379,25 @@ template <int MODE>
 static bool spline_chunks(cudaStream_t s, const LevelDims& d, const uint8_t* eactive, const SplineDev& sp,
                           const float2* coeff_df, double rho_min, double penal, double* rho, double* rhop,
                           float* rhop32, double* partial, double* out, unsigned* ctr, const OcStep& st) {
-  if (d.ex > ROW_MAX || sp.order > MAX_ORDER) return false;
+  if (d.ex > ROW_MAX || sp.order < 2 || sp.order > MAX_ORDER) return false;
   int ych = (int)std::min<int64_t>(CHUNK_Y, std::max<int64_t>(1, (int64_t)d.ey * d.ez / CHUNK_CTAS));
   auto cap = [&](int r) { return std::min(sp.nb[1], r + sp.order - 1); };
   auto bytes = [&](int r) { return sizeof(float2) * (size_t)sp.nb[0] * (cap(r) + r); };
   while (ych > 1 && bytes(ych) > 96 * 1024) --ych;
   const size_t smem = bytes(ych);
   if (smem > 200 * 1024) return false;
+  auto* fn = sp.order == 2   ? k_spline_chunks<MODE, 2>
+             : sp.order == 3 ? k_spline_chunks<MODE, 3>
+                             : k_spline_chunks<MODE, 4>;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_spline_chunks<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess) {
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   const int nb = (int)std::min<int64_t>(VOL_BLOCKS, (int64_t)((d.ey + ych - 1) / ych) * d.ez);
-  k_spline_chunks<MODE><<<nb, (d.ex + 31) / 32 * 32, smem, s>>>(d, eactive, sp, coeff_df, ych, cap(ych), rho_min,
-                                                                penal, rho, rhop, rhop32, partial, out, ctr, st);
+  const int ip = penal >= 0.0 && penal <= 8.0 && (double)(int)penal == penal ? (int)penal : -1;
+  fn<<<nb, (d.ex + 31) / 32 * 32, smem, s>>>(d, eactive, sp, coeff_df, ych, cap(ych), rho_min, penal, ip, rho, rhop,
+                                             rhop32, partial, out, ctr, st);
   return true;
 }
 

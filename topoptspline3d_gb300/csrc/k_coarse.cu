@@ -696,8 +696,13 @@ __global__ void k_restrict(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
 // vertex, and warp 0 sums the seven partial sums in a fixed order.  Seven
 // times the threads of a vertex-per-thread gather keep the loads in flight.
 constexpr int R4_WARPS = 7;
+// FLAT asks for a warp's 49 taps together instead of a row of 7 at a time: fewer
+// waits, which is what a grid of less than two CTAs per SM spends its time on
+// (20 CTAs: 10.7 -> 8.3 us); a full chip has the loads in flight anyway and the
+// row form's shorter code wins (8 x 133 CTAs: 20 us, flat 25).
+constexpr unsigned R4_FLAT_CTAS = 304;
 
-template <typename T>
+template <typename T, bool FLAT>
 __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
                                                              T* __restrict__ fc) {
   __shared__ T part[R4_WARPS][3][32];
@@ -713,20 +718,22 @@ __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, Level
     const int dz = w - 3, fz = 4 * z + dz;
     if (fz >= 0 && fz < fd.vz) {
       const T wz = T(4 - (dz < 0 ? -dz : dz));
+      const int64_t plane = (int64_t)fd.vx * fd.vy * fz;
+#pragma unroll(FLAT ? 7 : 1)
       for (int dy = -3; dy <= 3; ++dy) {
         const int fy = 4 * y + dy;
-        if (fy < 0 || fy >= fd.vy) continue;
+        if (!FLAT && (fy < 0 || fy >= fd.vy)) continue;
+        const bool iny = fy >= 0 && fy < fd.vy;
         const T wyz = wz * T(4 - (dy < 0 ? -dy : dy));
-        const int64_t rowv = (int64_t)fd.vx * (fy + (int64_t)fd.vy * fz);
 #pragma unroll
         for (int dx = -3; dx <= 3; ++dx) {
           const int fx = 4 * x + dx;
-          if (fx < 0 || fx >= fd.vx) continue;
+          const bool in = iny && fx >= 0 && fx < fd.vx;
           const T wt = wyz * T(4 - (dx < 0 ? -dx : dx));
-          const int64_t fv = rowv + fx;
-          s0 += wt * rf[fv];
-          s1 += wt * rf[fd.nv + fv];
-          s2 += wt * rf[2 * fd.nv + fv];
+          const int64_t fv = plane + (int64_t)fd.vx * fy + fx;
+          s0 += wt * (in ? rf[fv] : T(0));
+          s1 += wt * (in ? rf[fd.nv + fv] : T(0));
+          s2 += wt * (in ? rf[2 * fd.nv + fv] : T(0));
         }
       }
     }
@@ -793,7 +800,11 @@ template <typename T>
 void launch_restrict(cudaStream_t s, const LevelDims& fine, const LevelDims& coarse, const T* rf,
                      T* fc, int nb) {
   if (coarse.factor == 4) {
-    k_restrict4<T><<<dim3(nblk(coarse.nv, 32), nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
+    const unsigned g = nblk(coarse.nv, 32);
+    if (g * (unsigned)nb < R4_FLAT_CTAS)
+      k_restrict4<T, true><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
+    else
+      k_restrict4<T, false><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
   } else {
     k_restrict<T, 2><<<dim3(nblk(coarse.nv, 128), nb), 128, 0, s>>>(fine, coarse, rf, fc);
   }

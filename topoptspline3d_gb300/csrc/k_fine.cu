@@ -194,13 +194,12 @@ __device__ __forceinline__ void wht3_bwd<df>(df g[3][8]) {
   wht_bwd<df>(g[2]);
 }
 
-// In: c[3][8] nodal values per component.  Out: c[3][8] nodal forces of pe*Ke*u.
+// Modal forces g of pe*Ke from the modal displacements c (g[i][0] = 0, and
+// c[i][0] is not read).
 template <typename T>
-__device__ __forceinline__ void modal_element(T c[3][8], T pe) {
-  wht3_fwd<T>(c);
+__device__ __forceinline__ void modal_forces(const T c[3][8], T pe, T g[3][8]) {
   const T L = modal_c<T>(0) * pe, M = modal_c<T>(1) * pe;
   const T k0 = modal_c<T>(2), k1 = modal_c<T>(3), k2 = modal_c<T>(4);
-  T g[3][8];
 #pragma unroll
   for (int i = 0; i < 3; ++i) g[i][0] = T(0);
   {  // constant part of the gradient
@@ -247,6 +246,14 @@ __device__ __forceinline__ void modal_element(T c[3][8], T pe) {
     const T kk = k2 * (L + T(4) * M);
     g[0][7] = kk * c[0][7]; g[1][7] = kk * c[1][7]; g[2][7] = kk * c[2][7];
   }
+}
+
+// In: c[3][8] nodal values per component.  Out: c[3][8] nodal forces of pe*Ke*u.
+template <typename T>
+__device__ __forceinline__ void modal_element(T c[3][8], T pe) {
+  T g[3][8];
+  wht3_fwd<T>(c);
+  modal_forces<T>(c, pe, g);
   wht3_bwd<T>(g);
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -619,19 +626,27 @@ __global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE 
 // ---------------------------------------------------------------------------
 // FP32 form with one barrier per element layer.  A CTA is TYE warps; lane i of
 // warp j computes element (i, j) of the layer and owns vertex (i, j), the
-// element's (+x, +y) corner.  The element's nodal forces are combined along x
-// with a warp shuffle (vertex column i takes the x = 1 nodes of element i and
-// the x = 0 nodes of element i + 1); the y = 1 half stays in the lane's
-// registers and the y = 0 half (6 floats) goes through a double-buffered
-// shared exchange to warp j - 1.  The owned vertex's sum for plane ez is then
-// formed in the next layer's step, after its single barrier: its own y = 1
-// part, row j + 1's exchanged y = 0 part, and the top-node part carried from
-// the layer below.  Vertex planes sit in a 4-slot ring and only the element
-// phase reads them (the owned vertex's own value is taken into registers
-// there), so the copy issued at the top of a step never lands in a plane that
-// a warp still in the previous step may read.
-// Against the 2-barrier form: a quarter of the shared-memory traffic per
-// element, half the barriers.
+// element's (+x, +y) corner.  The kernel is bound by instruction issue (75% of
+// the slots at 256x128x128), so the transforms are split between layers: a
+// vertex plane's x-y modes are formed once and kept for the layer above it, and
+// the z = 1 forces of a layer wait as x-y modes (each lane its own, in shared
+// memory) for the z = 0 forces of the next, so the inverse x-y transform, the x
+// combine and the y exchange run once per vertex plane and not once per layer
+// and side.  Per plane: the x nodes, combined along x with a warp shuffle
+// (vertex column i takes the x = 1 nodes of element i and the x = 0 nodes of
+// element i + 1), then y: the y = 1 half stays in the lane's registers and the
+// y = 0 half (3 floats) goes through a double-buffered shared exchange to warp
+// j - 1.  The owned vertex's sum for plane ez is formed in the next layer's
+// step, after its single barrier: its own y = 1 part and row j + 1's exchanged
+// y = 0 part.  Vertex planes sit in a 4-slot ring and only the element phase
+// reads them (the owned vertex's own value is taken out there), so the copy
+// issued at the top of a step never lands in a plane that a warp still in the
+// previous step may read.
+// At 256x128x128 against whole transforms per layer: operator 96.6 -> 82.2 us,
+// residual 82.3 -> 76.8, Chebyshev step 100.6 -> 98.8 (its vertex operands are
+// another 200 MB).  Tried on the Chebyshev step: its operands by cp.async into a
+// per-lane slot 122 us (4-byte copies); the block inverse asked for before the
+// barrier 98.2 us, but 54.8 against 53.5 us at 8 x 96x48x48.
 // ---------------------------------------------------------------------------
 // Owned vertex (gx, gy) of the FP32 kernel over void planes [pa, pb): the
 // output of MODE for zero forces (kept out of line: inlined, its live values
@@ -673,12 +688,37 @@ __device__ __noinline__ void fine32_void_planes(const LevelDims& d, const uint8_
   }
 }
 
-template <int TYE>
+// The x-y modes (1, X, Y, XY) of a vertex plane's four values at an element:
+// components 0 and 1 in the lanes of p, component 2 in q.
+struct PlaneModes {
+  float2 p[4];
+  float q[4];
+};
+__device__ __forceinline__ void plane_modes(const float4* pl, int px, PlaneModes& m) {
+  const float2 m1 = make_float2(-1.f, -1.f);
+  const float4 a = pl[0], b = pl[1], c = pl[px], e = pl[px + 1];
+  const float2 pa = make_float2(a.x, a.y), pb = make_float2(b.x, b.y), pc = make_float2(c.x, c.y),
+               pd = make_float2(e.x, e.y);
+  const float2 s0 = __fadd2_rn(pa, pb), d0 = __ffma2_rn(pa, m1, pb), s1 = __fadd2_rn(pc, pd),
+               d1 = __ffma2_rn(pc, m1, pd);
+  m.p[0] = __fadd2_rn(s0, s1);
+  m.p[1] = __fadd2_rn(d0, d1);
+  m.p[2] = __ffma2_rn(s0, m1, s1);
+  m.p[3] = __ffma2_rn(d0, m1, d1);
+  const float t0 = a.z + b.z, e0 = b.z - a.z, t1 = c.z + e.z, e1 = e.z - c.z;
+  m.q[0] = t0 + t1;
+  m.q[1] = e0 + e1;
+  m.q[2] = t1 - t0;
+  m.q[3] = e1 - e0;
+}
+
+template <int TYE, bool DOTS>
 struct Modal32Smem {
   static constexpr int TXE = 32, NT = TXE * TYE, PX = TXE + 1, PY = TYE + 1, NP = PX * PY;
   float4 plane[4][NP];  // vertex planes (u0, u1, u2, -) in a 4-slot ring
-  float4 xa[2][NT];     // exchanged y = 0 forces: (z = 0: c0, c1, c2; z = 1: c0)
-  float2 xb[2][NT];     //                         (z = 1: c1, c2)
+  float4 xa[2][NT];     // exchanged y = 0 forces of a vertex plane (c0, c1, c2, -)
+  float4 top[3][NT];    // per component, x-y modes of the last layer's z = 1 forces (each lane its own)
+  float4 uo[DOTS ? NT : 1];  // MODE 3: the owned vertex's value at the last layer's lower plane (each lane its own)
   float coef[2];        // Chebyshev (c_old, c_new), read after each plane's barrier
 };
 
@@ -693,7 +733,7 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   // ne below 2^31), one instruction per address instead of two.
   constexpr bool CHEB = MODE >= 2, DOTS = MODE == 3;
   using I = typename std::conditional<I32, int, int64_t>::type;
-  using S = Modal32Smem<TYE>;
+  using S = Modal32Smem<TYE, DOTS>;
   constexpr int TXE = 32, NT = S::NT, PX = S::PX, NP = S::NP;
   extern __shared__ __align__(16) unsigned char m32_smem[];
   S& sm = *reinterpret_cast<S*>(m32_smem);
@@ -765,9 +805,8 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
       for (int c = 0; c < 3; ++c) dv_n[c] = dvin[c * nv + v];
     }
   };
-  float own1[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};  // own y = 1 forces of the last layer, z = 0 / 1
-  float top[3] = {0.f, 0.f, 0.f};                          // z = 1 forces of the layer below the last
-  float uo[3] = {0.f, 0.f, 0.f};                           // owned vertex's own value at the last layer's plane
+  float own1[3] = {0.f, 0.f, 0.f};  // own y = 1 forces at the last layer's lower plane
+  float uo[3] = {0.f, 0.f, 0.f};    // owned vertex's own value at the last layer's plane
   float dsum = 0.f;
   if (VOID && (zb0 < z0 || zend < zb1)) {  // void planes: the step's output for zero forces
     if (CHEB) __syncthreads();      // the step coefficients in shared memory
@@ -777,10 +816,13 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
     }
   }
   float pe_n = load_pe(z0 - 1);
+  PlaneModes lm;  // x-y modes of plane st
   if (z0 < zend) {
     prefetch(z0 - 1);
     prefetch(z0);
-    // step st: finish vertex plane st - 1 (layers st - 2, st - 1), then compute element layer st
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sm.top[c][t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // step st: finish vertex plane st - 1 (its forces left by layer st - 1), then compute element layer st
     for (int st = z0 - 1; st <= zend; ++st) {
       prefetch(st + 2);
       const float pe = pe_n;
@@ -793,21 +835,18 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
       cp_async_wait1();
       __syncthreads();
       // ---- vertex plane p = st - 1
-      if (st >= z0) {
-        const int p = st - 1, xs = (st - 1) & 1;
-        float y[3];
+      if (st > z0) {
+        const int p = st - 1;
         if (own) {
-          const float4 ra = sm.xa[xs][t + TXE];
-          const float2 rb = sm.xb[xs][t + TXE];
-          const float r0[3] = {ra.x, ra.y, ra.z}, r1[3] = {ra.w, rb.x, rb.y};
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            y[c] = top[c] + (own1[0][c] + r0[c]);
-            top[c] = own1[1][c] + r1[c];
-          }
-          if (p >= z0) {
+          const float4 ra = sm.xa[p & 1][t + TXE];
+          const float y[3] = {own1[0] + ra.x, own1[1] + ra.y, own1[2] + ra.z};
+          {
             const I v = gx + (I)d.vx * (gy + (I)d.vy * p);
             const uint8_t m = vm_c;
+            if (DOTS) {
+              const float4 q = sm.uo[t];
+              uo[0] = q.x; uo[1] = q.y; uo[2] = q.z;
+            }
             const float uv[3] = {uo[0], uo[1], uo[2]};
             if (!CHEB) {
 #pragma unroll
@@ -841,38 +880,46 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
       if (st < zend) {
         if (CHEB || (MODE == 0 && ch.dotp)) {
           const float4 q = sm.plane[(st + 4) & 3][(i + 1) + PX * (j + 1)];
-          uo[0] = q.x; uo[1] = q.y; uo[2] = q.z;
+          if (DOTS) sm.uo[t] = q;  // (in registers across the barrier these three spilled)
+          else { uo[0] = q.x; uo[1] = q.y; uo[2] = q.z; }
         }
-        float c[3][8];
+        const int k0 = i + PX * j;
+        if (st == z0 - 1) plane_modes(sm.plane[(st + 4) & 3] + k0, PX, lm);
+        PlaneModes um;
+        plane_modes(sm.plane[(st + 5) & 3] + k0, PX, um);
+        const float2 m1 = make_float2(-1.f, -1.f);
+        float g[3][8];
         if (pe != 0.f) {
+          float c[3][8];
 #pragma unroll
-          for (int a = 0; a < 8; ++a) {
-            const int k = (i + (a & 1)) + PX * (j + ((a >> 1) & 1));
-            const float4 q = sm.plane[(st + (a >> 2) + 4) & 3][k];
-            c[0][a] = q.x; c[1][a] = q.y; c[2][a] = q.z;
+          for (int a = 0; a < 4; ++a) {
+            const float2 sp = __fadd2_rn(lm.p[a], um.p[a]), dp = __ffma2_rn(lm.p[a], m1, um.p[a]);
+            c[0][a] = sp.x; c[1][a] = sp.y; c[2][a] = lm.q[a] + um.q[a];
+            c[0][a + 4] = dp.x; c[1][a + 4] = dp.y; c[2][a + 4] = um.q[a] - lm.q[a];
           }
-          modal_element<float>(c, pe);
+          modal_forces<float>(c, pe, g);
         } else {
 #pragma unroll
-          for (int a = 0; a < 8; ++a) c[0][a] = c[1][a] = c[2][a] = 0.f;
+          for (int a = 0; a < 8; ++a) g[0][a] = g[1][a] = g[2][a] = 0.f;
         }
-        // x combine: vertex column i takes the x = 1 nodes of element i and the
-        // x = 0 nodes of element i + 1 (lane 31's column is not owned)
-        float xc[2][2][3];  // [y bit][z bit][component]
+        lm = um;
+        // plane st: the layer's z = 0 forces on top of the layer below's z = 1
+        // forces, both as x-y modes; then x (nodes and the combine across
+        // lanes: vertex column i takes the x = 1 nodes of element i and the x = 0
+        // nodes of element i + 1, lane 31's column is not owned), then y
+        float y0f[3];
 #pragma unroll
-        for (int yb = 0; yb < 2; ++yb)
-#pragma unroll
-          for (int zb = 0; zb < 2; ++zb)
-#pragma unroll
-            for (int cc = 0; cc < 3; ++cc)
-              xc[yb][zb][cc] = c[cc][1 + 2 * yb + 4 * zb] +
-                               __shfl_down_sync(0xffffffffu, c[cc][2 * yb + 4 * zb], 1);
-#pragma unroll
-        for (int zb = 0; zb < 2; ++zb)
-#pragma unroll
-          for (int cc = 0; cc < 3; ++cc) own1[zb][cc] = xc[1][zb][cc];
-        sm.xa[st & 1][t] = make_float4(xc[0][0][0], xc[0][0][1], xc[0][0][2], xc[0][1][0]);
-        sm.xb[st & 1][t] = make_float2(xc[0][1][1], xc[0][1][2]);
+        for (int cc = 0; cc < 3; ++cc) {
+          const float4 tp = sm.top[cc][t];
+          const float G0 = tp.x - g[cc][4], G1 = (tp.y + g[cc][1]) - g[cc][5], G2 = (tp.z + g[cc][2]) - g[cc][6],
+                      G3 = (tp.w + g[cc][3]) - g[cc][7];
+          sm.top[cc][t] = make_float4(g[cc][4], g[cc][1] + g[cc][5], g[cc][2] + g[cc][6], g[cc][3] + g[cc][7]);
+          const float X0 = (G0 + G1) + __shfl_down_sync(0xffffffffu, G0 - G1, 1);
+          const float X1 = (G2 + G3) + __shfl_down_sync(0xffffffffu, G2 - G3, 1);
+          own1[cc] = X0 + X1;
+          y0f[cc] = X0 - X1;
+        }
+        sm.xa[st & 1][t] = make_float4(y0f[0], y0f[1], y0f[2], 0.f);
       }
     }
   }
@@ -1691,7 +1738,7 @@ dim3 modal_grid(const LevelDims& d, int tz, int nb) {
 template <int ROWS, int MODE, bool VOID>
 void launch_modal32_rows(cudaStream_t s, const LevelDims& d, const float* rhop, const uint8_t* vmask, const float* u,
                          const float* f, float* out, const ZSplit& zs, const dim3& grid, const ChebArgs& ch) {
-  const size_t smem = sizeof(Modal32Smem<ROWS>);
+  const size_t smem = sizeof(Modal32Smem<ROWS, MODE == 3>);
   static PerDeviceOnce once;
   once_per_device(once, [smem] {
     cudaError_t e = cudaFuncSetAttribute(k_fine_modal32<ROWS, MODE, true, VOID>,

@@ -1731,7 +1731,8 @@ dim3 modal_grid(const LevelDims& d, int tz, int nb) {
   const int rows = modal_rows<T>(d, tz);
   const int xs = modal_tc<T>(d, tz) ? MODAL_TXE - 2 : MODAL_TXE - 1;  // owned vertex columns per CTA
   const int gx = (d.vx + xs - 1) / xs, gy = (d.vy + rows - 2) / (rows - 1);
-  return dim3(gx, gy, fine_zblocks(d.vz, modal_depth(tz), (int64_t)gx * gy * nb) * nb);
+  const int resident = modal_tc<T>(d, tz) ? 0 : (sizeof(T) == 4 ? TOPO_FINE32_THREADS_PER_SM : 512) / (MODAL_TXE * rows);
+  return dim3(gx, gy, fine_zblocks(d.vz, modal_depth(tz), (int64_t)gx * gy * nb, resident) * nb);
 }
 
 // One launch of the FP32 modal kernel with a CTA tile of ROWS element rows.
@@ -1848,7 +1849,7 @@ static void launch_fine_apply_df_v(cudaStream_t s, const LevelDims& d, const dou
                                    const double* u, const double* f, double* out, bool residual, int nb, int tz) {
   if (tz <= 0) tz = MODAL_TZ;
   const int gx = (d.vx + MODAL_TXE - 2) / (MODAL_TXE - 1), gy = (d.vy + MODAL_TYE - 2) / (MODAL_TYE - 1);
-  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz, (int64_t)gx * gy * nb));
+  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz, (int64_t)gx * gy * nb, 0));
   const dim3 grid(gx, gy, zs.n * nb);
   constexpr int NT = MODAL_TXE * MODAL_TYE;
   const size_t smem = sizeof(DfSmem<MODAL_TXE, MODAL_TYE>);

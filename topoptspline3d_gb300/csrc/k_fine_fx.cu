@@ -34,6 +34,7 @@ void upload_fx(double lam, double mu, double h) {
 
 namespace {
 
+constexpr int FX_CTAS = 2;  // resident on an SM (128 registers a thread)
 constexpr int TX = FINE_TILE_X, TY = FINE_TILE_Y, NT = TX * TY, PX = TX + 1, NP = PX * (TY + 1);
 constexpr int KS = (NP + NT - 1) / NT;  // vertices of a plane a thread stages
 
@@ -61,7 +62,7 @@ struct FxCheb {
 
 // MODE 0: out = K u, 1: out = f - K u, 2: Chebyshev step
 template <int MODE, bool VOID>
-__global__ void __launch_bounds__(NT, 2) k_fine_fx(LevelDims d, const double* __restrict__ rhop,
+__global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const double* __restrict__ rhop,
                                                    const uint8_t* __restrict__ vmask, const double* __restrict__ u,
                                                    const double* __restrict__ f, double* __restrict__ out, ZSplit zs,
                                                    FxCheb ch) {
@@ -288,7 +289,7 @@ void launch(cudaStream_t s, const LevelDims& d, const double* rhop, const uint8_
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSmem));
   });
   const int gx = (d.vx + TX - 2) / (TX - 1), gy = (d.vy + TY - 2) / (TY - 1);
-  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz > 0 ? tz : 16, (int64_t)gx * gy * nb));
+  const ZSplit zs(d.vz, fine_zblocks(d.vz, tz > 0 ? tz : 16, (int64_t)gx * gy * nb, FX_CTAS));
   fn<<<dim3(gx, gy, zs.n * nb), NT, sizeof(FxSmem), s>>>(d, rhop, vmask, u, f, out, zs, ch);
 }
 

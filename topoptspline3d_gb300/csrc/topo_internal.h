@@ -76,19 +76,39 @@ inline int fine_rows_flag(int rows) {
 }
 
 // z blocks of the fine z-marching kernels over `tiles` columns of CTAs (all
-// right-hand sides): vz / tz of them, more where that leaves the chip idle, up
-// to two CTAs on each of the 152 SMs or one plane a block.  A block of few
-// planes recomputes the element layer below it, but a march costs 2 to 5 us a
-// plane whatever the grid (16x8x8: FP32 step 11.9 us with 4 planes a block,
+// right-hand sides): about vz / tz of them, more where that leaves the chip
+// idle, up to two CTAs on each of the 152 SMs or one plane a block.  A block of
+// few planes recomputes the element layer below it, but a march costs 2 to 5 us
+// a plane whatever the grid (16x8x8: FP32 step 11.9 us with 4 planes a block,
 // 8.1 with 1; fixed-point step 30.5 / 14.1; 77x44x42 with 304 CTAs 38 us, with
 // 441 43 us).  The planes are dealt evenly (ZSplit); a last block that takes
 // the remainder of vz / tz marches up to twice as long as the others (77x44x42,
 // 4 planes: 57 us).
+// Fewer blocks, down to 2/5 of vz / tz, where the last wave of CTAs would be
+// nearly empty (`resident` CTAs of the kernel on an SM; 0: as many as said).
+// The estimate: a wave of full SMs costs its planes and the two steps more that
+// a block marches, one with k of `resident` CTAs on an SM 0.4 + 0.6 k / resident
+// of that (a march alone on an SM is bound by latency).  It orders the measured
+// counts: FP32 Chebyshev step at 256x128x128 with 16 blocks (4.5 waves) 104 us,
+// 14 (3.9) 102, 7 (1.97) 98, 6 (1.7) 107, 4 (1.1) 126; at 159x79x77 with 9
+// (1.07) 36.8, 8 (0.95) 32.9, 7 (0.83) 35.7.  Outputs do not depend on the split.
 constexpr int FINE_FILL_CTAS = 304;
-inline int fine_zblocks(int vz, int tz, int64_t tiles) {
-  const int64_t by_depth = vz / tz > 1 ? vz / tz : 1, fill = FINE_FILL_CTAS / (tiles > 0 ? tiles : 1);
+inline int fine_zblocks(int vz, int tz, int64_t tiles, int resident) {
+  if (tiles < 1) tiles = 1;
+  const int64_t by_depth = vz / tz > 1 ? vz / tz : 1, fill = FINE_FILL_CTAS / tiles;
   const int64_t most = fill < vz ? fill : vz;
-  return (int)(by_depth > most ? by_depth : most);
+  const int64_t hi = by_depth > most ? by_depth : most;
+  if (resident <= 0) return (int)hi;
+  const int64_t shallow = (2 * by_depth + 4) / 5, lo = shallow > most ? shallow : most;
+  auto cost = [&](int64_t n) {
+    const int64_t ctas = tiles * n, slots = (int64_t)152 * resident, rem = ctas % slots;
+    const double last = rem ? 0.4 + 0.6 * (double)((rem + 151) / 152) / resident : 0.0;
+    return ((double)(ctas / slots) + last) * (double)((vz + n - 1) / n + 2);
+  };
+  int64_t best = hi;
+  for (int64_t n = hi - 1; n >= lo; --n)
+    if (cost(n) < cost(best)) best = n;
+  return (int)best;
 }
 // n blocks of vz planes: the first r of them have q + 1, the others q (worked
 // out on the host: a division in the FP32 kernel costs it a register, and the

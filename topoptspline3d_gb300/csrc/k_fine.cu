@@ -24,14 +24,11 @@ __device__ __forceinline__ float ke<float>(int i) { return cKe32[i]; }
 
 // Modal constants: lambda, mu, k0 = h/16, k1 = h/48, k2 = h/144 (see k_fine_modal).
 __constant__ double cModal64[5];
-__constant__ float cModal32[5];
 
 template <typename T>
 __device__ __forceinline__ T modal_c(int i);
 template <>
 __device__ __forceinline__ double modal_c<double>(int i) { return cModal64[i]; }
-template <>
-__device__ __forceinline__ float modal_c<float>(int i) { return cModal32[i]; }
 
 // Modal constants split into hi + lo floats.
 __constant__ float2 cModalDF[5];
@@ -41,21 +38,30 @@ __device__ __forceinline__ df modal_c<df>(int i) {
   return df(c.x, c.y);
 }
 
+// Products of the modal constants for the FP32 kernel, split into hi + lo floats:
+// lambda k0, mu k0 (= 3 mu k1), lambda k1, mu k1, (lambda + 4 mu) k2.
+__constant__ float2 cModalP[5];
+
 void upload_template(const double* Ke576, double lam, double mu, double h) {
   float k32[576];
   for (int i = 0; i < 576; ++i) k32[i] = (float)Ke576[i];
   cudaMemcpyToSymbol(cKe64, Ke576, sizeof(double) * 576);
   cudaMemcpyToSymbol(cKe32, k32, sizeof(float) * 576);
   const double m64[5] = {lam, mu, h / 16.0, h / 48.0, h / 144.0};
-  const float m32[5] = {(float)m64[0], (float)m64[1], (float)m64[2], (float)m64[3], (float)m64[4]};
   cudaMemcpyToSymbol(cModal64, m64, sizeof(m64));
-  cudaMemcpyToSymbol(cModal32, m32, sizeof(m32));
   float2 mdf[5];
   for (int i = 0; i < 5; ++i) {
     mdf[i].x = (float)m64[i];
     mdf[i].y = (float)(m64[i] - (double)mdf[i].x);
   }
   cudaMemcpyToSymbol(cModalDF, mdf, sizeof(mdf));
+  const double p[5] = {lam * h / 16.0, mu * h / 16.0, lam * h / 48.0, mu * h / 48.0, (lam + 4.0 * mu) * h / 144.0};
+  float2 pf[5];
+  for (int i = 0; i < 5; ++i) {
+    pf[i].x = (float)p[i];
+    pf[i].y = (float)(p[i] - (double)pf[i].x);
+  }
+  cudaMemcpyToSymbol(cModalP, pf, sizeof(pf));
   upload_fx(lam, mu, h);
 }
 
@@ -96,11 +102,7 @@ __device__ __forceinline__ void wht_bwd(T v[8]) {
       }
 }
 
-// The transforms of the three displacement components.  FP32: components 0
-// and 1 go through the packed two-lane FP32 instructions of sm_100 and later
-// (__fadd2_rn, __ffma2_rn; per lane the same rounding as the scalar forms, so
-// the results are identical), which halves their instruction count in an
-// issue-bound kernel.
+// The transforms of the three displacement components.
 template <typename T>
 __device__ __forceinline__ void wht3_fwd(T c[3][8]) {
   wht_fwd<T>(c[0]); wht_fwd<T>(c[1]); wht_fwd<T>(c[2]);
@@ -109,45 +111,6 @@ template <typename T>
 __device__ __forceinline__ void wht3_bwd(T g[3][8]) {
   wht_bwd<T>(g[0]); wht_bwd<T>(g[1]); wht_bwd<T>(g[2]);
 }
-template <>
-__device__ __forceinline__ void wht3_fwd<float>(float c[3][8]) {
-  const float2 m1 = make_float2(-1.f, -1.f);
-  float2 p[8];
-#pragma unroll
-  for (int a = 0; a < 8; ++a) p[a] = make_float2(c[0][a], c[1][a]);
-#pragma unroll
-  for (int hb = 1; hb < 8; hb <<= 1)
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (!(i & hb)) {
-        const float2 a = p[i], b = p[i | hb];
-        p[i] = __fadd2_rn(a, b);
-        p[i | hb] = __ffma2_rn(a, m1, b);  // b - a
-      }
-#pragma unroll
-  for (int a = 0; a < 8; ++a) { c[0][a] = p[a].x; c[1][a] = p[a].y; }
-  wht_fwd<float>(c[2]);
-}
-template <>
-__device__ __forceinline__ void wht3_bwd<float>(float g[3][8]) {
-  const float2 m1 = make_float2(-1.f, -1.f);
-  float2 p[8];
-#pragma unroll
-  for (int a = 0; a < 8; ++a) p[a] = make_float2(g[0][a], g[1][a]);
-#pragma unroll
-  for (int hb = 1; hb < 8; hb <<= 1)
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (!(i & hb)) {
-        const float2 a = p[i], b = p[i | hb];
-        p[i] = __ffma2_rn(b, m1, a);  // a - b
-        p[i | hb] = __fadd2_rn(a, b);
-      }
-#pragma unroll
-  for (int a = 0; a < 8; ++a) { g[0][a] = p[a].x; g[1][a] = p[a].y; }
-  wht_bwd<float>(g[2]);
-}
-
 // Double-float: components 0 and 1 in the lanes of df2.
 template <>
 __device__ __forceinline__ void wht3_fwd<df>(df c[3][8]) {
@@ -246,6 +209,41 @@ __device__ __forceinline__ void modal_forces(const T c[3][8], T pe, T g[3][8]) {
     const T kk = k2 * (L + T(4) * M);
     g[0][7] = kk * c[0][7]; g[1][7] = kk * c[1][7]; g[2][7] = kk * c[2][7];
   }
+}
+
+// modal_forces in FP32 with the parts that act on one mode added up first: mode
+// XY gets lambda k1 tr + 3 mu k1 c (3 k1 = k0) from the X and Y parts together, and the
+// three shear terms of modes XY, XZ, YZ share one sum.  About 20 operations
+// fewer than part by part.  Each product of pe and the constants is rounded
+// once (a rounding there scales a whole element's forces): the operator's error
+// against FP64 on random displacements is 6.6e-8, 7.0e-8 part by part with the
+// forces summed at the nodes and 7.3e-8 with them summed as modes.
+__device__ __forceinline__ void modal_forces32(const float c[3][8], float pe, float g[3][8]) {
+  auto times = [&](int i) { return fmaf(pe, cModalP[i].x, pe * cModalP[i].y); };
+  const float L0 = times(0), M0 = times(1), L1 = times(2), M1 = times(3), K7 = times(4);
+  const float M02 = 2.f * M0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) g[i][0] = 0.f;
+  const float t0 = L0 * (c[0][1] + c[1][2] + c[2][4]);
+  g[0][1] = fmaf(M02, c[0][1], t0);
+  g[1][2] = fmaf(M02, c[1][2], t0);
+  g[2][4] = fmaf(M02, c[2][4], t0);
+  g[0][2] = g[1][1] = M0 * (c[0][2] + c[1][1]);
+  g[0][4] = g[2][1] = M0 * (c[0][4] + c[2][1]);
+  g[1][4] = g[2][2] = M0 * (c[1][4] + c[2][2]);
+  const float tx = L1 * (c[1][3] + c[2][5]), ty = L1 * (c[0][3] + c[2][6]), tz = L1 * (c[0][5] + c[1][6]);
+  g[1][3] = fmaf(M0, c[1][3], tx);
+  g[2][5] = fmaf(M0, c[2][5], tx);
+  g[0][3] = fmaf(M0, c[0][3], ty);
+  g[2][6] = fmaf(M0, c[2][6], ty);
+  g[0][5] = fmaf(M0, c[0][5], tz);
+  g[1][6] = fmaf(M0, c[1][6], tz);
+  const float sh = c[0][6] + c[1][5] + c[2][3];
+  g[2][3] = M1 * (sh + c[2][3]);
+  g[1][5] = M1 * (sh + c[1][5]);
+  g[0][6] = M1 * (sh + c[0][6]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) g[i][7] = K7 * c[i][7];
 }
 
 // In: c[3][8] nodal values per component.  Out: c[3][8] nodal forces of pe*Ke*u.
@@ -644,7 +642,8 @@ __global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE 
 // previous step may read.
 // At 256x128x128 against whole transforms per layer: operator 96.6 -> 82.2 us,
 // residual 82.3 -> 76.8, Chebyshev step 100.6 -> 98.8 (its vertex operands are
-// another 200 MB).  Tried on the Chebyshev step: its operands by cp.async into a
+// another 200 MB); with modal_forces32 and the z blocks of fine_zblocks 73.4,
+// 70.3 and 93.8 us.  Tried on the Chebyshev step: its operands by cp.async into a
 // per-lane slot 122 us (4-byte copies); the block inverse asked for before the
 // barrier 98.2 us, but 54.8 against 53.5 us at 8 x 96x48x48.
 // ---------------------------------------------------------------------------
@@ -689,7 +688,9 @@ __device__ __noinline__ void fine32_void_planes(const LevelDims& d, const uint8_
 }
 
 // The x-y modes (1, X, Y, XY) of a vertex plane's four values at an element:
-// components 0 and 1 in the lanes of p, component 2 in q.
+// components 0 and 1 in the lanes of p, component 2 in q.  The packed two-lane
+// FP32 instructions of sm_100 and later (__fadd2_rn, __ffma2_rn) round as the
+// scalar forms and take one issue slot for two.
 struct PlaneModes {
   float2 p[4];
   float q[4];
@@ -897,7 +898,7 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
             c[0][a] = sp.x; c[1][a] = sp.y; c[2][a] = lm.q[a] + um.q[a];
             c[0][a + 4] = dp.x; c[1][a + 4] = dp.y; c[2][a + 4] = um.q[a] - lm.q[a];
           }
-          modal_forces<float>(c, pe, g);
+          modal_forces32(c, pe, g);
         } else {
 #pragma unroll
           for (int a = 0; a < 8; ++a) g[0][a] = g[1][a] = g[2][a] = 0.f;
@@ -911,8 +912,8 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc) {
           const float4 tp = sm.top[cc][t];
-          const float G0 = tp.x - g[cc][4], G1 = (tp.y + g[cc][1]) - g[cc][5], G2 = (tp.z + g[cc][2]) - g[cc][6],
-                      G3 = (tp.w + g[cc][3]) - g[cc][7];
+          const float G0 = tp.x - g[cc][4], G1 = tp.y + (g[cc][1] - g[cc][5]), G2 = tp.z + (g[cc][2] - g[cc][6]),
+                      G3 = tp.w + (g[cc][3] - g[cc][7]);
           sm.top[cc][t] = make_float4(g[cc][4], g[cc][1] + g[cc][5], g[cc][2] + g[cc][6], g[cc][3] + g[cc][7]);
           const float X0 = (G0 + G1) + __shfl_down_sync(0xffffffffu, G0 - G1, 1);
           const float X1 = (G2 + G3) + __shfl_down_sync(0xffffffffu, G2 - G3, 1);

@@ -647,44 +647,49 @@ __global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE 
 // per-lane slot 122 us (4-byte copies); the block inverse asked for before the
 // barrier 98.2 us, but 54.8 against 53.5 us at 8 x 96x48x48.
 // ---------------------------------------------------------------------------
-// Owned vertex (gx, gy) of the FP32 kernel over void planes [pa, pb): the
-// output of MODE for zero forces (kept out of line: inlined, its live values
-// pushed the z march past its register budget).
+// Owned vertex of the FP32 kernel over n void planes: the output of MODE for
+// zero forces (kept out of line: inlined, its live values pushed the z march
+// past its register budget), and MODE 3's share of f.out.  v: the vertex at
+// the first of them, plane: vertices a plane.  Everything by value, and called
+// before the march's own values are live: with references to the sum and to the
+// arguments the march kept those in local memory (MODE 3 on the ellipsoid solid at
+// 159x79x77: 50 -> 36 us).
 template <int MODE>
-__device__ __noinline__ void fine32_void_planes(const LevelDims& d, const uint8_t* __restrict__ vmask,
-                                                const float* __restrict__ u, const float* __restrict__ f,
-                                                float* __restrict__ out, const ChebArgs& ch, int rhs, int gx, int gy,
-                                                int pa, int pb, const float* coef, float& dsum) {
+__device__ __noinline__ float fine32_void_planes(int64_t nv, int64_t v, int64_t plane, int n,
+                                                 const uint8_t* __restrict__ vmask, const float* __restrict__ u,
+                                                 const float* __restrict__ f, float* __restrict__ out,
+                                                 const float* __restrict__ dinv, const float* __restrict__ dvin,
+                                                 float* __restrict__ dv, bool first, bool d_is_u, float c_old,
+                                                 float c_new) {
   constexpr bool CHEB = MODE >= 2, DOTS = MODE == 3;
-  const int64_t nv = d.nv;
-  const float* __restrict__ dvin =
-      (CHEB && !ch.first && !ch.d_is_u) ? static_cast<const float*>(ch.dvec) + (int64_t)rhs * 3 * nv : nullptr;
-  for (int p = pa; p < pb; ++p) {
-    const int64_t v = gx + (int64_t)d.vx * (gy + (int64_t)d.vy * p);
+  float dsum = 0.f;
+#pragma unroll 2
+  for (int p = 0; p < n; ++p, v += plane) {
     const uint8_t m = vmask[v];
     if (!CHEB) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) out[c * nv + v] = (MODE == 1 && ((m >> c) & 1)) ? f[c * nv + v] : 0.f;
     } else {
-      float* __restrict__ dv = static_cast<float*>(ch.dvec) + (int64_t)rhs * 3 * nv;
-      float r[3], zc[3], uv[3];
+      float r[3], zc[3], uv[3], fv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        r[c] = ((m >> c) & 1) ? f[c * nv + v] : 0.f;
+        fv[c] = f[c * nv + v];
+        r[c] = ((m >> c) & 1) ? fv[c] : 0.f;
         uv[c] = u[c * nv + v];
       }
-      dinv_sym_apply(static_cast<const float*>(ch.dinv), nv, v, r, zc);
+      dinv_sym_apply(dinv, nv, v, r, zc);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float dold = ch.d_is_u ? uv[c] : (dvin ? dvin[c * nv + v] : 0.f);
-        const float dn = ch.first ? coef[1] * zc[c] : coef[0] * dold + coef[1] * zc[c];
+        const float dold = d_is_u ? uv[c] : (dvin ? dvin[c * nv + v] : 0.f);
+        const float dn = first ? c_new * zc[c] : c_old * dold + c_new * zc[c];
         dv[c * nv + v] = dn;
         const float o = uv[c] + dn;
         out[c * nv + v] = o;
-        if (DOTS) dsum += f[c * nv + v] * o;
+        if (DOTS) dsum += fv[c] * o;
       }
     }
   }
+  return dsum;
 }
 
 // The x-y modes (1, X, Y, XY) of a vertex plane's four values at an element:
@@ -720,6 +725,7 @@ struct Modal32Smem {
   float4 xa[2][NT];     // exchanged y = 0 forces of a vertex plane (c0, c1, c2, -)
   float4 top[3][NT];    // per component, x-y modes of the last layer's z = 1 forces (each lane its own)
   float4 uo[DOTS ? NT : 1];  // MODE 3: the owned vertex's value at the last layer's lower plane (each lane its own)
+  float ds[DOTS ? NT : 1];   // MODE 3: each lane's share of f.out (in a register across the march it spilled)
   float coef[2];        // Chebyshev (c_old, c_new), read after each plane's barrier
 };
 
@@ -755,6 +761,23 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   const bool own = (i < TXE - 1) && (j < TYE - 1) && gx < d.vx && gy < d.vy;
   int z0, zend;  // the planes marched: [zb0, zb1) less the void
   fine_active_planes<VOID>(d, zb0, zb1, z0, zend);
+  const float* __restrict__ dvin =
+      (CHEB && !ch.first && !ch.d_is_u) ? static_cast<const float*>(ch.dvec) + (int64_t)rhs * 3 * d.nv : nullptr;
+  float dsum = 0.f;
+  if (VOID && (zb0 < z0 || zend < zb1)) {  // void planes: the step's output for zero forces
+    if (CHEB) __syncthreads();      // the step coefficients in shared memory
+    if (own) {
+      const int64_t pl = (int64_t)d.vx * d.vy, v = gx + (int64_t)d.vx * gy;
+      const float* __restrict__ dinv = static_cast<const float*>(ch.dinv);
+      float* __restrict__ dv = CHEB ? static_cast<float*>(ch.dvec) + (int64_t)rhs * 3 * d.nv : nullptr;
+      const float c_old = CHEB ? sm.coef[0] : 0.f, c_new = CHEB ? sm.coef[1] : 0.f;
+      dsum = fine32_void_planes<MODE>(d.nv, v + pl * zb0, pl, z0 - zb0, vmask, u, f, out, dinv, dvin, dv, ch.first,
+                                      ch.d_is_u, c_old, c_new);
+      dsum += fine32_void_planes<MODE>(d.nv, v + pl * zend, pl, zb1 - zend, vmask, u, f, out, dinv, dvin, dv,
+                                       ch.first, ch.d_is_u, c_old, c_new);
+    }
+  }
+  if (DOTS) sm.ds[t] = dsum;
   constexpr int KS = (NP + NT - 1) / NT;
   int pxy[KS];
 #pragma unroll
@@ -788,8 +811,6 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   auto load_pe = [&](int ez) -> float {
     return (pe_xy && ez >= 0 && ez < d.ez) ? rhop[pex + (I)d.ex * (pey + (I)d.ey * ez)] : 0.f;
   };
-  const float* __restrict__ dvin =
-      (CHEB && !ch.first && !ch.d_is_u) ? static_cast<const float*>(ch.dvec) + (int64_t)rhs * 3 * d.nv : nullptr;
   // operands of the owned vertex at plane z, read in step z and used in step z + 1
   uint8_t vm_n = 0;
   float f_n[3] = {0.f, 0.f, 0.f}, dv_n[3] = {0.f, 0.f, 0.f};
@@ -808,14 +829,6 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   };
   float own1[3] = {0.f, 0.f, 0.f};  // own y = 1 forces at the last layer's lower plane
   float uo[3] = {0.f, 0.f, 0.f};    // owned vertex's own value at the last layer's plane
-  float dsum = 0.f;
-  if (VOID && (zb0 < z0 || zend < zb1)) {  // void planes: the step's output for zero forces
-    if (CHEB) __syncthreads();      // the step coefficients in shared memory
-    if (own) {
-      fine32_void_planes<MODE>(d, vmask, u, f, out, ch, rhs, gx, gy, zb0, z0, sm.coef, dsum);
-      fine32_void_planes<MODE>(d, vmask, u, f, out, ch, rhs, gx, gy, zend, zb1, sm.coef, dsum);
-    }
-  }
   float pe_n = load_pe(z0 - 1);
   PlaneModes lm;  // x-y modes of plane st
   if (z0 < zend) {
@@ -859,7 +872,7 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
               }
             } else {
               float* __restrict__ dv = static_cast<float*>(ch.dvec) + (int64_t)rhs * 3 * d.nv;
-              float r[3], zc[3];
+              float r[3], zc[3], ds = DOTS ? sm.ds[t] : 0.f;
 #pragma unroll
               for (int c = 0; c < 3; ++c) r[c] = ((m >> c) & 1) ? f_c[c] - y[c] : 0.f;
               dinv_sym_apply(static_cast<const float*>(ch.dinv), nv, v, r, zc);
@@ -871,8 +884,9 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
                 dv[c * nv + v] = dn;
                 const float o = uv[c] + dn;
                 out[c * nv + v] = o;
-                if (DOTS) dsum += f_c[c] * o;
+                if (DOTS) ds += f_c[c] * o;
               }
+              if (DOTS) sm.ds[t] = ds;
             }
           }
         }
@@ -927,7 +941,7 @@ __global__ void __launch_bounds__(32 * TYE, modal_min_ctas(32 * TYE, MODE >= 2 ?
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   const int64_t cta = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
   if ((MODE == 0 || DOTS) && ch.dotp) {
-    const double bs = modal_block_sum((double)dsum);
+    const double bs = modal_block_sum((double)(DOTS ? sm.ds[t] : dsum));
     if (t == 0) ch.dotp[cta] = bs;
     if (ch.ctr) modal_finish_sum(ch.dotp, (int64_t)gridDim.x * gridDim.y * gridDim.z, ch.dot, ch.ctr, ch.rt);
   }

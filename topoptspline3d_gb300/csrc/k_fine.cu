@@ -309,10 +309,10 @@ __device__ __forceinline__ double modal_block_sum(double v);
 __device__ __forceinline__ void modal_finish_sum(const double* partial, int64_t n, double* out, unsigned* ctr,
                                                  const SumRatio& rt) {
   __shared__ bool last;
-  if (threadIdx.x == 0) {  // thread 0 wrote the block's partial: fence, then take a ticket
-    __threadfence();
-    last = atomicAdd(ctr, 1u) == (unsigned)(n - 1);
-    if (last) __threadfence();
+  RatioOps ops{};
+  if (threadIdx.x == 0) {  // thread 0 wrote the block's partial
+    ops = ratio_load(rt);
+    last = last_ticket(ctr, (unsigned)n);
   }
   __syncthreads();
   if (!last) return;
@@ -321,7 +321,7 @@ __device__ __forceinline__ void modal_finish_sum(const double* partial, int64_t 
   s = modal_block_sum(s);
   if (threadIdx.x == 0) {
     *out = s;
-    write_ratio(rt);
+    ratio_write(rt, ops, out, s);
     *ctr = 0u;
   }
 }

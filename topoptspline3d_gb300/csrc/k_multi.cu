@@ -51,11 +51,7 @@ __device__ __forceinline__ void bfinish(const double (&v)[N], double* part, doub
     const double s = bsum(v[k]);
     if (threadIdx.x == 0) part[((int64_t)k * gridDim.y + rhs) * nblk + blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(ctr + rhs, 1u) == (unsigned)(nblk - 1);
-    if (last) __threadfence();
-  }
+  if (threadIdx.x == 0) last = last_ticket(ctr + rhs, (unsigned)nblk);
   __syncthreads();
   if (!last) return;
 #pragma unroll

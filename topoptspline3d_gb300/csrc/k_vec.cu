@@ -16,8 +16,10 @@ constexpr int RED_MAX_BLOCKS = 1024;
 
 static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
+// Four values a thread: with eight, vectors of a small level (100 k) were on
+// too few SMs and waited for each value in turn.
 int reduce_blocks(int64_t n) {
-  int64_t b = (n + RED_THREADS * 8 - 1) / (RED_THREADS * 8);
+  int64_t b = (n + RED_THREADS * 4 - 1) / (RED_THREADS * 4);
   if (b < 1) b = 1;
   if (b > RED_MAX_BLOCKS) b = RED_MAX_BLOCKS;
   return (int)b;
@@ -34,7 +36,7 @@ __device__ __forceinline__ double block_sum(double v) {
   if (w == 0) {
     s = lane < RED_THREADS / 32 ? ws[lane] : 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    for (int o = RED_THREADS / 64; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   }
   return s;  // valid in thread 0
 }
@@ -45,25 +47,27 @@ __device__ __forceinline__ double block_sum(double v) {
 // depend on which block finishes last) and resets the counter for the next use.
 // Saves the separate finalising launch.  ctr: one counter per stream in order.
 // One call sums K sets of partials, set k at partial + k nb, into *out[k] (null:
-// not wanted); true in thread 0 of the last block, which goes on from there.
+// not wanted) and tot[k]; true in thread 0 of the last block, which goes on from
+// there.
 template <int K>
-__device__ __forceinline__ bool finish_sums(const double* partial, int nb, double* const (&out)[K], unsigned* ctr) {
+__device__ __forceinline__ bool finish_sums(const double* partial, int nb, double* const (&out)[K], double (&tot)[K],
+                                            unsigned* ctr) {
   __shared__ bool last;
-  if (threadIdx.x == 0) {  // thread 0 wrote the block's partials: fence, then take a ticket
-    __threadfence();
-    last = atomicAdd(ctr, 1u) == (unsigned)(nb - 1);
-    if (last) __threadfence();
-  }
+  if (threadIdx.x == 0) last = last_ticket(ctr, (unsigned)nb);  // thread 0 wrote the block's partials
   __syncthreads();
   if (!last) return false;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
+    tot[k] = 0.0;
     if (!out[k]) continue;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += __ldcg(partial + (int64_t)k * nb + i);
-    s = block_sum(s);
-    __syncthreads();  // block_sum's shared words are free again
-    if (threadIdx.x == 0) *out[k] = s;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) tot[k] += __ldcg(partial + (int64_t)k * nb + i);
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (!out[k]) continue;
+    if (k > 0) __syncthreads();  // block_sum's shared words are free again
+    tot[k] = block_sum(tot[k]);
+    if (threadIdx.x == 0) *out[k] = tot[k];
   }
   if (threadIdx.x == 0) *ctr = 0u;
   return threadIdx.x == 0;
@@ -86,7 +90,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot_partial(const T* __restrict
   if (threadIdx.x == 0) partial[blockIdx.x] = bs;
   if (ctr) {
     double* const outs[1] = {out};
-    if (finish_sums(partial, gridDim.x, outs, ctr)) write_ratio(rt);
+    double tot[1];
+    RatioOps ops{};
+    if (threadIdx.x == 0) ops = ratio_load(rt);
+    if (finish_sums(partial, gridDim.x, outs, tot, ctr)) ratio_write(rt, ops, out, tot[0]);
   }
 }
 
@@ -114,7 +121,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot2(const T* __restrict__ a, c
     if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = bt;
   }
   double* const outs[2] = {out_ab, two ? out_bc : nullptr};
-  if (finish_sums(partial, gridDim.x, outs, ctr) && two) write_ratio(rt);
+  double tot[2];
+  RatioOps ops{};
+  if (threadIdx.x == 0) ops = ratio_load(rt);
+  if (finish_sums(partial, gridDim.x, outs, tot, ctr) && two) ratio_write(rt, ops, out_ab, tot[0], out_bc, tot[1]);
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_finalize_sum(const double* __restrict__ partial, int nb, double* out,
@@ -124,7 +134,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_finalize_sum(const double* __re
   s = block_sum(s);
   if (threadIdx.x == 0) {
     *out = s;
-    write_ratio(rt);
+    ratio_write(rt, ratio_load(rt), out, s);
   }
 }
 
@@ -310,9 +320,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update_rr(T* __restrict__ x
   const double bs = block_sum((double)acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = bs;
   double* const outs[1] = {rr};
-  if (finish_sums(partial, gridDim.x, outs, ctr)) {
-    sc[rzold_slot] = sc[rz_slot];
-    if (lc.loop) loop_step(lc, *rr);
+  double tot[1], rz = 0.0;
+  LoopSlots ls{};
+  if (threadIdx.x == 0) {
+    rz = __ldcg(sc + rz_slot);
+    ls = loop_load(lc);
+  }
+  if (finish_sums(partial, gridDim.x, outs, tot, ctr)) {
+    sc[rzold_slot] = rz;
+    if (lc.loop) loop_step(lc, ls, tot[0]);
   }
 }
 
@@ -348,7 +364,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_inner_start(const double* __res
   const double bs = block_sum((double)s);
   if (threadIdx.x == 0) partial[blockIdx.x] = bs;
   double* const outs[1] = {rr};
-  if (finish_sums(partial, gridDim.x, outs, ctr)) loop_start(lc, *bb, *rr);
+  double tot[1];
+  const double b2 = threadIdx.x == 0 ? __ldcg(bb) : 0.0;
+  if (finish_sums(partial, gridDim.x, outs, tot, ctr)) loop_start(lc, b2, tot[0]);
 }
 
 void launch_inner_start(cudaStream_t s, const double* r, float* r32, float* x32, int64_t n, double* partial,
@@ -404,7 +422,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_power_step(int64_t nv, const T*
   const double b1 = block_sum((double)szz);
   if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = b1;
   double* const outs[2] = {xz, nrm};
-  if (finish_sums(partial, gridDim.x, outs, ctr)) *xx = n2;
+  double tot[2];
+  if (finish_sums(partial, gridDim.x, outs, tot, ctr)) *xx = n2;
 }
 
 template <typename T>

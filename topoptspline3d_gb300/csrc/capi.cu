@@ -2575,7 +2575,7 @@ int topo_multi_reserve(topo_handle* h, int capacity) {
     m->U.push_back(a); m->F.push_back(b); m->R.push_back(c); m->U2.push_back(d); m->cd.push_back(e);
   }
   const size_t n64 = (size_t)capacity * 3 * h->lv[0].d.nv * sizeof(double);
-  for (double** v : {&m->x, &m->f, &m->r, &m->d, &m->q, &m->rold, &m->z})
+  for (double** v : {&m->x, &m->f, &m->r, &m->d, &m->q, &m->rold})
     if (rc == TOPO_OK) rc = alloc((void**)v, n64);
   for (float** v : {&m->x32, &m->d32, &m->q32})
     if (rc == TOPO_OK) rc = alloc((void**)v, n64 / 2);
@@ -2629,8 +2629,8 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
       h->nb = 1;
     }
   } swap(h, m, nb);
-  enum { B_RR, B_FF, B_RZ, B_ZROLD, B_RZOLD, B_DQ, B_ALPHA, B_BETA,
-         I_RR, I_FF, I_RZ, I_RZOLD, I_DQ, I_ALPHA, I_BETA, I_ZERO };  // outer, inner (16 slots)
+  enum { B_RR, B_FF, B_RZ, B_RZOLD, B_DQ, B_ALPHA, B_BETA,
+         I_RR, I_FF, I_RZ, I_RZOLD, I_DQ, I_ALPHA, I_BETA };  // outer, inner (of 16 slots)
   const int inner_max = o->inner_max > 1 ? o->inner_max : 1;
   const double inner_rtol = o->inner_rtol > 0 ? o->inner_rtol : 1e-1;
   double* sb = m.sc;
@@ -2655,16 +2655,19 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
     return true;
   };
   int it = 0, nvc = 0;
-  if (inner_max > 1) CK(cudaMemsetAsync(slot(I_ZERO), 0, sizeof(double) * nb, h->stream));
   while (!converged() && it < o->max_iter) {
-    launch_d2f(h->stream, m.r, L0.F32, n3 * nb);
+    // r in FP32 for the preconditioner; later steps' by launch_bupdate
+    if (it == 0) {
+      launch_d2f(h->stream, m.r, L0.F32, n3 * nb);
+      count_launch();
+    }
+    const float* z = inner_max <= 1 ? L0.U32 : m.x32;
     if (inner_max <= 1) {
       // z = V(r): one FP32 V-cycle for the whole batch
       if (!cheb_zero_start(TOPO_SMOOTH_CHEBYSHEV, o->pre, cp))
         CK(cudaMemsetAsync(L0.U32, 0, sizeof(float) * n3 * nb, h->stream));
       vcycle32(h, o->pre, o->post, TOPO_SMOOTH_CHEBYSHEV, cp, true);
       ++nvc;
-      k_to_double<float><<<nb256(n3 * nb), 256, 0, h->stream>>>(n3 * nb, L0.U32, m.z);
     } else {
       // z = inner_max iterations of an FP32 CG per right-hand side on A z = r,
       // preconditioned by the batched V-cycle (a fixed symmetric operator, so
@@ -2683,29 +2686,27 @@ int topo_solve_multi(topo_handle* h, int nrhs, const topo_solve_opts* o, topo_mu
           CK(cudaMemsetAsync(z32, 0, sizeof(float) * n3 * nb, h->stream));
         vcycle32(h, o->pre, o->post, TOPO_SMOOTH_CHEBYSHEV, cp, true);
         ++nvc;
-        launch_bdot<float>(h->stream, r32, z32, n3, nb, m.part, m.ctr, slot(I_RZ));
-        launch_bbeta(h->stream, nb, slot(I_RZ), slot(I_ZERO), slot(I_RZOLD), j == 0, slot(I_BETA));
+        launch_bdot_beta<float>(h->stream, r32, z32, nullptr, n3, nb, m.part, m.ctr, slot(I_RZ), slot(I_RZOLD), j == 0,
+                                slot(I_BETA));
         launch_bdir<float>(h->stream, n3, nb, z32, m.d32, slot(I_BETA));
         launch_fine_apply<float>(h->stream, L0.d, h->rhop32, L0.vmask, m.d32, nullptr, m.q32, false, nb,
                                  tz32_arg(h));
-        launch_bdot<float>(h->stream, m.d32, m.q32, n3, nb, m.part, m.ctr, slot(I_DQ));
-        launch_balpha(h->stream, nb, slot(I_RZ), slot(I_DQ), slot(I_RR), slot(I_FF), inner_rtol * inner_rtol,
-                      slot(I_ALPHA), slot(I_RZOLD));
-        launch_bupdate<float>(h->stream, n3, nb, m.x32, r32, nullptr, m.d32, m.q32, slot(I_ALPHA), m.part, m.ctr,
+        launch_bdot_alpha<float>(h->stream, m.d32, m.q32, n3, nb, m.part, m.ctr, slot(I_DQ), slot(I_RZ), slot(I_RR),
+                                 slot(I_FF), inner_rtol * inner_rtol, slot(I_ALPHA), slot(I_RZOLD));
+        launch_bupdate<float>(h->stream, n3, nb, m.x32, r32, nullptr, nullptr, m.d32, m.q32, slot(I_ALPHA), m.part, m.ctr,
                               slot(I_RR));
-        count_launch(7);
+        count_launch(5);
       }
-      k_to_double<float><<<nb256(n3 * nb), 256, 0, h->stream>>>(n3 * nb, m.x32, m.z);
     }
-    launch_bdot<double>(h->stream, m.r, m.z, n3, nb, m.part, m.ctr, slot(B_RZ), it > 0 ? m.rold : nullptr, slot(B_ZROLD));
-    launch_bbeta(h->stream, nb, slot(B_RZ), slot(B_ZROLD), slot(B_RZOLD), it == 0, slot(B_BETA));
-    launch_bdir<double>(h->stream, n3, nb, m.z, m.d, slot(B_BETA));
+    launch_bdot_beta<double>(h->stream, m.r, z, it > 0 ? m.rold : nullptr, n3, nb, m.part, m.ctr, slot(B_RZ),
+                             slot(B_RZOLD), it == 0, slot(B_BETA));
+    launch_bdir<double>(h->stream, n3, nb, z, m.d, slot(B_BETA));
     fine64(h, L0.d, m.d, nullptr, m.q, false, nb);
-    launch_bdot<double>(h->stream, m.d, m.q, n3, nb, m.part, m.ctr, slot(B_DQ));
-    launch_balpha(h->stream, nb, slot(B_RZ), slot(B_DQ), slot(B_RR), slot(B_FF), rtol2, slot(B_ALPHA),
-                  slot(B_RZOLD));
-    launch_bupdate<double>(h->stream, n3, nb, m.x, m.r, m.rold, m.d, m.q, slot(B_ALPHA), m.part, m.ctr, slot(B_RR));
-    count_launch(9);
+    launch_bdot_alpha<double>(h->stream, m.d, m.q, n3, nb, m.part, m.ctr, slot(B_DQ), slot(B_RZ), slot(B_RR),
+                              slot(B_FF), rtol2, slot(B_ALPHA), slot(B_RZOLD));
+    launch_bupdate<double>(h->stream, n3, nb, m.x, m.r, m.rold, L0.F32, m.d, m.q, slot(B_ALPHA), m.part, m.ctr,
+                           slot(B_RR));
+    count_launch(5);
     CKL();
     CK(cudaMemcpyAsync(rr.data(), slot(B_RR), sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));

@@ -3,6 +3,7 @@
 // Reductions are deterministic: per-(CTA, rhs) partials that the right-hand
 // side's last CTA adds in a fixed order.
 #include <algorithm>
+#include <type_traits>
 
 #include "topo_internal.h"
 
@@ -41,9 +42,10 @@ __device__ __forceinline__ double bsum(double v) {
 
 // Publishes the CTA's sums; the CTA that takes the right-hand side's last
 // ticket adds its partials in index order (the result does not depend on which
-// CTA is last) and resets the counter.  part: [N][nb][gridDim.x].
-template <int N>
-__device__ __forceinline__ void bfinish(const double (&v)[N], double* part, double* const (&out)[N], unsigned* ctr) {
+// CTA is last), resets the counter and calls fin with the totals in one thread.
+// part: [N][nb][gridDim.x].
+template <int N, typename Fin>
+__device__ __forceinline__ void bfinish(const double (&v)[N], double* part, unsigned* ctr, Fin&& fin) {
   __shared__ bool last;
   const int rhs = blockIdx.y, nblk = gridDim.x;
 #pragma unroll
@@ -54,24 +56,56 @@ __device__ __forceinline__ void bfinish(const double (&v)[N], double* part, doub
   if (threadIdx.x == 0) last = last_ticket(ctr + rhs, (unsigned)nblk);
   __syncthreads();
   if (!last) return;
+  double tot[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nblk; i += kThreads) s += __ldcg(part + ((int64_t)k * gridDim.y + rhs) * nblk + i);
-    s = bsum(s);
-    if (threadIdx.x == 0) out[k][rhs] = s;
+    tot[k] = 0.0;
+    for (int i = threadIdx.x; i < nblk; i += kThreads) tot[k] += __ldcg(part + ((int64_t)k * gridDim.y + rhs) * nblk + i);
   }
-  if (threadIdx.x == 0) ctr[rhs] = 0u;
+#pragma unroll
+  for (int k = 0; k < N; ++k) tot[k] = bsum(tot[k]);
+  if (threadIdx.x == 0) {
+    ctr[rhs] = 0u;
+    fin(tot);
+  }
 }
 
-// a.b per right-hand side and, TWO, b.c with the same read of b.  The sums were
-// finished by one thread a right-hand side, 256 dependent FP64 additions: 19 us
-// after every 23 us of partial sums (eight vectors of 96x48x48).
-template <typename T, bool TWO>
-__global__ void __launch_bounds__(kThreads) k_bdot(const T* __restrict__ a, const T* __restrict__ b,
+// What a dot is followed by, per right-hand side, in the thread that has its
+// total (a kernel of its own took 3 to 4 us a scalar).
+struct BNone {};
+// beta = (rz - zrold) / rzold (0 at first, and for a right-hand side of rzold = 0)
+struct BBeta {
+  const double* rzold;
+  double* beta;
+  int first;
+};
+// alpha = rz / dq while rr > rtol^2 ff, else 0 (the right-hand side has
+// converged and its iterate is frozen); rzold = rz
+struct BAlpha {
+  const double *rz, *rr, *ff;
+  double rtol2;
+  double *alpha, *rzold;
+};
+
+// out = a.b per right-hand side, and the step St; TWO: with b.c by the same read
+// of b, for beta.  b may be of the other precision (the preconditioner's FP32
+// result in the FP64 iteration: widening it in memory first cost a pass of 12
+// bytes a value and twice the reads here).  Bound: two FP64 lanes a clock and SM
+// against 8 to 20 bytes a value, so four values are in flight a thread.
+template <typename T, typename TB, bool TWO, typename St>
+__global__ void __launch_bounds__(kThreads) k_bdot(const T* __restrict__ a, const TB* __restrict__ b,
                                                    const T* __restrict__ c, int64_t n, double* __restrict__ part,
-                                                   double* out0, double* out1, unsigned* ctr) {
-  const int64_t off = (int64_t)blockIdx.y * n;
+                                                   double* out, unsigned* ctr, St st) {
+  const int rhs = blockIdx.y;
+  const int64_t off = (int64_t)rhs * n;
+  double w0 = 0.0, w1 = 0.0, w2 = 0.0;  // the step's operands, read ahead
+  if constexpr (std::is_same<St, BBeta>::value) {
+    w0 = st.rzold[rhs];
+  } else if constexpr (std::is_same<St, BAlpha>::value) {
+    w0 = st.rz[rhs];
+    w1 = st.rr[rhs];
+    w2 = st.ff[rhs];
+  }
   double s = 0.0, t = 0.0;
 #pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
@@ -79,58 +113,63 @@ __global__ void __launch_bounds__(kThreads) k_bdot(const T* __restrict__ a, cons
     s += (double)a[off + i] * v;
     if (TWO) t += v * (double)c[off + i];
   }
-  if constexpr (TWO) {
-    bfinish<2>({s, t}, part, {out0, out1}, ctr);
-  } else {
-    bfinish<1>({s}, part, {out0}, ctr);
+  auto fin = [&](double ab, double bc) {
+    out[rhs] = ab;
+    if constexpr (std::is_same<St, BBeta>::value) {
+      st.beta[rhs] = st.first || !(w0 != 0.0) ? 0.0 : (ab - bc) / w0;
+    } else if constexpr (std::is_same<St, BAlpha>::value) {
+      st.alpha[rhs] = w1 > st.rtol2 * w2 && ab != 0.0 ? w0 / ab : 0.0;
+      st.rzold[rhs] = w0;
+    }
+  };
+  if constexpr (TWO) bfinish<2>({s, t}, part, ctr, [&](const double(&q)[2]) { fin(q[0], q[1]); });
+  else bfinish<1>({s}, part, ctr, [&](const double(&q)[1]) { fin(q[0], 0.0); });
+}
+
+template <typename T>
+void launch_bdot(cudaStream_t s, const T* a, const T* b, int64_t n, int nb, double* partial, unsigned* ctr,
+                 double* out) {
+  k_bdot<T, T, false, BNone><<<dim3(bdot_blocks(n, nb), nb), kThreads, 0, s>>>(a, b, nullptr, n, partial, out, ctr,
+                                                                              BNone{});
+}
+template <typename T>
+void launch_bdot_beta(cudaStream_t s, const T* r, const float* z, const T* rold, int64_t n, int nb, double* partial,
+                      unsigned* ctr, double* rz, const double* rzold, bool first, double* beta) {
+  const dim3 g(bdot_blocks(n, nb), nb);
+  const BBeta st{rzold, beta, first ? 1 : 0};
+  if (rold) k_bdot<T, float, true, BBeta><<<g, kThreads, 0, s>>>(r, z, rold, n, partial, rz, ctr, st);
+  else k_bdot<T, float, false, BBeta><<<g, kThreads, 0, s>>>(r, z, nullptr, n, partial, rz, ctr, st);
+}
+template <typename T>
+void launch_bdot_alpha(cudaStream_t s, const T* d, const T* q, int64_t n, int nb, double* partial, unsigned* ctr,
+                       double* dq, const double* rz, const double* rr, const double* ff, double rtol2, double* alpha,
+                       double* rzold) {
+  k_bdot<T, T, false, BAlpha><<<dim3(bdot_blocks(n, nb), nb), kThreads, 0, s>>>(
+      d, q, nullptr, n, partial, dq, ctr, BAlpha{rz, rr, ff, rtol2, alpha, rzold});
+}
+
+// d = z + beta d, z in FP32
+constexpr int kDirEach = 4;  // values of a thread, in flight together
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_bdir(int64_t n, const float* __restrict__ z, T* __restrict__ d,
+                                                   const double* __restrict__ beta) {
+  const int64_t off = (int64_t)blockIdx.y * n, i0 = (int64_t)blockIdx.x * (kDirEach * kThreads) + threadIdx.x;
+  const T b = (T)beta[blockIdx.y];
+#pragma unroll
+  for (int k = 0; k < kDirEach; ++k) {
+    const int64_t i = i0 + k * kThreads;
+    if (i < n) d[off + i] = (T)z[off + i] + b * d[off + i];
   }
 }
 
-template <typename T>
-void launch_bdot(cudaStream_t s, const T* a, const T* b, int64_t n, int nb, double* partial, unsigned* ctr, double* out,
-                 const T* c, double* out_bc) {
-  const dim3 g(bdot_blocks(n, nb), nb);
-  if (c) k_bdot<T, true><<<g, kThreads, 0, s>>>(a, b, c, n, partial, out, out_bc, ctr);
-  else k_bdot<T, false><<<g, kThreads, 0, s>>>(a, b, nullptr, n, partial, out, nullptr, ctr);
-}
-template void launch_bdot<double>(cudaStream_t, const double*, const double*, int64_t, int, double*, unsigned*, double*,
-                                  const double*, double*);
-template void launch_bdot<float>(cudaStream_t, const float*, const float*, int64_t, int, double*, unsigned*, double*,
-                                 const float*, double*);
-
-// Per right-hand side: beta = (rz - zrold) / rzold (first: 0).
-__global__ void k_bbeta(int nb, const double* rz, const double* zrold, const double* rzold, int first, double* beta) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nb) return;
-  beta[k] = first || !(rzold[k] != 0.0) ? 0.0 : (rz[k] - zrold[k]) / rzold[k];
-}
-
-// Per right-hand side: alpha = rz / dq while rr > rtol^2 ff, else 0 (the
-// right-hand side has converged and its iterate is frozen); rzold = rz.
-__global__ void k_balpha(int nb, const double* rz, const double* dq, const double* rr, const double* ff, double rtol2,
-                         double* alpha, double* rzold) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nb) return;
-  const bool active = rr[k] > rtol2 * ff[k] && dq[k] != 0.0;
-  alpha[k] = active ? rz[k] / dq[k] : 0.0;
-  rzold[k] = rz[k];
-}
-
-// d = z + beta d
-template <typename T>
-__global__ void k_bdir(int64_t n, int nb, const T* __restrict__ z, T* __restrict__ d, const double* __restrict__ beta) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * nb) return;
-  const T b = (T)beta[i / n];
-  d[i] = z[i] + b * d[i];
-}
-
-// x += alpha d, rold = r (when kept), r -= alpha q, and r.r of the new r
+// x += alpha d, rold = r (when kept), r -= alpha q, r.r of the new r, and the
+// new r in FP32 for the preconditioner (when wanted: it is in registers here)
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_bupdate(int64_t n, T* __restrict__ x, T* __restrict__ r,
-                                                      T* __restrict__ rold, const T* __restrict__ d,
-                                                      const T* __restrict__ q, const double* __restrict__ alpha,
-                                                      double* __restrict__ part, double* rr, unsigned* ctr) {
+                                                      T* __restrict__ rold, float* __restrict__ r32,
+                                                      const T* __restrict__ d, const T* __restrict__ q,
+                                                      const double* __restrict__ alpha, double* __restrict__ part,
+                                                      double* rr, unsigned* ctr) {
   const int64_t off = (int64_t)blockIdx.y * n;
   const T a = (T)alpha[blockIdx.y];
   double s = 0.0;
@@ -142,33 +181,32 @@ __global__ void __launch_bounds__(kThreads) k_bupdate(int64_t n, T* __restrict__
     if (rold) rold[i] = r0;
     const T rn = r0 - a * q[i];
     r[i] = rn;
+    if (r32) r32[i] = (float)rn;
     s += (double)rn * (double)rn;
   }
-  bfinish<1>({s}, part, {rr}, ctr);
+  bfinish<1>({s}, part, ctr, [&](const double(&t)[1]) { rr[blockIdx.y] = t[0]; });
 }
 
-void launch_bbeta(cudaStream_t s, int nb, const double* rz, const double* zrold, const double* rzold, bool first,
-                  double* beta) {
-  k_bbeta<<<nblk(nb, 64), 64, 0, s>>>(nb, rz, zrold, rzold, first ? 1 : 0, beta);
-}
-void launch_balpha(cudaStream_t s, int nb, const double* rz, const double* dq, const double* rr, const double* ff,
-                   double rtol2, double* alpha, double* rzold) {
-  k_balpha<<<nblk(nb, 64), 64, 0, s>>>(nb, rz, dq, rr, ff, rtol2, alpha, rzold);
+template <typename T>
+void launch_bdir(cudaStream_t s, int64_t n, int nb, const float* z, T* d, const double* beta) {
+  k_bdir<T><<<dim3(nblk(n, kDirEach * kThreads), nb), kThreads, 0, s>>>(n, z, d, beta);
 }
 template <typename T>
-void launch_bdir(cudaStream_t s, int64_t n, int nb, const T* z, T* d, const double* beta) {
-  k_bdir<T><<<nblk(n * nb, kThreads), kThreads, 0, s>>>(n, nb, z, d, beta);
-}
-template <typename T>
-void launch_bupdate(cudaStream_t s, int64_t n, int nb, T* x, T* r, T* rold, const T* d, const T* q,
+void launch_bupdate(cudaStream_t s, int64_t n, int nb, T* x, T* r, T* rold, float* r32, const T* d, const T* q,
                     const double* alpha, double* partial, unsigned* ctr, double* rr) {
-  k_bupdate<T><<<dim3(bdot_blocks(n, nb), nb), kThreads, 0, s>>>(n, x, r, rold, d, q, alpha, partial, rr, ctr);
+  k_bupdate<T><<<dim3(bdot_blocks(n, nb), nb), kThreads, 0, s>>>(n, x, r, rold, r32, d, q, alpha, partial, rr, ctr);
 }
-template void launch_bdir<double>(cudaStream_t, int64_t, int, const double*, double*, const double*);
-template void launch_bdir<float>(cudaStream_t, int64_t, int, const float*, float*, const double*);
-template void launch_bupdate<double>(cudaStream_t, int64_t, int, double*, double*, double*, const double*,
-                                     const double*, const double*, double*, unsigned*, double*);
-template void launch_bupdate<float>(cudaStream_t, int64_t, int, float*, float*, float*, const float*, const float*,
-                                    const double*, double*, unsigned*, double*);
+#define TOPO_MULTI(T)                                                                                                  \
+  template void launch_bdot<T>(cudaStream_t, const T*, const T*, int64_t, int, double*, unsigned*, double*);           \
+  template void launch_bdot_beta<T>(cudaStream_t, const T*, const float*, const T*, int64_t, int, double*, unsigned*,  \
+                                    double*, const double*, bool, double*);                                            \
+  template void launch_bdot_alpha<T>(cudaStream_t, const T*, const T*, int64_t, int, double*, unsigned*, double*,      \
+                                     const double*, const double*, const double*, double, double*, double*);           \
+  template void launch_bdir<T>(cudaStream_t, int64_t, int, const float*, T*, const double*);                           \
+  template void launch_bupdate<T>(cudaStream_t, int64_t, int, T*, T*, T*, float*, const T*, const T*, const double*,   \
+                                  double*, unsigned*, double*);
+TOPO_MULTI(double)
+TOPO_MULTI(float)
+#undef TOPO_MULTI
 
 }  // namespace topo

@@ -581,27 +581,32 @@ cudaError_t unet_host_pass(UNetState* u, cudaStream_t s, int X, int Y, int Z, in
                            const uint8_t* m, float* y, double* loss, float* grad);
 
 // k_multi.cu: batched vectors of the multi-right-hand-side solver.
-// out[k] = a_k.b_k and, with c, out_bc[k] = b_k.c_k; ctr: one zeroed ticket
-// counter per right-hand side (reset by the last CTA)
+// out[k] = a_k.b_k; ctr: one zeroed ticket counter per right-hand side (reset by
+// the last CTA)
 template <typename T>
-void launch_bdot(cudaStream_t s, const T* a, const T* b, int64_t n, int nb, double* partial, unsigned* ctr, double* out,
-                 const T* c = nullptr, double* out_bc = nullptr);
-void launch_bbeta(cudaStream_t s, int nb, const double* rz, const double* zrold, const double* rzold, bool first,
-                  double* beta);
-void launch_balpha(cudaStream_t s, int nb, const double* rz, const double* dq, const double* rr, const double* ff,
-                   double rtol2, double* alpha, double* rzold);
+void launch_bdot(cudaStream_t s, const T* a, const T* b, int64_t n, int nb, double* partial, unsigned* ctr, double* out);
+// rz = r.z and beta = (rz - z.rold) / rzold (rold null: Fletcher-Reeves; 0 at first)
 template <typename T>
-void launch_bdir(cudaStream_t s, int64_t n, int nb, const T* z, T* d, const double* beta);
-// x += alpha d, rold = r (when kept), r -= alpha q, rr[k] = r_k.r_k
+void launch_bdot_beta(cudaStream_t s, const T* r, const float* z, const T* rold, int64_t n, int nb, double* partial,
+                      unsigned* ctr, double* rz, const double* rzold, bool first, double* beta);
+// dq = d.q, alpha = rz / dq while rr > rtol2 ff (else 0), rzold = rz
 template <typename T>
-void launch_bupdate(cudaStream_t s, int64_t n, int nb, T* x, T* r, T* rold, const T* d, const T* q,
+void launch_bdot_alpha(cudaStream_t s, const T* d, const T* q, int64_t n, int nb, double* partial, unsigned* ctr,
+                       double* dq, const double* rz, const double* rr, const double* ff, double rtol2, double* alpha,
+                       double* rzold);
+template <typename T>
+void launch_bdir(cudaStream_t s, int64_t n, int nb, const float* z, T* d, const double* beta);
+// x += alpha d, rold = r (when kept), r -= alpha q, rr[k] = r_k.r_k, r32 = the new
+// r in FP32 (may be null)
+template <typename T>
+void launch_bupdate(cudaStream_t s, int64_t n, int nb, T* x, T* r, T* rold, float* r32, const T* d, const T* q,
                     const double* alpha, double* partial, unsigned* ctr, double* rr);
 
 // Batched buffers of the multi-right-hand-side solver (topo_multi_reserve).
 struct MultiRhs {
   int cap = 0;
   std::vector<float*> U, F, R, U2, cd;  // per level, cap * 3 nv
-  double *x = nullptr, *f = nullptr, *r = nullptr, *d = nullptr, *q = nullptr, *rold = nullptr, *z = nullptr;
+  double *x = nullptr, *f = nullptr, *r = nullptr, *d = nullptr, *q = nullptr, *rold = nullptr;
   float *x32 = nullptr, *d32 = nullptr, *q32 = nullptr;  // inner FP32 CG, level 0, cap * 3 nv
   double* part = nullptr;  // reduction partials, two sums [cap][256]
   unsigned* ctr = nullptr;  // ticket counters of the reductions [cap]

@@ -854,8 +854,10 @@ __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, c
     }
   }
   const T inv = T(1) / T(64);
+  // (4 - rx) a + rx b with one rounding: the product by 3, if there is one, goes
+  // into the fused multiply-add, the other weight is a power of two or 0
   const int rx = lane & 3;
-  const T w0 = T(4 - rx), w1 = T(rx);
+  const T wm = T(rx == 3 ? 3 : 4 - rx), wq = T(rx == 3 ? 1 : rx);
 #pragma unroll
   for (int k = 0; k < P4_EACH; ++k) {
     const uint8_t m = (mm[k] & 8) ? mm[k] : 0;
@@ -864,7 +866,8 @@ __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, c
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const T a = __shfl_sync(0xffffffffu, cyz[c], from), b = __shfl_sync(0xffffffffu, cyz[c], from + 1);
-      if ((m >> c) & 1) uf[c * fd.nv + v] = uo[k][c] + (w0 * a + w1 * b) * inv;
+      const T t = fma(wm, rx == 3 ? b : a, wq * (rx == 3 ? a : b));
+      if ((m >> c) & 1) uf[c * fd.nv + v] = uo[k][c] + t * inv;
     }
   }
 }

@@ -696,9 +696,9 @@ __global__ void k_restrict(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
 // vertex, and warp 0 sums the seven partial sums in a fixed order.  Seven
 // times the threads of a vertex-per-thread gather keep the loads in flight.
 constexpr int R4_WARPS = 7;
-// FLAT asks for a warp's 49 taps together instead of a row of 7 at a time: fewer
-// waits, which is what a grid of less than two CTAs per SM spends its time on
-// (20 CTAs: 10.7 -> 8.3 us); a full chip has the loads in flight anyway and the
+// FLAT (FP64) asks for a warp's 49 taps together instead of a row of 7 at a time:
+// fewer waits, which is what a grid of less than two CTAs per SM spends its time on
+// (FP32, 20 CTAs: 10.7 -> 8.3 us); a full chip has the loads in flight anyway and the
 // row form's shorter code wins (8 x 133 CTAs: 20 us, flat 25).
 constexpr unsigned R4_FLAT_CTAS = 304;
 
@@ -754,6 +754,59 @@ __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, Level
   }
 }
 
+// The same with a coarse vertex on eight lanes, one x tap each (seven used): a
+// lane has 21 taps instead of 147 and a warp's loads are 19 neighbouring values,
+// so a grid of a few CTAs becomes eight times as many that each wait once.
+template <typename T>
+__global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4_lanes(LevelDims fd, LevelDims cd,
+                                                                   const T* __restrict__ rf, T* __restrict__ fc) {
+  __shared__ T part[R4_WARPS][3][4];
+  rf += (int64_t)blockIdx.y * 3 * fd.nv;  // right-hand side of the batch
+  fc += (int64_t)blockIdx.y * 3 * cd.nv;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 3, tap = lane & 7;
+  const int64_t v0 = (int64_t)blockIdx.x * 4, v = v0 + g;
+  T s0 = T(0), s1 = T(0), s2 = T(0);
+  if (v < cd.nv && tap < 7) {
+    const int t = (int)(v / cd.vx), x = (int)(v - (int64_t)t * cd.vx), z = t / cd.vy, y = t - z * cd.vy;
+    const int fx = 4 * x + tap - 3, fz = 4 * z + w - 3;
+    if (fx >= 0 && fx < fd.vx && fz >= 0 && fz < fd.vz) {
+#pragma unroll
+      for (int dy = -3; dy <= 3; ++dy) {
+        const int fy = 4 * y + dy;
+        const bool in = fy >= 0 && fy < fd.vy;
+        const T wy = T(4 - (dy < 0 ? -dy : dy));
+        const int64_t fv = in ? fx + (int64_t)fd.vx * (fy + (int64_t)fd.vy * fz) : 0;
+        s0 += wy * (in ? rf[fv] : T(0));
+        s1 += wy * (in ? rf[fd.nv + fv] : T(0));
+        s2 += wy * (in ? rf[2 * fd.nv + fv] : T(0));
+      }
+      const T wt = T((w < 3 ? w + 1 : 7 - w) * (tap < 3 ? tap + 1 : 7 - tap));
+      s0 *= wt;
+      s1 *= wt;
+      s2 *= wt;
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  if (tap == 0) {
+    part[w][0][g] = s0;
+    part[w][1][g] = s1;
+    part[w][2][g] = s2;
+  }
+  __syncthreads();
+  if (tid < 12 && v0 + (tid & 3) < cd.nv) {
+    const int c = tid >> 2, q = tid & 3;
+    T a = T(0);
+#pragma unroll
+    for (int k = 0; k < R4_WARPS; ++k) a += part[k][c][q];
+    fc[c * cd.nv + v0 + q] = a * (T(1) / T(64));
+  }
+}
+
 template <typename T, int FCT>
 __global__ void k_prolong(LevelDims fd, LevelDims cd, const T* __restrict__ uc, T* __restrict__ uf,
                           const uint8_t* __restrict__ vmask) {
@@ -796,13 +849,25 @@ __global__ void k_prolong(LevelDims fd, LevelDims cd, const T* __restrict__ uc, 
   if (m & 4) uf[2 * fd.nv + v] += s2;
 }
 
+// Up to three CTAs of the row form per SM the lanes form is the faster one (CTAs
+// of the row form, us lanes / row or flat: 20 3.9 / 8.5, 95 5.2 / 9, 565 14.2 /
+// 14.0, 1,064 24 / 20, 2,212 47 / 43: it reads each fine plane by more CTAs).
+// FP32 only: the FP64 forms keep the order of their sums, which callers of
+// nearly converged cycles see in the residual's last digits.
+constexpr unsigned R4_LANES_CTAS = 456;
 template <typename T>
 void launch_restrict(cudaStream_t s, const LevelDims& fine, const LevelDims& coarse, const T* rf,
                      T* fc, int nb) {
   if (coarse.factor == 4) {
     const unsigned g = nblk(coarse.nv, 32);
-    if (g * (unsigned)nb < R4_FLAT_CTAS)
-      k_restrict4<T, true><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
+    if constexpr (sizeof(T) == 4) {
+      if (g * (unsigned)nb < R4_LANES_CTAS) {
+        k_restrict4_lanes<T><<<dim3(nblk(coarse.nv, 4), nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
+        return;
+      }
+    }
+    if (sizeof(T) == 8 && g * (unsigned)nb < R4_FLAT_CTAS)
+      k_restrict4<T, sizeof(T) == 8><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
     else
       k_restrict4<T, false><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
   } else {

@@ -10,15 +10,19 @@
 // Its error is below the FP64 kernel's: the transforms are exact and only the
 // 22 products of an element round.
 //
-// Per step (element layer ez), two barriers:
-//   A  publishes the last layer's y = 0 forces, and frees the oldest converted
-//      plane;
-//   -  each thread splits its staged vertices of plane ez + 1 into mantissas and
-//      exponents, and finishes its vertex of plane ez - 1 from the two layers
-//      next to it;
-//   C  the converted plane is complete; each thread computes its element.
-// A thread stages and converts the same vertices, so their copies need no
-// barrier.
+// Per step (element layer ez), one barrier:
+//   before it each thread splits its staged vertices of plane ez + 1 into
+//     mantissas and exponents, into a slot of three that no thread of the step
+//     before reads (it stages and converts the same vertices, so their copies
+//     need no barrier);
+//   after it, with plane ez + 1 converted and the last layer's y = 0 forces
+//     published, it finishes its vertex of plane ez - 1 from the two layers next
+//     to it and computes its element: the FP64 chain of the one and the integer
+//     work of the other are in one phase, where the 16 warps of an SM fill each
+//     other's gaps.
+// With a barrier on either side of the vertex, and two converted planes, the
+// Chebyshev step at 128x64x64 took 100.9 us (now 97.9), K u 67.6 (66.1): issue
+// slots 45% busy there, the FP64 pipe 31%, a sixth of the stalls at barriers.
 #include "topo_internal.h"
 
 #include "fx.cuh"
@@ -39,8 +43,8 @@ constexpr int TX = FINE_TILE_X, TY = FINE_TILE_Y, NT = TX * TY, PX = TX + 1, NP 
 constexpr int KS = (NP + NT - 1) / NT;  // vertices of a plane a thread stages
 
 struct FxSmem {
-  longlong2 qa[2][NP];     // converted planes: mantissas of components 0 and 1
-  longlong2 qb[2][NP];     //                   of component 2, exponents (16 bits each)
+  longlong2 qa[3][NP];     // converted planes: mantissas of components 0 and 1
+  longlong2 qb[3][NP];     //                   of component 2, exponents (16 bits each)
   double raw[3][3][NP];    // staged planes
   longlong2 xa[2][3][NT];  // y = 0 forces of a layer: z = 0 (c0, c1), (c2, z = 1 c0), z = 1 (c1, c2)
   int xe[2][NT];           // their exponent
@@ -86,7 +90,7 @@ __global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const doub
     zend = max(z0, min(zb1, cz.y + 2));
   }
   // What the owned vertex of plane p needs besides its element forces.  Loaded
-  // before the step's first barrier, so that the loads' latency passes there.
+  // before the step's barrier, so that the loads' latency passes there.
   struct Vertex {
     int64_t v;
     uint8_t m;
@@ -170,8 +174,8 @@ __global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const doub
       if (k < NP) {
         int e0, e1, e2;
         const int64_t q0 = fx_split(src[0][k], e0), q1 = fx_split(src[1][k], e1), q2 = fx_split(src[2][k], e2);
-        sm.qa[z & 1][k] = make_longlong2(q0, q1);
-        sm.qb[z & 1][k] = make_longlong2(q2, (long long)((uint64_t)(unsigned)(e0 | e1 << 16) | (uint64_t)e2 << 32));
+        sm.qa[(z + 3) % 3][k] = make_longlong2(q0, q1);
+        sm.qb[(z + 3) % 3][k] = make_longlong2(q2, (long long)((uint64_t)(unsigned)(e0 | e1 << 16) | (uint64_t)e2 << 32));
       }
     }
   };
@@ -197,8 +201,8 @@ __global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const doub
       if (st + 1 < zend) pe_n = load_pe(st + 1);
       asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane st + 1 has arrived
     }
-    __syncthreads();  // A
     if (st < zend) convert(st + 1);
+    __syncthreads();
     if (st >= z0 && own) {
       const int xs = (st - 1) & 1, n = t + TX;
       const longlong2 a = sm.xa[xs][0][n], b = sm.xa[xs][1][n], c2 = sm.xa[xs][2][n];
@@ -216,7 +220,6 @@ __global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const doub
       if (st - 1 >= z0) finish(V, y);
     }
     if (st == zend) break;
-    __syncthreads();  // C
     {
       int64_t v[3][8];
       int fe = FX_ZERO;
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(NT, FX_CTAS) k_fine_fx(LevelDims d, const doub
         int e2[8], m2 = 0;
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
-          const int k = (i + (a & 1)) + PX * (j + ((a >> 1) & 1)), z = (st + (a >> 2)) & 1;
+          const int k = (i + (a & 1)) + PX * (j + ((a >> 1) & 1)), z = (st + 3 + (a >> 2)) % 3;
           const longlong2 p = sm.qa[z][k], q = sm.qb[z][k];
           v[0][a] = p.x; v[1][a] = p.y; v[2][a] = q.x;
           e01[a] = (unsigned)q.y;

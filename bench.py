@@ -747,7 +747,7 @@ def main():
     p.profile_enable(False)
     d0 = p.level_dims(0)[0]
     nv, ne = (d0[0] + 1) * (d0[1] + 1) * (d0[2] + 1), d0[0] * d0[1] * d0[2]
-    fams = {capi.K_FINE_APPLY64: ("k_fine_modal_df (FP64 K.u in double-float, outer CG)",
+    fams = {capi.K_FINE_APPLY64: ("k_fine_fx (FP64 K.u in 64-bit fixed point, outer CG)",
                                   nv * (24 + 24 + 1) + ne * 8, ne * 240.0),
             # u in, f in, d out, u out (FP32 x3 each), vertex mask, the stored 3x3
             # block-Jacobi inverse (FP32, 6 of the symmetric 3x3), rho^p; d is read by one step in three
@@ -813,7 +813,7 @@ def main():
            "config": {"workload": f"{wl.name} spline OC design iteration", "grid": [nx, ny, nz],
                       "dofs": 3 * nv, "active_fraction": float(np.mean(wl.eactive)) if wl.eactive is not None else 1.0,
                       "lattice": [q + wl.order for q in wl.partition],
-                      "solver": f"FP64 flexible CG (fine matvec in double-float, ~1e-14 of FP64) + "
+                      "solver": f"FP64 flexible CG (fine matvec in 64-bit fixed point, within FP64 rounding) + "
                                 f"{opts['inner_max']} FP32 CG its (to {opts.get('inner_rtol', 0.1):g}) with "
                                 f"{args.smoother} V({opts['pre']},"
                                 f"{opts['post']}) degree-{opts['cheb_degree']} on "

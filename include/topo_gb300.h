@@ -243,8 +243,10 @@ int topo_apply_fine(topo_handle* h, int precision);
  * topo_set_operator_precision must have built. */
 int topo_apply_level(topo_handle* h, int level, int precision);
 /* Arithmetic of the FP64 fine operator used by the solvers (residuals and the
- * outer CG matvec): 0 = native FP64, 1 = double-float (pairs of floats with
- * error-free transformations, ~48-bit significands, on the FP32 pipe; default).
+ * outer CG matvec): 0 = native FP64, 1 = emulated (default): 64-bit fixed point
+ * in the CG solvers (error within that of FP64), double-float (pairs of floats
+ * with error-free transformations, ~48-bit significands) in topo_residual,
+ * topo_vcycle and solves by repeated cycles.
  * Vectors, dot products and step lengths stay FP64 either way. */
 int topo_set_fine_arithmetic(topo_handle* h, int arith);
 /* Element products of the FP32 fine kernels (the multigrid smoother, residual

@@ -216,6 +216,7 @@ constexpr int ROW_MAX = 1024;  // elements of a row, one thread each
 constexpr int CHUNK_Y = 16;    // most rows of a chunk (a warp holds their y-basis indices)
 // CTAs aimed at by shortening the chunks of small grids: four on each SM
 constexpr int CHUNK_CTAS = 608;
+constexpr size_t CHUNK_SMEM = 200 * 1024;  // most shared memory of a CTA's tables
 
 template <int K>
 __device__ __forceinline__ df spline_yz_at(const LevelDims& d, const SplineDev& sp, const float2* __restrict__ coeff,
@@ -385,12 +386,16 @@ static bool spline_chunks(cudaStream_t s, const LevelDims& d, const uint8_t* eac
   auto bytes = [&](int r) { return sizeof(float2) * (size_t)sp.nb[0] * (cap(r) + r); };
   while (ych > 1 && bytes(ych) > 96 * 1024) --ych;
   const size_t smem = bytes(ych);
-  if (smem > 200 * 1024) return false;
+  if (smem > CHUNK_SMEM) return false;
   auto* fn = sp.order == 2   ? k_spline_chunks<MODE, 2>
              : sp.order == 3 ? k_spline_chunks<MODE, 3>
                              : k_spline_chunks<MODE, 4>;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  // once a device and kernel, for the largest tables: the limit is the kernel's,
+  // not the launch's, and designs on other host threads need their own
+  static PerDeviceOnce once[MAX_ORDER + 1];
+  if (once_per_device(once[sp.order], [fn]() -> cudaError_t {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
+      }) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

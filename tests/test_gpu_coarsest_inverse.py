@@ -1,0 +1,81 @@
+"""Error of the mixed path's coarsest inverse against solves refined in extended precision, on its own matrix (FP32
+stencils): one tile of 32 pivots, a last tile of a few rows, several tiles a CTA, odd boxes, light designs (most of
+the box near the lowest density)."""
+import numpy as np
+import pytest
+
+from topoptspline3d_gb300 import capi, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(p, level):
+    """The FP32 operator of a level, exactly: unit vectors at every third vertex do not meet in a row."""
+    vx, vy, vz = (n + 1 for n in p.level_dims(level)[0])
+    nv = vx * vy * vz
+    z, y, x = (a.ravel() for a in np.meshgrid(range(vz), range(vy), range(vx), indexing="ij"))
+    A = np.zeros((3 * nv, 3 * nv))
+    near = lambda a, c: a - np.array([0, 1, -1])[(a - c) % 3]
+    for c in range(27):
+        cx, cy, cz = c % 3, c // 3 % 3, c // 9
+        ox, oy, oz = near(x, cx), near(y, cy), near(z, cz)
+        rows = np.flatnonzero((ox >= 0) & (oy >= 0) & (oz >= 0) & (ox < vx) & (oy < vy) & (oz < vz))
+        of = (ox + vx * (oy + vy * oz))[rows]
+        on = (x % 3 == cx) & (y % 3 == cy) & (z % 3 == cz)
+        for j in range(3):
+            u = np.zeros((3, nv))
+            u[j, on] = 1
+            r = p.apply_level(level, u.ravel(), 1).reshape(3, nv)
+            for i in range(3):
+                A[3 * rows + i, 3 * of + j] = r[i, rows]
+    return 0.5 * (A + A.T)
+
+
+def inverse_error(size, cap, mean, std, seed):
+    """Relative error of three solutions with the inverse, and the number of unknowns."""
+    nx, ny, nz = size
+    wl = workloads.cantilever(nx, ny, nz, lattice=tuple(max(4, s // 4 + 1) for s in size))
+    p = capi.Problem(nx, ny, nz, max_coarse_elements=cap)
+    p.set_bc(wl.fixed, wl.loads)
+    p.set_spline(wl.order, wl.partition, *wl.spline_box())
+    rng = np.random.default_rng(seed)
+    p.put("coeff", np.clip(mean + std * rng.standard_normal(p.num_coeffs()), 0.0, 1.0))
+    p.coeff_to_density()
+    p.set_operator_precision(2)
+    p.update_operators()
+    level = p.num_levels() - 1
+    A = _matrix(p, level)
+    n = len(A)
+    f = rng.standard_normal((n, 3))
+    x = np.zeros((n, 3))
+    for k in range(3):
+        p.put("f", f[:, k].reshape(-1, 3).T.ravel(), level)
+        p.coarsest_solve()
+        x[:, k] = p.get("u", level).reshape(3, -1).T.ravel()
+    p.close()
+    inv, AL = np.linalg.inv(A), A.astype(np.longdouble)
+    exact = (inv @ f).astype(np.longdouble)
+    for _ in range(4):
+        exact += inv @ (f - AL @ exact).astype(float)
+    return float(np.linalg.norm((x - exact).astype(float)) / np.linalg.norm(exact.astype(float))), n
+
+
+def mean_error(size, cap, mean, std):
+    e = [inverse_error(size, cap, mean, std, seed) for seed in range(8)]
+    return float(np.exp(np.mean(np.log([v for v, _ in e])))), e[0][1]
+
+
+# Means of the form that keeps the matrix, the pivots and the panels in FP64 and takes only the rank-32 updates in
+# double-float (k_gj_blocked<true>, which serves sizes beyond the SMs' shared memory), measured on the same matrices.
+# A mean of eight has a standard error of about 0.18 of its logarithm on either side: two of their difference are 1.6.
+@pytest.mark.parametrize("size, cap, mean, std, n, fp64_panels", [
+    ((4, 4, 4), 1, 0.6, 0.2, 24, 8.8e-16), ((4, 4, 4), 1, 0.1, 0.2, 24, 7.6e-16),
+    ((8, 4, 4), 8, 0.6, 0.2, 36, 2.3e-14), ((8, 4, 4), 8, 0.1, 0.2, 36, 1.9e-14),
+    ((8, 8, 8), 8, 0.4, 0.3, 81, 2.1e-14), ((16, 8, 8), 16, 0.1, 0.2, 135, 3.3e-13),
+    ((33, 17, 15), 40, 0.4, 0.3, 216, 1.9e-14), ((24, 12, 12), 400, 0.4, 0.3, 336, 7.2e-13),
+    ((16, 8, 8), 400, 0.6, 0.2, 675, 6.7e-13), ((33, 17, 15), 400, 0.1, 0.2, 900, 1.5e-13),
+])
+def test_no_further_off_than_with_fp64_panels(size, cap, mean, std, n, fp64_panels):
+    error, unknowns = mean_error(size, cap, mean, std)
+    assert unknowns == n
+    assert error < 1.6 * fp64_panels

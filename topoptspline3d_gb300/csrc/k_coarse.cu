@@ -1455,19 +1455,28 @@ __global__ void __launch_bounds__(256) k_gj_blocked(int n, double* __restrict__ 
 // Gauss-Jordan on the full matrix.  Each CTA owns consecutive tiles of that
 // triangle in shared memory for the whole inversion (n = 1617: nine tiles a
 // SM, n = 675: two), so a panel moves only the panel itself through L2:
-//   B: W_j = C_j D, eight rows of a tile at a time spread over all CTAs, with
-//      C_j = A_jK and D = A_KK^-1 published by the phase before;
+//   B: W_j = C_j D^-1, the panel's rows dealt evenly over all CTAs, with
+//      C_j = A_jK and D = A_KK published by the phase before;
 //   C: every tile's update; the owners of the next panel's tiles publish them.
 // CTA 0 owns no tile: during C it forms the next diagonal tile from the
 // published parts and inverts it.  Two grid barriers a panel.
-// Everything is double-float arithmetic on the FP32 pipe, for matrices that come
-// from FP32 stencils: even the conversions of a form with FP64 panels cost more
-// than the panels (n = 675: 0.65 against 0.36 ms).  Its bounds: at n = 675 the
-// chain of a panel (C for the diagonal tile 3 us, its inversion 7 us, B 2 us,
-// barriers 2.5 us), at n = 1617 the updates (480 FP32 instructions an element
-// and panel).  Against k_gj_blocked<true>: n = 336 0.64 -> 0.18 ms, 675
-// 1.31 -> 0.36 ms, 1617 5.17 -> 1.6 ms; ||A X - 1|| no larger on coarsest matrices
-// of designs (n = 675: 6.6e-13 against 8.0e-13).
+// Precision: tiles and updates are double-float, as the updates of
+// k_gj_blocked<true> are (an FP64 tile between two of them holds no more).  The
+// panel has FP64 accuracy, as there: the block's inverse X is formed in
+// double-float, where its pivots' serial chain is short, and B corrects
+// W0 = C_j X by the FP64 residual C_j - W0 D, which takes X's error squared; for
+// j = K that refines the inverse itself.  Error of the inverse on matrices of
+// designs, this / k_gj_blocked<true> / panels in double-float: n = 24 6.4e-16 /
+// 8.8e-16 / 1.8e-14, 36 2.5e-14 / 2.3e-14 / 1.3e-13, 135 0.9e-13 / 3.3e-13 /
+// 5.6e-13, 675 2.0e-13 / 6.7e-13 / 7.5e-13, 1617 2.9e-14 / 1.9e-13 / 1.9e-13
+// (the updates' terms are summed apart from the element).
+// Bounds: at n = 675 the chain of a panel (C for the diagonal tile 3 us, its
+// inversion 7 us, B 5 us, barriers 2.5 us), at n = 1617 the updates (480 FP32
+// instructions an element and panel) and B's FP64 products (2.7 us of 4 us a
+// panel).  Inversion alone, this / k_gj_blocked<true> / panels in double-float:
+// n = 135 0.13 / 0.30 / 0.10 ms, 336 0.24 / 0.67 / 0.19, 675 0.45 / 1.51 / 0.37,
+// 1617 1.90 / 5.23 / 1.66, 2520 6.1 / 17.2 / 5.3.  (The block's pivots in FP64
+// too: 0.67 ms at n = 675.)
 // The pivot-drop rule and status are k_gj_blocked's.
 // ---------------------------------------------------------------------------
 constexpr int GJT = GJB * GJB;         // elements of a tile
@@ -1503,17 +1512,19 @@ __device__ __forceinline__ df df_rcp(df p) {
   return df_fast2sum(r, __fmul_rn(r, __fmaf_rn(e, e, e)));
 }
 
-// Inverts the kb x kb symmetric block in the lower triangle of sd (rows and
-// columns from kb on are zero) and writes the full inverse to out[GJT].
-// Called by all threads of a CTA.  k0: index of the first pivot (status).
+// Inverts the kb x kb symmetric block T (pitch GJP, lower triangle; rows and
+// columns from kb on are zero) and writes the full inverse to out[GJT] and the
+// block itself in FP64 to d64[GJT].  Called by all threads of a CTA.  k0: index
+// of the first pivot (status).
 // Four pivots at a time: warp 0 sweeps them on their own four columns, held in
 // registers (lane r: row r), so a pivot costs shuffles and arithmetic but no
 // barrier, and the other elements then get their rank-4 update from all warps.
 // (One barrier a pivot took twice as long.)
-__device__ __forceinline__ void sweep_block(df (*sd)[GJP], df (*sv)[SB][GJB], int kb, int k0, float tol, int* status,
-                                            df* out) {
+__device__ __forceinline__ void sweep_block(const df* T, df (*sd)[GJP], df (*sv)[SB][GJB], int kb, int k0, df tol,
+                                            int* status, df* out, double* d64) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const df zero(0.f, 0.f);
+  for (int e = tid; e < GJT; e += GJ_THREADS) sd[e / GJB][e % GJB] = T[(e / GJB) * GJP + e % GJB];
   // this thread's element of the lower triangle with the four panel rows taken
   // out: rows r and 27 - r of that 28-row triangle together hold 29
   constexpr int R = GJB - SB;
@@ -1534,7 +1545,7 @@ __device__ __forceinline__ void sweep_block(df (*sd)[GJP], df (*sv)[SB][GJB], in
           continue;
         }
         const df p = df_shfl(v[q], j + q);
-        const bool drop = p.hi <= tol;
+        const bool drop = p.hi < tol.hi || (p.hi == tol.hi && p.lo <= tol.lo);
         df rp = df_rcp(p);
         if (drop) rp = zero;
         const df w = drop ? zero : v[q] * rp;
@@ -1549,7 +1560,7 @@ __device__ __forceinline__ void sweep_block(df (*sd)[GJP], df (*sv)[SB][GJB], in
         }
         v[q] = m;
         if (drop && lane == 0) {
-          if (p.hi < -tol) status[1] = k0 + j + q + 1;
+          if (p.hi < -tol.hi || (p.hi == -tol.hi && p.lo < -tol.lo)) status[1] = k0 + j + q + 1;
           else status[0] += 1;
         }
       }
@@ -1557,6 +1568,11 @@ __device__ __forceinline__ void sweep_block(df (*sd)[GJP], df (*sv)[SB][GJB], in
       for (int q = 0; q < SB; ++q)
         if (lane >= j + q) sd[lane][j + q] = v[q];
         else if (lane < j) sd[j + q][lane] = v[q];
+    } else if (j == 0) {  // (the warps that wait for the first pivots)
+      for (int e = tid - 32; e < GJT; e += GJ_THREADS - 32) {
+        const int r = e / GJB, c = e % GJB;
+        d64[e] = df_to(r >= c ? T[r * GJP + c] : T[c * GJP + r]);
+      }
     }
     __syncthreads();
     if (mine) {
@@ -1585,12 +1601,16 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
   __shared__ df sv[2][SB][GJB];
   __shared__ double smax[GJ_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = (n + GJB - 1) / GJB;
-  // published panels: C_j transposed ([2][nt][m][r]), W_j ([nt][r][m]), the
-  // inverse block ([2]) and the next but one diagonal tile ([2])
+  // published panels: C_j transposed ([2][nt][m][r]), W_j ([nt][r][m], the
+  // block's inverse for j = K), the block before its refinement, the block itself
+  // in FP64, the last block's inverse in FP64, and the next but one diagonal
+  // tile ([2])
   df* Cg = reinterpret_cast<df*>(work);
   df* Wg = Cg + (int64_t)2 * nt * GJT;
-  df* Dg = Wg + (int64_t)nt * GJT;
-  df* Qg = Dg + 2 * GJT;
+  df* Xg = Wg + (int64_t)nt * GJT;
+  double* D64 = reinterpret_cast<double*>(Xg + GJT);
+  double* X64 = D64 + GJT;
+  df* Qg = reinterpret_cast<df*>(X64 + GJT);
   double dmax = 0.0;
   for (int k = tid; k < n; k += GJ_THREADS) dmax = fmax(dmax, fabs(A[(int64_t)k * n + k]));
 #pragma unroll
@@ -1598,7 +1618,7 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
   if (lane == 0) smax[warp] = dmax;
   __syncthreads();
   for (int k = 0; k < GJ_THREADS / 32; ++k) dmax = fmax(dmax, smax[k]);
-  const float tol = (float)(1e-10 * dmax);
+  const df tol = df_from(1e-10 * dmax);
   // tiles t0 .. t1 of the triangle in row order; CTA 0 has none unless alone
   const int nb = (int)gridDim.x, own = nb > 1 ? nb - 1 : 1, me = nb > 1 ? (int)blockIdx.x - 1 : 0;
   const int64_t ntri = (int64_t)nt * (nt + 1) / 2;
@@ -1632,39 +1652,59 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
       if (++j > i) { ++i; j = 0; }
     }
   }
+  df* sQ = nb > 1 ? sT : sC;  // CTA 0's diagonal tile (it owns none, or the panels have not begun)
   if (blockIdx.x == 0) {
-    for (int e = tid; e < GJT; e += GJ_THREADS) sd[e / GJB][e % GJB] = df_from(entry(e / GJB, e % GJB));
-    sweep_block(sd, sv, min(GJB, n), 0, tol, status, Dg);
+    for (int e = tid; e < GJT; e += GJ_THREADS) sQ[(e / GJB) * GJP + e % GJB] = df_from(entry(e / GJB, e % GJB));
+    __syncthreads();
+    sweep_block(sQ, sd, sv, min(GJB, n), 0, tol, status, Xg, D64);
   }
   grid.sync();
   for (int k = 0; k < nt; ++k) {
     if (__ldcg(status + 1)) return;  // indefinite pivot: every CTA sees it after the barrier
     const df* Ck = Cg + (int64_t)(k & 1) * nt * GJT;
-    const df* Dk = Dg + (k & 1) * GJT;
-    // ---- B: W_j = C_j D, eight rows of one tile a unit: half the products of
-    // an element a thread, the halves added through shared memory
-    if ((int)blockIdx.x < 4 * nt) {
-      df* D = sW;
-      df* H = sC;
+    // ---- B: W_j = C_j D^-1, the panel's rows dealt evenly over the CTAs, a warp
+    // a row (lane m holds C_j(r, m), then W_j(r, m)): W0 = C_j X with the block's
+    // inverse X as it came, the residual C_j - W0 D in FP64, W = W0 + residual X.
+    // For j = K, C is the identity and W the inverse itself.
+    const int rows = nt * GJB, per = (rows + nb - 1) / nb, r0 = (int)blockIdx.x * per, r1 = min(rows, r0 + per);
+    if (r0 < r1) {
+      df* X = sW;
+      double* D = reinterpret_cast<double*>(sW + GJT);
+      auto load_c = [&](int g) {
+        return g / GJB == k ? df(lane == g % GJB ? 1 : 0) : df_ldcg(Ck + (int64_t)(g / GJB) * GJT + lane * GJB + g % GJB);
+      };
+      df cn = r0 + warp < r1 ? load_c(r0 + warp) : df(0);  // in flight with the block
 #pragma unroll
-      for (int q = 0; q < GJT / GJ_THREADS; ++q) D[tid + q * GJ_THREADS] = df_ldcg(Dk + tid + q * GJ_THREADS);
-      const int rr = warp & 7, half = warp >> 3;
-      for (int u = blockIdx.x; u < 4 * nt; u += nb) {
-        const int j = u >> 2, r = (u & 3) * 8 + rr;
-        df c[GJB / 2];
+      for (int q = 0; q < GJT / GJ_THREADS; ++q) {
+        X[tid + q * GJ_THREADS] = df_ldcg(Xg + tid + q * GJ_THREADS);
+        D[tid + q * GJ_THREADS] = __ldcg(D64 + tid + q * GJ_THREADS);
+      }
+      __syncthreads();
+      for (int g = r0 + warp; g < r1; g += GJ_THREADS / 32) {
+        const int j = g / GJB, r = g % GJB;
+        const df c = cn;
+        if (g + GJ_THREADS / 32 < r1) cn = load_c(g + GJ_THREADS / 32);
+        df a[4] = {df(0), df(0), df(0), df(0)};  // four chains of each sum
+#pragma unroll 2
+        for (int m = 0; m < GJB; m += 4)
 #pragma unroll
-        for (int m = 0; m < GJB / 2; ++m) c[m] = df_ldcg(Ck + (int64_t)j * GJT + (half * (GJB / 2) + m) * GJB + r);
-        __syncthreads();
-        df a(0), b(0);  // two chains
+          for (int i = 0; i < 4; ++i) a[i] = df_nfma(a[i], df_shfl(c, m + i), X[(m + i) * GJB + lane]);
+        const double w = -df_to((a[0] + a[1]) + (a[2] + a[3]));
+        double e[4] = {df_to(c), 0.0, 0.0, 0.0};
+#pragma unroll 2
+        for (int m = 0; m < GJB; m += 4)
 #pragma unroll
-        for (int m = 0; m < GJB / 2; m += 2) {
-          a = df_nfma(a, c[m], D[(half * (GJB / 2) + m) * GJB + lane]);
-          b = df_nfma(b, c[m + 1], D[(half * (GJB / 2) + m + 1) * GJB + lane]);
+          for (int i = 0; i < 4; ++i) e[i] = fma(-__shfl_sync(0xffffffffu, w, m + i), D[(m + i) * GJB + lane], e[i]);
+        const float res = (float)((e[0] + e[1]) + (e[2] + e[3]));
+        float p = 0.f, q = 0.f;
+#pragma unroll 4
+        for (int m = 0; m < GJB; m += 2) {
+          p = fmaf(__shfl_sync(0xffffffffu, res, m), X[m * GJB + lane].hi, p);
+          q = fmaf(__shfl_sync(0xffffffffu, res, m + 1), X[(m + 1) * GJB + lane].hi, q);
         }
-        a = a + b;
-        if (half) H[rr * GJB + lane] = a;
-        __syncthreads();
-        if (!half && j != k) Wg[(int64_t)j * GJT + r * GJB + lane] = df_neg(a + H[rr * GJB + lane]);
+        const double v = w + (double)(p + q);
+        Wg[(int64_t)j * GJT + r * GJB + lane] = df_from(v);
+        if (k + 1 == nt && j == k) X64[r * GJB + lane] = v;
       }
     }
     grid.sync();
@@ -1683,7 +1723,7 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
       const df* W = sW + buf * GJT + warp * GJB;
       const df* C = sC + buf * GJT + lane;
       df* t = T + warp * GJP + lane;
-      df v0 = t[0], v1 = t[16 * GJP], w0(0), w1(0);  // even and odd m apart: shorter sums, smaller error
+      df v0(0), v1(0), w0(0), w1(0);  // even and odd m apart, and from the element: smaller sums, smaller error
 #pragma unroll 4
       for (int m = 0; m < GJB; m += 2) {
         const df c = C[m * GJB], e = C[(m + 1) * GJB];
@@ -1692,18 +1732,18 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
         w0 = df_nfma(w0, W[m + 1], e);
         w1 = df_nfma(w1, W[16 * GJB + m + 1], e);
       }
-      t[0] = v0 + w0;
-      t[16 * GJP] = v1 + w1;
+      t[0] = t[0] + (v0 + w0);
+      t[16 * GJP] = t[16 * GJP] + (v1 + w1);
     };
     if (blockIdx.x == 0 && k1 < nt) {
       stage(0, k1, k1);
       asm volatile("cp.async.commit_group;\n" ::: "memory");
-      df* T = &sd[0][0];
-      for (int e = tid; e < GJT; e += GJ_THREADS) T[(e / GJB) * GJP + e % GJB] = df_ldcg(Qg + (k1 & 1) * GJT + e);
+      for (int e = tid; e < GJT; e += GJ_THREADS) sQ[(e / GJB) * GJP + e % GJB] = df_ldcg(Qg + (k1 & 1) * GJT + e);
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       __syncthreads();
-      update(T, 0);
-      sweep_block(sd, sv, min(GJB, n - k1 * GJB), k1 * GJB, tol, status, Dg + (k1 & 1) * GJT);
+      update(sQ, 0);
+      __syncthreads();
+      sweep_block(sQ, sd, sv, min(GJB, n - k1 * GJB), k1 * GJB, tol, status, Xg, D64);
     }
     int i = i0, j = j0;
     if (t0 < t1 && i != k && j != k) stage(0, i, j);
@@ -1716,8 +1756,9 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
       df* T = sT + (int64_t)(t - t0) * GJ_TILE;
       if (i != k && j != k) {
         update(T, buf);
-      } else if (i == j) {  // -D
-        for (int e = tid; e < GJT; e += GJ_THREADS) T[(e / GJB) * GJP + e % GJB] = df_neg(df_ldcg(Dk + e));
+      } else if (i == j) {  // -D^-1
+        for (int e = tid; e < GJT; e += GJ_THREADS)
+          T[(e / GJB) * GJP + e % GJB] = df_neg(df_ldcg(Wg + (int64_t)k * GJT + e));
       } else {  // W_i, or W_j transposed
         const df* W = Wg + (int64_t)(j == k ? i : j) * GJT;
         for (int e = tid; e < GJT; e += GJ_THREADS) {
@@ -1733,22 +1774,24 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __res
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     grid.sync();
   }
-  // ---- A <- the inverse, both triangles, and its FP32 copy
+  // ---- A <- the inverse, both triangles, and its FP32 copy (the last block,
+  // which no update followed, as it was formed in FP64)
   int i = i0, j = j0;
   for (int t = t0; t < t1; ++t) {
     const df* T = sT + (int64_t)(t - t0) * GJ_TILE;
+    const bool lastb = i == nt - 1 && j == i;
     for (int e = tid; e < GJT; e += GJ_THREADS) {
       const int a = e / GJB, b = e % GJB;
       int r = i * GJB + a, c = j * GJB + b;
       if (r < n && c < n && (i != j || r >= c)) {
-        const double v = -df_to(T[a * GJP + b]);
+        const double v = lastb ? __ldcg(X64 + e) : -df_to(T[a * GJP + b]);
         A[(int64_t)r * n + c] = v;
         A32[(int64_t)r * n + c] = (float)v;
       }
       r = i * GJB + b;
       c = j * GJB + a;
       if (r < n && c < n && (i != j || r > c)) {
-        const double v = -df_to(T[b * GJP + a]);
+        const double v = lastb ? __ldcg(X64 + b * GJB + a) : -df_to(T[b * GJP + a]);
         A[(int64_t)c * n + r] = v;
         A32[(int64_t)c * n + r] = (float)v;
       }

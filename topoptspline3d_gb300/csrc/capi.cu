@@ -37,6 +37,17 @@ using namespace topo;
 #define TOPO_FUSED_DOT_TICKET 1
 #endif
 
+// CTAs per SM of the blocked coarsest inversion (FP64 operators) when it runs on
+// the side stream next to the solve's set-up kernels: one up to
+// TOPO_GJ_SIDE_LARGE_N unknowns, where the set-up kernels need the SMs as much as
+// the inversion, two above, where the inversion outlasts the set-up by far
+#ifndef TOPO_GJ_SIDE_PER_SM
+#define TOPO_GJ_SIDE_PER_SM 1
+#endif
+#ifndef TOPO_GJ_SIDE_LARGE_N
+#define TOPO_GJ_SIDE_LARGE_N 1000
+#endif
+
 #include "handle.h"
 
 // z-march depth argument of the handle's FP32 fine-kernel launches
@@ -1629,7 +1640,8 @@ int topo_update_operators(topo_handle* h) {
       }
       CK(cudaEventRecord(h->ev_ops, h->stream));
       CK(cudaStreamWaitEvent(h->side, h->ev_ops, 0));
-      const int e = coarsest_invert(h->side, h->ndense, h->A, h->A32, h->gjwork, h->status, !b64);
+      const int e = coarsest_invert(h->side, h->ndense, h->A, h->A32, h->gjwork, h->status, !b64,
+                                    h->ndense > TOPO_GJ_SIDE_LARGE_N ? 2 : TOPO_GJ_SIDE_PER_SM);
       count_launch();
       if (e != (int)cudaSuccess)
         return fail(h, TOPO_E_CUDA, "coarsest inversion launch failed: %s", cudaGetErrorString((cudaError_t)e));

@@ -1861,44 +1861,65 @@ void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t
 
 bool stencil_by_vertex(const LevelDims& d) { return d.nv < STENCIL_WARP_MAX_NV; }
 
+// Whether k_gj_sweep inverts a matrix of n unknowns (df_update: from FP32
+// stencils) and, in blocks and smem, its launch: the triangle has to fit into the
+// SMs' shared memory (n up to about 2,500).  Else, and for FP64 operators, the
+// blocked Gauss-Jordan on A in place.
+static bool coarsest_sweeps(int n, bool df_update, int nsm, int* blocks, size_t* smem) {
+  const int64_t nt = (n + GJB - 1) / GJB, ntri = nt * (nt + 1) / 2;
+  *blocks = nt == 1 ? 1 : (int)std::min<int64_t>(nsm, ntri + 1);
+  const int64_t own = nt == 1 ? 1 : (ntri + *blocks - 2) / (*blocks - 1);
+  *smem = (size_t)(8 * (4 * GJT + own * GJ_TILE));
+  return df_update && *smem <= (size_t)GJ_SWEEP_SMEM;
+}
+static int sm_count() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+
+// The matrix of the coarsest stencils; its symmetric part for the blocked form
+// (the sweeps take that as they read).  Both here, before the inversion's stream
+// starts: k_symmetrize in that stream let the set-up kernels of the design
+// iteration onto the SMs first, and the blocked form's CTAs, two an SM, then came
+// to lie unevenly (FP64 operators, 77x44x42: 18.8 against 15.0 ms an iteration).
 template <typename T>
 void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const T* st, double* A) {
   const int64_t n = 3 * d.nv;
   cudaMemsetAsync(A, 0, sizeof(double) * n * n, s);
   k_dense_from_stencil<T><<<nblk(243 * d.nv, 256), 256, 0, s>>>(d, st, st_idx<T>(d), A);
+  int blocks;
+  size_t smem;
+  if (!coarsest_sweeps((int)n, sizeof(T) == 4, sm_count(), &blocks, &smem))
+    k_symmetrize<<<nblk(n * n, 256), 256, 0, s>>>((int)n, A);
 }
 
-// A: the coarsest matrix (its symmetric part is inverted in place), A32: the
-// inverse in FP32.  df_update: the sweeps where the triangle fits into the SMs'
-// shared memory (n up to about 2,500).  Else, and for FP64 operators, the
-// blocked Gauss-Jordan on A in place.
-int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update) {
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int threads = 256;
-  if (df_update) {
-    const int64_t nt = (n + GJB - 1) / GJB, ntri = nt * (nt + 1) / 2;
-    const int blocks = nt == 1 ? 1 : (int)std::min<int64_t>(nsm, ntri + 1);
-    const int64_t own = nt == 1 ? 1 : (ntri + blocks - 2) / (blocks - 1);
-    const int64_t smem = 8 * (4 * GJT + own * GJ_TILE);
-    if (smem <= GJ_SWEEP_SMEM) {
-      static PerDeviceOnce once;
-      const cudaError_t e = once_per_device(once, []() -> cudaError_t {
-        return cudaFuncSetAttribute(k_gj_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SWEEP_SMEM);
-      });
-      if (e != cudaSuccess) return (int)e;
-      cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
-      void* args[] = {&n, &A, &A32, &work, &status_dev};
-      return (int)cudaLaunchCooperativeKernel((void*)k_gj_sweep, dim3(blocks), dim3(GJ_THREADS), args, (size_t)smem, s);
-    }
+// A: the coarsest matrix (launch_dense_from_stencil; its symmetric part is
+// inverted in place), A32: the inverse in FP32.  max_per_sm: CTAs an SM of the
+// blocked form.
+int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update,
+                    int max_per_sm) {
+  int blocks;
+  size_t smem;
+  const int nsm = sm_count();
+  if (coarsest_sweeps(n, df_update, nsm, &blocks, &smem)) {
+    static PerDeviceOnce once;
+    const cudaError_t e = once_per_device(once, []() -> cudaError_t {
+      return cudaFuncSetAttribute(k_gj_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SWEEP_SMEM);
+    });
+    if (e != cudaSuccess) return (int)e;
+    cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
+    void* args[] = {&n, &A, &A32, &work, &status_dev};
+    return (int)cudaLaunchCooperativeKernel((void*)k_gj_sweep, dim3(blocks), dim3(GJ_THREADS), args, smem, s);
   }
-  k_symmetrize<<<nblk((int64_t)n * n, 256), 256, 0, s>>>(n, A);
+  const int threads = 256;
+  int per_sm = 0;
   void* fn = df_update ? (void*)k_gj_blocked<true> : (void*)k_gj_blocked<false>;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
   if (per_sm < 1) return (int)cudaErrorCooperativeLaunchTooLarge;
   const int tiles = ((n + GJB - 1) / GJB) * ((n + GJB - 1) / GJB);
-  const int blocks = std::max(1, std::min(tiles, nsm * std::min(per_sm, 2)));
+  blocks = std::max(1, std::min(tiles, nsm * std::min(per_sm, std::max(1, max_per_sm))));
   cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), s);
   void* args[] = {&n, &A, &work, &status_dev};
   const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, 0, s);

@@ -371,8 +371,10 @@ template <typename T>
 void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const T* st, double* A);
 // Inverts the symmetric part of A in place and writes its FP32 copy to A32.
 // work: published panels (128 n + 8192 doubles); df_update: in double-float
-// arithmetic (matrices from FP32 stencils).
-int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update);
+// arithmetic (matrices from FP32 stencils).  max_per_sm caps the blocked form's
+// CTAs an SM (beside other work on a second stream).
+int coarsest_invert(cudaStream_t s, int n, double* A, float* A32, double* work, int* status_dev, bool df_update,
+                    int max_per_sm = 2);
 void launch_to_float(cudaStream_t s, const double* a, float* b, int64_t n);
 template <typename T>
 void launch_dense_gemv(cudaStream_t s, int n, const T* Ainv, const T* f_soa, T* u_soa, int64_t nv, int nb = 1);

@@ -14,15 +14,18 @@
 //  - its modes are sums of eight of them, |c| <= 2^60, exact.  The components
 //    are then brought to a common unit in which the largest mode is just below
 //    2^60 (X: its exponent), and the products with rho^p times the modal
-//    constants, 59-bit integers of exponent x, are rounded to the nearest 2^-57
-//    of that largest mode.
+//    constants, 59-bit integers of exponent x, come out within 1.25 units, a
+//    unit being 2^-57 of that largest mode by the largest constant.
 //  - the force is an integer of exponent X + x (fx_to), below 2^63 for any u;
 //    each of the three additions that combine the elements of a vertex first
 //    halves its operands (fx_down), so no sum can leave 64 bits.
-// Everything is relative to the element's own values, as in floating point: a
-// large displacement of the void does not blunt a stiff element next to it.
-// Adding forces of different exponents shifts the smaller one further, as a
-// floating addition would.
+// Everything is relative to the element's own largest mode: a large displacement
+// of the void does not blunt a stiff element next to it.  The three components of
+// an element share that unit (FP64 would keep a component that is 2^40 smaller,
+// and not coupled to the others, to more digits of its own).  Adding forces of
+// different exponents shifts the smaller one further, as a floating addition
+// would.  Shifts round down.  Displacements below the normal range count as 0,
+// and so do forces (the double-float form lost all below 2^-126).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -96,11 +99,13 @@ __host__ __device__ __forceinline__ int64_t fx_factor(double p, int x) {
   return (b >> 63) ? -q : q;
 }
 
-// a p / 2^62 to the nearest, |a| < 2^62, |p| < 2^59
+// a p / 2^62 for |a| < 2^62, |p| < 2^59, off by -1.25 to 0.75 units and unbiased:
+// the product of the low halves is left out (0 to 1 unit, a quarter in the mean,
+// which the rounding constant adds back)
 __host__ __device__ __forceinline__ int64_t fx_mul(int64_t a, int64_t p) {
   const int ph = (int)(p >> 31), pl = (int)(p & 0x7fffffff);
   const int ah = (int)(a >> 31), al = (int)(a & 0x7fffffff);
-  const int64_t m = (int64_t)ah * pl + ((int64_t)al * ph + (1 << 30));
+  const int64_t m = (int64_t)ah * pl + ((int64_t)al * ph + ((1 << 30) + (1 << 29)));
   return (int64_t)ah * ph + (m >> 31);
 }
 

@@ -79,3 +79,12 @@ def test_no_further_off_than_with_fp64_panels(size, cap, mean, std, n, fp64_pane
     error, unknowns = mean_error(size, cap, mean, std)
     assert unknowns == n
     assert error < 1.6 * fp64_panels
+
+
+@pytest.mark.parametrize("size, cap, n, fp64_panels", [((26, 18, 10), 700, 2520, 1.4e-12), ((32, 18, 8), 600, 2550, 1.5e-11)])
+def test_either_side_of_the_shared_memory_limit(size, cap, n, fp64_panels):
+    """The largest triangle that the SMs hold (21 tiles a CTA), and the smallest that goes to the blocked form (nt = 80).
+    Single solves: their logarithm's spread of 0.5 on either side, twice, is 4."""
+    error, unknowns = inverse_error(size, cap, 0.6, 0.2, 0)
+    assert unknowns == n
+    assert error < 4 * fp64_panels

@@ -522,12 +522,12 @@ void launch_stencil_cheb(cudaStream_t s, const LevelDims& d, const T* st, const 
                                                                                 dvec, coef, first);
       return;
     }
-  }
-  if (d.nv < STENCIL_WARP_MAX_NV)
+  } else if (d.nv < STENCIL_WARP_MAX_NV) {
     k_stencil_cheb_warp<T><<<dim3(nblk(d.nv, WV), nb), 32 * WV, 0, s>>>(d, st, u, f, uout, dinv, dvec, coef, first);
-  else
-    k_stencil_cheb<T><<<dim3(nblk(d.nv, SV), nb), 3 * SV, 0, s>>>(d, st, st_idx<T>(d), u, f, uout, dinv, dvec, coef,
-                                                                  first);
+    return;
+  }
+  k_stencil_cheb<T><<<dim3(nblk(d.nv, SV), nb), 3 * SV, 0, s>>>(d, st, st_idx<T>(d), u, f, uout, dinv, dvec, coef,
+                                                                first);
 }
 
 template void launch_stencil_cheb<double>(cudaStream_t, const LevelDims&, const double*, const double*,

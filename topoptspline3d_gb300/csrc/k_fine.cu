@@ -410,10 +410,7 @@ __device__ __forceinline__ void dinv_sym_apply(const float* __restrict__ dinv, I
 constexpr int modal_min_ctas(int threads, int per_sm) { return per_sm / threads > 0 ? per_sm / threads : 1; }
 
 template <typename T, int TXE, int TYE, int MODE, bool VOID>
-__global__ void __launch_bounds__(TXE* TYE, sizeof(T) == 4 ? modal_min_ctas(TXE * TYE, MODE == 2
-                                                                                          ? TOPO_FINE32_CHEB_THREADS_PER_SM
-                                                                                          : TOPO_FINE32_THREADS_PER_SM)
-                                                           : modal_min_ctas(TXE * TYE, 512))
+__global__ void __launch_bounds__(TXE* TYE, modal_min_ctas(TXE * TYE, 512))
     k_fine_modal(LevelDims d, const T* __restrict__ rhop,
                                                          const uint8_t* __restrict__ vmask,
                                                          const T* __restrict__ u, const T* __restrict__ f,

@@ -602,10 +602,13 @@ static int gs_cluster_size() {
   return e == cudaSuccess ? size[dev].load() : 8;
 }
 
-// A colour of at least this many vertices runs thread per vertex.  FP64, us a
-// colour, nine lanes against one thread a vertex: 400 vertices 10.4 / 24.7,
-// 1,200 12.2 / 24.7, 8,800 29.5 / 45.8, 20,000 58.4 / 53.6, 29,000 83 / 57.
-constexpr int GS_THREAD_MIN = 16384;
+// A colour of at least this many vertices runs thread per vertex.  Us a colour,
+// nine lanes against one thread a vertex, FP64: 400 vertices 10.4 / 24.7, 1,200
+// 12.2 / 24.7, 8,800 29.5 / 45.8, 20,000 58.4 / 53.6, 29,000 83 / 57; FP32: 1,200
+// 4.8 / 18, 8,800 8.6 / 23, 17,000 13.7 / 24, 29,000 20.4 / 25, 43,500 29 / 28,
+// 56,000 38 / 32.
+template <typename T>
+constexpr int GS_THREAD_MIN = sizeof(T) == 8 ? 16384 : 40960;
 
 // `sweeps` Gauss-Seidel sweeps, colours 0..7 or 7..0.  Returns the launches made.
 template <typename T>
@@ -634,7 +637,7 @@ int launch_stencil_gs(cudaStream_t s, const LevelDims& d, const T* st, const uin
       const int col = reverse ? 7 - cc : cc;
       const GsColour g = gs_colour(d, col);
       if (g.cnt <= 0) continue;
-      if (big.cnt >= GS_THREAD_MIN)
+      if (big.cnt >= GS_THREAD_MIN<T>)
         k_stencil_gs<T><<<nblk(g.cnt, 128), 128, 0, s>>>(d, st, st_idx<T>(d), vmask, u, f, g.cx, g.cy, g.cz, g.hx, g.hy,
                                                        g.cnt, reverse);
       else

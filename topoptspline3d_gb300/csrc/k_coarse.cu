@@ -699,15 +699,15 @@ __global__ void k_restrict(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
 // vertex, and warp 0 sums the seven partial sums in a fixed order.  Seven
 // times the threads of a vertex-per-thread gather keep the loads in flight.
 constexpr int R4_WARPS = 7;
-// FLAT (FP64) asks for a warp's 49 taps together instead of a row of 7 at a time:
-// fewer waits, which is what a grid of less than two CTAs per SM spends its time on
-// (FP32, 20 CTAs: 10.7 -> 8.3 us); a full chip has the loads in flight anyway and the
-// row form's shorter code wins (8 x 133 CTAs: 20 us, flat 25).
-constexpr unsigned R4_FLAT_CTAS = 304;
+// FP64 asks for a warp's 49 taps together instead of a row of 7 at a time, which
+// waits less at every size (CTAs: us row / all; 20: 18.0 / 14.4, 133 18.5 / 14.4, 299
+// 26.7 / 24.5, 566 51.6 / 43.1, 2,213 175 / 147).  FP32 has enough of them in flight
+// by the row on the grids that it takes (8 x 133 CTAs: 20 us, all 25).
 
-template <typename T, bool FLAT>
+template <typename T>
 __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
                                                              T* __restrict__ fc) {
+  constexpr bool FLAT = sizeof(T) == 8;
   __shared__ T part[R4_WARPS][3][32];
   rf += (int64_t)blockIdx.y * 3 * fd.nv;  // right-hand side of the batch
   fc += (int64_t)blockIdx.y * 3 * cd.nv;
@@ -853,8 +853,9 @@ __global__ void k_prolong(LevelDims fd, LevelDims cd, const T* __restrict__ uc, 
 }
 
 // Up to three CTAs of the row form per SM the lanes form is the faster one (CTAs
-// of the row form, us lanes / row or flat: 20 3.9 / 8.5, 95 5.2 / 9, 565 14.2 /
-// 14.0, 1,064 24 / 20, 2,212 47 / 43: it reads each fine plane by more CTAs).
+// of the row form, us lanes / row: 20 3.2 / 9.7, 95 4.8 / 10.8, 232 8.1 / 11.7, 299
+// 9.0 / 12.8, 354 10.3 / 11.9, 418 11.5 / 12.7, 566 14.5 / 14.3, 1,064 24 / 20, 2,212
+// 47 / 43: it reads each fine plane by more CTAs).
 // FP32 only: the FP64 forms keep the order of their sums, which callers of
 // nearly converged cycles see in the residual's last digits.
 constexpr unsigned R4_LANES_CTAS = 456;
@@ -869,10 +870,7 @@ void launch_restrict(cudaStream_t s, const LevelDims& fine, const LevelDims& coa
         return;
       }
     }
-    if (sizeof(T) == 8 && g * (unsigned)nb < R4_FLAT_CTAS)
-      k_restrict4<T, sizeof(T) == 8><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
-    else
-      k_restrict4<T, false><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
+    k_restrict4<T><<<dim3(g, nb), 32 * R4_WARPS, 0, s>>>(fine, coarse, rf, fc);
   } else {
     k_restrict<T, 2><<<dim3(nblk(coarse.nv, 128), nb), 128, 0, s>>>(fine, coarse, rf, fc);
   }

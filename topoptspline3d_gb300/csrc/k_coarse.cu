@@ -1250,9 +1250,10 @@ constexpr int GJB = 32;
 // ran 5.4 ms, and the update on packed two-lane FP32 instructions cut the
 // instructions by a quarter but ran 5.6 ms: the panel barriers and the serial
 // panel work then set the pace.)
+// (No __restrict__ on what the CTAs hand each other between grid barriers: it
+// lets the compiler keep a value across a barrier.)
 template <bool DFC>
-__global__ void __launch_bounds__(256) k_gj_blocked(int n, double* __restrict__ A, double* __restrict__ work,
-                                                    int* __restrict__ status) {
+__global__ void __launch_bounds__(256) k_gj_blocked(int n, double* A, double* work, int* status) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double sd[GJB][GJB + 1];
   __shared__ df scd[DFC ? GJB : 1][GJB + 1];
@@ -1322,7 +1323,9 @@ __global__ void __launch_bounds__(256) k_gj_blocked(int n, double* __restrict__ 
   grid.sync();
   for (int k0 = 0; k0 < n; k0 += GJB) {
     const int kb = min(GJB, n - k0);
-    if (status[1]) return;  // indefinite pivot: every CTA sees it after the barrier
+    // indefinite pivot: every thread of every CTA has to see it, or the others
+    // wait for this one at the next barrier
+    if (*(volatile int*)(status + 1)) return;
     for (int e = tid; e < GJB * GJB; e += blockDim.x) sd[e / GJB][e % GJB] = work[e];
     __syncthreads();
     // ---- B: row panel P = D^-1 A[K,:] (columns outside K) and column panel C = A[:,K]
@@ -1591,8 +1594,7 @@ __device__ __forceinline__ void sweep_block(const df* T, df (*sd)[GJP], df (*sv)
   }
 }
 
-__global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* __restrict__ A, float* __restrict__ A32,
-                                                         double* __restrict__ work, int* __restrict__ status) {
+__global__ void __launch_bounds__(GJ_THREADS, 1) k_gj_sweep(int n, double* A, float* A32, double* work, int* status) {
   cg::grid_group grid = cg::this_grid();
   extern __shared__ __align__(16) unsigned char gj_smem[];
   df* sW = reinterpret_cast<df*>(gj_smem);  // [2][GJT] staged W_i, [r][m]

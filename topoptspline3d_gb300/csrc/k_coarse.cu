@@ -876,64 +876,85 @@ void launch_restrict(cudaStream_t s, const LevelDims& fine, const LevelDims& coa
   }
 }
 
-// Prolongation by a factor of 4: a warp takes 96 fine vertices of a row.  Lane l
-// forms the y-z combination of coarse column cx0 + l once (25 of them cover the
-// piece), and a fine vertex takes its two by shuffles; masks, fine values and
-// stores are lane by lane along x, whole lines: 103 MB at 256x128x128 in 23 us.  (A
-// thread per four neighbouring vertices wrote every fourth value of a line at a
-// time, 40 us; 48x24x24 5.2 -> 3.8 us.)
-constexpr int P4_EACH = 3, P4_X = 32 * P4_EACH;  // fine vertices of a lane, of a warp
-static_assert(P4_X / 4 + 1 <= 32, "a lane per coarse column of a piece");
+// Prolongation by a factor of 4: a warp takes a piece of a row, up to 96 fine
+// vertices.  Lane l forms the y-z combination of coarse column cx0 + l once (25 of
+// them cover a piece), and a fine vertex takes its two by shuffles; masks, fine
+// values and stores are lane by lane along x, whole lines: 103 MB at 256x128x128 in
+// 23 us.  (A thread per four neighbouring vertices wrote every fourth value of a
+// line at a time, 40 us; 48x24x24 5.2 -> 3.8 us.)
+// FP64 is bound by its pipe, 16 clocks of an SM for an instruction of a warp
+// whatever its lanes do: a row's units of 32 vertices are dealt evenly to its
+// pieces and no others are worked on, a value and component takes two
+// operations, and the weights come from integers without conversion.  FP64, us,
+// a thread per four vertices / pieces of 96 from the row's start with three
+// operations / this: 61x37x29 8.3 / 6.5 / 6.3, 128x64x64 21.7 / 24.8 / 16.8,
+// 192x96x96 55.5 / 73.9 / 43.0, 256x128x128 119 / 128 / 82.
+constexpr int P4_EACH = 3;  // units of 32 fine vertices of a warp, at most
+static_assert(32 * P4_EACH / 4 + 1 <= 32, "a lane per coarse column of a piece");
+
+// w as T, 1 <= w <= 16
+template <typename T>
+__device__ __forceinline__ T small_weight(int w) {
+  const float f = (float)w;
+  if constexpr (sizeof(T) == 4) return f;
+  else return __hiloint2double((__float_as_int(f) >> 3) + (896 << 20), 0);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, const T* __restrict__ uc,
-                                                   T* __restrict__ uf, const uint8_t* __restrict__ vmask, int pieces) {
+                                                   T* __restrict__ uf, const uint8_t* __restrict__ vmask, int units,
+                                                   int pieces) {
   uc += (int64_t)blockIdx.y * 3 * cd.nv;  // right-hand side of the batch
   uf += (int64_t)blockIdx.y * 3 * fd.nv;
   const int lane = threadIdx.x & 31;
   const int64_t q = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // this warp's piece
   const int64_t row = q / pieces;
   if (row >= (int64_t)fd.vy * fd.vz) return;
-  const int x0 = (int)(q - row * pieces) * P4_X, z = (int)(row / fd.vy), y = (int)(row - (int64_t)z * fd.vy);
+  const int piece = (int)(q - row * pieces), uq = units / pieces, ur = units - uq * pieces;
+  const int n = uq + (piece < ur ? 1 : 0);  // units of this piece
+  const int x0 = 32 * (piece * uq + min(piece, ur)), z = (int)(row / fd.vy), y = (int)(row - (int64_t)z * fd.vy);
   const int64_t v0 = row * fd.vx;
   uint8_t mm[P4_EACH];
   T uo[P4_EACH][3];
 #pragma unroll
   for (int k = 0; k < P4_EACH; ++k) {
     const int x = x0 + 32 * k + lane;
-    mm[k] = x < fd.vx ? vmask[v0 + x] : 0;
+    const bool in = k < n && x < fd.vx;
+    mm[k] = in ? vmask[v0 + x] : 0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) uo[k][c] = x < fd.vx ? uf[c * fd.nv + v0 + x] : T(0);
+    for (int c = 0; c < 3; ++c) uo[k][c] = in ? uf[c * fd.nv + v0 + x] : T(0);
   }
   const int cx = x0 / 4 + lane, cy = y / 4, cz = z / 4, ry = y % 4, rz = z % 4;
   // corners with a zero weight are not read (they may lie outside the coarse grid)
   T cyz[3] = {T(0), T(0), T(0)};  // sum over oy, oz of wy wz u_c
-  if (lane <= P4_X / 4 && cx < cd.vx) {
+  if (lane <= 8 * n && cx < cd.vx) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int oy = k & 1, oz = k >> 1;
       const int w = (oy ? ry : 4 - ry) * (oz ? rz : 4 - rz);
       if (w == 0) continue;
+      const T wt = small_weight<T>(w);
       const int64_t cv = cx + (int64_t)cd.vx * ((cy + oy) + (int64_t)cd.vy * (cz + oz));
-      cyz[0] += T(w) * uc[cv];
-      cyz[1] += T(w) * uc[cd.nv + cv];
-      cyz[2] += T(w) * uc[2 * cd.nv + cv];
+      cyz[0] += wt * uc[cv];
+      cyz[1] += wt * uc[cd.nv + cv];
+      cyz[2] += wt * uc[2 * cd.nv + cv];
     }
   }
-  const T inv = T(1) / T(64);
-  // (4 - rx) a + rx b with one rounding: the product by 3, if there is one, goes
-  // into the fused multiply-add, the other weight is a power of two or 0
+  // ((4 - rx) a + rx b) / 64 with one rounding: rx = 0, 2 as a, a + b and 1, 3 as
+  // 3 a + b, a + 3 b in a fused multiply-add, the power of two with the 1 / 64
   const int rx = lane & 3;
-  const T wm = T(rx == 3 ? 3 : 4 - rx), wq = T(rx == 3 ? 1 : rx);
+  const T wm = rx & 1 ? T(3) : T(1), sc = rx == 0 ? T(1) / T(16) : rx == 2 ? T(1) / T(32) : T(1) / T(64);
 #pragma unroll
   for (int k = 0; k < P4_EACH; ++k) {
+    if (k >= n) break;  // the whole warp
     const uint8_t m = (mm[k] & 8) ? mm[k] : 0;
     const int from = 8 * k + (lane >> 2);
     const int64_t v = v0 + x0 + 32 * k + lane;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const T a = __shfl_sync(0xffffffffu, cyz[c], from), b = __shfl_sync(0xffffffffu, cyz[c], from + 1);
-      const T t = fma(wm, rx == 3 ? b : a, wq * (rx == 3 ? a : b));
-      if ((m >> c) & 1) uf[c * fd.nv + v] = uo[k][c] + t * inv;
+      const T t = fma(wm, rx == 3 ? b : a, rx == 0 ? T(0) : rx == 3 ? a : b);
+      if ((m >> c) & 1) uf[c * fd.nv + v] = fma(t, sc, uo[k][c]);
     }
   }
 }
@@ -942,9 +963,9 @@ template <typename T>
 void launch_prolong(cudaStream_t s, const LevelDims& fine, const LevelDims& coarse, const T* uc,
                     T* uf, const uint8_t* vmask_fine, int nb) {
   if (coarse.factor == 4) {
-    const int pieces = (fine.vx + P4_X - 1) / P4_X;
+    const int units = (fine.vx + 31) / 32, pieces = (units + P4_EACH - 1) / P4_EACH;
     k_prolong4x<T><<<dim3(nblk((int64_t)pieces * fine.vy * fine.vz, 8), nb), 256, 0, s>>>(fine, coarse, uc, uf,
-                                                                                         vmask_fine, pieces);
+                                                                                         vmask_fine, units, pieces);
   } else
     k_prolong<T, 2><<<dim3(nblk(fine.nv, 256), nb), 256, 0, s>>>(fine, coarse, uc, uf, vmask_fine);
 }

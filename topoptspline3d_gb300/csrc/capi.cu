@@ -1166,8 +1166,8 @@ int topo_create(const topo_config* cfg, const uint8_t* eactive, topo_handle** ou
     A(dalloc(hp, &L.U2, 3 * nv)); A(dalloc(hp, &L.U2_32, 3 * nv));
     if (l > 0) {
       A(dalloc(hp, &L.kel, 576 * ne)); A(dalloc(hp, &L.kel32, 576 * ne));
-      A(dalloc(hp, &L.stencil, 243 * nv));
-      if (stencil_by_vertex(L.d)) A(dalloc(hp, &L.stencilv, 243 * nv));
+      // small levels: by vertex; TOPO_STENCIL's form when it is first asked for (stencil_planes)
+      A(dalloc(hp, stencil_by_vertex(L.d) ? &L.stencilv : &L.stencil, 243 * nv));
       // FP32: room for the tiled layout (243 x 32 values per started group of 32 vertices)
       A(dalloc(hp, &L.stencil32, 243 * ((nv + 31) / 32 * 32)));
     }
@@ -1511,6 +1511,22 @@ static int array_info(topo_handle* h, int which, int level, void** dptr, size_t*
   return TOPO_OK;
 }
 
+// TOPO_STENCIL of a small level, whose kernels read the stencils by vertex: kept
+// from the first call that asks for it (written by every operator update, for
+// nobody mostly, it took up to 64 MB a level and 9 us of 2.3 ms at 192x96x96).
+static int stencil_planes(topo_handle* h, int which, int level, void** dptr) {
+  if (which != TOPO_STENCIL) return TOPO_OK;
+  DevLevel& L = h->lv[level];
+  if (!L.stencil) {
+    RET(dalloc(h, &L.stencil, 243 * L.d.nv));
+    launch_stencil_planes(h->stream, L.d, L.stencilv, L.stencil);
+    count_launch();
+    CKL();
+  }
+  *dptr = L.stencil;
+  return TOPO_OK;
+}
+
 int topo_array_size(const topo_handle* h, int which, int level, size_t* count) {
   DEVICE_SCOPE(h);
   if (!h || !count) return TOPO_E_BAD_INPUT;
@@ -1543,6 +1559,7 @@ int topo_get_array(topo_handle* h, int which, int level, void* dst, size_t count
   if (rc != TOPO_OK) return fail(h, rc, "bad array id/level %d/%d", which, level);
   if (count != n) return fail(h, TOPO_E_BAD_INPUT, "array %d has %zu elements, asked %zu", which, n, count);
   if (which == TOPO_RHOP) RET(update_penalised_if_stale(h));
+  RET(stencil_planes(h, which, level, &p));
   CK(cudaMemcpyAsync(dst, p, n * es, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return TOPO_OK;
@@ -1552,7 +1569,8 @@ int topo_device_ptr(topo_handle* h, int which, int level, void** dptr) {
   DEVICE_SCOPE(h);
   if (!h || !dptr) return TOPO_E_BAD_INPUT;
   size_t n, es;
-  return array_info(h, which, level, dptr, &n, &es);
+  RET(array_info(h, which, level, dptr, &n, &es));
+  return stencil_planes(h, which, level, dptr);
 }
 
 int topo_coeff_to_density(topo_handle* h) {

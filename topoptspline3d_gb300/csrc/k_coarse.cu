@@ -1167,16 +1167,32 @@ __global__ void __launch_bounds__(576) k_galerkin_dyadic(LevelDims fd, LevelDims
 }
 
 // Stencil assembly from element matrices: thread per (neighbour d, vertex v),
-// consecutive threads along what the layout stores together.  planes: also the
-// [243][nv] form that callers read (FP64, null: none).
+// consecutive threads along what the layout stores together; FP64 by vertex, a warp
+// one neighbour of 32 vertices: its blocks are sums of as many elements (1 to 8)
+// in every lane, which counts for more there than whole lines (operator update
+// at 192x96x96, FP64 2,310 -> 2,284 us, FP32 358 -> 429).  planes: also the [243][nv]
+// form that callers read (FP64, null: none).
 template <typename T>
 __global__ void k_assemble_stencil(LevelDims d, const uint8_t* __restrict__ eactive,
                                    const uint8_t* __restrict__ vmask, const T* __restrict__ kel,
                                    T* __restrict__ st, StIdx si, T* __restrict__ planes) {
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 27 * d.nv) return;
-  const int k = (int)(si.form == 2 ? gid % 27 : gid / d.nv);
-  const int64_t v = si.form == 2 ? gid / 27 : gid % d.nv;
+  int k;
+  int64_t v;
+  if (sizeof(T) == 4 && si.form == 2) {
+    v = gid / 27;
+    k = (int)(gid - 27 * v);
+    if (v >= d.nv) return;
+  } else if (si.form == 2) {
+    const int64_t w = gid >> 5, g = w / 27;
+    k = (int)(w - 27 * g);
+    v = 32 * g + (gid & 31);
+    if (v >= d.nv) return;
+  } else {
+    if (gid >= 27 * d.nv) return;
+    k = (int)(gid / d.nv);
+    v = gid % d.nv;
+  }
   const int x = (int)(v % d.vx);
   const int64_t t = v / d.vx;
   const int y = (int)(t % d.vy), z = (int)(t / d.vy);
@@ -1216,6 +1232,13 @@ __global__ void k_assemble_stencil(LevelDims d, const uint8_t* __restrict__ eact
     st[si.base(v) + k * si.ks() + q * si.es()] = blk[q];
     if (planes) planes[(int64_t)(k * 9 + q) * d.nv + v] = blk[q];
   }
+}
+
+__global__ void k_stencil_planes(int64_t nv, const double* __restrict__ st, StIdx si, double* __restrict__ planes) {
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= 243 * nv) return;
+  const int64_t q = gid / nv, v = gid - q * nv;
+  planes[gid] = st[si.base(v) + q / 9 * si.ks() + q % 9 * si.es()];
 }
 
 template <typename T>
@@ -1880,7 +1903,11 @@ void launch_galerkin_dyadic_t(cudaStream_t s, const LevelDims& fd, const LevelDi
 template <typename T>
 void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t* eactive,
                                const uint8_t* vmask, const T* kel, T* st, T* planes) {
-  k_assemble_stencil<T><<<nblk(27 * d.nv, 256), 256, 0, s>>>(d, eactive, vmask, kel, st, st_idx<T>(d), planes);
+  k_assemble_stencil<T><<<nblk(27 * ((d.nv + 31) / 32 * 32), 256), 256, 0, s>>>(d, eactive, vmask, kel, st, st_idx<T>(d), planes);
+}
+
+void launch_stencil_planes(cudaStream_t s, const LevelDims& d, const double* st, double* planes) {
+  k_stencil_planes<<<nblk(243 * d.nv, 256), 256, 0, s>>>(d.nv, st, st_idx<double>(d), planes);
 }
 
 bool stencil_by_vertex(const LevelDims& d) { return d.nv < STENCIL_WARP_MAX_NV; }

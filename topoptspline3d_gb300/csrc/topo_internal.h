@@ -151,8 +151,8 @@ struct DevLevel {
   float *U32 = nullptr, *F32 = nullptr, *R32 = nullptr;  // FP32 [3nv]
   double* kel = nullptr;        // coarse: FP64 element matrices [ne][576]
   float* kel32 = nullptr;       // coarse: FP32 element matrices [ne][576]
-  double* stencil = nullptr;    // coarse: FP64 [243][nv], as callers read it
-  double* stencilv = nullptr;   // coarse: the kernels' copy on small levels, by vertex (StIdx form 2; else null)
+  double* stencil = nullptr;    // coarse: FP64 [243][nv]; small levels: null until a caller asks for it
+  double* stencilv = nullptr;   // coarse: the kernels' form on small levels, by vertex (StIdx form 2; else null)
   float* stencil32 = nullptr;   // coarse: FP32, by vertex on small levels, tiled on the others (StIdx)
   double* dinv = nullptr;       // FP64 inverse diagonal blocks [9][nv] (Chebyshev)
   float* dinv32 = nullptr;      // FP32 inverse diagonal blocks [9][nv]; level 0: packed symmetric (float4 d00 d01 d02 d11 [nv], float2 d12 d22 [nv])
@@ -367,6 +367,8 @@ void launch_assemble_stencil_t(cudaStream_t s, const LevelDims& d, const uint8_t
                                const uint8_t* vmask, const T* kel, T* st, T* planes = nullptr);
 // whether a level's stencils are stored by vertex
 bool stencil_by_vertex(const LevelDims& d);
+// [243][nv] from stencils by vertex
+void launch_stencil_planes(cudaStream_t s, const LevelDims& d, const double* st, double* planes);
 template <typename T>
 void launch_dense_from_stencil(cudaStream_t s, const LevelDims& d, const T* st, double* A);
 // Inverts the symmetric part of A in place and writes its FP32 copy to A32.

@@ -391,9 +391,10 @@ static bool spline_chunks(cudaStream_t s, const LevelDims& d, const uint8_t* eac
              : sp.order == 3 ? k_spline_chunks<MODE, 3>
                              : k_spline_chunks<MODE, 4>;
   // once a device and kernel, for the largest tables: the limit is the kernel's,
-  // not the launch's, and designs on other host threads need their own
+  // not the launch's, and designs on other host threads need their own.  Only once
+  // tables need it: a raised limit costs the small ones 1 us a launch (191x95x93)
   static PerDeviceOnce once[MAX_ORDER + 1];
-  if (once_per_device(once[sp.order], [fn]() -> cudaError_t {
+  if (smem > 48 * 1024 && once_per_device(once[sp.order], [fn]() -> cudaError_t {
         return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
       }) != cudaSuccess) {
     cudaGetLastError();

@@ -42,6 +42,7 @@ namespace topo {
 
 constexpr int kMmaMaxM = 4;        // constraints handled by the GPU kernel
 constexpr int kMmaBlock = 256;     // threads of a CTA, at most (mma_alloc)
+constexpr int kMmaFew = 8192;      // variables up to which CTAs have half of them
 constexpr int kMmaWarps = kMmaBlock / 32;
 constexpr int kMmaSlots = 32;      // reduction slots per grid-wide reduction
 constexpr double kStepFrac = 0.99; // asym_clamp_factor, optimization/mma_t.h:20
@@ -509,10 +510,12 @@ static int mma_alloc(topo_mma* o) {
   // One CTA per SM at most: enough threads for the design sizes the spline
   // lattices give, and a cheaper grid barrier than a fully populated grid.  A
   // variable's Newton step has some 30 FP64 divisions, which the warps of an SM
-  // take one after another, so few variables are spread over small CTAs (n =
-  // 637: 4.0 ms an update on 3 CTAs of 256 threads, 2.7 on 10 of 64).
-  o->threads = 64;
-  while (o->threads < kMmaBlock && (long long)o->n > (long long)o->threads * sms) o->threads *= 2;
+  // take one after another, so few variables are spread over small CTAs; many are
+  // not, since a barrier and the sums after it cost more on more CTAs.  us an
+  // update with CTAs of 64 / 128 / 256 threads, one constraint: n = 637 868 / 846 /
+  // 1131, 3000 1287 / 1092 / 1298, 6500 1920 / 1435 / 1488, 9000 2318 / 1655 / 1593,
+  // 18081 2886 / 2453 / 2087; four: 6500 2802 / 2319 / 2693, 18081 4103 / 3395 / 3330.
+  o->threads = o->n <= kMmaFew ? kMmaBlock / 2 : kMmaBlock;
   const long long want = ((long long)o->n + o->threads - 1) / o->threads;
   o->nblocks = (int)std::max(1LL, std::min<long long>(want, (long long)sms * std::min(per_sm, 1)));
   const size_t n = o->n, m1 = o->m + 1;

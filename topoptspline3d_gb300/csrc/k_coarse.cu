@@ -702,7 +702,8 @@ constexpr int R4_WARPS = 7;
 // FP64 asks for a warp's 49 taps together instead of a row of 7 at a time, which
 // waits less at every size (CTAs: us row / all; 20: 18.0 / 14.4, 133 18.5 / 14.4, 299
 // 26.7 / 24.5, 566 51.6 / 43.1, 2,213 175 / 147).  FP32 has enough of them in flight
-// by the row on the grids that it takes (8 x 133 CTAs: 20 us, all 25).
+// by the row on the grids that it takes (8 x 133 CTAs: 20 us, all 25), with branches
+// past the grid's sides (159x79x77: 13.5 us, with selects 15.5).
 
 template <typename T>
 __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, LevelDims cd, const T* __restrict__ rf,
@@ -721,23 +722,34 @@ __global__ void __launch_bounds__(32 * R4_WARPS) k_restrict4(LevelDims fd, Level
     const int dz = w - 3, fz = 4 * z + dz;
     if (fz >= 0 && fz < fd.vz) {
       const T wz = T(4 - (dz < 0 ? -dz : dz));
-      const int64_t plane = (int64_t)fd.vx * fd.vy * fz;
-#pragma unroll(FLAT ? 7 : 1)
-      for (int dy = -3; dy <= 3; ++dy) {
+      auto taps = [&](int dy) {
         const int fy = 4 * y + dy;
-        if (!FLAT && (fy < 0 || fy >= fd.vy)) continue;
         const bool iny = fy >= 0 && fy < fd.vy;
+        if (!FLAT && !iny) return;
         const T wyz = wz * T(4 - (dy < 0 ? -dy : dy));
+        const int64_t rowv = (int64_t)fd.vx * (fy + (int64_t)fd.vy * fz);
 #pragma unroll
         for (int dx = -3; dx <= 3; ++dx) {
           const int fx = 4 * x + dx;
           const bool in = iny && fx >= 0 && fx < fd.vx;
           const T wt = wyz * T(4 - (dx < 0 ? -dx : dx));
-          const int64_t fv = plane + (int64_t)fd.vx * fy + fx;
-          s0 += wt * (in ? rf[fv] : T(0));
-          s1 += wt * (in ? rf[fd.nv + fv] : T(0));
-          s2 += wt * (in ? rf[2 * fd.nv + fv] : T(0));
+          const int64_t fv = rowv + fx;
+          if constexpr (FLAT) {
+            s0 += wt * (in ? rf[fv] : T(0));
+            s1 += wt * (in ? rf[fd.nv + fv] : T(0));
+            s2 += wt * (in ? rf[2 * fd.nv + fv] : T(0));
+          } else if (in) {
+            s0 += wt * rf[fv];
+            s1 += wt * rf[fd.nv + fv];
+            s2 += wt * rf[2 * fd.nv + fv];
+          }
         }
+      };
+      if constexpr (FLAT) {
+#pragma unroll
+        for (int dy = -3; dy <= 3; ++dy) taps(dy);
+      } else {
+        for (int dy = -3; dy <= 3; ++dy) taps(dy);
       }
     }
   }
@@ -883,9 +895,11 @@ void launch_restrict(cudaStream_t s, const LevelDims& fine, const LevelDims& coa
 // 23 us.  (A thread per four neighbouring vertices wrote every fourth value of a
 // line at a time, 40 us; 48x24x24 5.2 -> 3.8 us.)
 // FP64 is bound by its pipe, 16 clocks of an SM for an instruction of a warp
-// whatever its lanes do: a row's units of 32 vertices are dealt evenly to its
-// pieces and no others are worked on, a value and component takes two
-// operations, and the weights come from integers without conversion.  FP64, us,
+// whatever its lanes do: there a row's units of 32 vertices are dealt evenly to its
+// pieces and no others are worked on (FP32 keeps pieces of 96: dealt, 28 against
+// 24 us at 256x128x128), a value and
+// component takes two operations, and the weights come from integers without
+// conversion.  FP64, us,
 // a thread per four vertices / pieces of 96 from the row's start with three
 // operations / this: 61x37x29 8.3 / 6.5 / 6.3, 128x64x64 21.7 / 24.8 / 16.8,
 // 192x96x96 55.5 / 73.9 / 43.0, 256x128x128 119 / 128 / 82.
@@ -910,16 +924,20 @@ __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, c
   const int64_t q = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // this warp's piece
   const int64_t row = q / pieces;
   if (row >= (int64_t)fd.vy * fd.vz) return;
-  const int piece = (int)(q - row * pieces), uq = units / pieces, ur = units - uq * pieces;
-  const int n = uq + (piece < ur ? 1 : 0);  // units of this piece
-  const int x0 = 32 * (piece * uq + min(piece, ur)), z = (int)(row / fd.vy), y = (int)(row - (int64_t)z * fd.vy);
+  const int piece = (int)(q - row * pieces), z = (int)(row / fd.vy), y = (int)(row - (int64_t)z * fd.vy);
+  int n = P4_EACH, x0 = 32 * P4_EACH * piece;  // units of this piece and its first vertex
+  if constexpr (sizeof(T) == 8) {
+    const int uq = units / pieces, ur = units - uq * pieces;
+    n = uq + (piece < ur ? 1 : 0);
+    x0 = 32 * (piece * uq + min(piece, ur));
+  }
   const int64_t v0 = row * fd.vx;
   uint8_t mm[P4_EACH];
   T uo[P4_EACH][3];
 #pragma unroll
   for (int k = 0; k < P4_EACH; ++k) {
     const int x = x0 + 32 * k + lane;
-    const bool in = k < n && x < fd.vx;
+    const bool in = (sizeof(T) == 4 || k < n) && x < fd.vx;
     mm[k] = in ? vmask[v0 + x] : 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) uo[k][c] = in ? uf[c * fd.nv + v0 + x] : T(0);
@@ -927,7 +945,7 @@ __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, c
   const int cx = x0 / 4 + lane, cy = y / 4, cz = z / 4, ry = y % 4, rz = z % 4;
   // corners with a zero weight are not read (they may lie outside the coarse grid)
   T cyz[3] = {T(0), T(0), T(0)};  // sum over oy, oz of wy wz u_c
-  if (lane <= 8 * n && cx < cd.vx) {
+  if (lane <= 8 * (sizeof(T) == 8 ? n : P4_EACH) && cx < cd.vx) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int oy = k & 1, oz = k >> 1;
@@ -940,21 +958,33 @@ __global__ void __launch_bounds__(256) k_prolong4x(LevelDims fd, LevelDims cd, c
       cyz[2] += wt * uc[2 * cd.nv + cv];
     }
   }
-  // ((4 - rx) a + rx b) / 64 with one rounding: rx = 0, 2 as a, a + b and 1, 3 as
-  // 3 a + b, a + 3 b in a fused multiply-add, the power of two with the 1 / 64
+  // ((4 - rx) a + rx b) / 64 with one rounding.  FP64: rx = 0, 2 as a, a + b and 1, 3
+  // as 3 a + b, a + 3 b in a fused multiply-add, the power of two with the 1 / 64.
+  // FP32: the product by 3, if there is one, in the fused multiply-add, the other
+  // weight a power of two or 0 (by the FP64 form 26 against 24 us at 256x128x128).
   const int rx = lane & 3;
-  const T wm = rx & 1 ? T(3) : T(1), sc = rx == 0 ? T(1) / T(16) : rx == 2 ? T(1) / T(32) : T(1) / T(64);
+  T wm, sc, wq = T(0);
+  if constexpr (sizeof(T) == 8) {
+    wm = rx & 1 ? T(3) : T(1);
+    sc = rx == 0 ? T(1) / T(16) : rx == 2 ? T(1) / T(32) : T(1) / T(64);
+  } else {
+    wm = T(rx == 3 ? 3 : 4 - rx);
+    wq = T(rx == 3 ? 1 : rx);
+    sc = T(1) / T(64);
+  }
 #pragma unroll
   for (int k = 0; k < P4_EACH; ++k) {
-    if (k >= n) break;  // the whole warp
+    if (sizeof(T) == 8 && k >= n) break;  // the whole warp
     const uint8_t m = (mm[k] & 8) ? mm[k] : 0;
     const int from = 8 * k + (lane >> 2);
     const int64_t v = v0 + x0 + 32 * k + lane;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const T a = __shfl_sync(0xffffffffu, cyz[c], from), b = __shfl_sync(0xffffffffu, cyz[c], from + 1);
-      const T t = fma(wm, rx == 3 ? b : a, rx == 0 ? T(0) : rx == 3 ? a : b);
-      if ((m >> c) & 1) uf[c * fd.nv + v] = fma(t, sc, uo[k][c]);
+      T t;
+      if constexpr (sizeof(T) == 8) t = fma(wm, rx == 3 ? b : a, rx == 0 ? T(0) : rx == 3 ? a : b);
+      else t = fma(wm, rx == 3 ? b : a, wq * (rx == 3 ? a : b));
+      if ((m >> c) & 1) uf[c * fd.nv + v] = uo[k][c] + t * sc;
     }
   }
 }

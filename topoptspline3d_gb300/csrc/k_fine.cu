@@ -621,8 +621,8 @@ __global__ void __launch_bounds__(TXE* TYE, modal_min_ctas(TXE * TYE, 512))
 // ---------------------------------------------------------------------------
 // FP32 form with one barrier per element layer.  A CTA is TYE warps; lane i of
 // warp j computes element (i, j) of the layer and owns vertex (i, j), the
-// element's (+x, +y) corner.  The kernel is bound by instruction issue (75% of
-// the slots at 256x128x128), so the transforms are split between layers: a
+// element's (+x, +y) corner.  The kernel spends its time issuing
+// instructions (76% of the slots at 256x128x128 before, 70% now), so the transforms are split between layers: a
 // vertex plane's x-y modes are formed once and kept for the layer above it, and
 // the z = 1 forces of a layer wait as x-y modes (each lane its own, in shared
 // memory) for the z = 0 forces of the next, so the inverse x-y transform, the x
